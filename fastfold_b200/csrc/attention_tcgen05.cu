@@ -1,4 +1,5 @@
-// Fused gated-attention core for the Evoformer's axial attentions (forward):
+// Fused attention core for the Evoformer's axial attentions: forward pass of training (inference: attention_infer.cu) and
+// backward pass.  Forward:
 //
 //   O[b,i,h,:] = softmax_j( scale * <Q[b,i,h,:], K[b,j,h,:]> + bias[h,i,j]  |  key mask[b,j] ) V[b,j,h,:]
 //
@@ -31,7 +32,7 @@
 // Replaces logits matmul + fused_softmax + weights*v of the reference
 // (fastfold/model/fastnn/ops.py:304-319) and its unused Triton forward-only
 // attention core (kernel/triton/attention_core.py:12-121).
-#include "common.cuh"
+#include "attention_common.cuh"
 #include "tmap.h"
 
 namespace ffb {
@@ -40,7 +41,6 @@ constexpr int AT_BQ = 128;      // queries per tile
 constexpr int AT_BK = 128;      // keys per block
 constexpr int AT_THREADS = 320; // producer warp, MMA warp, 8 softmax / gradient warps
 constexpr int AT_KV_STAGES = 3;
-constexpr float LOG2E = 1.4426950408889634f;
 
 struct AttnArgs {
   int B, H, n_q, n_k;            // batch rows, heads, query / key lengths
@@ -55,49 +55,6 @@ struct AttnArgs {
   float* lse2;                   // [B][H][n_q] or null
   int has_bias;
 };
-
-// descriptor with explicit layout code: 2 = 128B swizzle, 4 = 64B swizzle
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(layout) << 61;
-  return d;
-}
-
-__device__ __forceinline__ float ex2f(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// two bf16 packed in a word -> two floats (low half first)
-__device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
-
-// Keep-bits of 64 consecutive keys starting at kbase: bit c of (lo | hi << 32) is set when key kbase + c is inside the
-// sequence and its mask entry is non-zero.  `valid` gets the in-sequence bits alone.  One warp-wide call.
-__device__ __forceinline__ void key_bits(const bf16* mrow, int kbase, int n_k, int lane, uint32_t& keep_lo, uint32_t& keep_hi,
-                                         uint32_t& valid_lo, uint32_t& valid_hi) {
-  const int k_a = kbase + lane, k_b = kbase + 32 + lane;
-  const bool in_a = k_a < n_k, in_b = k_b < n_k;
-  bool on_a = in_a, on_b = in_b;
-  if (mrow) {
-    if (in_a) on_a = __bfloat162float(mrow[k_a]) != 0.f;
-    if (in_b) on_b = __bfloat162float(mrow[k_b]) != 0.f;
-  }
-  valid_lo = __ballot_sync(0xffffffffu, in_a);
-  valid_hi = __ballot_sync(0xffffffffu, in_b);
-  keep_lo = __ballot_sync(0xffffffffu, on_a);
-  keep_hi = __ballot_sync(0xffffffffu, on_b);
-}
-
-// Masked keys take this logit (replaced, not added).  -2^30 instead of the reference's -1e9: its product with log2(e) is
-// exact in fp32, so a fully masked row still comes out as exactly uniform weights from the fused multiply-add form
-// exp2(v * log2e - m * log2e); any finite logit next to it underflows to weight 0 either way.
-constexpr float MASKED_LOGIT = -1073741824.f;
 
 // Per-warp table of the 64 keys of a half block: (keep, penalty) with logit' = logit * keep + penalty, i.e. (1, 0) for a
 // normal key, (0, MASKED_LOGIT) for a masked one, (0, -inf) past the end of the sequence.  One FMA per logit instead of
@@ -524,7 +481,6 @@ int ffb_attention_fwd(const void* q, const void* k, const void* v, long long q_b
   if (D != 32) return -2;
   if ((q_rstride % 8) || (kv_rstride % 8) || (q_bstride % 8) || (kv_bstride % 8) || (out_rstride % 8) || (out_bstride % 8)) return -3;
   if (bias && (n_k % 8)) return -4;
-  if (mask && (mask_bstride % 8)) return -5;
   AttnArgs a;
   a.B = B; a.H = H; a.n_q = n_q; a.n_k = n_k;
   a.n_qt = (n_q + AT_BQ - 1) / AT_BQ;
@@ -1002,7 +958,7 @@ int ffb_attention_bwd_strided(const void* q, const void* k, const void* v, long 
   using namespace ffb;
   if (D != 32) return -2;
   if (n_q > 512) return -3;
-  if ((q_rstride % 8) || (kv_rstride % 8) || (q_bstride % 8) || (kv_bstride % 8) || (n_k % 8)) return -4;
+  if ((q_rstride % 8) || (kv_rstride % 8) || (q_bstride % 8) || (kv_bstride % 8) || ((bias || ds) && n_k % 8)) return -4;
   if ((dq_rstride % 8) || (dkv_rstride % 8) || (dq_bstride % 8) || (dkv_bstride % 8) || (o_bstride % 8) || (o_rstride % 8)) return -5;
   AttnBwdArgs a;
   a.B = B; a.H = H; a.n_q = n_q; a.n_k = n_k;

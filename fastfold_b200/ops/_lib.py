@@ -52,6 +52,7 @@ def _declare(lib):
         "ffb_gemm_bf16_peer": [P, P, I, I, L, L, L, L, I, ctypes.POINTER(GemmArgs), I, ctypes.POINTER(c_void_p), I, P],
         "ffb_read_status": [ctypes.POINTER(c_int), I],
         "ffb_attention_fwd": [P, P, P, L, L, L, L, P, P, L, P, L, L, P, I, I, I, I, I, F, P],
+        "ffb_attention_infer": [P, P, P, L, L, L, L, P, L, P, L, P, L, L, I, I, I, I, I, F, P],
         "ffb_attention_bwd": [P, P, P, L, L, L, L, P, P, L, P, P, P, P, P, I, I, I, I, I, F, P],
         "ffb_attention_bwd_strided": [P, P, P, L, L, L, L, P, P, L, P, P, L, L, P, P, P, P, L, L, L, L, P, I, I, I, I, I, F, P],
         "ffb_layernorm_fwd": [P, P, P, P, P, P, L, I, F, I, P],

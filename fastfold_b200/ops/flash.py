@@ -1,4 +1,4 @@
-"""Fused tcgen05 attention (csrc/attention_tcgen05.cu): dispatch, autograd wrapper.
+"""Fused tcgen05 attention (csrc/attention_tcgen05.cu with gradients, csrc/attention_infer.cu without): dispatch, autograd wrapper.
 
 ``q, k, v`` arrive as ``[1, B, H, n, d]`` views of the fused QKV projection output ``[1, B, n, 3, H, d]``; the
 kernel reads them in place through TMA (no head transposes) and writes ``[1, B, n, H*d]``, which is returned as
@@ -65,9 +65,13 @@ def _fwd(q, k, v, mask, bias, scale, want_lse):
     lse = torch.empty(B, H, n_q, device=q.device, dtype=torch.float32) if want_lse else None
     b3 = bias.reshape(H, n_q, n_k).contiguous() if bias is not None else None
     m2 = mask.reshape(B, n_k).to(torch.bfloat16).contiguous() if mask is not None else None
-    rc = lib.ffb_attention_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), qbs, qrs, kbs, krs, _lib.ptr(b3), _lib.ptr(m2), n_k,
-                               _lib.ptr(out), n_q * H * d, H * d, _lib.ptr(lse), B, H, n_q, n_k, d, float(scale), _lib.stream_ptr())
-    _lib.check(rc, "ffb_attention_fwd(B=%d,H=%d,n=%d/%d)" % (B, H, n_q, n_k))
+    if want_lse:
+        rc = lib.ffb_attention_fwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), qbs, qrs, kbs, krs, _lib.ptr(b3), _lib.ptr(m2), n_k,
+                                   _lib.ptr(out), n_q * H * d, H * d, _lib.ptr(lse), B, H, n_q, n_k, d, float(scale), _lib.stream_ptr())
+    else:
+        rc = lib.ffb_attention_infer(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), qbs, qrs, kbs, krs, _lib.ptr(b3), n_k, _lib.ptr(m2), n_k,
+                                     _lib.ptr(out), n_q * H * d, H * d, B, H, n_q, n_k, d, float(scale), _lib.stream_ptr())
+    _lib.check(rc, "ffb_attention_%s(B=%d,H=%d,n=%d/%d)" % ("fwd" if want_lse else "infer", B, H, n_q, n_k))
     return out, lse, (q, k, v, b3, m2)
 
 
@@ -159,8 +163,12 @@ def _packed_fwd(qkv, mask, bias, scale, want_lse, transposed):
     b3 = bias.reshape(H, n, n).contiguous() if bias is not None else None
     m2 = mask.reshape(B, n).to(torch.bfloat16).contiguous() if mask is not None else None
     base = qkv.data_ptr()
-    rc = lib.ffb_attention_fwd(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, _lib.ptr(b3), _lib.ptr(m2), n,
-                               _lib.ptr(out), obs, ors, _lib.ptr(lse), B, H, n, n, d, float(scale), _lib.stream_ptr())
+    if want_lse:
+        rc = lib.ffb_attention_fwd(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, _lib.ptr(b3), _lib.ptr(m2), n,
+                                   _lib.ptr(out), obs, ors, _lib.ptr(lse), B, H, n, n, d, float(scale), _lib.stream_ptr())
+    else:
+        rc = lib.ffb_attention_infer(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, _lib.ptr(b3), n, _lib.ptr(m2), n,
+                                     _lib.ptr(out), obs, ors, B, H, n, n, d, float(scale), _lib.stream_ptr())
     _lib.check(rc, "ffb_attention_fwd packed (B=%d,H=%d,n=%d)" % (B, H, n))
     return out, lse, b3, m2
 

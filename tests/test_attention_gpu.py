@@ -37,6 +37,32 @@ def test_forward(B, n, H, use_bias, use_mask, device_status):
     assert err < 2e-2, "max abs err %g" % err
 
 
+@pytest.mark.parametrize("B,n,H,use_bias", [(1, 64, 4, True), (5, 72, 4, True), (6, 256, 8, True), (7, 320, 4, False), (9, 640, 4, True)])
+def test_forward_rows_that_leave_the_exponent_range(B, n, H, use_bias, device_status):
+    """Rows whose reference point has to move: logits of several hundred, a much larger (smaller) level from some key on,
+    leading blocks that are masked as a whole, a fully masked row.  Bound: |v| < 5.5; the
+    output is rounded to bf16 (half a step of 2^-5 at 4 .. 8), and P is (2^-9 relative, so up to 2 x 2^-9 x 5.5 between a
+    row's keys): 1.6e-2 + 2.2e-2; the logits agree to fp32."""
+    torch.manual_seed(n + B)
+    q, k, v = _qkv(B, n, H)
+    q = q * 8.0
+    bias = None
+    if use_bias:
+        bias = torch.randn(1, 1, H, n, n, device=DEV)
+        bias[..., : n // 3, n // 2:] += 300.0
+        bias[..., n // 3: 2 * (n // 3), n // 2:] -= 300.0
+        bias[:, :, 0] -= 500.0
+        bias = bias.to(torch.bfloat16)
+    mask = torch.ones(1, B, n, device=DEV, dtype=torch.bfloat16)
+    mask[0, 0, : (n * 3) // 4] = 0
+    if B > 1:
+        mask[0, 1] = 0
+    with torch.no_grad():
+        out = attention_core(q, k, v, mask, bias)
+    ref = attention_core_ref(q.float(), k.float(), v.float(), mask.float(), None if bias is None else bias.float())
+    assert (out.float() - ref).abs().max().item() < 3.8e-2
+
+
 @pytest.mark.parametrize("B,n,H,use_bias,use_mask", [
     (4, 128, 8, True, True), (16, 256, 8, True, True), (7, 256, 4, False, True), (5, 384, 4, True, False), (3, 200, 4, True, True),
     (6, 512, 4, True, True),
