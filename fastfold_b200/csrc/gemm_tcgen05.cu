@@ -454,9 +454,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_kernel(const __grid
                           (long long)(m1 % g.cq_mdiv) * g.cq_sr1 + (long long)(col0 >> 5) * g.cq_sc1;
               asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], 2048;" ::"l"(dst), "r"(epi_smem + out_buf * 4096)
                            : "memory");
-              asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], 2048;" ::"l"(dst + g.cq_sc1),
-                           "r"(epi_smem + out_buf * 4096 + 2048)
-                           : "memory");
+              if (col0 + 32 < g.N)                           // N is a multiple of 32: the last chunk may hold one block only
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], 2048;" ::"l"(dst + g.cq_sc1),
+                             "r"(epi_smem + out_buf * 4096 + 2048)
+                             : "memory");
             } else {
               asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(&tmC),
                            "r"(epi_smem + out_buf * 4096), "r"(col0), "r"(row0), "r"(tc.batch)
@@ -639,9 +640,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_kernel(const __grid
                           (long long)(m1 % g.cq_mdiv) * g.cq_sr1 + (long long)(col0 >> 5) * g.cq_sc1;
               asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], 2048;" ::"l"(dst), "r"(epi_smem + out_buf * 4096)
                            : "memory");
-              asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], 2048;" ::"l"(dst + g.cq_sc1),
-                           "r"(epi_smem + out_buf * 4096 + 2048)
-                           : "memory");
+              if (col0 + 32 < g.N)                           // N is a multiple of 32: the last chunk may hold one block only
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], 2048;" ::"l"(dst + g.cq_sc1),
+                             "r"(epi_smem + out_buf * 4096 + 2048)
+                             : "memory");
             } else {
               asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(&tmC),
                            "r"(epi_smem + out_buf * 4096), "r"(col0), "r"(row0), "r"(tc.batch)
@@ -956,7 +958,7 @@ static int gemm_launch(const void* A, const void* B, int a_mn, int b_mn, long lo
   if (tma_epi && g.resid && !(al16(g.resid, g.ldres, g.res_bstride) && (batch == 1 || g.res_bstride != 0))) tma_epi = 0;
   if (g.cq) {
     // block-permuted store: bf16, whole 32 x 64 warp tiles only, no mul / residual tiles (they would be fetched in matrix layout)
-    if (g.out_mode != OUT_BF16 || g.trans_out || g.glu || g.mul || g.resid || (g.M % 32) || (g.N % 64)) return -23;
+    if (g.out_mode != OUT_BF16 || g.trans_out || g.glu || g.mul || g.resid || (g.M % 32) || (g.N % 32)) return -23;
     if ((reinterpret_cast<uintptr_t>(g.C) & 15) || (g.cq_sr1 % 8) || (g.cq_sr2 % 8) || (g.cq_sc1 % 8) || (g.c_bstride % 8) || g.cq_mdiv < 1) return -23;
     tma_epi = 1;
   } else if (tma_epi) {

@@ -39,9 +39,7 @@ class MSAColumnAttention(nn.Module):
         from . import ops as fops
         if fops.CHUNK_SIZE is not None:
             return False
-        if not (like.is_cuda and like.dtype == torch.bfloat16 and self.c == flash.HEAD_DIM and n_seq % 8 == 0):
-            return False
-        return True
+        return like.is_cuda and like.dtype == torch.bfloat16 and self.c == flash.HEAD_DIM
 
     def forward(self, M_raw, M_mask, M_norm_t=None, strided=None):
         """``M_norm_t``: ``layernormM`` of the input when the caller already has it - transposed ``[1, N/P, S, c]`` unless

@@ -194,11 +194,13 @@ class OutProductMean(nn.Module):
         N, e = right_all.shape[2], right_all.shape[3]
         l2 = left.reshape(S, ni * d)
         r2 = right_all.reshape(S, N * e)
-        if (Z_raw.is_cuda and Z_raw.dtype == torch.bfloat16 and d == 32 and e == 32 and N % 32 == 0 and ni * d >= 64
-                and self.o_linear.bias is not None):
+        need_grad = torch.is_grad_enabled() and any(t.requires_grad for t in (l2, r2, Z_raw, self.o_linear.weight))
+        if (Z_raw.is_cuda and Z_raw.dtype == torch.bfloat16 and d == 32 and e == 32 and (N % 32 == 0 or not need_grad) and ni * d >= 64
+                and N * e >= 64 and self.o_linear.bias is not None):
             # the product [(i d), (j e)] leaves the GEMM epilogue already laid out as [i, j, d, e], the operand layout of
-            # the output projection; its gradient comes back the other way through the same block-permuting store
-            if torch.is_grad_enabled() and any(t.requires_grad for t in (l2, r2, Z_raw, self.o_linear.weight)):
+            # the output projection; its gradient comes back the other way through the same block-permuting store, which
+            # cuts the (i j) rows into blocks of 32 and so wants whole ones
+            if need_grad:
                 out = _OpmCore.apply(l2, r2, self.o_linear.weight, self.o_linear.bias, inv_norm.reshape(-1), Z_raw.reshape(ni * N, -1))
             else:
                 out = _opm_forward(l2, r2, self.o_linear.weight, self.o_linear.bias, inv_norm.reshape(-1), Z_raw.reshape(ni * N, -1))[0]
@@ -322,6 +324,16 @@ class _OpmCore(torch.autograd.Function):
 # ---------------------------------------------------------------------------
 # Gated self attention
 # ---------------------------------------------------------------------------
+def _key_contiguous(b):
+    """``b [1, h, q, k]`` with the keys contiguous; without gradients the rows are laid out at the 8-element pitch that the
+    attention kernel's bias tiles are read at, so that odd lengths need no second copy."""
+    n = b.shape[-1]
+    if n % 8 == 0 or not b.is_cuda or torch.is_grad_enabled():
+        return b.contiguous()
+    buf = b.new_empty(*b.shape[:-1], (n + 7) // 8 * 8)[..., :n]
+    return buf.copy_(b)
+
+
 class SelfAttention(nn.Module):
     """Multi-head gated self attention on ``[b1, b2, n, c]`` (attention along ``n``)."""
 
@@ -344,18 +356,22 @@ class SelfAttention(nn.Module):
             return nonbatched_bias[0]          # already ``[b, h, q, k]`` (``pair_bias_hqk``)
         if transposed:      # projected from the un-transposed pair tensor [k, q_local, h]: gather the query axis
             b = gather_async_opp(*nonbatched_bias, dim=2)
-            return b.permute(0, 3, 2, 1).contiguous()      # 'b k q h -> b h q k'
+            return _key_contiguous(b.permute(0, 3, 2, 1))      # 'b k q h -> b h q k'
         b = gather_async_opp(*nonbatched_bias, dim=1)
-        return b.permute(0, 3, 1, 2).contiguous()          # 'b q k h -> b h q k'
+        return _key_contiguous(b.permute(0, 3, 1, 2))          # 'b q k h -> b h q k'
 
-    def _padded_heads(self):
-        """Weights of the same layer with every head widened to the fused attention kernel's 32 channels by zero rows /
+    def _padded_dim(self):
+        """Head width that the forward attention kernel runs narrow heads at: the smallest of its widths that holds them."""
+        return min(D for D in flash.FWD_HEAD_DIMS if D >= self.c)
+
+    def _padded_heads(self, D=flash.HEAD_DIM):
+        """Weights of the same layer with every head widened to ``D`` channels - a width of the fused attention kernel - by zero rows /
         columns (the extra-MSA stack has 8-channel heads): zero q / k channels leave the logits unchanged, zero v
         channels give zero outputs that the zero columns of the output projection ignore.  Inference only; cached."""
-        H, d, D = self.n_head, self.c, flash.HEAD_DIM
+        H, d = self.n_head, self.c
         # Cached in eval mode only: an optimiser that updates the parameters through raw pointers (the flat fused Adam)
         # changes neither ``_version`` nor ``data_ptr``, so in training the widened copies are rebuilt on every call.
-        key = (self.to_qkv.weight.data_ptr(), self.to_qkv.weight._version, self.o_linear.weight._version,
+        key = (D, self.to_qkv.weight.data_ptr(), self.to_qkv.weight._version, self.o_linear.weight._version,
                self.gating_linear.weight._version if self.gating else 0)
         if self.training or getattr(self, "_pad_cache", None) is None or self._pad_cache[0] != key:
             def rows(w, groups):                      # [groups * H * d, ...] -> [groups * H * D, ...]
@@ -405,8 +421,8 @@ class SelfAttention(nn.Module):
 
     def _one_padded(self, x, mask, bias, tail):
         """No-grad GPU path for heads narrower than the fused kernel's: see ``_padded_heads``."""
-        H, D = self.n_head, flash.HEAD_DIM
-        wq, wg, bg, wo = self._padded_heads()
+        H, D = self.n_head, self._padded_dim()
+        wq, wg, bg, wo = self._padded_heads(D)
         b1, b2, n, _ = x.shape
         x2 = x.reshape(-1, x.shape[-1])
         qkv = K.gemm(x2, wq).reshape(b1, b2, n, 3, H, D)
@@ -427,7 +443,7 @@ class SelfAttention(nn.Module):
     def _one(self, x, mask, bias, tail, transposed=False):
         """``transposed``: ``x [b1, n, b2, c]`` and the attention runs along dim 1 (``mask [b1, b2, n]``)."""
         H, d = self.n_head, self.c
-        if d < flash.HEAD_DIM and not transposed and _fusable(x) and x.shape[-2] % 8 == 0:
+        if d < flash.HEAD_DIM and not transposed and _fusable(x):
             res = self._one_padded(x, mask, bias, tail)
             if res is not None:
                 return res
@@ -610,6 +626,31 @@ class _TriangleMultiplication(nn.Module):
             p = _bmm_tn(lt, rt)                              # [c, i, j]
         return p.permute(1, 2, 0).unsqueeze(0)
 
+    def _fused_nograd_any(self, Z_raw, Z_mask, dropmask, Z_norm=None):
+        """``_fused_nograd`` on one GPU for extents that are no multiple of 8: the same kernels, with the first pair axis as
+        the batch of the projections, so that the channel-major operands and the contraction's result get rows at an
+        8-element pitch (TMA wants 16-byte strides).  Extents stay exact - the padding is neither written nor read, except
+        by the second LayerNorm, whose rows there are not used."""
+        c = self.c
+        A, B = Z_raw.shape[1], Z_raw.shape[2]
+        Z = self.layernorm1(Z_raw) if Z_norm is None else Z_norm
+        w, b = self._glu_weights()
+        lr_t = torch.empty(2 * c, A, (B + 7) // 8 * 8, device=Z.device, dtype=Z.dtype)[:, :, :B]
+        K.gemm(Z.reshape(A, B, -1), w, bias=b, glu=True, rowscale=Z_mask.reshape(A, B), trans_out=True, out=lr_t.permute(1, 0, 2))
+        g = K.gemm(Z.reshape(A * B, -1), self.output_gate.weight, bias=self.output_gate.bias, act="sigmoid")
+        n_i = n_j = A if self.outgoing else B
+        pitch = (n_j + 7) // 8 * 8
+        p = torch.empty(c, n_i, pitch, device=Z.device, dtype=Z.dtype)
+        if self.outgoing:
+            K.gemm(lr_t[:c], lr_t[c:], out=p[:, :, :n_j])
+        else:
+            K.gemm(lr_t[:c], lr_t[c:], a_mn=True, b_mn=True, out=p[:, :, :n_j])
+        ab = K.layer_norm_transposed(p.reshape(c, n_i * pitch), self.layernorm2.weight, self.layernorm2.bias, self.layernorm2.eps)
+        zr3 = Z_raw.reshape(A, B, -1)
+        out = K.gemm(ab.view(n_i, pitch, c)[:, :n_j], self.output_projection.weight, bias=self.output_bias, mul=g.view(A, B, -1),
+                     dmask=None if dropmask is None else _mask_idx(Z_raw, dropmask), resid=zr3, out=_res_out(zr3))
+        return out.reshape(Z_raw.shape)
+
     def _fused_nograd(self, Z_raw, Z_mask, dropmask, Z_norm=None):
         """Inference / checkpoint first pass: 7 kernels, no transposed copies."""
         c = self.c
@@ -710,13 +751,20 @@ class _TriangleMultiplication(nn.Module):
             dropmask = F.dropout(torch.ones_like(Z_raw[:, 0:1, :, :]), p=self.p_drop, training=True)
         if not training:
             dropmask = None
-        can_fuse = _fusable(Z_raw) and (Z_raw.shape[1] * Z_raw.shape[2]) % 8 == 0 and Z_raw.shape[1] % 8 == 0 and Z_raw.shape[2] % 8 == 0
+        A, B = Z_raw.shape[1], Z_raw.shape[2]
+        can_fuse = _fusable(Z_raw) and A % 8 == 0 and B % 8 == 0
+        # one GPU, square pair tensor, a dropout mask that is shared along the first axis: the row index within a batch
+        # row of the projections is then the mask's row
+        can_fuse_any = (_fusable(Z_raw) and not can_fuse and core.get_dap_size() == 1 and A == B and Z_raw.shape[0] == 1 and self.c % 8 == 0
+                        and (dropmask is None or (dropmask.dim() == 4 and dropmask.shape[1] == 1)))
         if CHUNK_SIZE is not None and not torch.is_grad_enabled():
             # The slab pipeline bounds memory (its temporaries are one rank's slab) but pays permuted copies of both
             # operands; the dense no-grad path has none and needs about eight times the local pair tensor, so it is
             # taken whenever that is a small part of the GPU's memory.
-            if not (can_fuse and _dense_fits(Z_raw)):
+            if not ((can_fuse or can_fuse_any) and _dense_fits(Z_raw)):
                 return self._chunked(Z_raw, Z_mask)
+        if can_fuse_any:
+            return self._fused_nograd_any(Z_raw, Z_mask, dropmask, Z_norm)
         if can_fuse:
             return self._fused_nograd(Z_raw, Z_mask, dropmask, Z_norm)
         c = self.c
@@ -869,9 +917,9 @@ class _TriangleAttention(nn.Module):
         """``n_attn``: length of the axis the ending node attends along (the full first pair axis)."""
         if self.starting or CHUNK_SIZE is not None:
             return False
-        if not (like.is_cuda and like.dtype == torch.bfloat16 and self.c == flash.HEAD_DIM and n_attn % 8 == 0):
+        if not (like.is_cuda and like.dtype == torch.bfloat16 and self.c == flash.HEAD_DIM):
             return False
-        return True
+        return n_attn % 8 == 0 or not torch.is_grad_enabled()          # backward wants 16-byte rows of the pair bias
 
     def inplace(self, Z_raw, Z_mask, dropmask=None):
         with inplace_scope():

@@ -9,6 +9,7 @@ import torch
 from . import _lib
 
 HEAD_DIM = 32
+FWD_HEAD_DIMS = (32,)      # head widths of the forward pass without gradients
 MAX_BWD_QUERIES = 512      # queries of one (row, head) whose gradient the backward kernel holds in tensor memory
 
 
@@ -130,17 +131,33 @@ def flash_attention(q, k, v, mask, bias, scale):
 # ---------------------------------------------------------------------------
 def packed_supported(qkv, mask, bias, transposed=False):
     """``qkv [1, B, n, 3, H, d]`` (or ``[1, n, B, 3, H, d]``) contiguous bf16 on a GPU, self attention."""
+    need_grad = torch.is_grad_enabled() and (qkv.requires_grad or (bias is not None and bias.requires_grad))
     if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 6 and qkv.shape[0] == 1 and qkv.shape[3] == 3
-            and qkv.shape[-1] == HEAD_DIM and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0):
+            and qkv.shape[-1] in ((HEAD_DIM,) if need_grad else FWD_HEAD_DIMS) and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0):
         return False
     if not (_lib.has("ffb_attention_fwd") and _lib.has("ffb_attention_bwd_strided")):
         return False
     n = qkv.shape[1] if transposed else qkv.shape[2]
-    if n % 8:
-        return False
+    if n % 8 and bias is not None and need_grad:
+        return False            # the backward kernel stores the logit gradient in 16-byte pieces of un-padded rows
     if bias is not None and (bias.dim() != 5 or bias.shape[0] != 1 or bias.shape[1] != 1):
         return False
     return True
+
+
+def _pitched_bias(bias, H, n_q, n_k):
+    """The pair bias as the forward kernel reads it: rows of ``n_k`` values at a pitch that is a multiple of 8 (TMA wants
+    16-byte strides).  Returns ``(tensor, pitch)``; a bias that is laid out like that already is passed on as it is."""
+    if bias is None:
+        return None, n_k
+    b3 = bias.reshape(H, n_q, n_k) if bias.dim() != 3 else bias
+    pitch = b3.stride(1)
+    if (b3.stride(2) == 1 and pitch % 8 == 0 and pitch >= n_k and (H == 1 or b3.stride(0) == n_q * pitch) and b3.data_ptr() % 16 == 0):
+        return b3, pitch
+    pitch = (n_k + 7) // 8 * 8
+    buf = b3.new_empty(H, n_q, pitch)
+    buf[:, :, :n_k].copy_(b3)
+    return buf, pitch
 
 
 def _packed_geometry(qkv, transposed):
@@ -160,14 +177,17 @@ def _packed_fwd(qkv, mask, bias, scale, want_lse, transposed):
     HD = H * d
     out = torch.empty((1, n, B, HD) if transposed else (1, B, n, HD), device=qkv.device, dtype=qkv.dtype)
     lse = torch.empty(B, H, n, device=qkv.device, dtype=torch.float32) if want_lse else None
-    b3 = bias.reshape(H, n, n).contiguous() if bias is not None else None
+    if want_lse:                                          # the backward kernel reads un-padded rows
+        b3, pitch = (bias.reshape(H, n, n).contiguous() if bias is not None else None), n
+    else:
+        b3, pitch = _pitched_bias(bias, H, n, n)
     m2 = mask.reshape(B, n).to(torch.bfloat16).contiguous() if mask is not None else None
     base = qkv.data_ptr()
     if want_lse:
         rc = lib.ffb_attention_fwd(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, _lib.ptr(b3), _lib.ptr(m2), n,
                                    _lib.ptr(out), obs, ors, _lib.ptr(lse), B, H, n, n, d, float(scale), _lib.stream_ptr())
     else:
-        rc = lib.ffb_attention_infer(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, _lib.ptr(b3), n, _lib.ptr(m2), n,
+        rc = lib.ffb_attention_infer(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, _lib.ptr(b3), pitch, _lib.ptr(m2), n,
                                      _lib.ptr(out), obs, ors, B, H, n, n, d, float(scale), _lib.stream_ptr())
     _lib.check(rc, "ffb_attention_fwd packed (B=%d,H=%d,n=%d)" % (B, H, n))
     return out, lse, b3, m2

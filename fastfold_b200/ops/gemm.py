@@ -72,7 +72,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, alpha=1.0, bias=None, act=None, glu=Fa
     with ``m = 32 m1 + m0`` and ``n = 32 n1 + n0``, element ``(m, n)`` lands at flat index
     ``(m1 // mdiv) sr2 + (m1 % mdiv) sr1 + n1 sc1 + 32 m0 + n0`` (every 32 x 32 block contiguous).  With ``d = e = 32``:
     ``[(i d), (j e)] -> [i, j, d, e]`` is ``(1, 1024 J, 0, 1024)`` and ``[(i j), (d e)] -> [(i d), (j e)]`` is
-    ``(J // 32, 1024 J, 1024, 32 J)``.  Needs ``M % 32 == 0``, ``N % 64 == 0``.
+    ``(J // 32, 1024 J, 1024, 32 J)``.  Needs ``M % 32 == 0``, ``N % 32 == 0``.
     """
     if block_out is not None:
         assert out is None and not trans_out and not glu and mul is None and resid is None and a.dim() == 2 and b.dim() == 2
@@ -131,7 +131,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, alpha=1.0, bias=None, act=None, glu=Fa
     blocked = None
     if block_out is not None:
         shape, mdiv, sr2, sr1, sc1 = block_out
-        assert M % 32 == 0 and n_out % 64 == 0 and (M // 32) % mdiv == 0 and out_dtype in (None, torch.bfloat16)
+        assert M % 32 == 0 and n_out % 32 == 0 and (M // 32) % mdiv == 0 and out_dtype in (None, torch.bfloat16)
         blocked = torch.empty(shape, device=a.device, dtype=torch.bfloat16)
         assert blocked.numel() == M * n_out
         out = blocked.view(-1).as_strided((M, n_out), (8, 1))          # carries shape and dtype through the checks; the kernel ignores ldc

@@ -1,0 +1,129 @@
+"""Lengths that are no multiple of 8: the fused no-grad path of every trunk module against the module in fp32 on the CPU."""
+import copy
+
+import pytest
+import torch
+
+from fastfold_b200.models.fastnn import ops as fops
+from fastfold_b200.models.fastnn.msa import ExtraMSACore, MSAColumnAttention, MSARowAttentionWithPairBias
+from fastfold_b200.models.fastnn.triangle import (TriangleAttentionEndingNode, TriangleAttentionStartingNode, TriangleMultiplicationIncoming,
+                                                  TriangleMultiplicationOutgoing)
+from fastfold_b200.ops import flash
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _random_parameters(mod):
+    with torch.no_grad():
+        for name, p in mod.named_parameters():
+            p.normal_(std=p.shape[-1] ** -0.5 if p.dim() >= 2 else 0.1)
+            if "norm" in name and name.endswith("weight"):
+                p.add_(1.0)
+    return mod.to(torch.bfloat16).float()        # weights that bf16 holds exactly
+
+
+def _check(mod, inputs, call, tol=2e-2):
+    """Relative 2-norm error of the module's update; bf16 roundings of a handful of chained tensors, 2^-9 each."""
+    gpu = copy.deepcopy(mod).to(DEV, torch.bfloat16)
+    with torch.no_grad():
+        ref = call(mod, [t.float() for t in inputs])
+        got = call(gpu, [t.to(DEV, torch.bfloat16) for t in inputs]).float().cpu()
+    assert got.shape == ref.shape
+    err = ((got - ref).norm() / ref.norm()).item()
+    assert err < tol, err
+
+
+def _masks(n, s=0):
+    pm = torch.ones(1, n, n)
+    pm[:, :, n - 3:] = 0
+    pm[:, 1] = 0                                 # a row without any key: uniform weights over the true length
+    if not s:
+        return pm
+    mm = torch.ones(1, s, n)
+    mm[:, :, n - 2:] = 0
+    mm[:, s // 2] = 0
+    return pm, mm
+
+
+@pytest.mark.parametrize("n", [33, 61, 68, 129, 203, 261])
+@pytest.mark.parametrize("cls", [TriangleAttentionStartingNode, TriangleAttentionEndingNode, TriangleMultiplicationOutgoing, TriangleMultiplicationIncoming])
+def test_pair_modules(cls, n, device_status):
+    torch.manual_seed(n)
+    att = cls in (TriangleAttentionStartingNode, TriangleAttentionEndingNode)
+    mod = _random_parameters(cls(128, p_drop=0.25, c=32 if att else 128, **({"n_head": 4} if att else {}))).eval()
+    _check(mod, [torch.randn(1, n, n, 128).bfloat16(), _masks(n)], lambda m, x: m(*x))
+    fops.set_chunk_size(16)
+    try:
+        _check(mod, [torch.randn(1, n, n, 128).bfloat16(), _masks(n)], lambda m, x: m(*x))
+    finally:
+        fops.set_chunk_size(None)
+
+
+@pytest.mark.parametrize("n", [16, 45, 64, 200, 320])
+@pytest.mark.parametrize("cls", [TriangleAttentionStartingNode, TriangleAttentionEndingNode])
+def test_sixteen_channel_heads(cls, n, device_status):
+    """Heads of 16 channels (template pair stack) have their own instance of the forward attention kernel."""
+    torch.manual_seed(n)
+    mod = _random_parameters(cls(64, p_drop=0.25, c=16, n_head=4)).eval()
+    _check(mod, [torch.randn(1, n, n, 64).bfloat16(), _masks(n)], lambda m, x: m(*x))
+
+
+@pytest.mark.parametrize("n", [61, 130])
+def test_triangle_multiplication_with_dropout_mask(n, device_status):
+    """The first pass of activation checkpointing: no gradients, training mode, a mask shared along the first axis."""
+    torch.manual_seed(n)
+    mod = _random_parameters(TriangleMultiplicationOutgoing(128, p_drop=0.25, c=128)).train()
+    drop = ((torch.rand(1, 1, n, 128) > 0.25).float() / 0.75).bfloat16()
+    _check(mod, [torch.randn(1, n, n, 128).bfloat16(), _masks(n), drop], lambda m, x: m(*x))
+
+
+@pytest.mark.parametrize("s,n", [(5, 33), (29, 61), (130, 71)])
+def test_msa_modules(s, n, device_status):
+    torch.manual_seed(s + n)
+    pm, mm = _masks(n, s)
+    m, z = torch.randn(1, s, n, 256).bfloat16(), torch.randn(1, n, n, 128).bfloat16()
+    _check(_random_parameters(MSARowAttentionWithPairBias(256, 128)).eval(), [m, z, mm], lambda f, x: f(*x))
+    _check(_random_parameters(MSAColumnAttention(256)).eval(), [m, mm], lambda f, x: f(*x))
+    _check(_random_parameters(ExtraMSACore(64, 128)).eval(), [m[..., :64], z, mm], lambda f, x: f(*x))
+
+
+@pytest.mark.parametrize("s,n", [(7, 2), (16, 3), (24, 33), (40, 77), (128, 100)])
+def test_outer_product_mean(s, n, device_status):
+    torch.manual_seed(s + n)
+    mod = _random_parameters(fops.OutProductMean(256, 128, 32)).eval()
+    _check(mod, [torch.randn(1, s, n, 256).bfloat16(), torch.ones(1, s, n), torch.randn(1, n, n, 128).bfloat16()], lambda m, x: m(*x))
+
+
+@pytest.mark.parametrize("S,n", [(5, 16), (83, 24), (131, 40), (517, 8)])
+def test_column_attention_gradients_for_any_number_of_sequences(S, n, device_status):
+    torch.manual_seed(S)
+    mod = _random_parameters(MSAColumnAttention(256)).eval()
+    x, up = torch.randn(1, S, n, 256).bfloat16(), torch.randn(1, S, n, 256).bfloat16()
+    mask = torch.ones(1, S, n)
+    mask[:, S - S // 8:] = 0
+    grads = []
+    for dev, dt in (("cpu", torch.float32), (DEV, torch.bfloat16)):
+        m = copy.deepcopy(mod).to(dev, dt)
+        xi = x.to(dev, dt).requires_grad_(True)
+        out = m(xi, mask.to(dev, dt))
+        grads.append([out.float().cpu()] + [g.float().cpu() for g in torch.autograd.grad(out, [xi] + list(m.parameters()), up.to(dev, dt))])
+    for a, b in zip(*grads):
+        assert ((a - b).norm() / a.norm()).item() < 3e-2
+
+
+def test_bias_pitch(device_status):
+    """Every layout of the pair bias that the forward kernel takes gives the result of the contiguous one."""
+    torch.manual_seed(0)
+    H, n = 4, 75
+    qkv = torch.randn(1, 6, n, 3, H, 32, device=DEV).bfloat16()
+    bias = torch.randn(1, 1, H, n, n, device=DEV).bfloat16()
+    with torch.no_grad():
+        want = flash.flash_attention_packed(qkv, None, bias, 32 ** -0.5)
+        for pitch in (80, 88, 200):
+            wide = torch.full((1, 1, H, n, pitch), float("nan"), device=DEV, dtype=torch.bfloat16)
+            wide[..., :n] = bias
+            assert torch.equal(flash.flash_attention_packed(qkv, None, wide[..., :n], 32 ** -0.5), want)
+        odd = torch.full((1, 1, H, n, 81), float("nan"), device=DEV, dtype=torch.bfloat16)
+        odd[..., :n] = bias
+        assert torch.equal(flash.flash_attention_packed(qkv, None, odd[..., :n], 32 ** -0.5), want)
