@@ -9,7 +9,7 @@ import torch
 from . import _lib
 
 HEAD_DIM = 32
-FWD_HEAD_DIMS = (32,)      # head widths of the forward pass without gradients
+FWD_HEAD_DIMS = (16, 32)   # head widths of the forward kernel without gradients (the kernels with gradients have 32 only)
 MAX_BWD_QUERIES = 512      # queries of one (row, head) whose gradient the backward kernel holds in tensor memory
 
 
