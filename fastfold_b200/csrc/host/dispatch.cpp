@@ -1,0 +1,346 @@
+// Host side of the operator calls: argument checks, output allocation and the launch, from tensors to the C entry points
+// of libffb200.so, without a trip through Python objects for every pointer, stride and flag.
+//
+// Why it is native: a block of the trunk is 60 - 90 launches (a training step of it 250), and with the argument block of
+// a launch filled through ctypes each cost the host 20 - 35 us, so that calls of up to 256 residues were bound by the host:
+// a block of 32 x 64 took 1.98 ms and takes 0.95 ms (65 launches), 128 x 256 the same, the training pass of the pair half at
+// 256 residues 5.3 and 3.5 ms (198 launches).
+//
+// Nothing is kept between calls.  Work goes to the caller's current stream; tensors are allocated by PyTorch's allocator
+// on that stream, exactly as the Python code did.
+#include <torch/extension.h>
+
+#include <c10/cuda/CUDAStream.h>
+
+#include "gemm_api.h"
+
+extern "C" {
+int ffb_gemm_bf16(const void* A, const void* B, int a_mn, int b_mn, long long lda, long long ldb, long long a_bstride, long long b_bstride,
+                  int batch, int bn, GemmArgs* args, void* stream);
+int ffb_layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd, long long rows, int C, float eps,
+                      int dtype, void* stream);
+int ffb_layernorm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx, float* part, int nblocks,
+                      void* dgamma, void* dbeta, long long rows, int C, int dtype, void* stream);
+int ffb_layernorm_fwd_transposed(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd, long long rows, int C,
+                                 float eps, void* stream);
+int ffb_attention_fwd(const void* q, const void* k, const void* v, long long q_bstride, long long q_rstride, long long kv_bstride,
+                      long long kv_rstride, const void* bias, const void* mask, long long mask_bstride, void* out, long long out_bstride,
+                      long long out_rstride, float* lse2, int B, int H, int n_q, int n_k, int D, float scale, void* stream);
+int ffb_attention_infer(const void* q, const void* k, const void* v, long long q_bstride, long long q_rstride, long long kv_bstride,
+                        long long kv_rstride, const void* bias, long long bias_rstride, const void* mask, long long mask_bstride, void* out,
+                        long long out_bstride, long long out_rstride, int B, int H, int n_q, int n_k, int D, float scale, void* stream);
+int ffb_bias_sigmoid_mul_fwd(const void* g, const void* b, const void* o, void* y, long long rows, int C, void* stream);
+int ffb_bias_sigmoid_mul_bwd(const void* dy, const void* g, const void* b, const void* o, void* dg, void* dob, long long rows, int C, void* stream);
+int ffb_bias_dropout_add_fwd(const void* x, const void* b, const void* m, const void* r, void* y, long long rows, int C, int div, int mod, void* stream);
+int ffb_mask_mul(const void* dy, const void* m, void* dx, long long rows, int C, int div, int mod, void* stream);
+int ffb_bias_ele_dropout_res_fwd(const void* ab, const void* b, const void* g, const void* m, const void* r, void* y, long long rows, int C, int div,
+                                 int mod, void* stream);
+int ffb_bias_ele_dropout_res_bwd(const void* dy, const void* ab, const void* b, const void* g, const void* m, void* dab, void* dg, long long rows,
+                                 int C, int div, int mod, void* stream);
+int ffb_glu_mask_t_fwd(const void* pre, const void* mask, void* out, int C2, long long R, void* stream);
+int ffb_glu_mask_t_bwd(const void* dout, const void* pre, const void* mask, void* dpre, int C2, long long R, void* stream);
+int ffb_act_bwd(const void* dy, const void* y, void* dx, long long rows, int C, int mode, void* stream);
+int ffb_colsum(const void* x, float* out, long long rows, int C, void* stream);
+}
+
+namespace {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+long long g_launches = 0;        // guarded by the interpreter lock: every entry below holds it
+
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+void* ptr(const Tensor& t) { return t.data_ptr(); }
+void* ptr(const OptTensor& t) { return t ? t->data_ptr() : nullptr; }
+
+// The checks that the Python wrappers made with ``assert`` raise the same exception type here.
+void expect(bool ok, const char* what) {
+  if (!ok) {
+    PyErr_SetString(PyExc_AssertionError, what);
+    throw pybind11::error_already_set();
+  }
+}
+
+void check(int rc, const char* what) {
+  ++g_launches;
+  TORCH_CHECK(rc == 0, "fastfold_b200 kernel launch failed: ", what, " returned ", rc);
+}
+
+Tensor f32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+
+// See ``gemm`` in ops/gemm.py for the meaning of the arguments.
+Tensor gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, double alpha, OptTensor bias, int act, bool glu, OptTensor rowscale, OptTensor mul,
+            OptTensor dmask, int64_t dm_div, int64_t dm_mod, OptTensor resid, bool trans_out, OptTensor out, bool out_f32, int64_t splits,
+            bool accumulate, int64_t bn, std::optional<std::vector<int64_t>> block_out) {
+  expect(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16, "tcgen05 GEMM takes bf16 operands");
+  if (a.stride(-1) != 1) a = a.contiguous();
+  if (b.stride(-1) != 1) b = b.contiguous();
+  const bool a3 = a.dim() == 3, b3 = b.dim() == 3, batched = a3 || b3;
+  expect((a3 || a.dim() == 2) && (b3 || b.dim() == 2), "operands are matrices or batches of matrices");
+  int64_t batch = 1;
+  if (a3) batch = a.size(0);
+  if (b3) batch = std::max(batch, b.size(0));
+  const int64_t K = a_mn ? a.size(-2) : a.size(-1), M = a_mn ? a.size(-1) : a.size(-2);
+  const int64_t Kb = b_mn ? b.size(-2) : b.size(-1), N = b_mn ? b.size(-1) : b.size(-2);
+  expect(K == Kb, "contraction extents differ");
+  const int64_t n_out = glu ? N / 2 : N;
+  GemmArgs g = {};
+  Tensor result;
+  std::vector<int64_t> oshape;
+  if (batched) oshape.push_back(batch);
+  oshape.push_back(trans_out ? n_out : M);
+  oshape.push_back(trans_out ? M : n_out);
+  if (block_out) {
+    const auto& q = *block_out;      // [shape ..., mdiv, sr2, sr1, sc1]
+    const size_t n = q.size() - 4;
+    expect(!out && M % 32 == 0 && n_out % 32 == 0 && (M / 32) % q[n] == 0 && !out_f32, "block-permuted output");
+    result = at::empty(at::IntArrayRef(q.data(), n), a.options());
+    expect(result.numel() == M * n_out, "block-permuted output");
+    g.cq = 1;
+    g.cq_mdiv = (int)q[n];
+    g.cq_sr2 = q[n + 1];
+    g.cq_sr1 = q[n + 2];
+    g.cq_sc1 = q[n + 3];
+    g.ldc = 8;
+    g.out_mode = OUT_BF16;
+  } else {
+    if (out) {
+      result = *out;
+      expect(result.sizes() == at::IntArrayRef(oshape), "out has another shape than the result");
+      expect(result.stride(-1) == 1, "out rows must be contiguous");
+    } else {
+      result = out_f32 ? f32(oshape, a) : at::empty(oshape, a.options());
+    }
+    if (result.scalar_type() == at::kBFloat16) {
+      expect(!accumulate, "accumulation needs an fp32 output");
+      g.out_mode = OUT_BF16;
+    } else {
+      expect(result.scalar_type() == at::kFloat, "output type");
+      g.out_mode = accumulate ? OUT_F32_ATOMIC : OUT_F32;
+    }
+    g.ldc = result.stride(-2);
+    g.c_bstride = batched ? result.stride(0) : 0;
+  }
+  g.M = (int)M;
+  g.N = (int)N;
+  g.K = (int)K;
+  g.splits = accumulate ? (int)splits : 1;
+  g.trans_out = trans_out;
+  g.act = act;
+  g.glu = glu;
+  g.alpha = (float)alpha;
+  g.C = ptr(result);
+  g.dm_div = g.dm_mod = 1;
+  if (bias) {
+    bias = bias->to(at::kBFloat16).contiguous();
+    expect(bias->numel() == N, "bias length");
+    g.bias = ptr(bias);
+  }
+  if (rowscale) {
+    rowscale = rowscale->to(at::kFloat).contiguous();
+    g.rowscale = static_cast<const float*>(ptr(rowscale));
+    g.rs_bstride = (batched && rowscale->dim() == 2) ? M : 0;
+  }
+  if (mul) {
+    expect(mul->scalar_type() == at::kBFloat16 && mul->stride(-1) == 1, "mul operand");
+    g.mul = ptr(mul);
+    g.ldmul = mul->stride(-2);
+    g.mul_bstride = (batched && mul->dim() == 3) ? mul->stride(0) : 0;
+  }
+  if (dmask) {
+    expect(dmask->scalar_type() == at::kBFloat16 && dmask->stride(-1) == 1 && dmask->size(-1) == n_out, "dropout mask");
+    g.dmask = ptr(dmask);
+    g.lddm = dmask->dim() >= 2 ? dmask->stride(-2) : 0;
+    g.dm_div = (int)dm_div;
+    g.dm_mod = (int)dm_mod;
+  }
+  if (resid) {
+    expect(resid->scalar_type() == at::kBFloat16 && resid->stride(-1) == 1, "residual");
+    g.resid = ptr(resid);
+    g.ldres = resid->stride(-2);
+    g.res_bstride = (batched && resid->dim() == 3) ? resid->stride(0) : 0;
+  }
+  const int rc = ffb_gemm_bf16(ptr(a), ptr(b), a_mn, b_mn, a.stride(-2), b.stride(-2), a3 ? a.stride(0) : 0, b3 ? b.stride(0) : 0, (int)batch,
+                               (int)bn, &g, stream());
+  ++g_launches;
+  TORCH_CHECK(rc == 0, "fastfold_b200 kernel launch failed: ffb_gemm_bf16(M=", M, ",N=", N, ",K=", K, ",batch=", batch, ") returned ", rc);
+  return result;
+}
+
+// Gradients of y = x W^T + b on [rows, c]: each None unless asked for.  The weight gradient is a split-K product into fp32
+// that is then rounded, the bias gradient column sums in fp32.
+std::tuple<OptTensor, OptTensor, OptTensor> linear_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, bool need_x, bool need_w, bool need_b,
+                                                       int64_t splits) {
+  OptTensor dx, dw, db;
+  const OptTensor none;
+  if (need_x) dx = gemm(dy, w, false, true, 1.0, none, ACT_NONE, false, none, none, none, 1, 1, none, false, none, false, 1, false, 0, std::nullopt);
+  if (need_w) {
+    const Tensor acc = at::zeros({dy.size(1), x.size(1)}, dy.options().dtype(at::kFloat));
+    gemm(dy, x, true, true, 1.0, none, ACT_NONE, false, none, none, none, 1, 1, none, false, acc, false, splits, true, 0, std::nullopt);
+    dw = acc.to(w.scalar_type());
+  }
+  if (need_b) {
+    const Tensor acc = at::zeros({dy.size(1)}, dy.options().dtype(at::kFloat));
+    check(ffb_colsum(ptr(dy), static_cast<float*>(ptr(acc)), dy.size(0), (int)dy.size(1), stream()), "colsum");
+    db = acc.to(w.scalar_type());
+  }
+  return {dx, dw, db};
+}
+
+int dtype_code(const Tensor& t) {
+  return t.scalar_type() == at::kFloat ? 0 : (t.scalar_type() == at::kHalf ? 1 : 2);
+}
+
+// y, and mean / rstd when `stats`
+std::tuple<Tensor, OptTensor, OptTensor> layer_norm_fwd(const Tensor& x, const Tensor& weight, const Tensor& bias, double eps, bool stats) {
+  const Tensor w = weight.contiguous(), b = bias.contiguous();
+  const int64_t C = x.size(-1), rows = x.numel() / C;
+  Tensor y = at::empty_like(x);
+  OptTensor mean, rstd;
+  if (stats) {
+    mean = f32({rows}, x);
+    rstd = f32({rows}, x);
+  }
+  check(ffb_layernorm_fwd(ptr(x), ptr(w), ptr(b), ptr(y), static_cast<float*>(ptr(mean)), static_cast<float*>(ptr(rstd)), rows, (int)C, (float)eps,
+                          dtype_code(x), stream()),
+        "layernorm_fwd");
+  return {y, mean, rstd};
+}
+
+std::tuple<Tensor, Tensor, Tensor> layer_norm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd,
+                                                  int64_t nblocks) {
+  const int64_t C = x.size(-1), rows = x.numel() / C;
+  Tensor dx = at::empty_like(x), dg = at::empty_like(w), db = at::empty_like(w), part = f32({nblocks * 2 * C}, x);
+  check(ffb_layernorm_bwd(ptr(dy), ptr(x), ptr(w), static_cast<const float*>(ptr(mean)), static_cast<const float*>(ptr(rstd)), ptr(dx),
+                          static_cast<float*>(ptr(part)), (int)nblocks, ptr(dg), ptr(db), rows, (int)C, dtype_code(x), stream()),
+        "layernorm_bwd");
+  return {dx, dg, db};
+}
+
+std::tuple<Tensor, OptTensor, OptTensor> layer_norm_transposed_fwd(const Tensor& x_cm, const Tensor& weight, const Tensor& bias, double eps,
+                                                                   bool stats) {
+  const Tensor w = weight.contiguous(), b = bias.contiguous();
+  const int64_t C = x_cm.size(0), rows = x_cm.size(1);
+  Tensor y = at::empty({rows, C}, x_cm.options());
+  OptTensor mean, rstd;
+  if (stats) {
+    mean = f32({rows}, x_cm);
+    rstd = f32({rows}, x_cm);
+  }
+  check(ffb_layernorm_fwd_transposed(ptr(x_cm), ptr(w), ptr(b), ptr(y), static_cast<float*>(ptr(mean)), static_cast<float*>(ptr(rstd)), rows, (int)C,
+                                     (float)eps, stream()),
+        "layernorm_fwd_transposed");
+  return {y, mean, rstd};
+}
+
+// qkv [1, B, n, 3, H, d] (transposed: [1, n, B, 3, H, d]); bias [H, n, n] at row pitch `pitch`; mask [B, n] bf16
+std::tuple<Tensor, OptTensor> attention_packed_fwd(const Tensor& qkv, const OptTensor& mask, const OptTensor& bias, int64_t pitch, double scale,
+                                                   bool want_lse, bool transposed) {
+  const int64_t B = qkv.size(transposed ? 2 : 1), n = qkv.size(transposed ? 1 : 2), H = qkv.size(4), d = qkv.size(5), HD = H * d;
+  Tensor out = transposed ? at::empty({1, n, B, HD}, qkv.options()) : at::empty({1, B, n, HD}, qkv.options());
+  OptTensor lse;
+  if (want_lse) lse = f32({B, H, n}, qkv);
+  const int64_t bs = transposed ? 3 * HD : n * 3 * HD, rs = transposed ? B * 3 * HD : 3 * HD;
+  char* base = static_cast<char*>(ptr(qkv));
+  const int64_t obs = transposed ? HD : n * HD, ors = transposed ? B * HD : HD;
+  if (want_lse)           // a pass with gradients: contiguous bias rows
+    check(ffb_attention_fwd(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, ptr(bias), ptr(mask), n, ptr(out), obs, ors,
+                            static_cast<float*>(ptr(lse)), (int)B, (int)H, (int)n, (int)n, (int)d, (float)scale, stream()),
+          "ffb_attention_fwd packed");
+  else
+    check(ffb_attention_infer(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, ptr(bias), pitch, ptr(mask), n, ptr(out), obs, ors, (int)B, (int)H,
+                              (int)n, (int)n, (int)d, (float)scale, stream()),
+          "ffb_attention_infer packed");
+  return {out, lse};
+}
+
+int64_t rows_of(const Tensor& x) { return x.numel() / x.size(-1); }
+
+Tensor bias_sigmoid_mul_fwd(const Tensor& g, const Tensor& b, const Tensor& o) {
+  Tensor y = at::empty_like(g);
+  check(ffb_bias_sigmoid_mul_fwd(ptr(g), ptr(b), ptr(o), ptr(y), rows_of(g), (int)g.size(-1), stream()), "bias_sigmoid_mul_fwd");
+  return y;
+}
+
+std::tuple<Tensor, Tensor> bias_sigmoid_mul_bwd(const Tensor& dy, const Tensor& g, const Tensor& b, const Tensor& o) {
+  Tensor dg = at::empty_like(g), dob = at::empty_like(o);
+  check(ffb_bias_sigmoid_mul_bwd(ptr(dy), ptr(g), ptr(b), ptr(o), ptr(dg), ptr(dob), rows_of(g), (int)g.size(-1), stream()), "bias_sigmoid_mul_bwd");
+  return {dg, dob};
+}
+
+Tensor bias_dropout_add_fwd(const Tensor& x, const OptTensor& b, const OptTensor& m, const Tensor& r, int64_t div, int64_t mod) {
+  Tensor y = at::empty_like(x);
+  check(ffb_bias_dropout_add_fwd(ptr(x), ptr(b), ptr(m), ptr(r), ptr(y), rows_of(x), (int)x.size(-1), (int)div, (int)mod, stream()),
+        "bias_dropout_add_fwd");
+  return y;
+}
+
+Tensor mask_mul(const Tensor& dy, const Tensor& m, int64_t div, int64_t mod) {
+  Tensor dx = at::empty_like(dy);
+  check(ffb_mask_mul(ptr(dy), ptr(m), ptr(dx), rows_of(dy), (int)dy.size(-1), (int)div, (int)mod, stream()), "mask_mul");
+  return dx;
+}
+
+Tensor bias_ele_dropout_res_fwd(const Tensor& ab, const Tensor& b, const Tensor& g, const OptTensor& m, const Tensor& r, int64_t div, int64_t mod) {
+  Tensor y = at::empty_like(ab);
+  check(ffb_bias_ele_dropout_res_fwd(ptr(ab), ptr(b), ptr(g), ptr(m), ptr(r), ptr(y), rows_of(ab), (int)ab.size(-1), (int)div, (int)mod, stream()),
+        "bias_ele_dropout_res_fwd");
+  return y;
+}
+
+std::tuple<Tensor, Tensor> bias_ele_dropout_res_bwd(const Tensor& dy, const Tensor& ab, const Tensor& b, const Tensor& g, const OptTensor& m,
+                                                    int64_t div, int64_t mod) {
+  Tensor dab = at::empty_like(ab), dg = at::empty_like(g);
+  check(ffb_bias_ele_dropout_res_bwd(ptr(dy), ptr(ab), ptr(b), ptr(g), ptr(m), ptr(dab), ptr(dg), rows_of(ab), (int)ab.size(-1), (int)div, (int)mod,
+                                     stream()),
+        "bias_ele_dropout_res_bwd");
+  return {dab, dg};
+}
+
+Tensor glu_mask_t_fwd(const Tensor& pre, const Tensor& mask) {
+  const int64_t C2 = pre.size(0) / 2, R = pre.size(1);
+  Tensor out = at::empty({C2, R}, pre.options());
+  check(ffb_glu_mask_t_fwd(ptr(pre), ptr(mask), ptr(out), (int)C2, R, stream()), "glu_mask_t_fwd");
+  return out;
+}
+
+Tensor glu_mask_t_bwd(const Tensor& dout, const Tensor& pre, const Tensor& mask) {
+  Tensor dpre = at::empty_like(pre);
+  check(ffb_glu_mask_t_bwd(ptr(dout), ptr(pre), ptr(mask), ptr(dpre), (int)(pre.size(0) / 2), pre.size(1), stream()), "glu_mask_t_bwd");
+  return dpre;
+}
+
+Tensor act_bwd(const Tensor& dy, const Tensor& y, int mode) {
+  Tensor dx = at::empty_like(dy);
+  check(ffb_act_bwd(ptr(dy), ptr(y), ptr(dx), rows_of(dy), (int)dy.size(-1), mode, stream()), "act_bwd");
+  return dx;
+}
+
+Tensor colsum(const Tensor& x, OptTensor out) {
+  if (!out) out = at::zeros({x.size(1)}, x.options().dtype(at::kFloat));
+  check(ffb_colsum(ptr(x), static_cast<float*>(ptr(*out)), x.size(0), (int)x.size(1), stream()), "colsum");
+  return *out;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_ffb_dispatch, m) {
+  m.def("gemm", &gemm);
+  m.def("linear_bwd", &linear_bwd);
+  m.def("layer_norm_fwd", &layer_norm_fwd);
+  m.def("layer_norm_bwd", &layer_norm_bwd);
+  m.def("layer_norm_transposed_fwd", &layer_norm_transposed_fwd);
+  m.def("attention_packed_fwd", &attention_packed_fwd);
+  m.def("bias_sigmoid_mul_fwd", &bias_sigmoid_mul_fwd);
+  m.def("bias_sigmoid_mul_bwd", &bias_sigmoid_mul_bwd);
+  m.def("bias_dropout_add_fwd", &bias_dropout_add_fwd);
+  m.def("mask_mul", &mask_mul);
+  m.def("bias_ele_dropout_res_fwd", &bias_ele_dropout_res_fwd);
+  m.def("bias_ele_dropout_res_bwd", &bias_ele_dropout_res_bwd);
+  m.def("glu_mask_t_fwd", &glu_mask_t_fwd);
+  m.def("glu_mask_t_bwd", &glu_mask_t_bwd);
+  m.def("act_bwd", &act_bwd);
+  m.def("colsum", &colsum);
+  m.def("launches", []() { return g_launches; });
+}

@@ -7,6 +7,8 @@ CPU-only machine the ops use their PyTorch reference implementations and this
 module is never asked for the library.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import threading
 
@@ -14,8 +16,9 @@ import torch
 
 from .. import _build
 
-_lock = threading.Lock()
+_lock = threading.RLock()
 _lib = None
+_native = None
 
 c_void_p = ctypes.c_void_p
 c_int = ctypes.c_int
@@ -113,6 +116,23 @@ def get():
     return _lib
 
 
+def native():
+    """The extension module of csrc/host/dispatch.cpp: the frequent operator calls, tensors in and out."""
+    global _native
+    if _native is not None:
+        return _native
+    with _lock:
+        if _native is None:
+            get()                                    # builds both libraries when they are missing
+            path = _build.dispatch_path()
+            if not os.path.exists(path):
+                _build.build(verbose=False)
+            loader = importlib.machinery.ExtensionFileLoader(_build.DISPATCH, path)
+            _native = importlib.util.module_from_spec(importlib.util.spec_from_loader(_build.DISPATCH, loader))
+            loader.exec_module(_native)
+    return _native
+
+
 def has(name):
     return hasattr(get(), name)
 
@@ -132,11 +152,25 @@ def dtype_code(dt):
     return _DT[dt]
 
 
-LAUNCHES = [0]   # number of native launcher calls made through this module (bench.py reports it)
+class _Launches:
+    """Number of native launcher calls as ``LAUNCHES[0]`` (bench.py reports it): those made through ctypes and those that
+    the extension module counts."""
+
+    def __init__(self):
+        self.here = 0
+
+    def __getitem__(self, i):
+        return self.here + (_native.launches() if _native is not None else 0)
+
+    def __setitem__(self, i, n):
+        self.here = n - (_native.launches() if _native is not None else 0)
+
+
+LAUNCHES = _Launches()
 
 
 def check(code, what):
-    LAUNCHES[0] += 1
+    LAUNCHES.here += 1
     if code != 0:
         raise RuntimeError("fastfold_b200 kernel launch failed: %s returned %d" % (what, code))
 

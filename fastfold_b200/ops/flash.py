@@ -172,24 +172,13 @@ def _packed_geometry(qkv, transposed):
 
 
 def _packed_fwd(qkv, mask, bias, scale, want_lse, transposed):
-    lib = _lib.get()
-    B, n, H, d, (bs, rs), (obs, ors) = _packed_geometry(qkv, transposed)
-    HD = H * d
-    out = torch.empty((1, n, B, HD) if transposed else (1, B, n, HD), device=qkv.device, dtype=qkv.dtype)
-    lse = torch.empty(B, H, n, device=qkv.device, dtype=torch.float32) if want_lse else None
+    B, n, H = _packed_geometry(qkv, transposed)[:3]
     if want_lse:                                          # the backward kernel reads un-padded rows
         b3, pitch = (bias.reshape(H, n, n).contiguous() if bias is not None else None), n
     else:
         b3, pitch = _pitched_bias(bias, H, n, n)
     m2 = mask.reshape(B, n).to(torch.bfloat16).contiguous() if mask is not None else None
-    base = qkv.data_ptr()
-    if want_lse:
-        rc = lib.ffb_attention_fwd(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, _lib.ptr(b3), _lib.ptr(m2), n,
-                                   _lib.ptr(out), obs, ors, _lib.ptr(lse), B, H, n, n, d, float(scale), _lib.stream_ptr())
-    else:
-        rc = lib.ffb_attention_infer(base, base + 2 * HD, base + 4 * HD, bs, rs, bs, rs, _lib.ptr(b3), pitch, _lib.ptr(m2), n,
-                                     _lib.ptr(out), obs, ors, B, H, n, n, d, float(scale), _lib.stream_ptr())
-    _lib.check(rc, "ffb_attention_fwd packed (B=%d,H=%d,n=%d)" % (B, H, n))
+    out, lse = _lib.native().attention_packed_fwd(qkv, m2, b3, pitch, scale, want_lse, transposed)
     return out, lse, b3, m2
 
 

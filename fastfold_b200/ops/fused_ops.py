@@ -52,26 +52,17 @@ def _mask_index(x, mask):
 class _BiasSigmoidMul(torch.autograd.Function):
     @staticmethod
     def forward(ctx, g, bias, o):
-        lib = _lib.get()
         gc, oc, bc = g.contiguous(), o.contiguous(), bias.contiguous()
-        rows, C = _rows_c(gc)
-        y = torch.empty_like(gc)
-        _lib.check(lib.ffb_bias_sigmoid_mul_fwd(_lib.ptr(gc), _lib.ptr(bc), _lib.ptr(oc), _lib.ptr(y), rows, C, _lib.stream_ptr()),
-                   "bias_sigmoid_mul_fwd")
+        y = _lib.native().bias_sigmoid_mul_fwd(gc, bc, oc)
         ctx.save_for_backward(gc, bc, oc)
         ctx.bias_param = bias
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        lib = _lib.get()
         gc, bc, oc = ctx.saved_tensors
         rows, C = _rows_c(gc)
-        dg = torch.empty_like(gc)
-        do = torch.empty_like(oc)
-        dyc = dy.contiguous()
-        _lib.check(lib.ffb_bias_sigmoid_mul_bwd(_lib.ptr(dyc), _lib.ptr(gc), _lib.ptr(bc), _lib.ptr(oc), _lib.ptr(dg), _lib.ptr(do),
-                                                rows, C, _lib.stream_ptr()), "bias_sigmoid_mul_bwd")
+        dg, do = _lib.native().bias_sigmoid_mul_bwd(dy.contiguous(), gc, bc, oc)
         db = _bias_grad(ctx.bias_param, dg.reshape(rows, C), bc.dtype) if ctx.needs_input_grad[1] else None
         return dg, db, do
 
@@ -86,12 +77,7 @@ def bias_sigmod_ele(y, bias, z):
 class _BiasDropoutAdd(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, bias, m2, div, mod, resid):
-        lib = _lib.get()
-        xc, rc = x.contiguous(), resid.contiguous()
-        rows, C = _rows_c(xc)
-        y = torch.empty_like(xc)
-        _lib.check(lib.ffb_bias_dropout_add_fwd(_lib.ptr(xc), _lib.ptr(bias), _lib.ptr(m2), _lib.ptr(rc), _lib.ptr(y), rows, C,
-                                                div, mod, _lib.stream_ptr()), "bias_dropout_add_fwd")
+        y = _lib.native().bias_dropout_add_fwd(x.contiguous(), bias, m2, resid.contiguous(), div, mod)
         ctx.save_for_backward(m2)
         ctx.dm = (div, mod)
         ctx.has_bias = bias is not None
@@ -100,14 +86,11 @@ class _BiasDropoutAdd(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        lib = _lib.get()
         (m2,) = ctx.saved_tensors
         dyc = dy.contiguous()
         rows, C = _rows_c(dyc)
         if m2 is not None:
-            dx = torch.empty_like(dyc)
-            _lib.check(lib.ffb_mask_mul(_lib.ptr(dyc), _lib.ptr(m2), _lib.ptr(dx), rows, C, ctx.dm[0], ctx.dm[1], _lib.stream_ptr()),
-                       "mask_mul")
+            dx = _lib.native().mask_mul(dyc, m2, *ctx.dm)
         else:
             dx = dyc
         db = _bias_grad(ctx.bias_param, dx.reshape(rows, C), dyc.dtype) if (ctx.has_bias and ctx.needs_input_grad[1]) else None
@@ -136,12 +119,8 @@ def bias_dropout_add(x, bias, dropmask, residual, prob, training=True):
 class _BiasEleDropoutRes(torch.autograd.Function):
     @staticmethod
     def forward(ctx, ab, b, g, m2, div, mod, resid):
-        lib = _lib.get()
-        abc, gc, rc, bc = ab.contiguous(), g.contiguous(), resid.contiguous(), b.contiguous()
-        rows, C = _rows_c(abc)
-        y = torch.empty_like(abc)
-        _lib.check(lib.ffb_bias_ele_dropout_res_fwd(_lib.ptr(abc), _lib.ptr(bc), _lib.ptr(gc), _lib.ptr(m2), _lib.ptr(rc), _lib.ptr(y),
-                                                    rows, C, div, mod, _lib.stream_ptr()), "bias_ele_dropout_res_fwd")
+        abc, gc, bc = ab.contiguous(), g.contiguous(), b.contiguous()
+        y = _lib.native().bias_ele_dropout_res_fwd(abc, bc, gc, m2, resid.contiguous(), div, mod)
         ctx.save_for_backward(abc, bc, gc, m2)
         ctx.dm = (div, mod)
         ctx.bias_param = b
@@ -149,15 +128,10 @@ class _BiasEleDropoutRes(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        lib = _lib.get()
         abc, bc, gc, m2 = ctx.saved_tensors
         dyc = dy.contiguous()
         rows, C = _rows_c(dyc)
-        dab = torch.empty_like(abc)
-        dg = torch.empty_like(gc)
-        _lib.check(lib.ffb_bias_ele_dropout_res_bwd(_lib.ptr(dyc), _lib.ptr(abc), _lib.ptr(bc), _lib.ptr(gc), _lib.ptr(m2),
-                                                    _lib.ptr(dab), _lib.ptr(dg), rows, C, ctx.dm[0], ctx.dm[1], _lib.stream_ptr()),
-                   "bias_ele_dropout_res_bwd")
+        dab, dg = _lib.native().bias_ele_dropout_res_bwd(dyc, abc, bc, gc, m2, *ctx.dm)
         db = _bias_grad(ctx.bias_param, dab.reshape(rows, C), bc.dtype) if ctx.needs_input_grad[1] else None
         return dab, db, dg, None, None, None, dyc
 
@@ -224,17 +198,13 @@ class _GluMaskT(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, pre, mask, split):
-        lib = _lib.get()
-        C2, R = pre.shape[0] // 2, pre.shape[1]
-        out = torch.empty(C2, R, device=pre.device, dtype=pre.dtype)
-        _lib.check(lib.ffb_glu_mask_t_fwd(_lib.ptr(pre), _lib.ptr(mask), _lib.ptr(out), C2, R, _lib.stream_ptr()), "glu_mask_t_fwd")
+        out = _lib.native().glu_mask_t_fwd(pre, mask)
         ctx.save_for_backward(pre, mask)
         ctx.split = split
         return out[:split], out[split:]
 
     @staticmethod
     def backward(ctx, d_lo, d_hi):
-        lib = _lib.get()
         pre, mask = ctx.saved_tensors
         C2, R = pre.shape[0] // 2, pre.shape[1]
         if d_lo is None:
@@ -242,9 +212,7 @@ class _GluMaskT(torch.autograd.Function):
         if d_hi is None:
             d_hi = pre.new_zeros(C2 - ctx.split, R)
         dout = torch.cat([d_lo.reshape(ctx.split, R), d_hi.reshape(C2 - ctx.split, R)], dim=0)
-        dpre = torch.empty_like(pre)
-        _lib.check(lib.ffb_glu_mask_t_bwd(_lib.ptr(dout), _lib.ptr(pre), _lib.ptr(mask), _lib.ptr(dpre), C2, R, _lib.stream_ptr()), "glu_mask_t_bwd")
-        return dpre, None, None
+        return _lib.native().glu_mask_t_bwd(dout, pre, mask), None, None
 
 
 def glu_mask_t(pre, mask, split=None):
@@ -343,12 +311,7 @@ def act_backward(dy2, y2, act):
     """dy * act'(pre-activation), expressed through the saved activation output."""
     mode = 1 if act == "relu" else 2
     if _bf16_cuda(dy2, y2) and dy2.shape[-1] % 8 == 0:
-        lib = _lib.get()
-        dyc, yc = dy2.contiguous(), y2.contiguous()
-        rows, C = _rows_c(dyc)
-        dx = torch.empty_like(dyc)
-        _lib.check(lib.ffb_act_bwd(_lib.ptr(dyc), _lib.ptr(yc), _lib.ptr(dx), rows, C, mode, _lib.stream_ptr()), "act_bwd")
-        return dx
+        return _lib.native().act_bwd(dy2.contiguous(), y2.contiguous(), mode)
     if mode == 1:
         return dy2 * (y2 > 0).to(dy2.dtype)
     return dy2 * y2 * (1 - y2)
@@ -357,12 +320,7 @@ def act_backward(dy2, y2, act):
 def colsum(x2, out=None):
     """fp32 column sums of a 2-D tensor; with ``out`` (fp32 ``[C]``) the sums are ADDED into it."""
     if x2.is_cuda and x2.dtype == torch.bfloat16 and x2.shape[-1] % 2 == 0:
-        lib = _lib.get()
-        xc = x2.contiguous()
-        if out is None:
-            out = torch.zeros(xc.shape[-1], device=xc.device, dtype=torch.float32)
-        _lib.check(lib.ffb_colsum(_lib.ptr(xc), _lib.ptr(out), xc.shape[0], xc.shape[1], _lib.stream_ptr()), "colsum")
-        return out
+        return _lib.native().colsum(x2.contiguous(), out)
     r = x2.float().sum(dim=0)
     if out is not None:
         out.add_(r)

@@ -95,6 +95,12 @@ def gemm(a, b, *, a_mn=False, b_mn=False, alpha=1.0, bias=None, act=None, glu=Fa
                 out.copy_(r)
             return out
         return r
+    if peer is None:
+        assert out_dtype in (None, torch.bfloat16, torch.float32)
+        blocked = None if block_out is None else [*block_out[0], *block_out[1:]]
+        m, div, mod = dmask if dmask is not None else (None, 1, 1)
+        return _lib.native().gemm(a, b, a_mn, b_mn, alpha, bias, _ACT[act], glu, rowscale, mul, m, div, mod, resid, trans_out, out,
+                                  out_dtype == torch.float32, splits, accumulate, bn, blocked)
     lib = _lib.get()
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "tcgen05 GEMM takes bf16 operands"
     if a.stride(-1) != 1:
@@ -116,13 +122,11 @@ def gemm(a, b, *, a_mn=False, b_mn=False, alpha=1.0, bias=None, act=None, glu=Fa
     else:
         N, Kb = b3.shape[1], b3.shape[2]
     assert K == Kb, "contraction extents differ: %d vs %d" % (K, Kb)
-    peer_slab = 0
-    if peer is not None:
-        which, addrs = peer
-        if which == "a":
-            peer_slab, M = M, M * len(addrs)
-        else:
-            peer_slab, N = N, N * len(addrs)
+    which, addrs = peer
+    if which == "a":
+        peer_slab, M = M, M * len(addrs)
+    else:
+        peer_slab, N = N, N * len(addrs)
     n_out = N // 2 if glu else N
     batched = a.dim() == 3 or b.dim() == 3
     oshape = (n_out, M) if trans_out else (M, n_out)
@@ -189,20 +193,13 @@ def gemm(a, b, *, a_mn=False, b_mn=False, alpha=1.0, bias=None, act=None, glu=Fa
         g.resid = resid.data_ptr()
         g.ldres = resid.stride(-2)
         g.res_bstride = resid.stride(0) if (batched and resid.dim() == 3) else 0
-    if peer is not None:
-        import ctypes
-        which, addrs = peer
-        g.peer_slab = peer_slab
-        arr = (ctypes.c_void_p * len(addrs))(*[int(x) for x in addrs])
-        rc = lib.ffb_gemm_bf16_peer(_lib.ptr(a3), _lib.ptr(b3), 1 if a_mn else 0, 1 if b_mn else 0, a3.stride(1), b3.stride(1),
-                                    a3.stride(0) if a.dim() == 3 else 0, b3.stride(0) if b.dim() == 3 else 0, batch, g,
-                                    1 if which == "a" else 2, arr, len(addrs), _lib.stream_ptr())
-        _lib.check(rc, "ffb_gemm_bf16_peer(M=%d,N=%d,K=%d,batch=%d,slab=%d)" % (M, N, K, batch, peer_slab))
-        return blocked if blocked is not None else out
-    rc = lib.ffb_gemm_bf16(_lib.ptr(a3), _lib.ptr(b3), 1 if a_mn else 0, 1 if b_mn else 0, a3.stride(1), b3.stride(1),
-                           a3.stride(0) if a.dim() == 3 else 0, b3.stride(0) if b.dim() == 3 else 0, batch, bn, g,
-                           _lib.stream_ptr())
-    _lib.check(rc, "ffb_gemm_bf16(M=%d,N=%d,K=%d,batch=%d)" % (M, N, K, batch))
+    import ctypes
+    g.peer_slab = peer_slab
+    arr = (ctypes.c_void_p * len(addrs))(*[int(x) for x in addrs])
+    rc = lib.ffb_gemm_bf16_peer(_lib.ptr(a3), _lib.ptr(b3), 1 if a_mn else 0, 1 if b_mn else 0, a3.stride(1), b3.stride(1),
+                                a3.stride(0) if a.dim() == 3 else 0, b3.stride(0) if b.dim() == 3 else 0, batch, g,
+                                1 if which == "a" else 2, arr, len(addrs), _lib.stream_ptr())
+    _lib.check(rc, "ffb_gemm_bf16_peer(M=%d,N=%d,K=%d,batch=%d,slab=%d)" % (M, N, K, batch, peer_slab))
     return blocked if blocked is not None else out
 
 
@@ -239,6 +236,13 @@ class _Linear(torch.autograd.Function):
         if ctx.act:
             dy2 = fused_ops.act_backward(dy2, y, ctx.act)
         dx = dw = db = None
+        n_out, n_in = w.shape
+        if (dy2.is_cuda and grad_sink(w) is None and ctx.bias_ref is None and n_out >= 64 and n_in >= 64 and n_out % 8 == 0 and n_in % 8 == 0
+                and x2.is_contiguous() and w.is_contiguous()):
+            tiles = ((n_out + 127) // 128) * ((n_in + 127) // 128)
+            dx, dw, db = _lib.native().linear_bwd(dy2, x2, w, ctx.needs_input_grad[0], ctx.needs_input_grad[1],
+                                                  ctx.has_bias and ctx.needs_input_grad[2], _wgrad_splits(dy2.shape[0], tiles))
+            return None if dx is None else dx.view(ctx.xshape), dw, db, None
         if ctx.needs_input_grad[0]:
             dx = gemm(dy2, w, b_mn=True).reshape(ctx.xshape)
         if ctx.needs_input_grad[1] and not sink_weight_grad(w, dy2, x2):

@@ -11,6 +11,7 @@ import numbers
 
 import torch
 from torch import nn
+from torch.autograd import forward_ad
 
 from . import _lib
 
@@ -26,21 +27,11 @@ def _native_ok(x, weight):
 class _LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, eps):
-        lib = _lib.get()
         xc = x.contiguous()
-        C = xc.shape[-1]
-        rows = xc.numel() // C
-        y = torch.empty_like(xc)
-        need_stats = torch.is_grad_enabled() or ctx.needs_input_grad[0] or ctx.needs_input_grad[1]
-        mean = torch.empty(rows, device=x.device, dtype=torch.float32)
-        rstd = torch.empty(rows, device=x.device, dtype=torch.float32)
         w = weight.contiguous()
-        b = bias.contiguous()
-        _lib.check(lib.ffb_layernorm_fwd(_lib.ptr(xc), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), _lib.ptr(mean), _lib.ptr(rstd),
-                                         rows, C, float(eps), _lib.dtype_code(x.dtype), _lib.stream_ptr()), "layernorm_fwd")
+        y, mean, rstd = _lib.native().layer_norm_fwd(xc, w, bias, eps, True)
         ctx.save_for_backward(xc, w, mean, rstd)
         ctx.params = (weight, bias)
-        del need_stats
         return y
 
     @staticmethod
@@ -50,29 +41,33 @@ class _LayerNormFn(torch.autograd.Function):
         dyc = dy.contiguous()
         C = xc.shape[-1]
         rows = xc.numel() // C
-        dx = torch.empty_like(xc)
         nblocks = int(min(1184, max(1, (rows + 3) // 4)))   # 8 blocks per SM: enough warps in flight to hide the per-row reductions
-        part = torch.empty(nblocks * 2 * C, device=xc.device, dtype=torch.float32)
         from .gemm import grad_sink
         sg, sb = grad_sink(ctx.params[0]), grad_sink(ctx.params[1])
         if sg is not None and sb is not None and xc.dtype == torch.bfloat16 and _lib.has("ffb_layernorm_bwd_acc"):
             # gamma / beta gradients go straight into the trainer's fp32 buffer
+            dx = torch.empty_like(xc)
+            part = torch.empty(nblocks * 2 * C, device=xc.device, dtype=torch.float32)
             _lib.check(lib.ffb_layernorm_bwd_acc(_lib.ptr(dyc), _lib.ptr(xc), _lib.ptr(w), _lib.ptr(mean), _lib.ptr(rstd), _lib.ptr(dx),
                                                  _lib.ptr(part), nblocks, _lib.ptr(sg), _lib.ptr(sb), rows, C, _lib.stream_ptr()),
                        "layernorm_bwd_acc")
             return dx, None, None, None
-        dg = torch.empty_like(w)
-        db = torch.empty_like(w)
-        _lib.check(lib.ffb_layernorm_bwd(_lib.ptr(dyc), _lib.ptr(xc), _lib.ptr(w), _lib.ptr(mean), _lib.ptr(rstd), _lib.ptr(dx),
-                                         _lib.ptr(part), nblocks, _lib.ptr(dg), _lib.ptr(db), rows, C,
-                                         _lib.dtype_code(xc.dtype), _lib.stream_ptr()), "layernorm_bwd")
+        dx, dg, db = _lib.native().layer_norm_bwd(dyc, xc, w, mean, rstd, nblocks)
         return dx, dg, db, None
 
 
 def layer_norm(x, weight, bias, eps=1e-5):
     if not _native_ok(x, weight):
         return torch.nn.functional.layer_norm(x, (x.shape[-1],), weight.to(x.dtype), bias.to(x.dtype), eps)
+    if not _needs_graph(x, weight, bias):
+        return _lib.native().layer_norm_fwd(x.contiguous(), weight, bias, eps, False)[0]
     return _LayerNormFn.apply(x, weight, bias, eps)
+
+
+def _needs_graph(*ts):
+    """False when no gradient can be asked for: the autograd function is then passed by (inside a forward-mode level it is
+    not - it raises there, and must go on doing so)."""
+    return (torch.is_grad_enabled() and any(t.requires_grad for t in ts)) or forward_ad._current_level >= 0
 
 
 def _ln_t_supported(x_cm):
@@ -80,15 +75,8 @@ def _ln_t_supported(x_cm):
 
 
 def _ln_t_forward(x_cm, weight, bias, eps, want_stats):
-    lib = _lib.get()
-    C, rows = x_cm.shape
     x_cm = x_cm.contiguous()
-    y = torch.empty(rows, C, device=x_cm.device, dtype=x_cm.dtype)
-    mean = torch.empty(rows, device=x_cm.device, dtype=torch.float32) if want_stats else None
-    rstd = torch.empty(rows, device=x_cm.device, dtype=torch.float32) if want_stats else None
-    _lib.check(lib.ffb_layernorm_fwd_transposed(_lib.ptr(x_cm), _lib.ptr(weight.contiguous()), _lib.ptr(bias.contiguous()),
-                                                _lib.ptr(y), _lib.ptr(mean), _lib.ptr(rstd), rows, C, float(eps), _lib.stream_ptr()),
-               "layernorm_fwd_transposed")
+    y, mean, rstd = _lib.native().layer_norm_transposed_fwd(x_cm, weight, bias, eps, want_stats)
     return y, x_cm, mean, rstd
 
 
