@@ -1,6 +1,6 @@
 // Invariant point attention core (AlphaFold Algorithm 22, lines 7-11) as one flash-style kernel.
 //
-// For every query residue i (one CTA per query row) the kernel streams the keys j in chunks and keeps, per head h,
+// For every query residue i (two or four per CTA) the kernel streams the keys j in chunks and keeps, per head h,
 // an online softmax over
 //     logit[h][j] = w_C * q_i.k_j  +  sqrt(1/3) * (z[i][j] . W_b[h] + b_b[h])
 //                   - 0.5 * gamma_h * sum_p |q_pt[i][h][p] - k_pt[j][h][p]|^2  +  inf * (mask_i * mask_j - 1)
@@ -17,9 +17,8 @@
 
 namespace ffb {
 
-constexpr int IPA_THREADS = 256;
+constexpr int IPA_THREADS = 384;   // one warp per head
 constexpr int IPA_J = 64;          // keys per chunk
-constexpr int IPA_MAXH = 16;
 constexpr int IPA_ZP = 8;          // padding (bf16) of a z row in shared memory: consecutive keys fall into different banks
 
 struct IpaArgs {
@@ -41,157 +40,363 @@ struct IpaArgs {
   float w_c, w_b, inf;
 };
 
-template <int H, int C, int PQ, int PV, int CZ>
-__global__ void __launch_bounds__(IPA_THREADS) ipa_fwd_kernel(const IpaArgs a) {
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in_range) {
+  const int bytes = in_range ? 16 : 0;                         // 0: the 16 bytes are filled with zeros, nothing is read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// R query rows per CTA, 12 warps.
+//   logits : warp = head, lane = key (two per chunk); k, k_pts once per key for all R rows, z and w_b from shared memory.
+//            The softmax of a (row, head) stays in the warp's registers.
+//   sums   : warps 0 .. 2R-1 own (row, two pair channels) for all heads, the others the 480 scalar / point channels for all
+//            rows, so that v and v_pts are read once per CTA.
+// The z chunk after next is on its way (cp.async) while this one is used; two barriers per chunk.
+//
+// What bounds it: instruction issue (about 50 issue slots x SM sub-partition per (query, key) pair for all heads) and, below
+// some 150 CTAs, the number of SMs in use.  One row per CTA with one key-value read per row, which this replaces, spent its
+// time waiting for L2: every row re-read 3.2 KB of keys, values and points per key, a quarter of the warps in flight.
+// R = 2 with two CTAs per SM below 1024 rows, where R = 4 would leave SMs without a CTA; R = 4 (half the key / value traffic)
+// from there on.
+//   Measured (B200, N = 512): 349 us with one row per CTA, 200 us with R = 2.
+template <int R, int H, int C, int PQ, int PV, int CZ>
+__global__ void __launch_bounds__(IPA_THREADS, R == 2 ? 2 : 1) ipa_fwd_kernel(const IpaArgs a) {
   pdl_launch_dependents();
   pdl_wait();
+  static_assert(H * 32 == IPA_THREADS && CZ == 128, "one warp per head");
   constexpr int ZROW = CZ + IPA_ZP;
-  constexpr int VC = C + 3 * PV;                 // value channels per head that do not come from z
-  extern __shared__ uint8_t ipa_smem[];
-  bf16* zs = reinterpret_cast<bf16*>(ipa_smem);                                  // [J][ZROW]
-  float* wbt = reinterpret_cast<float*>(ipa_smem + IPA_J * ZROW * 2);            // [CZ][H + 1]  (transposed, padded)
-  float* qs = wbt + CZ * (H + 1);                                                // [H][C]
-  float* qp = qs + H * C;                                                        // [H][PQ * 3]
-  float* ps = qp + H * PQ * 3;                                                   // [H][J]  logits, then probabilities
-  float* mrun = ps + H * IPA_J;                                                  // [H] running max
-  float* lrun = mrun + H;                                                        // [H] running sum
-  float* alph = lrun + H;                                                        // [H] rescale factor of this chunk
+  constexpr int VC = H * C, VT = H * PV * 3;                 // value channels from v and from v_pts
+  constexpr int ZT = R * (CZ / 2);                           // threads on the pair channels
+  constexpr int NV_T = IPA_THREADS - ZT;                     // threads on the value channels
+  constexpr int NVA = (VC + VT + NV_T - 1) / NV_T;           // value channels per such thread
+  extern __shared__ __align__(16) uint8_t ipa_smem[];
+  bf16* zs = reinterpret_cast<bf16*>(ipa_smem);                                  // [2][R][J][ZROW]
+  float* wbs = reinterpret_cast<float*>(ipa_smem + 2 * R * IPA_J * ZROW * 2);    // [H][CZ]
+  float* qs = wbs + H * CZ;                                                      // [R][H][C]
+  float* qp = qs + R * H * C;                                                    // [R][H][PQ * 3]
+  float* ps = qp + R * H * PQ * 3;                                               // [R][J][H] probabilities of the chunk
+  float* alph = ps + R * IPA_J * H;                                              // [R][H] rescale factor of the chunk
+  float* lfin = alph + R * H;                                                    // [R][H] row sums at the end
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int r = blockIdx.x;
-  if (r >= a.rows) return;
-  const int i = a.row0 + r;
+  const int r0 = blockIdx.x * R;
   const int N = a.N;
-  for (int t = tid; t < H * CZ; t += IPA_THREADS) {
-    const int h = t / CZ, c = t - h * CZ;
-    wbt[c * (H + 1) + h] = a.wb[t];
-  }
-  for (int t = tid; t < H * C; t += IPA_THREADS) qs[t] = a.q[(long long)i * H * C + t];
-  for (int t = tid; t < H * PQ * 3; t += IPA_THREADS) qp[t] = a.q_pts[(long long)i * H * PQ * 3 + t];
-  if (tid < H) {
-    mrun[tid] = -INFINITY;
-    lrun[tid] = 0.f;
-  }
-  const float mask_i = a.mask ? a.mask[i] : 1.f;
-  // accumulators: threads [0, CZ) own pair channel `tid` for every head; threads [CZ, 256) own the scalar / point channels
-  float acc_z[H];
-#pragma unroll
-  for (int h = 0; h < H; ++h) acc_z[h] = 0.f;
-  constexpr int NV_T = IPA_THREADS - CZ;                      // threads on the value channels
-  constexpr int NVA = (H * VC + NV_T - 1) / NV_T;             // accumulators per such thread
-  float acc_v[NVA];
-#pragma unroll
-  for (int u = 0; u < NVA; ++u) acc_v[u] = 0.f;
-  const bf16* zrow = a.z + (long long)r * N * CZ;
-  __syncthreads();
-
-  for (int j0 = 0; j0 < N; j0 += IPA_J) {
-    const int jn = (N - j0) < IPA_J ? (N - j0) : IPA_J;
-    // ---- stage the chunk of the pair row: [jn][CZ] bf16, 16-byte loads ----
-    for (int t = tid; t < IPA_J * (CZ / 8); t += IPA_THREADS) {
-      const int j = t / (CZ / 8), c8 = t - j * (CZ / 8);
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (j < jn) val = *reinterpret_cast<const uint4*>(zrow + (long long)(j0 + j) * CZ + c8 * 8);
-      *reinterpret_cast<uint2*>(zs + j * ZROW + c8 * 8) = make_uint2(val.x, val.y);
-      *reinterpret_cast<uint2*>(zs + j * ZROW + c8 * 8 + 4) = make_uint2(val.z, val.w);
+  const uint32_t zs_addr = smem_u32(zs);
+  auto load_z = [&](int chunk) {
+    const int j0 = chunk * IPA_J;
+    for (int t = tid; t < R * IPA_J * (CZ / 8); t += IPA_THREADS) {
+      const int c8 = t % (CZ / 8), j = t / (CZ / 8) % IPA_J, r = t / (CZ / 8 * IPA_J);
+      const bool ok = j0 + j < N && r0 + r < a.rows;
+      const bf16* src = ok ? a.z + ((long long)(r0 + r) * N + j0 + j) * CZ + c8 * 8 : a.z;
+      cp_async16(zs_addr + (((chunk & 1) * R + r) * IPA_J + j) * ZROW * 2 + c8 * 16, src, ok);
     }
-    __syncthreads();
-    // ---- logits: one (key, head) pair per thread and step ----
-    for (int t = tid; t < IPA_J * H; t += IPA_THREADS) {
-      const int j = t / H, h = t - j * H;
-      float logit = -INFINITY;
-      if (j < jn) {
-        const int jj = j0 + j;
-        const float4* kp = reinterpret_cast<const float4*>(a.k + ((long long)jj * H + h) * C);
-        float qk = 0.f;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load_z(0);
+  for (int t = tid; t < H * CZ; t += IPA_THREADS) wbs[t] = a.wb[t];
+  for (int t = tid; t < R * H * C; t += IPA_THREADS) {
+    const int r = t / (H * C);
+    qs[t] = r0 + r < a.rows ? a.q[(long long)(a.row0 + r0 + r) * H * C + t % (H * C)] : 0.f;
+  }
+  for (int t = tid; t < R * H * PQ * 3; t += IPA_THREADS) {
+    const int r = t / (H * PQ * 3);
+    qp[t] = r0 + r < a.rows ? a.q_pts[(long long)(a.row0 + r0 + r) * H * PQ * 3 + t % (H * PQ * 3)] : 0.f;
+  }
+  float mrun[R], lrun[R], mask_i[R];
 #pragma unroll
-        for (int c = 0; c < C / 4; ++c) {
-          const float4 kv = kp[c];
-          qk += qs[h * C + 4 * c] * kv.x + qs[h * C + 4 * c + 1] * kv.y + qs[h * C + 4 * c + 2] * kv.z + qs[h * C + 4 * c + 3] * kv.w;
-        }
-        const float* kpt = a.k_pts + ((long long)jj * H + h) * PQ * 3;
-        float d2 = 0.f;
+  for (int r = 0; r < R; ++r) {
+    mrun[r] = -INFINITY;
+    lrun[r] = 0.f;
+    mask_i[r] = (a.mask && r0 + r < a.rows) ? a.mask[a.row0 + r0 + r] : 1.f;
+  }
+  const float bb_h = a.bb[warp], ghalf = 0.5f * a.gamma[warp];
+  // accumulators: pair channels 2 * cp, 2 * cp + 1 of one row for every head, or NVA value channels for every row
+  const int zr = tid / (CZ / 2), cp = tid % (CZ / 2);
+  constexpr int NACC = 2 * H > NVA * R ? 2 * H : NVA * R;
+  float acc[NACC];
 #pragma unroll
-        for (int p = 0; p < PQ * 3; ++p) {
-          const float d = qp[h * PQ * 3 + p] - kpt[p];
-          d2 += d * d;
-        }
-        float bz = a.bb[h];
-        const bf16* zr = zs + j * ZROW;
-#pragma unroll 8
-        for (int c = 0; c < CZ; c += 2) {
-          const float2 zf = __bfloat1622float2(*reinterpret_cast<const bf162*>(zr + c));
-          bz += zf.x * wbt[c * (H + 1) + h] + zf.y * wbt[(c + 1) * (H + 1) + h];
-        }
-        const float mj = a.mask ? a.mask[jj] : 1.f;
-        logit = a.w_c * qk + a.w_b * bz - 0.5f * a.gamma[h] * d2 + a.inf * (mask_i * mj - 1.f);
+  for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
+  int vhead[NVA], vstep[NVA];
+  const float* vbase[NVA];
+#pragma unroll
+  for (int u = 0; u < NVA; ++u) {
+    const int ch = tid - ZT + u * NV_T;
+    const bool on = tid >= ZT && ch < VC + VT, pt = ch >= VC;
+    vhead[u] = on ? (pt ? (ch - VC) / (PV * 3) : ch / C) : 0;
+    vstep[u] = on ? (pt ? VT : VC) : 0;
+    vbase[u] = on ? (pt ? a.v_pts + (ch - VC) : a.v + ch) : a.v;
+  }
+  const int chunks = (N + IPA_J - 1) / IPA_J;
+  for (int ck = 0; ck < chunks; ++ck) {
+    const int j0 = ck * IPA_J, jn = (N - j0) < IPA_J ? (N - j0) : IPA_J;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                    // chunk landed; everyone is done with the previous chunk's sums
+    if (ck + 1 < chunks) load_z(ck + 1);
+    const bf16* zc = zs + (ck & 1) * R * IPA_J * ZROW;
+    // ---- logits and softmax: warp = head ----
+    float lg[R][2];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int j = half * 32 + lane;
+      const bool on = j < jn;
+      const long long jj = on ? j0 + j : 0;
+      float acc0[R], acc1[R];                           // even / odd pair channels
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        acc0[r] = bb_h;
+        acc1[r] = 0.f;
       }
-      ps[h * IPA_J + j] = logit;
+#pragma unroll 2
+      for (int c = 0; c < CZ; c += 8) {
+        const float4 w0 = *reinterpret_cast<const float4*>(wbs + warp * CZ + c), w1 = *reinterpret_cast<const float4*>(wbs + warp * CZ + c + 4);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint4 raw = *reinterpret_cast<const uint4*>(zc + (r * IPA_J + j) * ZROW + c);
+          acc0[r] = fmaf(__uint_as_float(raw.x << 16), w0.x, acc0[r]);
+          acc1[r] = fmaf(__uint_as_float(raw.x & 0xffff0000u), w0.y, acc1[r]);
+          acc0[r] = fmaf(__uint_as_float(raw.y << 16), w0.z, acc0[r]);
+          acc1[r] = fmaf(__uint_as_float(raw.y & 0xffff0000u), w0.w, acc1[r]);
+          acc0[r] = fmaf(__uint_as_float(raw.z << 16), w1.x, acc0[r]);
+          acc1[r] = fmaf(__uint_as_float(raw.z & 0xffff0000u), w1.y, acc1[r]);
+          acc0[r] = fmaf(__uint_as_float(raw.w << 16), w1.z, acc0[r]);
+          acc1[r] = fmaf(__uint_as_float(raw.w & 0xffff0000u), w1.w, acc1[r]);
+        }
+      }
+      const float mj = a.mask ? a.mask[jj] : 1.f;
+      float qk[R], d2[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) qk[r] = d2[r] = 0.f;
+      const float4* kp = reinterpret_cast<const float4*>(a.k + (jj * H + warp) * C);
+#pragma unroll
+      for (int c = 0; c < C / 4; ++c) {
+        const float4 kv = kp[c];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float4 qv = *reinterpret_cast<const float4*>(qs + (r * H + warp) * C + 4 * c);
+          qk[r] += qv.x * kv.x + qv.y * kv.y + qv.z * kv.z + qv.w * kv.w;
+        }
+      }
+      const float4* kpt = reinterpret_cast<const float4*>(a.k_pts + (jj * H + warp) * PQ * 3);
+#pragma unroll
+      for (int c = 0; c < PQ * 3 / 4; ++c) {
+        const float4 kv = kpt[c];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float4 qv = *reinterpret_cast<const float4*>(qp + (r * H + warp) * PQ * 3 + 4 * c);
+          const float dx = qv.x - kv.x, dy = qv.y - kv.y, dz = qv.z - kv.z, dw = qv.w - kv.w;
+          d2[r] += dx * dx + dy * dy + dz * dz + dw * dw;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        lg[r][half] = on ? a.w_c * qk[r] + a.w_b * (acc0[r] + acc1[r]) - ghalf * d2[r] + a.inf * (mask_i[r] * mj - 1.f) : -INFINITY;
     }
-    __syncthreads();
-    // ---- online softmax: warp w handles heads w, w + 8, ... ----
-    for (int h = warp; h < H; h += IPA_THREADS / 32) {
-      const float s0 = ps[h * IPA_J + lane], s1 = ps[h * IPA_J + 32 + lane];
-      const float mold = mrun[h];
-      const float mnew = fmaxf(mold, warp_max(fmaxf(s0, s1)));
-      const float p0 = __expf(s0 - mnew), p1 = __expf(s1 - mnew);      // -inf logits (beyond N) give 0
-      ps[h * IPA_J + lane] = p0;
-      ps[h * IPA_J + 32 + lane] = p1;
-      const float sum = warp_sum(p0 + p1);
-      if (lane == 0) {
-        const float al = __expf(mold - mnew);                            // 0 on the first chunk (mold = -inf)
-        alph[h] = al;
-        mrun[h] = mnew;
-        lrun[h] = lrun[h] * al + sum;
-      }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float mnew = fmaxf(mrun[r], warp_max(fmaxf(lg[r][0], lg[r][1])));
+      const float p0 = __expf(lg[r][0] - mnew), p1 = __expf(lg[r][1] - mnew);      // -inf logits (beyond N) give 0
+      const float al = __expf(mrun[r] - mnew);                                     // 0 on the first chunk (-inf)
+      ps[(r * IPA_J + lane) * H + warp] = p0;
+      ps[(r * IPA_J + 32 + lane) * H + warp] = p1;
+      lrun[r] = lrun[r] * al + warp_sum(p0 + p1);
+      mrun[r] = mnew;
+      if (lane == 0) alph[r * H + warp] = al;
     }
     __syncthreads();
     // ---- weighted sums ----
-    if (tid < CZ) {
+    if (tid < ZT) {
 #pragma unroll
-      for (int h = 0; h < H; ++h) acc_z[h] *= alph[h];
-      for (int j = 0; j < IPA_J; j += 4) {
-        const float z0 = __bfloat162float(zs[(j + 0) * ZROW + tid]), z1 = __bfloat162float(zs[(j + 1) * ZROW + tid]);
-        const float z2 = __bfloat162float(zs[(j + 2) * ZROW + tid]), z3 = __bfloat162float(zs[(j + 3) * ZROW + tid]);
+      for (int h = 0; h < H; ++h) {
+        const float al = alph[zr * H + h];
+        acc[2 * h] *= al;
+        acc[2 * h + 1] *= al;
+      }
+      const bf16* zp = zc + zr * IPA_J * ZROW + 2 * cp;
+      const float* pp = ps + zr * IPA_J * H;
+#pragma unroll 4
+      for (int j = 0; j < IPA_J; ++j) {                 // rows past N: z = 0 and p = 0
+        const uint32_t zz = *reinterpret_cast<const uint32_t*>(zp + j * ZROW);
+        const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xffff0000u);
 #pragma unroll
-        for (int h = 0; h < H; ++h) {
-          const float4 p = *reinterpret_cast<const float4*>(ps + h * IPA_J + j);     // same address in every lane
-          acc_z[h] += p.x * z0 + p.y * z1 + p.z * z2 + p.w * z3;
+        for (int h4 = 0; h4 < H / 4; ++h4) {
+          const float4 p = *reinterpret_cast<const float4*>(pp + j * H + h4 * 4);  // same address in every lane
+          acc[h4 * 8 + 0] = fmaf(p.x, z0, acc[h4 * 8 + 0]);
+          acc[h4 * 8 + 1] = fmaf(p.x, z1, acc[h4 * 8 + 1]);
+          acc[h4 * 8 + 2] = fmaf(p.y, z0, acc[h4 * 8 + 2]);
+          acc[h4 * 8 + 3] = fmaf(p.y, z1, acc[h4 * 8 + 3]);
+          acc[h4 * 8 + 4] = fmaf(p.z, z0, acc[h4 * 8 + 4]);
+          acc[h4 * 8 + 5] = fmaf(p.z, z1, acc[h4 * 8 + 5]);
+          acc[h4 * 8 + 6] = fmaf(p.w, z0, acc[h4 * 8 + 6]);
+          acc[h4 * 8 + 7] = fmaf(p.w, z1, acc[h4 * 8 + 7]);
         }
       }
     } else {
-      const int u0 = tid - CZ;
 #pragma unroll
-      for (int u = 0; u < NVA; ++u) {
-        const int ch = u0 + u * NV_T;
-        if (ch < H * VC) {
-          const int h = ch / VC, c = ch - h * VC;
-          const float* base = c < C ? a.v + (long long)h * C + c : a.v_pts + (long long)h * PV * 3 + (c - C);
-          const long long jstride = c < C ? (long long)H * C : (long long)H * PV * 3;
-          float acc = acc_v[u] * alph[h];
-          for (int j = 0; j < jn; ++j) acc += ps[h * IPA_J + j] * base[(long long)(j0 + j) * jstride];
-          acc_v[u] = acc;
-        }
+      for (int u = 0; u < NVA; ++u)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[u * R + r] *= alph[r * H + vhead[u]];
+      int j = 0;
+#pragma unroll 1
+      for (; j + 4 <= jn; j += 4) {
+        float v[NVA][4];
+#pragma unroll
+        for (int u = 0; u < NVA; ++u)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[u][e] = vbase[u][(j0 + j + e) * vstep[u]];
+#pragma unroll
+        for (int u = 0; u < NVA; ++u)
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[u * R + r] = fmaf(ps[(r * IPA_J + j + e) * H + vhead[u]], v[u][e], acc[u * R + r]);
       }
+#pragma unroll 1
+      for (; j < jn; ++j)
+#pragma unroll
+        for (int u = 0; u < NVA; ++u)
+#pragma unroll
+          for (int r = 0; r < R; ++r) acc[u * R + r] = fmaf(ps[(r * IPA_J + j) * H + vhead[u]], vbase[u][(j0 + j) * vstep[u]], acc[u * R + r]);
     }
-    __syncthreads();
   }
   // ---- normalise and store ----
-  if (tid < CZ) {
 #pragma unroll
-    for (int h = 0; h < H; ++h) a.o_pair[((long long)r * H + h) * CZ + tid] = acc_z[h] / lrun[h];
+  for (int r = 0; r < R; ++r)
+    if (lane == 0) lfin[r * H + warp] = lrun[r];
+  __syncthreads();
+  if (tid < ZT) {
+    if (r0 + zr < a.rows) {
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        const float l = lfin[zr * H + h];
+        *reinterpret_cast<float2*>(a.o_pair + ((long long)(r0 + zr) * H + h) * CZ + 2 * cp) = make_float2(acc[2 * h] / l, acc[2 * h + 1] / l);
+      }
+    }
   } else {
-    const int u0 = tid - CZ;
 #pragma unroll
     for (int u = 0; u < NVA; ++u) {
-      const int ch = u0 + u * NV_T;
-      if (ch < H * VC) {
-        const int h = ch / VC, c = ch - h * VC;
-        const float val = acc_v[u] / lrun[h];
-        if (c < C) a.o[((long long)r * H + h) * C + c] = val;
-        else a.o_pt[((long long)r * H + h) * PV * 3 + (c - C)] = val;
+      const int ch = tid - ZT + u * NV_T;
+      if (ch >= VC + VT) continue;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (r0 + r >= a.rows) continue;
+        const float val = acc[u * R + r] / lfin[r * H + vhead[u]];
+        if (ch < VC) a.o[(long long)(r0 + r) * VC + ch] = val;
+        else a.o_pt[(long long)(r0 + r) * VT + ch - VC] = val;
       }
     }
   }
+}
+
+template <int R>
+static int ipa_launch(const IpaArgs& a, cudaStream_t st) {
+  constexpr int HH = 12, CC = 16, PQ = 4, PV = 8, CZZ = 128;
+  constexpr size_t smem = 2 * R * IPA_J * (CZZ + IPA_ZP) * 2 + sizeof(float) * (HH * CZZ + R * HH * CC + R * HH * PQ * 3 + R * HH * IPA_J + 2 * R * HH);
+  auto kern = ipa_fwd_kernel<R, HH, CC, PQ, PV, CZZ>;
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -4;
+    attr = true;
+  }
+  launch_light(kern, (a.rows + R - 1) / R, IPA_THREADS, smem, st, a);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// ---------------------------------------------------------------------------
+// What surrounds the core: projections in, concatenated features out, one kernel each.  As PyTorch operations these are some
+// 200 launches of a few thousand elements (rotation matrices from quaternions, three-component sums, stacks, conversions),
+// which bound the layer: 1.75 ms at N = 512 where the kernels of all of them took 0.45 ms; with the two kernels here and the
+// core above 0.26 ms.
+// One CTA per residue; a few KB each, so the launch is what they cost.
+// ---------------------------------------------------------------------------
+struct Frame {
+  float r[3][3], t[3];
+};
+
+// rot: [N][9] matrices or [N][4] quaternions (w, x, y, z), in fp32
+__device__ __forceinline__ Frame load_frame(const float* rot, int is_quat, const float* trans, long long n) {
+  Frame f;
+  if (is_quat) {
+    const float w = rot[n * 4], x = rot[n * 4 + 1], y = rot[n * 4 + 2], z = rot[n * 4 + 3];
+    f.r[0][0] = w * w + x * x - y * y - z * z;
+    f.r[0][1] = 2.f * (x * y - w * z);
+    f.r[0][2] = 2.f * (x * z + w * y);
+    f.r[1][0] = 2.f * (x * y + w * z);
+    f.r[1][1] = w * w - x * x + y * y - z * z;
+    f.r[1][2] = 2.f * (y * z - w * x);
+    f.r[2][0] = 2.f * (x * z - w * y);
+    f.r[2][1] = 2.f * (y * z + w * x);
+    f.r[2][2] = w * w - x * x - y * y + z * z;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) f.r[i][j] = rot[n * 9 + i * 3 + j];
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) f.t[i] = trans[n * 3 + i];
+  return f;
+}
+
+struct IpaPrepArgs {
+  const bf16 *q, *kv, *q_pts, *kv_pts;   // projections [N][H*C], [N][H][2C], [N][3][H*Pq], [N][3][H][Pq+Pv] (x, y, z lie apart)
+  const float *rot, *trans;
+  int is_quat;
+  float *oq, *ok, *ov, *oq_pts, *ok_pts, *ov_pts;   // [N][H][C] x 3, [N][H][P][3] x 3 (global frame)
+  int N, H, C, Pq, Pv;
+};
+
+__global__ void __launch_bounds__(256) ipa_prep_kernel(const IpaPrepArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long n = blockIdx.x;
+  const int HC = a.H * a.C;
+  for (int i = threadIdx.x; i < HC; i += blockDim.x) {
+    const int h = i / a.C, c = i - h * a.C;
+    a.oq[n * HC + i] = __bfloat162float(a.q[n * HC + i]);
+    a.ok[n * HC + i] = __bfloat162float(a.kv[n * 2 * HC + h * 2 * a.C + c]);
+    a.ov[n * HC + i] = __bfloat162float(a.kv[n * 2 * HC + h * 2 * a.C + a.C + c]);
+  }
+  const Frame f = load_frame(a.rot, a.is_quat, a.trans, n);
+  const int nq = a.H * a.Pq, pk = a.Pq + a.Pv, nk = a.H * pk;
+  for (int i = threadIdx.x; i < nq + nk; i += blockDim.x) {
+    const bool isq = i < nq;
+    const int p = isq ? i : i - nq, np = isq ? nq : nk;
+    const bf16* src = (isq ? a.q_pts : a.kv_pts) + n * 3 * np + p;
+    const float x = __bfloat162float(src[0]), y = __bfloat162float(src[np]), z = __bfloat162float(src[2 * np]);
+    float* dst;
+    if (isq) {
+      dst = a.oq_pts + (n * nq + p) * 3;
+    } else {
+      const int h = p / pk, r = p - h * pk;
+      dst = r < a.Pq ? a.ok_pts + ((n * a.H + h) * a.Pq + r) * 3 : a.ov_pts + ((n * a.H + h) * a.Pv + r - a.Pq) * 3;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) dst[k] = f.r[k][0] * x + f.r[k][1] * y + f.r[k][2] * z + f.t[k];
+  }
+}
+
+// out [N][H*C | x, y, z of H*Pv local points | their norms | H*CZ] in bf16
+__global__ void __launch_bounds__(256) ipa_cat_kernel(const float* __restrict__ o, const float* __restrict__ o_pt, const float* __restrict__ o_pair,
+                                                      const float* __restrict__ rot, int is_quat, const float* __restrict__ trans,
+                                                      bf16* __restrict__ out, int H, int C, int Pv, int CZ, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long n = blockIdx.x;
+  const int HC = H * C, HP = H * Pv, HZ = H * CZ;
+  bf16* dst = out + n * (HC + 4 * HP + HZ);
+  for (int i = threadIdx.x; i < HC; i += blockDim.x) dst[i] = __float2bfloat16(o[n * HC + i]);
+  const Frame f = load_frame(rot, is_quat, trans, n);
+  for (int i = threadIdx.x; i < HP; i += blockDim.x) {
+    const float* p = o_pt + (n * HP + i) * 3;
+    const float x = p[0] - f.t[0], y = p[1] - f.t[1], z = p[2] - f.t[2];
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float v = f.r[0][k] * x + f.r[1][k] * y + f.r[2][k] * z;
+      dst[HC + k * HP + i] = __float2bfloat16(v);
+      s += v * v;
+    }
+    dst[HC + 3 * HP + i] = __float2bfloat16(sqrtf(s + eps));
+  }
+  for (int i = threadIdx.x; i < HZ; i += blockDim.x) dst[HC + 4 * HP + i] = __float2bfloat16(o_pair[n * HZ + i]);
 }
 
 }  // namespace ffb
@@ -199,6 +404,24 @@ __global__ void __launch_bounds__(IPA_THREADS) ipa_fwd_kernel(const IpaArgs a) {
 using namespace ffb;
 
 extern "C" {
+
+// Queries, keys, values and points of the core from the layer's bf16 projections and the frames (IpaPrepArgs).
+int ffb_ipa_prep(const void* q, const void* kv, const void* q_pts, const void* kv_pts, const float* rot, int is_quat, const float* trans, float* oq,
+                 float* ok, float* ov, float* oq_pts, float* ok_pts, float* ov_pts, int N, int H, int C, int Pq, int Pv, void* stream) {
+  if (N <= 0 || H <= 0 || C <= 0 || Pq <= 0 || Pv <= 0) return -2;
+  IpaPrepArgs a = {(const bf16*)q, (const bf16*)kv, (const bf16*)q_pts, (const bf16*)kv_pts, rot, trans, is_quat, oq, ok, ov, oq_pts, ok_pts, ov_pts,
+                   N, H, C, Pq, Pv};
+  launch_light(ipa_prep_kernel, N, 256, 0, reinterpret_cast<cudaStream_t>(stream), a);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// The core's outputs in the local frames, with the point norms, as the bf16 input of the output projection.
+int ffb_ipa_cat(const float* o, const float* o_pt, const float* o_pair, const float* rot, int is_quat, const float* trans, void* out, int N, int H,
+                int C, int Pv, int CZ, float eps, void* stream) {
+  if (N <= 0) return -2;
+  launch_light(ipa_cat_kernel, N, 256, 0, reinterpret_cast<cudaStream_t>(stream), o, o_pt, o_pair, rot, is_quat, trans, (bf16*)out, H, C, Pv, CZ, eps);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
 
 // All pointers are device memory; q / k / v / points / weights / outputs fp32, z bf16 (layouts in IpaArgs).
 // Supported configuration: H = 12 heads, C = 16 channels, 4 query / key points, 8 value points, c_z = 128 (AlphaFold's
@@ -208,7 +431,9 @@ int ffb_ipa_fwd(const float* q, const float* k, const float* v, const float* q_p
                 int C, int Pq, int Pv, int CZ, int row0, int rows, float w_c, float w_b, float inf, void* stream) {
   if (H != 12 || C != 16 || Pq != 4 || Pv != 8 || CZ != 128) return -2;
   if (rows <= 0) return 0;
-  if (N <= 0 || row0 < 0 || row0 + rows > N || (reinterpret_cast<uintptr_t>(z) & 15) || (reinterpret_cast<uintptr_t>(k) & 15)) return -3;
+  if (N <= 0 || row0 < 0 || row0 + rows > N || (reinterpret_cast<uintptr_t>(z) & 15) || (reinterpret_cast<uintptr_t>(k) & 15) ||
+      (reinterpret_cast<uintptr_t>(k_pts) & 15) || (reinterpret_cast<uintptr_t>(o_pair) & 7))
+    return -3;
   IpaArgs a;
   a.q = q; a.k = k; a.v = v; a.q_pts = q_pts; a.k_pts = k_pts; a.v_pts = v_pts;
   a.z = reinterpret_cast<const bf16*>(z);
@@ -216,10 +441,8 @@ int ffb_ipa_fwd(const float* q, const float* k, const float* v, const float* q_p
   a.o = o; a.o_pt = o_pt; a.o_pair = o_pair;
   a.N = N; a.H = H; a.C = C; a.Pq = Pq; a.Pv = Pv; a.CZ = CZ; a.row0 = row0; a.rows = rows;
   a.w_c = w_c; a.w_b = w_b; a.inf = inf;
-  constexpr int HH = 12, CC = 16, PQ = 4, PV = 8, CZZ = 128;
-  const size_t smem = IPA_J * (CZZ + IPA_ZP) * 2 + sizeof(float) * (CZZ * (HH + 1) + HH * CC + HH * PQ * 3 + HH * IPA_J + 3 * HH);
-  launch_light(ipa_fwd_kernel<HH, CC, PQ, PV, CZZ>, rows, IPA_THREADS, smem, reinterpret_cast<cudaStream_t>(stream), a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  return rows >= 1024 ? ipa_launch<4>(a, st) : ipa_launch<2>(a, st);
 }
 
 }  // extern "C"

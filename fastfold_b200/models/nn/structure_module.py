@@ -102,6 +102,13 @@ class InvariantPointAttention(nn.Module):
 
     def forward(self, s, z, r, mask):
         H = self.no_heads
+        if not self.is_multimer and z.is_cuda and not torch.is_grad_enabled() and (H, self.c_hidden, self.no_qk_points, self.no_v_points) == (12, 16, 4, 8):
+            from ...ops import ipa as ipa_op
+            proj = [f(s) for f in (self.linear_q, self.linear_kv, self.linear_q_points, self.linear_kv_points)]
+            if ipa_op.layer_supported(s, z, *proj, r):
+                head_w = self.softplus(self.head_weights) * math.sqrt(1.0 / (3 * (self.no_qk_points * 9.0 / 2)))
+                return self.linear_out(ipa_op.ipa_layer(*proj, r, z, self.linear_b.weight, self.linear_b.bias, head_w, mask,
+                                                        math.sqrt(1.0 / (3 * self.c_hidden)), math.sqrt(1.0 / 3), self.inf, self.eps))
         q = self.linear_q(s)
         q = q.view(q.shape[:-1] + (H, -1))
         if self.is_multimer:

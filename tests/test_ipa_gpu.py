@@ -71,3 +71,33 @@ def test_ipa_module_uses_kernel_and_matches_cpu(device_status):
         assert _lib.LAUNCHES[0] > n0            # the native kernel ran
     err = (got.float().cpu() - ref).abs().mean().item()
     assert err <= 5e-2 * max(1.0, ref.abs().mean().item()), err
+
+
+@pytest.mark.parametrize("N,fmt", [(1, "quat"), (33, "quat"), (96, "rot_mat"), (130, "quat")])
+def test_ipa_layer_in_three_kernels(N, fmt, device_status):
+    """Points, core and concatenated features against the operations they stand for, from the same bf16 projections.  The
+    features are rounded to bf16 (2^-9 relative); coordinates of up to ~50 cancel against translations in fp32."""
+    from fastfold_b200.ops import ipa as ipa_op
+    from fastfold_b200.utils.rigid_utils import Rigid, Rotation
+    g = torch.Generator().manual_seed(N)
+    H, C, PQ, PV, CZ = 12, 16, 4, 8, 128
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    b = lambda *s: r(*s).to(torch.bfloat16)
+    q, kv, qp, kvp, z = b(N, 192), b(N, 384), b(N, 144), b(N, 432), b(N, N, CZ)
+    rots = Rotation(quats=r(N, 4), normalize_quats=True)
+    if fmt == "rot_mat":
+        rots = Rotation(rot_mats=rots.get_rot_mats())
+    frames = Rigid(rots, r(N, 3) * 8)
+    wb, bb, gamma, mask = r(H, CZ) * 0.1, r(H) * 0.1, torch.rand(H, generator=g).to(DEV) * 0.1, (torch.rand(N, generator=g) > 0.2).float().to(DEV)
+    w = (math.sqrt(1.0 / 48), math.sqrt(1.0 / 3), 1e5)
+    with torch.no_grad():
+        assert ipa_op.layer_supported(torch.empty(N, 384, device=DEV), z, q, kv, qp, kvp, frames)
+        out = ipa_op.ipa_layer(q, kv, qp, kvp, frames, z, wb, bb, gamma, mask, *w, 1e-8)
+        k, v = kv.view(N, H, 2 * C).split(C, dim=-1)
+        pts = [frames[..., None].apply(torch.stack(p.split(p.shape[-1] // 3, dim=-1), dim=-1)).view(N, H, -1, 3) for p in (qp, kvp)]
+        o, o_pt, o_pair = ipa_op.ipa_core_ref(q.view(N, H, C), k, v, pts[0], pts[1][:, :, :PQ], pts[1][:, :, PQ:], z, wb, bb, gamma, mask, *w)
+        o_pt = frames[..., None, None].invert_apply(o_pt).reshape(N, -1, 3)
+        ref = torch.cat([o.flatten(1), *o_pt.unbind(-1), torch.sqrt((o_pt ** 2).sum(-1) + 1e-8), o_pair.flatten(1)], dim=-1)
+    assert out.shape == ref.shape and out.dtype == torch.bfloat16
+    assert ((out.float() - ref).norm() / ref.norm()).item() < 4e-3
+    assert (out.float() - ref).abs().max().item() < 2.0 ** -8 * ref.abs().max().item() + 1e-3
