@@ -20,7 +20,8 @@ struct GemmArgs {
   void* C;
   long long ldc, c_bstride;
   const void* bias;         // bf16 [N], added to alpha * acc
-  const float* rowscale;    // fp32 [batch][M], multiplies the row
+  const void* rowscale;     // [batch][M], multiplies the row: fp32, or bf16 when rs_bf16
+  int rs_bf16;
   long long rs_bstride;
   const void* mul;          // bf16, same indexing as the (non-transposed) output
   long long ldmul, mul_bstride;

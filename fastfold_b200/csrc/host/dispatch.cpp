@@ -138,8 +138,11 @@ Tensor gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, double alpha, OptTensor bi
     g.bias = ptr(bias);
   }
   if (rowscale) {
-    rowscale = rowscale->to(at::kFloat).contiguous();
-    g.rowscale = static_cast<const float*>(ptr(rowscale));
+    // bf16 masks are read as they are, which saves the conversion's launch; not so in the gated projection of the triangle
+    // multiplication, which is 3 % faster on the converted mask (1215 against 1250 us at 1024 residues)
+    g.rs_bf16 = rowscale->scalar_type() == at::kBFloat16 && !glu;
+    rowscale = (g.rs_bf16 ? *rowscale : rowscale->to(at::kFloat)).contiguous();
+    g.rowscale = ptr(rowscale);
     g.rs_bstride = (batched && rowscale->dim() == 2) ? M : 0;
   }
   if (mul) {

@@ -25,7 +25,7 @@ from ...utils import memo
 from ...utils.checkpointing import checkpoint_blocks
 from .msa import MSACore
 from .ops import Linear, OutProductMean
-from .triangle import PairCore, pad_amount
+from .triangle import PairCore, pad_amount, pad_or_pass
 from . import ops as fops
 
 
@@ -73,12 +73,12 @@ class Evoformer(nn.Module):
         seq_length = pair_mask.size(-1)
         pad = pad_amount(seq_length, P)
         if self.first_block:
-            m = F.pad(m.unsqueeze(0), (0, 0, 0, pad))
+            m = pad_or_pass(m.unsqueeze(0), (0, 0, 0, pad))
             m = scatter(m, dim=2) if self.is_multimer else scatter(m, dim=1)
             if P > 1 and pad == 0 and z.shape[0] * P == seq_length:
                 z = z.unsqueeze(0)                      # the caller keeps the pair tensor row-sharded between the stacks
             else:
-                z = F.pad(z.unsqueeze(0), (0, 0, 0, pad, 0, pad))
+                z = pad_or_pass(z.unsqueeze(0), (0, 0, 0, pad, 0, pad))
                 z = scatter(z, dim=1)
         msa_mask = memo.cached(("pad_msa", pad), (msa_mask,), lambda: F.pad(msa_mask.unsqueeze(0), (0, pad)))
         pair_mask = memo.cached(("pad_pair", pad), (pair_mask,), lambda: F.pad(pair_mask.unsqueeze(0), (0, pad, 0, pad)))

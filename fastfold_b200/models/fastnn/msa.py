@@ -12,7 +12,7 @@ from ...utils import memo
 from ...utils.checkpointing import checkpoint_blocks
 from .ops import (ChunkMSARowAttentionWithPairBias, ChunkMSAColumnGlobalAttention, ChunkTransition, GlobalAttention,
                   OutProductMean, SelfAttention, Transition, _fusable)
-from .triangle import PairCore, pad_amount
+from .triangle import PairCore, pad_amount, pad_or_pass as _pad
 from . import ops as fops
 
 
@@ -48,7 +48,10 @@ class MSAColumnAttention(nn.Module):
             strided = M_norm_t is None and self.strided_for(M_raw.shape[1], M_raw)
         if strided:
             M = self.layernormM(M_raw) if M_norm_t is None else M_norm_t
-            out, _ = self.attention(M, memo.cached("mask_t", (M_mask,), lambda: M_mask.transpose(-1, -2).contiguous()), transposed=True)
+            tail = (None, None, M_raw) if _fusable(M_raw) else None          # the residual joins in the output projection
+            out, done = self.attention(M, memo.cached("mask_t", (M_mask,), lambda: M_mask.transpose(-1, -2).contiguous()), tail=tail, transposed=True)
+            if done:
+                return out
             return M_raw.add_(out) if fops.INPLACE else M_raw + out
         M = self.layernormM(M_raw.transpose(-2, -3).contiguous()) if M_norm_t is None else M_norm_t
         out, _ = self.attention(M, memo.cached("mask_t", (M_mask,), lambda: M_mask.transpose(-1, -2).contiguous()))
@@ -121,12 +124,12 @@ class ExtraMSABlock(nn.Module):
         cnt_pad = pad_amount(msa_mask.size(-2), P)
         len_pad = pad_amount(pair_mask.size(-1), P)
         if self.first_block:
-            m = F.pad(m.unsqueeze(0), (0, 0, 0, len_pad, 0, cnt_pad))
+            m = _pad(m.unsqueeze(0), (0, 0, 0, len_pad, 0, cnt_pad))
             m = scatter(m, dim=1) if not self.is_multimer else scatter(m, dim=2)
             if P > 1 and len_pad == 0 and z.shape[0] * P == pair_mask.size(-1):
                 z = z.unsqueeze(0)                      # already this rank's row shard
             else:
-                z = F.pad(z.unsqueeze(0), (0, 0, 0, len_pad, 0, len_pad))
+                z = _pad(z.unsqueeze(0), (0, 0, 0, len_pad, 0, len_pad))
                 z = scatter(z, dim=1)
         msa_mask = memo.cached(("pad_msa", len_pad, cnt_pad), (msa_mask,), lambda: F.pad(msa_mask.unsqueeze(0), (0, len_pad, 0, cnt_pad)))
         pair_mask = memo.cached(("pad_pair", len_pad), (pair_mask,), lambda: F.pad(pair_mask.unsqueeze(0), (0, len_pad, 0, len_pad)))

@@ -188,6 +188,13 @@ class OutProductMean(nn.Module):
         self.o_linear = Linear(n_feat_proj * n_feat_proj, n_feat_out, initializer="zero", use_bias=True)
         self.n_feat_proj = n_feat_proj
 
+    @staticmethod
+    def _masked(proj, M, mask):
+        """``proj(M) * mask`` with one mask value per row; without gradients in the projection's epilogue."""
+        if not (_fusable(M) and proj.weight.dtype == M.dtype):
+            return proj(M) * mask
+        return K.gemm(M.reshape(-1, M.shape[-1]), proj.weight, bias=proj.bias, rowscale=mask.reshape(-1)).view(*M.shape[:-1], -1)
+
     def _outer(self, left, right_all, inv_norm, Z_raw):
         """left [1,S,ni,d], right_all [1,S,N,e] -> Z_raw + o_linear(outer) * inv_norm."""
         S, ni, d = left.shape[1], left.shape[2], left.shape[3]
@@ -256,11 +263,10 @@ class OutProductMean(nn.Module):
             if out is not None:
                 return out
         mask_col_a = memo.cached(("opm_mask_col_as", M.dtype), (src,), lambda: M_mask_col.to(M.dtype))
-        right_act = self.linear_b(M)
         # mask before the gather: identical result, and the gathered operand is ready to use
-        right_act = right_act * mask_col_a
+        right_act = self._masked(self.linear_b, M, mask_col_a)
         right_act_all, work = gather_async(right_act, dim=2)
-        left_act = self.linear_a(M) * mask_col_a
+        left_act = self._masked(self.linear_a, M, mask_col_a)
         inv_norm = memo.cached("opm_inv_norm", (src,), lambda: 1.0 / (torch.einsum("bsid,bsjd->bijd", M_mask_col.float(), M_mask.float()) + 1e-3))
         right_act_all = gather_async_opp(right_act_all, work, dim=2)
         if CHUNK_SIZE is None:
@@ -516,6 +522,24 @@ def pair_bias_hqk(Zn, weight):
         return None
     b_t = K.linear_t(Zn.reshape(A * N, Zn.shape[-1]), weight)            # [H, (q_local k)]
     return gather(b_t.view(1, H, A, N), dim=2, reduce_grad=True)
+
+
+def pair_bias_rows(Zn, weight, transposed):
+    """The pair bias ``[1, H, q, k]`` of an unsharded pair tensor without gradients, for any length and both nodes:
+    ``bias[h, q, k] = Zn[q, k] . weight[h]``, or ``Zn[k, q] . weight[h]`` with ``transposed``.
+
+    One GEMM with the query as its batch: its transposed epilogue stores each query's ``[H, k]`` slab at the 8-element row
+    pitch of the attention kernel's bias tiles, and the ending node's transpose is a matter of the operand's strides.
+    (A channel-last projection and a permuting copy, which this replaces, read and wrote the pair tensor's rows twice.)
+    Returns None where it does not apply."""
+    if not (Zn.shape[0] == 1 and _fusable(Zn) and weight.dtype == Zn.dtype and core.get_dap_size() == 1 and Zn.shape[-1] % 8 == 0
+            and Zn.stride(-1) == 1 and Zn.data_ptr() % 16 == 0 and Zn.stride(1) % 8 == 0 and Zn.stride(2) % 8 == 0):
+        return None
+    a = Zn[0].transpose(0, 1) if transposed else Zn[0]           # [q, k, c]
+    n_q, n_k, H = a.shape[0], a.shape[1], weight.shape[0]
+    buf = torch.empty(H, n_q, (n_k + 7) // 8 * 8, device=Zn.device, dtype=Zn.dtype)[:, :, :n_k]
+    K.gemm(a, weight, trans_out=True, out=buf.permute(1, 0, 2))
+    return buf.unsqueeze(0)
 
 
 class GlobalAttention(nn.Module):
@@ -891,6 +915,8 @@ class _TriangleAttention(nn.Module):
         else:
             Z = self.layernorm1(Z_raw if (self.starting or strided) else Z_raw.transpose(-2, -3).contiguous())
         b = pair_bias_hqk(Z, self.linear_b.weight) if not strided else None
+        if b is None:
+            b = pair_bias_rows(Z, self.linear_b.weight, strided)
         if b is not None:
             work = -1
         else:
@@ -957,6 +983,8 @@ class ChunkMSARowAttentionWithPairBias(nn.Module):
         M = self.layernormM(M_raw)
         Zn = self.layernormZ(Z)
         b = pair_bias_hqk(Zn, self.linear_b_weights)
+        if b is None:
+            b = pair_bias_rows(Zn, self.linear_b_weights, False)
         if b is not None:
             work = -1
         else:

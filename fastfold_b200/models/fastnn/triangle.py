@@ -1,5 +1,6 @@
 """Pair half of the Evoformer block (names as in fastfold/model/fastnn/triangle.py)."""
 import torch.nn as nn
+import torch.nn.functional as F
 
 from ...parallel.comm import scatter, scatter_mask, row_to_col, col_to_row
 from ...parallel.fused import a2a_layer_norm
@@ -15,6 +16,15 @@ def pad_amount(n, P):
     strips the padding with ``[:-pad]``; padded positions are masked, so the outputs are the same.
     """
     return (-n) % P
+
+
+def pad_or_pass(x, pad):
+    """``F.pad``, which copies even when there is nothing to add; the copy is only needed where the modules behind write
+    over their input."""
+    from . import ops as fops
+    if fops.INPLACE or any(pad):
+        return F.pad(x, pad)
+    return x
 
 
 class TriangleMultiplicationOutgoing(AsyncChunkTriangleMultiplicationOutgoing):

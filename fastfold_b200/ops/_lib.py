@@ -39,7 +39,7 @@ class GemmArgs(ctypes.Structure):
         ("alpha", c_float),
         ("C", c_void_p), ("ldc", c_ll), ("c_bstride", c_ll),
         ("bias", c_void_p),
-        ("rowscale", c_void_p), ("rs_bstride", c_ll),
+        ("rowscale", c_void_p), ("rs_bf16", c_int), ("rs_bstride", c_ll),
         ("mul", c_void_p), ("ldmul", c_ll), ("mul_bstride", c_ll),
         ("dmask", c_void_p), ("lddm", c_ll),
         ("resid", c_void_p), ("ldres", c_ll), ("res_bstride", c_ll),

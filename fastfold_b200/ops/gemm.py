@@ -60,6 +60,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, alpha=1.0, bias=None, act=None, glu=Fa
 
     ``a_mn`` / ``b_mn``: the operand is stored with the contraction index
     strided, i.e. A is given as ``[.., K, M]`` / B as ``[.., K, N]``.
+    ``rowscale``: one factor per row, fp32 or bf16.
     Epilogue order: ``+bias -> act -> glu -> *mul -> *rowscale -> *dmask -> +resid``.
     ``dmask=(mask[mod, N], div, mod)`` picks mask row ``(m // div) % mod``.
     ``accumulate=True`` adds into an fp32 ``out`` with atomics (allows ``splits > 1``).
