@@ -449,6 +449,102 @@ __global__ void __launch_bounds__(256) ln_fwd_transposed64_kernel(const bf16* __
   }
 }
 
+// C = 128, rows % 8 == 0, no statistics wanted (the triangle multiplication without gradients): the 64 x 128 tile lives in registers - a thread holds eight rows of
+// four adjacent channels from four 16-byte loads - and only the normalised values cross shared memory, as bf16, on their way
+// to 16-byte stores.  A bandwidth problem (one read, one write); the kernel above, which stages the tile as fp32 in shared
+// memory, reads it from there three times and fits six CTAs on an SM, keeps too few bytes in flight.
+//   Measured (B200): triangle multiplication at 1024 residues, of which this is one of six kernels, 1230 -> 1182 us.
+// Passes with gradients stay on the kernel above: another order of the sums moves single roundings of the output, which the
+// weight gradients of the attentions behind it carry on to 4 % of their norm.
+// Shared tile: [64 rows][32 pieces of 8 bytes], piece index XOR 4 * (row / 8): the eight row octets of a warp's store fall
+// into different banks, and pairs of pieces stay adjacent for the 16-byte reads.
+__global__ void __launch_bounds__(256, 3) ln_fwd_transposed128_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma,
+                                                                      const bf16* __restrict__ beta, bf16* __restrict__ y,
+                                                                      long long rows, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int C = 128;
+  __shared__ __align__(16) uint2 tile[LNT64 * 32];
+  __shared__ __align__(16) float s_part[8][LNT64];
+  __shared__ __align__(16) float s_mean[LNT64], s_rstd[LNT64];
+  const long long r0 = (long long)blockIdx.x * LNT64;
+  const int tid = threadIdx.x, o = tid & 7, cl = tid >> 3, warp = tid >> 5, lane = tid & 31;
+  const bool ok = r0 + 8 * o < rows;             // the octet is in range as a whole
+  float v[4][8];
+  {
+    uint4 raw[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      raw[i] = ok ? *reinterpret_cast<const uint4*>(x + (long long)(4 * cl + i) * rows + r0 + 8 * o) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        v[i][2 * k] = __uint_as_float(w[k] << 16);
+        v[i][2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+      }
+    }
+  }
+  // sums over the channels of every row: four in the thread, four threads of the warp, eight warps
+  auto fold = [&](float (&p)[8]) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      p[k] += __shfl_xor_sync(0xffffffffu, p[k], 8);
+      p[k] += __shfl_xor_sync(0xffffffffu, p[k], 16);
+    }
+    if (lane < 8) {
+      *reinterpret_cast<float4*>(&s_part[warp][8 * o]) = make_float4(p[0], p[1], p[2], p[3]);
+      *reinterpret_cast<float4*>(&s_part[warp][8 * o + 4]) = make_float4(p[4], p[5], p[6], p[7]);
+    }
+    __syncthreads();
+  };
+  auto total = [&](int r) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += s_part[w][r];
+    return t;
+  };
+  float p[8], m[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) p[k] = (v[0][k] + v[1][k]) + (v[2][k] + v[3][k]);
+  fold(p);
+  if (tid < LNT64) s_mean[tid] = total(tid) / C;
+  __syncthreads();
+  *reinterpret_cast<float4*>(m) = *reinterpret_cast<const float4*>(&s_mean[8 * o]);
+  *reinterpret_cast<float4*>(m + 4) = *reinterpret_cast<const float4*>(&s_mean[8 * o + 4]);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    p[k] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[i][k] -= m[k];
+      p[k] += v[i][k] * v[i][k];
+    }
+  }
+  fold(p);
+  if (tid < LNT64) s_rstd[tid] = rsqrtf(total(tid) / C + eps);
+  __syncthreads();
+  *reinterpret_cast<float4*>(m) = *reinterpret_cast<const float4*>(&s_rstd[8 * o]);
+  *reinterpret_cast<float4*>(m + 4) = *reinterpret_cast<const float4*>(&s_rstd[8 * o + 4]);
+  const uint2 ug = *reinterpret_cast<const uint2*>(gamma + 4 * cl), ub = *reinterpret_cast<const uint2*>(beta + 4 * cl);
+  const float g[4] = {__uint_as_float(ug.x << 16), __uint_as_float(ug.x & 0xffff0000u), __uint_as_float(ug.y << 16), __uint_as_float(ug.y & 0xffff0000u)};
+  const float b[4] = {__uint_as_float(ub.x << 16), __uint_as_float(ub.x & 0xffff0000u), __uint_as_float(ub.y << 16), __uint_as_float(ub.y & 0xffff0000u)};
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const bf162 lo = __floats2bfloat162_rn(v[0][k] * m[k] * g[0] + b[0], v[1][k] * m[k] * g[1] + b[1]);
+    const bf162 hi = __floats2bfloat162_rn(v[2][k] * m[k] * g[2] + b[2], v[3][k] * m[k] * g[3] + b[3]);
+    tile[(8 * o + k) * 32 + (cl ^ (4 * o))] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int idx = tid + it * 256, rr = idx >> 4, pc = idx & 15;
+    if (r0 + rr < rows)
+      *reinterpret_cast<uint4*>(y + (r0 + rr) * C + pc * 8) = *reinterpret_cast<const uint4*>(&tile[rr * 32 + ((2 * pc) ^ (4 * (rr >> 3)))]);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // bf16 rows of C = 8 * L elements, L in {8, 16, 32} lanes per row (C = 64, 128, 256 - every LayerNorm of the
 // Evoformer): a warp works on 32 / L rows side by side and on MR_U such groups per step, so that every lane has
@@ -710,6 +806,11 @@ int ffb_layernorm_fwd_transposed(const void* x, const void* gamma, const void* b
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (rows % 2 == 0 && C % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(gamma) |
                                        reinterpret_cast<uintptr_t>(beta)) & 15) == 0) {
+    if (C == 128 && rows % 8 == 0 && !mean && !rstd) {
+      launch_light(ln_fwd_transposed128_kernel, (unsigned)((rows + LNT64 - 1) / LNT64), 256, 0, st, (const bf16*)x, (const bf16*)gamma,
+                   (const bf16*)beta, (bf16*)y, rows, eps);
+      return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    }
     static bool attr = false;
     if (!attr) {
       if (cudaFuncSetAttribute(ln_fwd_transposed64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * 256 * (LNT64 + 1))) !=

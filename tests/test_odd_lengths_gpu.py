@@ -127,3 +127,17 @@ def test_bias_pitch(device_status):
         odd = torch.full((1, 1, H, n, 81), float("nan"), device=DEV, dtype=torch.bfloat16)
         odd[..., :n] = bias
         assert torch.equal(flash.flash_attention_packed(qkv, None, odd[..., :n], 32 ** -0.5), want)
+
+
+@pytest.mark.parametrize("rows", [8, 56, 64, 72, 4096, 203 * 208])
+@pytest.mark.parametrize("offset", [0.0, 30.0])
+def test_channel_major_layer_norm_of_128_channels(rows, offset, device_status):
+    """Tile edges, remainders and rows whose mean is large against their spread; bf16 output: 2^-8 of its range."""
+    from fastfold_b200 import ops as K
+    torch.manual_seed(rows)
+    x = (torch.randn(128, rows, device=DEV) + offset).bfloat16()
+    w, b = (1 + 0.1 * torch.randn(128, device=DEV)).bfloat16(), (0.1 * torch.randn(128, device=DEV)).bfloat16()
+    ref = torch.nn.functional.layer_norm(x.double().t(), (128,), w.double(), b.double(), 1e-5)
+    with torch.no_grad():
+        out = K.layer_norm_transposed(x, w, b, 1e-5)
+    assert (out.double() - ref).abs().max().item() <= 2.0 ** -8 * ref.abs().max().item()
