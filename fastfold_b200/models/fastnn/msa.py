@@ -37,7 +37,7 @@ class MSAColumnAttention(nn.Module):
         batch strides.  ``n_seq``: length of that axis."""
         from ...ops import flash
         from . import ops as fops
-        if fops.CHUNK_SIZE is not None:
+        if fops.CHUNK_SIZE is not None and (torch.is_grad_enabled() or like.shape[0] != 1):
             return False
         return like.is_cuda and like.dtype == torch.bfloat16 and self.c == flash.HEAD_DIM
 

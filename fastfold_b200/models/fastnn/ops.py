@@ -496,15 +496,53 @@ class SelfAttention(nn.Module):
     def forward(self, in_data, mask, nonbatched_bias=None, tail=None, transposed=False):
         """``tail=(out_bias, (mask2d, div, mod) or None, residual)`` lets the output projection absorb the
         bias / dropout / residual that follow it; the second return value says whether it did.
-        ``transposed``: attend along dim 1 of ``in_data`` instead of dim 2 (no chunking in that mode)."""
+        ``transposed``: attend along dim 1 of ``in_data`` instead of dim 2."""
         bias = self._bias(nonbatched_bias, transposed)
-        if transposed or CHUNK_SIZE is None or CHUNK_SIZE >= in_data.shape[1]:
+        if CHUNK_SIZE is None or CHUNK_SIZE >= in_data.shape[2 if transposed else 1]:
+            return self._one(in_data, mask, bias, tail, transposed)
+        if _fusable(in_data) and in_data.shape[0] == 1 and (tail is None or tail[1] is None or (tail[1][1] == 1 and not transposed)):
+            out = self._chunks_fused(in_data, mask, bias, tail, transposed)
+            if out is not None:
+                return out, tail is not None
+        if transposed:
             return self._one(in_data, mask, bias, tail, transposed)
         outs = []
         for ax in range(0, in_data.shape[1], CHUNK_SIZE):
             o, _ = self._one(in_data[:, ax:ax + CHUNK_SIZE], mask[:, ax:ax + CHUNK_SIZE], bias, None)
             outs.append(o)
         return torch.cat(outs, dim=1), False
+
+    def _chunks_fused(self, x, mask, bias, tail, transposed):
+        """``CHUNK_SIZE`` rows (columns with ``transposed``) at a time without gradients: every projection of a chunk reads
+        its slice of ``x`` and the last one writes its slice of the result, residual included, through the operands' strides,
+        so that nothing is gathered, concatenated or added afterwards.  Returns None where the kernels do not apply."""
+        H, D = self.n_head, self._padded_dim()
+        if D == self.c:
+            wq, wo = self.to_qkv.weight, self.o_linear.weight
+            wg, bg = (self.gating_linear.weight, self.gating_bias) if self.gating else (None, None)
+        else:
+            wq, wg, bg, wo = self._padded_heads(D)
+        bias5 = None if bias is None else bias.unsqueeze(1)
+        x3 = x[0]                                             # [rows, n, c] (transposed: [n, columns, c])
+        out_bias, dmask, resid = tail if tail is not None else (None, None, None)
+        out_bias = out_bias if out_bias is not None else self.o_linear.bias
+        if x3.stride(-1) != 1 or x3.stride(1) % 8 or (resid is not None and not resid.is_contiguous()) or wo.shape[0] < 64:
+            return None
+        out = x.new_empty(*x.shape[:-1], wo.shape[0]) if resid is None else (resid if INPLACE else torch.empty_like(resid))
+        for ax in range(0, x.shape[2 if transposed else 1], CHUNK_SIZE):
+            sl = (slice(None), slice(ax, ax + CHUNK_SIZE)) if transposed else (slice(ax, ax + CHUNK_SIZE),)
+            part = x3[sl]
+            # rows are contiguous: one matrix; columns are not: a batch of them, one per position along the attention
+            mat = (lambda t: t) if transposed else (lambda t: t.reshape(-1, t.shape[-1]))
+            qkv = K.gemm(mat(part), wq).view(1, *part.shape[:-1], 3, H, D)
+            m = mask[:, ax:ax + CHUNK_SIZE]
+            if not flash.packed_supported(qkv, m, bias5, transposed=transposed):
+                return None
+            o = flash.flash_attention_packed(qkv, m, bias5, self.scaling, transposed=transposed)[0]
+            if self.gating:
+                o = K.gemm(mat(part), wg, bias=bg, act="sigmoid", mul=mat(o))
+            K.gemm(mat(o), wo, bias=out_bias, dmask=dmask, resid=None if resid is None else mat(resid[0][sl]), out=mat(out[0][sl]))
+        return out
 
 
 def pair_bias_hqk(Zn, weight):
@@ -941,7 +979,7 @@ class _TriangleAttention(nn.Module):
 
     def strided_for(self, n_attn, like):
         """``n_attn``: length of the axis the ending node attends along (the full first pair axis)."""
-        if self.starting or CHUNK_SIZE is not None:
+        if self.starting or (CHUNK_SIZE is not None and (torch.is_grad_enabled() or self.training or like.shape[0] != 1)):
             return False
         if not (like.is_cuda and like.dtype == torch.bfloat16 and self.c == flash.HEAD_DIM):
             return False

@@ -141,3 +141,32 @@ def test_channel_major_layer_norm_of_128_channels(rows, offset, device_status):
     with torch.no_grad():
         out = K.layer_norm_transposed(x, w, b, 1e-5)
     assert (out.double() - ref).abs().max().item() <= 2.0 ** -8 * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("chunk", [1, 5, 16, 64])
+@pytest.mark.parametrize("n", [24, 61])
+def test_chunked_attention_is_the_unchunked_one(n, chunk, device_status):
+    """Chunks that divide the rows or do not, in place and not, for every attention module (the block in-place mode writes
+    each slice over its residual)."""
+    torch.manual_seed(n)
+    s = 37
+    pm, mm = _masks(n, s)
+    z, m = torch.randn(1, n, n, 128).bfloat16().to(DEV), torch.randn(1, s, n, 256).bfloat16().to(DEV)
+    pm, mm = pm.bfloat16().to(DEV), mm.bfloat16().to(DEV)
+    mods = [(TriangleAttentionStartingNode(128, p_drop=0.25, c=32, n_head=4), (z, pm)), (TriangleAttentionEndingNode(128, p_drop=0.25, c=32, n_head=4), (z, pm)),
+            (MSARowAttentionWithPairBias(256, 128), (m, z, mm)), (MSAColumnAttention(256), (m, mm)),
+            (TriangleAttentionEndingNode(128, p_drop=0.25, c=16, n_head=8), (z, pm))]
+    for mod, args in mods:
+        mod = _random_parameters(mod).eval().to(DEV, torch.bfloat16)
+        with torch.no_grad():
+            want = mod(*args).float()
+            fops.set_chunk_size(chunk)
+            try:
+                got = mod(*args).float()
+                with fops.inplace_scope():
+                    first = args[0].clone()
+                    over = mod(first, *args[1:])
+            finally:
+                fops.set_chunk_size(None)
+        assert ((got - want).norm() / want.norm()).item() < 4e-3
+        assert torch.equal(over.float(), got)
