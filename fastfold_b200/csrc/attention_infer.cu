@@ -179,6 +179,9 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, u
       : "memory");
 }
 
+// The logit of a masked key in the log2 domain of the reference points (exact, see MASKED_LOGIT).
+constexpr float MASKED_LOG2 = MASKED_LOGIT * LOG2E;
+
 constexpr float ROW_SUM_LO = 8.673617379884035e-19f, ROW_SUM_HI = 1.152921504606847e18f;   // 2^-60, 2^60
 
 template <int D, bool BIAS>   // head dim: 32 (64-byte rows, 64-byte swizzle) or 16 (32-byte)
@@ -439,8 +442,8 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
         uint64_t sum = pk2(0.f, 0.f);
         if (none) {
           // masked keys next to a real one have weight 0; where there has been no other key they all have the same logit
-          const bool alone = l == 0.f || M == MASKED_LOGIT;
-          if (alone) M = MASKED_LOGIT;
+          const bool alone = l == 0.f || M == MASKED_LOG2;
+          if (alone) M = MASKED_LOG2;
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             uint32_t p[16];

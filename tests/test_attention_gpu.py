@@ -63,6 +63,22 @@ def test_forward_rows_that_leave_the_exponent_range(B, n, H, use_bias, device_st
     assert (out.float() - ref).abs().max().item() < 3.8e-2
 
 
+@pytest.mark.parametrize("n", [128, 200, 640])
+@pytest.mark.parametrize("level", [-8e8, -1e9])
+def test_forward_masked_block_before_keys_of_a_low_bias(level, n, device_status):
+    """A wholly masked block of 64 keys, then keys that the pair bias pushes to the level that masks are written with: still
+    above the logit of a masked key (-2^30), so all weight is theirs.  Values of 1 there and -1 on masked keys: exactly 1."""
+    torch.manual_seed(n)
+    q, k, _ = _qkv(3, n, 4)
+    v = torch.ones_like(q)
+    v[..., :64, :] = -1
+    mask = torch.ones(1, 3, n, device=DEV, dtype=torch.bfloat16)
+    mask[..., :64] = 0
+    bias = torch.full((1, 1, 4, n, n), level, device=DEV, dtype=torch.bfloat16)
+    with torch.no_grad():
+        assert torch.equal(attention_core(q, k, v, mask, bias), torch.ones_like(v))
+
+
 @pytest.mark.parametrize("B,n,H,use_bias,use_mask", [
     (4, 128, 8, True, True), (16, 256, 8, True, True), (7, 256, 4, False, True), (5, 384, 4, True, False), (3, 200, 4, True, True),
     (6, 512, 4, True, True),
