@@ -48,13 +48,15 @@ constexpr int AF_BK = 64;       // keys per block
 constexpr int AF_THREADS = 128 + AF_GROUPS * 128;
 constexpr int AF_BSLOTS = 4;    // bias tiles in shared memory
 constexpr int AF_ISSUERS = 2;   // MMA issuer warps
+// tensor memory of group g: columns g * 128 + [0, 64) S, [64, 96) P (bf16 pairs), [96, 128) O
+constexpr uint32_t AF_TM_P = 64, AF_TM_O = 96;
 
 struct AttnInferArgs {
   int B, H, n_q, n_k;            // batch rows, heads, query / key lengths
   int n_qt, n_kb;                // query tiles (128), key blocks (64)
   int units;                     // H * n_qt * B (head, query tile, batch row) units
   int bias_resident;             // 1: n_kb <= AF_BSLOTS, bias tiles stay in shared memory across batch rows
-  float scale_log2e;             // logit scale * log2(e)
+  float scale, scale_log2e;      // logit scale, and times log2(e)
   const bf16* mask;              // [B][n_k] or null
   long long mask_bstride;
   bf16* out;                     // [B][n_q][H*D]
@@ -179,10 +181,112 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, u
       : "memory");
 }
 
-// The logit of a masked key in the log2 domain of the reference points (exact, see MASKED_LOGIT).
-constexpr float MASKED_LOG2 = MASKED_LOGIT * LOG2E;
-
 constexpr float ROW_SUM_LO = 8.673617379884035e-19f, ROW_SUM_HI = 1.152921504606847e18f;   // 2^-60, 2^60
+
+// Rows whose largest logit is this far out (log2 domain) are `far` rows.  There the two formulas of the ordinary path end:
+// masked keys no longer have weight 0 next to such a row's keys (a pair bias of -1e9, of the type's lowest value or -inf is
+// itself a mask), the log2 domain overflows for the lowest and largest bf16 values, and one ulp of a reference point is no
+// longer small against 1.  A far row's reference point is its running maximum in natural units, masked keys take part in it
+// with MASKED_LOGIT, and its logits are rounded as the kernel with gradients rounds them.
+constexpr float FAR_LOGIT = 1048576.f;
+
+struct RowState {
+  float M, l;                     // reference point (log2 domain; natural units in a far row), row sum relative to it
+  int far;                        // int: as a bool it takes a predicate and the ordinary path a spilled register more
+};
+
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, float (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "r"(taddr));
+}
+
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const float (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+               ::"f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "r"(taddr)
+               : "memory");
+}
+
+__device__ __forceinline__ void tmem_st_32x4(uint32_t taddr, const uint32_t (&v)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%4], {%0, %1, %2, %3};" ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(taddr) : "memory");
+}
+
+// A block of keys for a warp that holds a far row: the general softmax step.  Rows with `move` get a new reference point (the
+// output and the sum so far are rescaled to it), the others keep theirs.  Eight columns at a time and inlined: no row of a
+// model's own biases gets here, but the ordinary path uses all registers that five warps per scheduler leave, and a call or
+// wider pieces cost it 2 - 8 % (n 389, B 389, H 4 with bias: 192 us without this path, 193 us as it is, 205 us as a call).
+template <bool BIAS>
+__device__ __forceinline__ RowState far_block(RowState st, bool move, uint32_t tm, bool has_o, const uint8_t* brow, int r, uint32_t keep_lo,
+                                           uint32_t keep_hi, int keys, float scale, float scale_log2e) {
+  constexpr float LN2 = 0.6931471805599453f;
+  const uint64_t keep = keep_lo | (uint64_t)keep_hi << 32;        // `keys` of the 64 are in the sequence
+  auto load = [&](int c, float (&s)[8], float (&b)[8]) {
+    tmem_ld_32x8(tm + c * 8, s);
+    tmem_ld_wait();
+    if (BIAS) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(brow + ((c ^ (r & 7)) << 4));
+      b[0] = bf_lo(raw.x), b[1] = bf_hi(raw.x), b[2] = bf_lo(raw.y), b[3] = bf_hi(raw.y);
+      b[4] = bf_lo(raw.z), b[5] = bf_hi(raw.z), b[6] = bf_lo(raw.w), b[7] = bf_hi(raw.w);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) b[e] = 0.f;
+    }
+  };
+  auto logit = [&](int key, float s, float b) -> float {          // natural units
+    return (keep >> key) & 1u ? fmaf(s, scale, b) : (key < keys ? MASKED_LOGIT : -INFINITY);
+  };
+  tmem_st_wait();                          // what the ordinary path stored for this block is about to be replaced
+  float mx = -INFINITY, alpha = 1.f;
+#pragma unroll 1
+  for (int c = 0; c < 8; ++c) {
+    float s[8], b[8];
+    load(c, s, b);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) mx = fmaxf(mx, logit(c * 8 + e, s[e], b[e]));
+  }
+  if (move) {
+    const float top = st.l > 0.f ? fmaxf(mx, st.far ? st.M : (st.M + log2f(st.l)) * LN2) : mx;
+    if (top != -INFINITY) {                // a row without any key yet keeps its reference point
+      const bool far = !(fabsf(top * LOG2E) < FAR_LOGIT);
+      const float m2 = far ? top : top * LOG2E;
+      if (st.l > 0.f) alpha = ex2f(far ? ((st.far ? st.M : st.M * LN2) - top) * LOG2E : (st.far ? st.M * LOG2E : st.M) - m2);
+      st.M = m2;
+      st.far = far;
+    }
+  }
+  if (has_o) {
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {          // heads of 16 channels: the upper columns are nobody's
+      float o[8];
+      tmem_ld_32x8(tm + AF_TM_O + c * 8, o);
+      tmem_ld_wait();
+#pragma unroll
+      for (int e = 0; e < 8; ++e) o[e] *= alpha;
+      tmem_st_32x8(tm + AF_TM_O + c * 8, o);
+    }
+  }
+  float sum = 0.f;
+#pragma unroll 1
+  for (int c = 0; c < 8; ++c) {
+    float s[8], b[8];
+    uint32_t p[4];
+    load(c, s, b);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (st.far) s[e] = ex2f((logit(c * 8 + e, s[e], b[e]) - st.M) * LOG2E);
+      else s[e] = (keep >> (c * 8 + e)) & 1u ? ex2f(fmaf(s[e], scale_log2e, fmaf(b[e], LOG2E, -st.M))) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bf162 h = __floats2bfloat162_rn(s[2 * i], s[2 * i + 1]);
+      p[i] = *reinterpret_cast<const uint32_t*>(&h);
+      sum += bf_lo(p[i]) + bf_hi(p[i]);
+    }
+    tmem_st_32x4(tm + AF_TM_P + c * 4, p);
+  }
+  st.l = st.l * alpha + sum;
+  return st;
+}
 
 template <int D, bool BIAS>   // head dim: 32 (64-byte rows, 64-byte swizzle) or 16 (32-byte)
 __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_constant__ CUtensorMap tmQ,
@@ -239,8 +343,6 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  // tensor memory of group g: columns g * 128 + [0, 64) S, [64, 96) P (bf16 pairs), [96, 128) O
-  constexpr uint32_t TM_P = 64, TM_O = 96;
 
   // Contiguous range of units for this CTA; unit = (h * n_qt + qt) * B + b.  A round takes up to AF_GROUPS consecutive
   // batch rows of one (head, query tile); every role walks the same rounds.
@@ -367,7 +469,7 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
             const uint64_t v = dv + (e * 2 + st) * (8192 >> 4);
 #pragma unroll
             for (int k = 0; k < AF_BK / 16; ++k)
-              umma_bf16_ts(tmem + g * 128 + TM_O, tmem + g * 128 + TM_P + k * 8, v + ((k * 2 * GROUP) >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+              umma_bf16_ts(tmem + g * 128 + AF_TM_O, tmem + g * 128 + AF_TM_P + k * 8, v + ((k * 2 * GROUP) >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
             umma_commit(o_done + 8 * g);
             umma_commit(kv_empty + 8 * (g * 2 + st));
             ++pi[e];
@@ -400,7 +502,7 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
       prev = grp;
       // resident tiles are released in the last round that reads them, streamed ones at once
       const bool release = BIAS && (!a.bias_resident || u >= u_end || u / a.B != grp);
-      float M = 0.f, l = 0.f;                       // reference point (log2 domain) and row sum relative to it
+      RowState row = {0.f, 0.f, false};
       const bf16* mrow = (a.mask && active) ? a.mask + (long long)b * a.mask_bstride : nullptr;
       for (int j = 0; j < a.n_kb; ++j) {
         uint32_t slot = 0, bpar = 0;
@@ -442,68 +544,83 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
         uint64_t sum = pk2(0.f, 0.f);
         if (none) {
           // masked keys next to a real one have weight 0; where there has been no other key they all have the same logit
-          const bool alone = l == 0.f || M == MASKED_LOG2;
-          if (alone) M = MASKED_LOG2;
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            uint32_t p[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const uint32_t bits = ((c ? valid_hi : valid_lo) >> (2 * i)) & 3u;
-              p[i] = alone ? (bits & 1u) * 0x3f80u + (bits >> 1) * 0x3f800000u : 0u;
+          const bool alone = row.l == 0.f || (row.far && row.M == MASKED_LOGIT);
+          if (__any_sync(0xffffffffu, row.far && !alone)) {
+            row = far_block<BIAS>(row, alone || row.far, tm, j > 0, brow, r, 0u, 0u, a.n_k - j * AF_BK, a.scale, a.scale_log2e);
+          } else {
+            if (alone) {
+              row.M = MASKED_LOGIT;
+              row.far = 1;
+              row.l += (float)(__popc(valid_lo) + __popc(valid_hi));
             }
-            tmem_st_32x16(tm + TM_P + c * 16, p);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              uint32_t p[16];
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const uint32_t bits = ((c ? valid_hi : valid_lo) >> (2 * i)) & 3u;
+                p[i] = alone ? (bits & 1u) * 0x3f80u + (bits >> 1) * 0x3f800000u : 0u;
+              }
+              tmem_st_32x16(tm + AF_TM_P + c * 16, p);
+            }
           }
-          if (alone) sum = pk2((float)(__popc(valid_lo) + __popc(valid_hi)), 0.f);
-        } else if (plain) {
-          softmax_block<true, BIAS>(tm, tm + TM_P, brow, r, pen, a.scale_log2e, -M, sum);
         } else {
-          softmax_block<false, BIAS>(tm, tm + TM_P, brow, r, pen, a.scale_log2e, -M, sum);
-        }
-        float sx, sy;
-        up2(sum, sx, sy);
-        float ln = l + (sx + sy);
-        const bool bad = !(ln > ROW_SUM_LO && ln < ROW_SUM_HI);
-        if (!none && __any_sync(0xffffffffu, bad)) {
-          // some row's sum has left the safe range (first block of a row with large logits, only masked keys before this
-          // block, or a much larger logit in it): move that row's reference point and redo the block
-          if (plain) write_penalties(pen, lane, keep_lo, keep_hi);
-          float mx = -INFINITY, alpha = 1.f;
-#pragma unroll 1
-          for (int c = 0; c < 2; ++c) {
-            float s[32];
-            uint64_t t[16];
-            tmem_ld_32x32(tm + c * 32, s);
-            tmem_ld_wait();
-            logits32<false, BIAS>(t, s, brow, r, c * 32, pen, a.scale_log2e, 0.f);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              float x, y;
-              up2(t[i], x, y);
-              mx = fmaxf(mx, fmaxf(x, y));
-            }
-          }
-          if (bad) {
-            const float m2 = l > 0.f ? fmaxf(mx, M + log2f(l)) : mx;
-            if (m2 != -INFINITY) {                  // a row without any key yet keeps its reference point
-              if (l > 0.f) alpha = ex2f(M - m2);
-              M = m2;
-            }
-          }
-          if (j > 0) {
-            float o[32];                            // D = 16: the upper columns are nobody's
-            tmem_ld_32x32(tm + TM_O, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int c = 0; c < 32; ++c) o[c] *= alpha;
-            tmem_st_32x32(tm + TM_O, o);
-          }
-          sum = pk2(0.f, 0.f);
-          softmax_block<false, BIAS>(tm, tm + TM_P, brow, r, pen, a.scale_log2e, -M, sum);
+          if (plain) softmax_block<true, BIAS>(tm, tm + AF_TM_P, brow, r, pen, a.scale_log2e, -row.M, sum);
+          else softmax_block<false, BIAS>(tm, tm + AF_TM_P, brow, r, pen, a.scale_log2e, -row.M, sum);
+          float sx, sy;
           up2(sum, sx, sy);
-          ln = l * alpha + (sx + sy);
+          float ln = row.l + (sx + sy);
+          const bool bad = row.far || !(ln > ROW_SUM_LO && ln < ROW_SUM_HI);
+          if (__any_sync(0xffffffffu, bad)) {
+            // some row's sum has left the safe range (first block of a row with large logits, only masked keys before this
+            // block, or a much larger logit in it): move that row's reference point and redo the block
+            if (plain) write_penalties(pen, lane, 0xffffffffu, 0xffffffffu);
+            float mx = -INFINITY, alpha = 1.f;
+            tmem_st_wait();                         // the first attempt's P is about to be replaced
+#pragma unroll 1
+            for (int c = 0; c < 2; ++c) {
+              float s[32];
+              uint64_t t[16];
+              tmem_ld_32x32(tm + c * 32, s);
+              tmem_ld_wait();
+              logits32<false, BIAS>(t, s, brow, r, c * 32, pen, a.scale_log2e, 0.f);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                float x, y;
+                up2(t[i], x, y);
+                mx = fmaxf(mx, fmaxf(x, y));
+              }
+            }
+            const float m2 = (row.l > 0.f && !row.far) ? fmaxf(mx, row.M + log2f(row.l)) : mx;
+            // a row that leaves the domain of the ordinary path, or that has not re-entered it from above
+            const bool out = bad && (!(fabsf(m2) < FAR_LOGIT) || (row.far && row.M > 0.f));
+            if (__any_sync(0xffffffffu, out)) {
+              // the keys from the table: bits kept until here would be spilled
+              row = far_block<BIAS>(row, bad, tm, j > 0, brow, r, __ballot_sync(0xffffffffu, pen[lane] == 0.f),
+                                    __ballot_sync(0xffffffffu, pen[lane + 32] == 0.f), a.n_k - j * AF_BK, a.scale, a.scale_log2e);
+            } else {
+              if (bad) {
+                if (row.l > 0.f) alpha = ex2f((row.far ? row.M * LOG2E : row.M) - m2);
+                row.M = m2;
+                row.far = 0;
+              }
+              if (j > 0) {
+                float o[32];                        // D = 16: the upper columns are nobody's
+                tmem_ld_32x32(tm + AF_TM_O, o);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 32; ++c) o[c] *= alpha;
+                tmem_st_32x32(tm + AF_TM_O, o);
+              }
+              sum = pk2(0.f, 0.f);
+              softmax_block<false, BIAS>(tm, tm + AF_TM_P, brow, r, pen, a.scale_log2e, -row.M, sum);
+              up2(sum, sx, sy);
+              row.l = row.l * alpha + (sx + sy);
+            }
+          } else {
+            row.l = ln;
+          }
         }
-        l = ln;
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -523,11 +640,11 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
       }
       tc_fence_after();
       float o[32];
-      tmem_ld_32x32(tm + TM_O, o);
+      tmem_ld_32x32(tm + AF_TM_O, o);
       tmem_ld_wait();
       const int qrow = qt * AF_BQ + r;
       if (qrow < a.n_q) {
-        const float inv = 1.f / l;
+        const float inv = 1.f / row.l;
         bf16* dst = a.out + (long long)b * a.out_bstride + (long long)qrow * a.out_rstride + h * D;
 #pragma unroll
         for (int c = 0; c < D; c += 8) {
@@ -574,6 +691,7 @@ int ffb_attention_infer(const void* q, const void* k, const void* v, long long q
   if (units <= 0 || units > 0x7fffffffLL || a.n_kb <= 0) return -6;
   a.units = (int)units;
   a.bias_resident = (bias && a.n_kb <= AF_BSLOTS) ? 1 : 0;
+  a.scale = scale;
   a.scale_log2e = scale * LOG2E;
   a.mask = (const bf16*)mask;
   a.mask_bstride = mask_bstride;

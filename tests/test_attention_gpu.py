@@ -79,6 +79,32 @@ def test_forward_masked_block_before_keys_of_a_low_bias(level, n, device_status)
         assert torch.equal(attention_core(q, k, v, mask, bias), torch.ones_like(v))
 
 
+@pytest.mark.parametrize("B,n,H,d", [(1, 64, 4, 32), (5, 75, 4, 32), (6, 256, 8, 32), (9, 320, 4, 32), (9, 640, 4, 32), (6, 128, 4, 16), (7, 333, 4, 16)])
+def test_forward_biases_that_are_masks(B, n, H, d, device_status):
+    """Pair biases of -1e9, the lowest and the largest bf16 value, -inf and ordinary ones in blocks of keys, next to blocks that
+    are masked wholly, in part or not at all.  Rows without a single finite logit are NaN in both.  Bound as above: |v| < 5.5,
+    output and P rounded to bf16."""
+    g = torch.Generator().manual_seed(n + B + d)
+    qkv = torch.randn(1, B, n, 3, H, d, generator=g).to(DEV, torch.bfloat16)
+    low = torch.finfo(torch.bfloat16).min
+    levels = torch.tensor([0.0, -600.0, 600.0, -2e6, 2e6, -1e9, 1e9, low, -low, float("-inf")])
+    blocks = (n + 63) // 64
+    pick = torch.randint(0, len(levels), (1, 1, H, n, blocks), generator=g)
+    pick[..., : n // 2, :] = pick[..., : n // 2, :1]                # half of the rows at one level,
+    pick[..., : n // 4, :] = 5 + 2 * (pick[..., : n // 4, :] % 3)   # some of them at one that is a mask
+    bias = (levels[pick].repeat_interleave(64, -1)[..., :n] + torch.randn(1, 1, H, n, n, generator=g)).to(DEV, torch.bfloat16)
+    share = torch.tensor([0.0, 0.1, 0.5, 1.0])[torch.randint(0, 4, (1, B, blocks), generator=g)].repeat_interleave(64, -1)[..., :n]
+    mask = (torch.rand(1, B, n, generator=g) >= share).to(DEV, torch.bfloat16)
+    mask[0, 0] = 1
+    mask[0, -1, :64] = 0
+    with torch.no_grad():
+        out = flash.flash_attention_packed(qkv, mask, bias, d ** -0.5).float()
+    q, k, v = qkv.float().permute(3, 0, 1, 4, 2, 5)
+    ref = attention_core_ref(q, k, v, mask.float(), bias.float()).transpose(2, 3).flatten(3)
+    assert torch.equal(out.isnan(), ref.isnan())
+    assert (out - ref).nan_to_num().abs().max().item() < 3.8e-2
+
+
 @pytest.mark.parametrize("B,n,H,use_bias,use_mask", [
     (4, 128, 8, True, True), (16, 256, 8, True, True), (7, 256, 4, False, True), (5, 384, 4, True, False), (3, 200, 4, True, True),
     (6, 512, 4, True, True),
