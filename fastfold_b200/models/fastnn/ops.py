@@ -516,6 +516,8 @@ class SelfAttention(nn.Module):
         """``CHUNK_SIZE`` rows (columns with ``transposed``) at a time without gradients: every projection of a chunk reads
         its slice of ``x`` and the last one writes its slice of the result, residual included, through the operands' strides,
         so that nothing is gathered, concatenated or added afterwards.  Returns None where the kernels do not apply."""
+        if self.c > max(flash.FWD_HEAD_DIMS):
+            return None
         H, D = self.n_head, self._padded_dim()
         if D == self.c:
             wq, wo = self.to_qkv.weight, self.o_linear.weight

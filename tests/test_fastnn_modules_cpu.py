@@ -133,3 +133,24 @@ def test_extramsa_stack(chunk):
         z1 = ori(m, z, chunk_size=chunk, msa_mask=msa_mask, pair_mask=pair_mask, _mask_trans=False)
         z2 = fast(m, z, chunk_size=chunk, msa_mask=msa_mask, pair_mask=pair_mask, _mask_trans=False)
     assert torch.isfinite(z2).all() and (z1 - z2).abs().mean() < 2e-3 * max(1.0, float(z1.abs().mean()))
+
+
+@pytest.mark.parametrize("c", [8, 16, 24, 32, 40, 64])
+def test_chunked_attention_takes_any_head_width(c, monkeypatch):
+    """Chunked rows without gradients where the fused path may be tried: head widths that its kernels do not have - wider ones
+    among them - give what the plain evaluation gives."""
+    monkeypatch.setattr(fops, "_fusable", lambda x: not torch.is_grad_enabled())
+    torch.manual_seed(c)
+    att = fops.SelfAttention(qkv_dim=64, c=c, n_head=2, out_dim=64).eval()
+    with torch.no_grad():
+        for p in att.parameters():
+            p.normal_(std=0.1)
+        x, mask = torch.randn(1, 7, 12, 64), torch.ones(1, 7, 12)
+        mask[..., 9:] = 0
+        want = att(x, mask)[0]
+        fops.set_chunk_size(3)
+        try:
+            got = att(x, mask)[0]
+        finally:
+            fops.set_chunk_size(None)
+    torch.testing.assert_close(got, want, rtol=1e-4, atol=1e-5)
