@@ -1,4 +1,5 @@
 """Pair half of the Evoformer block (names as in fastfold/model/fastnn/triangle.py)."""
+import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
@@ -19,10 +20,11 @@ def pad_amount(n, P):
 
 
 def pad_or_pass(x, pad):
-    """``F.pad``, which copies even when there is nothing to add; the copy is only needed where the modules behind write
-    over their input."""
+    """``F.pad``, which copies even when there is nothing to add.  The copy is left out where nothing behind it needs one: the
+    modules write over their input in in-place mode, autograd keeps it for backward (the caller may go on writing to the
+    original), and the kernels want 16-byte aligned rows, which a view into a larger tensor need not have."""
     from . import ops as fops
-    if fops.INPLACE or any(pad):
+    if fops.INPLACE or torch.is_grad_enabled() or any(pad) or not x.is_contiguous() or x.data_ptr() % 16:
         return F.pad(x, pad)
     return x
 

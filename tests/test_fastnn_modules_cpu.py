@@ -154,3 +154,24 @@ def test_chunked_attention_takes_any_head_width(c, monkeypatch):
         finally:
             fops.set_chunk_size(None)
     torch.testing.assert_close(got, want, rtol=1e-4, atol=1e-5)
+
+
+def test_stack_entry_passes_on_only_what_needs_no_copy():
+    """Evoformer and extra-MSA stacks hand their input on without a copy only where it is dense, 16-byte aligned, not needed
+    by a backward pass and not written over."""
+    from fastfold_b200.models.fastnn.triangle import pad_or_pass
+    flat = torch.randn(8 * 16 * 32 + 8).bfloat16()
+    start = (-flat.data_ptr() // 2) % 8                       # first 16-byte boundary
+    dense = flat[start:start + 4096].view(1, 8, 16, 32)
+    views = {"off the boundary": flat[start + 1:start + 4097].view(1, 8, 16, 32), "every other channel": dense[..., ::2],
+             "expanded channel": dense[..., :1].expand(1, 8, 16, 8), "channels first": dense.permute(0, 1, 3, 2)}
+    with torch.no_grad():
+        assert pad_or_pass(dense, (0, 0, 0, 0)).data_ptr() == dense.data_ptr()
+        for name, v in views.items():
+            out = pad_or_pass(v, (0, 0, 0, 0))
+            assert torch.equal(out, v) and out.data_ptr() != v.data_ptr() and out.data_ptr() % 16 == 0, name
+        assert pad_or_pass(dense, (0, 0, 0, 2)).shape == (1, 8, 18, 32)
+        with fops.inplace_scope():
+            assert pad_or_pass(dense, (0, 0, 0, 0)).data_ptr() != dense.data_ptr()
+    kept = dense.detach().requires_grad_(True)
+    assert pad_or_pass(kept, (0, 0, 0, 0)).data_ptr() != dense.data_ptr()

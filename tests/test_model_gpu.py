@@ -169,3 +169,35 @@ def test_first_pass_uses_current_weights_after_optimizer_steps(device_status):
         err = (a.float() - b.detach().float()).abs().mean().item()
         assert moved > 1e-3, "the optimiser steps did not change the block's output"
         assert err < 0.1 * moved + 2e-2 * max(1.0, b.detach().float().abs().mean().item()), (err, moved)
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("S,N", [(8, 64), (5, 37)])
+def test_stack_entry_takes_views(S, N, grad, device_status):
+    """Inputs that start off a 16-byte boundary (a view into a flat buffer) and inputs whose channels are not adjacent give the
+    bits of dense ones, with and without gradients."""
+    from fastfold_b200.models.fastnn.evoformer import Evoformer
+    from fastfold_b200.models.fastnn.msa import ExtraMSABlock
+    torch.manual_seed(N)
+    for cls, c_m in ((Evoformer, 256), (ExtraMSABlock, 64)):
+        block = cls(c_m, 128, first_block=True, last_block=True).to("cuda", torch.bfloat16).eval()
+        with torch.no_grad():
+            for p in block.parameters():
+                if p.dim() >= 2:
+                    p.normal_(std=p.shape[-1] ** -0.5)
+        block.requires_grad_(grad)
+        m, z = torch.randn(S, N, c_m, device="cuda").bfloat16(), torch.randn(N, N, 128, device="cuda").bfloat16()
+        mm, pm = torch.ones(S, N, device="cuda").bfloat16(), torch.ones(N, N, device="cuda").bfloat16()
+
+        def off(t):
+            flat = torch.empty(t.numel() + 8, device="cuda", dtype=t.dtype)
+            return flat[1:t.numel() + 1].view(t.shape).copy_(t)
+
+        def wide(t):
+            return torch.stack([t, torch.zeros_like(t)], dim=-1).flatten(-2)[..., ::2]
+
+        with torch.set_grad_enabled(grad):
+            want = block(m, z, mm, pm)
+            for view in (off, wide):
+                got = block(view(m), view(z), mm, pm)
+                assert all(torch.equal(a, b) for a, b in zip(got, want)), (cls.__name__, view.__name__)
