@@ -11,7 +11,7 @@ from ...parallel.fused import a2a_layer_norm
 from ...utils import memo
 from ...utils.checkpointing import checkpoint_blocks
 from .ops import (ChunkMSARowAttentionWithPairBias, ChunkMSAColumnGlobalAttention, ChunkTransition, GlobalAttention,
-                  OutProductMean, SelfAttention, Transition, _fusable)
+                  OutProductMean, SelfAttention, Transition, _fusable, _residual)
 from .triangle import PairCore, pad_amount, pad_or_pass as _pad
 from . import ops as fops
 
@@ -48,7 +48,7 @@ class MSAColumnAttention(nn.Module):
             strided = M_norm_t is None and self.strided_for(M_raw.shape[1], M_raw)
         if strided:
             M = self.layernormM(M_raw) if M_norm_t is None else M_norm_t
-            tail = (None, None, M_raw) if _fusable(M_raw) else None          # the residual joins in the output projection
+            tail = (None, None, _residual(M_raw)) if _fusable(M_raw) else None          # the residual joins in the output projection
             out, done = self.attention(M, memo.cached("mask_t", (M_mask,), lambda: M_mask.transpose(-1, -2).contiguous()), tail=tail, transposed=True)
             if done:
                 return out

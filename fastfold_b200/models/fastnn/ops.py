@@ -60,6 +60,12 @@ def _res_out(resid2d):
     return resid2d if (INPLACE and resid2d.is_contiguous()) else None
 
 
+def _residual(x):
+    """``x`` as the residual of a GEMM epilogue, which reads rows of adjacent channels: other layouts (a pair tensor stored
+    channel-first) are copied."""
+    return x if x.stride(-1) == 1 else x.contiguous()
+
+
 def set_chunk_size(chunk_size):
     global CHUNK_SIZE
     CHUNK_SIZE = chunk_size
@@ -210,7 +216,7 @@ class OutProductMean(nn.Module):
             if need_grad:
                 out = _OpmCore.apply(l2, r2, self.o_linear.weight, self.o_linear.bias, inv_norm.reshape(-1), Z_raw.reshape(ni * N, -1))
             else:
-                out = _opm_forward(l2, r2, self.o_linear.weight, self.o_linear.bias, inv_norm.reshape(-1), Z_raw.reshape(ni * N, -1))[0]
+                out = _opm_forward(l2, r2, self.o_linear.weight, self.o_linear.bias, inv_norm.reshape(-1), _residual(Z_raw).reshape(ni * N, -1))[0]
             return out.reshape(Z_raw.shape)
         if left.is_cuda and left.dtype == torch.bfloat16 and (ni * d) % 8 == 0 and (N * e) % 64 == 0 and ni * d >= 64:
             o = K.gemm(l2, r2, a_mn=True, b_mn=True) if not torch.is_grad_enabled() else _bmm_tn(l2, r2)
@@ -710,7 +716,7 @@ class _TriangleMultiplication(nn.Module):
         else:
             K.gemm(lr_t[:c], lr_t[c:], a_mn=True, b_mn=True, out=p[:, :, :n_j])
         ab = K.layer_norm_transposed(p.reshape(c, n_i * pitch), self.layernorm2.weight, self.layernorm2.bias, self.layernorm2.eps)
-        zr3 = Z_raw.reshape(A, B, -1)
+        zr3 = _residual(Z_raw).reshape(A, B, -1)
         out = K.gemm(ab.view(n_i, pitch, c)[:, :n_j], self.output_projection.weight, bias=self.output_bias, mul=g.view(A, B, -1),
                      dmask=None if dropmask is None else _mask_idx(Z_raw, dropmask), resid=zr3, out=_res_out(zr3))
         return out.reshape(Z_raw.shape)
@@ -964,7 +970,7 @@ class _TriangleAttention(nn.Module):
             b, work = gather_async(b, dim=2 if strided else 1)
         tail = None
         if (self.starting or strided) and _fusable(Z_raw):
-            tail = (self.out_bias, None if dropmask is None else _mask_idx(Z_raw, dropmask), Z_raw)
+            tail = (self.out_bias, None if dropmask is None else _mask_idx(Z_raw, dropmask), _residual(Z_raw))
         out, done = self.attention(Z, mask, (b, work), tail=tail, transposed=strided)
         if done:
             return out

@@ -170,3 +170,25 @@ def test_chunked_attention_is_the_unchunked_one(n, chunk, device_status):
                 fops.set_chunk_size(None)
         assert ((got - want).norm() / want.norm()).item() < 4e-3
         assert torch.equal(over.float(), got)
+
+
+@pytest.mark.parametrize("chunk", [None, 16])
+def test_inputs_stored_channel_first(chunk, device_status):
+    """Residual inputs whose channels are not adjacent, at lengths that are no multiple of 8: the bits of dense ones."""
+    torch.manual_seed(0)
+    s, n = 29, 61
+    pm, mm = (t.bfloat16().to(DEV) for t in _masks(n, s))
+    z, m = torch.randn(1, n, n, 128, device=DEV).bfloat16(), torch.randn(1, s, n, 256, device=DEV).bfloat16()
+    zt, mt = (t.movedim(-1, 1).contiguous().movedim(1, -1) for t in (z, m))
+    mods = [(TriangleMultiplicationOutgoing(128, p_drop=0.25, c=128), (z, pm), (zt, pm)),
+            (TriangleAttentionEndingNode(128, p_drop=0.25, c=32, n_head=4), (z, pm), (zt, pm)),
+            (MSAColumnAttention(256), (m, mm), (mt, mm)), (fops.OutProductMean(256, 128, 32), (m, mm, z), (mt, mm, zt))]
+    for mod, dense, strided in mods:
+        mod = _random_parameters(mod).eval().to(DEV, torch.bfloat16)
+        with torch.no_grad():
+            fops.set_chunk_size(chunk)
+            try:
+                want, got = mod(*dense), mod(*strided)
+            finally:
+                fops.set_chunk_size(None)
+        assert torch.equal(got, want), type(mod).__name__
