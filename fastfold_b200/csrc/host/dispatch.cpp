@@ -144,6 +144,7 @@ Tensor gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, double alpha, OptTensor bi
     rowscale = (g.rs_bf16 ? *rowscale : rowscale->to(at::kFloat)).contiguous();
     g.rowscale = ptr(rowscale);
     g.rs_bstride = (batched && rowscale->dim() == 2) ? M : 0;
+    expect(rowscale->numel() >= (g.rs_bstride ? batch : 1) * M, "fewer row factors than rows");
   }
   if (mul) {
     expect(mul->scalar_type() == at::kBFloat16 && mul->stride(-1) == 1, "mul operand");

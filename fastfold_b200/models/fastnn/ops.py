@@ -199,7 +199,7 @@ class OutProductMean(nn.Module):
         """``proj(M) * mask`` with one mask value per row; without gradients in the projection's epilogue."""
         if not (_fusable(M) and proj.weight.dtype == M.dtype):
             return proj(M) * mask
-        return K.gemm(M.reshape(-1, M.shape[-1]), proj.weight, bias=proj.bias, rowscale=mask.reshape(-1)).view(*M.shape[:-1], -1)
+        return K.gemm(M.reshape(-1, M.shape[-1]), proj.weight, bias=proj.bias, rowscale=mask.expand(*M.shape[:-1], 1).reshape(-1)).view(*M.shape[:-1], -1)
 
     def _outer(self, left, right_all, inv_norm, Z_raw):
         """left [1,S,ni,d], right_all [1,S,N,e] -> Z_raw + o_linear(outer) * inv_norm."""
@@ -275,6 +275,7 @@ class OutProductMean(nn.Module):
         left_act = self._masked(self.linear_a, M, mask_col_a)
         inv_norm = memo.cached("opm_inv_norm", (src,), lambda: 1.0 / (torch.einsum("bsid,bsjd->bijd", M_mask_col.float(), M_mask.float()) + 1e-3))
         right_act_all = gather_async_opp(right_act_all, work, dim=2)
+        inv_norm = inv_norm.expand(-1, left_act.shape[2], right_act_all.shape[2], -1)      # of a mask that broadcasts
         if CHUNK_SIZE is None:
             return self._outer(left_act, right_act_all, inv_norm, Z_raw)
         out = Z_raw if INPLACE else torch.empty_like(Z_raw)
@@ -706,7 +707,7 @@ class _TriangleMultiplication(nn.Module):
         Z = self.layernorm1(Z_raw) if Z_norm is None else Z_norm
         w, b = self._glu_weights()
         lr_t = torch.empty(2 * c, A, (B + 7) // 8 * 8, device=Z.device, dtype=Z.dtype)[:, :, :B]
-        K.gemm(Z.reshape(A, B, -1), w, bias=b, glu=True, rowscale=Z_mask.reshape(A, B), trans_out=True, out=lr_t.permute(1, 0, 2))
+        K.gemm(Z.reshape(A, B, -1), w, bias=b, glu=True, rowscale=Z_mask.expand(1, A, B)[0], trans_out=True, out=lr_t.permute(1, 0, 2))
         g = K.gemm(Z.reshape(A * B, -1), self.output_gate.weight, bias=self.output_gate.bias, act="sigmoid")
         n_i = n_j = A if self.outgoing else B
         pitch = (n_j + 7) // 8 * 8

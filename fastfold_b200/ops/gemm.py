@@ -175,6 +175,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, alpha=1.0, bias=None, act=None, glu=Fa
         rowscale = rowscale.to(torch.float32).contiguous()
         g.rowscale = rowscale.data_ptr()
         g.rs_bstride = M if (batched and rowscale.dim() == 2) else 0
+        assert rowscale.numel() >= (batch if g.rs_bstride else 1) * M, "fewer row factors than rows"
         keep.append(rowscale)
     if mul is not None:
         assert mul.dtype == torch.bfloat16 and mul.stride(-1) == 1

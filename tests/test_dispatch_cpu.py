@@ -1,0 +1,23 @@
+"""Argument checks of the extension module: they come before any launch, so they need no GPU."""
+import os
+
+import pytest
+import torch
+
+from fastfold_b200 import _build
+from fastfold_b200.ops import _lib
+
+pytestmark = pytest.mark.skipif(not os.path.exists(_build.dispatch_path()), reason="extension module not built")
+
+
+def _gemm(a, b, rowscale):
+    return _lib.native().gemm(a, b, False, False, 1.0, None, 0, False, rowscale, None, None, 1, 1, None, False, None, False, 1, False, 0, None)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("batch,shape", [(0, (127,)), (0, (1, 16)), (3, (127,)), (3, (3, 127)), (3, (2, 128)), (3, (1, 128))])
+def test_gemm_refuses_fewer_row_factors_than_rows(batch, shape, dtype):
+    """The kernel reads one factor per row through a bare pointer."""
+    a = torch.zeros(*([batch] if batch else []), 128, 64, dtype=torch.bfloat16)
+    with pytest.raises(AssertionError, match="fewer row factors than rows"):
+        _gemm(a, torch.zeros(64, 64, dtype=torch.bfloat16), torch.ones(shape, dtype=dtype))

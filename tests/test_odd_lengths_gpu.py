@@ -192,3 +192,20 @@ def test_inputs_stored_channel_first(chunk, device_status):
             finally:
                 fops.set_chunk_size(None)
         assert torch.equal(got, want), type(mod).__name__
+
+
+@pytest.mark.parametrize("n", [33, 61])
+def test_masks_that_broadcast(n, device_status):
+    """Masks with an extent of 1 give the bits of the masks that they stand for."""
+    torch.manual_seed(n)
+    s = 29
+    z, m = torch.randn(1, n, n, 128, device=DEV).bfloat16(), torch.randn(1, s, n, 256, device=DEV).bfloat16()
+    tri = _random_parameters(TriangleMultiplicationIncoming(128, p_drop=0.25, c=128)).eval().to(DEV, torch.bfloat16)
+    opm = _random_parameters(fops.OutProductMean(256, 128, 32)).eval().to(DEV, torch.bfloat16)
+    with torch.no_grad():
+        for shape in ((1, 1, n), (1, n, 1), (1, 1, 1)):
+            mask = (torch.rand(shape, device=DEV) > 0.2).bfloat16()
+            assert torch.equal(tri(z, mask), tri(z, mask.expand(1, n, n).contiguous()))
+        mask = (torch.rand(1, s, 1, device=DEV) > 0.2).bfloat16()
+        mask[:, 0] = 1
+        assert torch.equal(opm(m, mask, z), opm(m, mask.expand(1, s, n).contiguous(), z))
