@@ -209,3 +209,19 @@ def test_masks_that_broadcast(n, device_status):
         mask = (torch.rand(1, s, 1, device=DEV) > 0.2).bfloat16()
         mask[:, 0] = 1
         assert torch.equal(opm(m, mask, z), opm(m, mask.expand(1, s, n).contiguous(), z))
+
+
+@pytest.mark.parametrize("n", [61, 64])
+def test_biases_of_another_type_or_extent(n, device_status):
+    """A pair bias in fp32, and one that all heads share, next to the bf16 ``[1, H, n, n]`` that the kernel reads.  bf16 roundings
+    of the logits (2^-9 of up to 8) and of the output."""
+    torch.manual_seed(n)
+    att = _random_parameters(fops.SelfAttention(qkv_dim=128, c=32, n_head=4, out_dim=128)).eval().to(DEV, torch.bfloat16)
+    x, mask = torch.randn(1, 9, n, 128, device=DEV).bfloat16(), torch.ones(1, 9, n, device=DEV).bfloat16()
+    shared = torch.randn(1, 1, n, n, device=DEV).bfloat16()
+    bias = shared.expand(1, 4, n, n).contiguous()
+    with torch.no_grad():
+        want = att(x, mask, (bias, -1))[0].float()
+        for b in (bias.float(), shared):
+            got = att(x, mask, (b, -1))[0].float()
+            assert ((got - want).norm() / want.norm()).item() < 2e-2
