@@ -225,3 +225,15 @@ def test_biases_of_another_type_or_extent(n, device_status):
         for b in (bias.float(), shared):
             got = att(x, mask, (b, -1))[0].float()
             assert ((got - want).norm() / want.norm()).item() < 2e-2
+
+
+@pytest.mark.parametrize("n", [24, 32])
+def test_outer_product_mean_with_only_its_bias_trainable(n, device_status):
+    torch.manual_seed(n)
+    mod = _random_parameters(fops.OutProductMean(256, 128, 32)).to(DEV, torch.bfloat16).requires_grad_(False)
+    mod.o_linear.bias.requires_grad_(True)
+    m, z, mask = torch.randn(1, 8, n, 256, device=DEV).bfloat16(), torch.randn(1, n, n, 128, device=DEV).bfloat16(), torch.ones(1, 8, n, device=DEV)
+    up = torch.randn(1, n, n, 128, device=DEV).bfloat16()
+    (grad,) = torch.autograd.grad(mod(m, mask.bfloat16(), z), [mod.o_linear.bias], up)
+    want = up.float().sum((0, 1, 2)) / (8 + 1e-3)                  # 1 / (sequences + 1e-3) for every pair
+    assert ((grad.float() - want).norm() / want.norm()).item() < 2e-2
