@@ -22,7 +22,7 @@ setup(
     version="0.2.0",
     description="AlphaFold training and inference on NVIDIA B200: tcgen05 / TMA kernels, NVLink symmetric-heap collectives, Dynamic Axial Parallelism",
     packages=find_packages(include=["fastfold_b200", "fastfold_b200.*", "fastfold", "fastfold.*"]),
-    package_data={"fastfold_b200": ["lib/*.so", "csrc/*", "common/data/*.json"]},
+    package_data={"fastfold_b200": ["lib/*.so", "csrc/*", "csrc/host/*", "common/data/*.json"]},
     python_requires=">=3.9",
     install_requires=["numpy", "einops", "scipy"],
     cmdclass={"build_py": BuildWithKernels},
