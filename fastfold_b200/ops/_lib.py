@@ -99,19 +99,14 @@ def available():
 
 
 def get():
-    """Returns the loaded library, building it first when a compiler is at hand."""
+    """Returns the loaded library.  What is missing, or was built from other sources than the ones here or for another
+    PyTorch, is built first - before anything is loaded, since a loaded library stays for the life of the process."""
     global _lib
     if _lib is not None:
         return _lib
     with _lock:
         if _lib is None:
-            if not available():
-                try:
-                    _build.build(verbose=False)
-                except Exception as e:  # no nvcc on the box
-                    raise RuntimeError(
-                        "fastfold_b200: native library %s is missing and could not be built (%s). "
-                        "Run `python -m fastfold_b200._build` on a machine with nvcc." % (lib_path(), e))
+            _build.ensure()
             _lib = _declare(ctypes.CDLL(lib_path()))
     return _lib
 
@@ -123,13 +118,16 @@ def native():
         return _native
     with _lock:
         if _native is None:
-            get()                                    # builds both libraries when they are missing
+            get()
             path = _build.dispatch_path()
-            if not os.path.exists(path):
-                _build.build(verbose=False)
-            loader = importlib.machinery.ExtensionFileLoader(_build.DISPATCH, path)
-            _native = importlib.util.module_from_spec(importlib.util.spec_from_loader(_build.DISPATCH, loader))
-            loader.exec_module(_native)
+            try:
+                loader = importlib.machinery.ExtensionFileLoader(_build.DISPATCH, path)
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader(_build.DISPATCH, loader))
+                loader.exec_module(module)
+            except ImportError as e:
+                raise RuntimeError("fastfold_b200: %s does not load under PyTorch %s (%s). Rebuild it with `python -m fastfold_b200._build "
+                                   "--force`." % (path, torch.__version__, e))
+            _native = module                     # only now: other threads take it without the lock
     return _native
 
 
