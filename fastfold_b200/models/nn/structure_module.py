@@ -102,14 +102,15 @@ class InvariantPointAttention(nn.Module):
 
     def forward(self, s, z, r, mask):
         H = self.no_heads
-        if not self.is_multimer and z.is_cuda and not torch.is_grad_enabled() and (H, self.c_hidden, self.no_qk_points, self.no_v_points) == (12, 16, 4, 8):
-            from ...ops import ipa as ipa_op
-            proj = [f(s) for f in (self.linear_q, self.linear_kv, self.linear_q_points, self.linear_kv_points)]
-            if ipa_op.layer_supported(s, z, *proj, r):
-                head_w = self.softplus(self.head_weights) * math.sqrt(1.0 / (3 * (self.no_qk_points * 9.0 / 2)))
-                return self.linear_out(ipa_op.ipa_layer(*proj, r, z, self.linear_b.weight, self.linear_b.bias, head_w, mask,
-                                                        math.sqrt(1.0 / (3 * self.c_hidden)), math.sqrt(1.0 / 3), self.inf, self.eps))
+        from ...ops import ipa as ipa_op
         q = self.linear_q(s)
+        if not self.is_multimer:
+            kv, q_pts, kv_pts = self.linear_kv(s), self.linear_q_points(s), self.linear_kv_points(s)
+            if ((H, self.c_hidden, self.no_qk_points, self.no_v_points) == (12, 16, 4, 8)
+                    and ipa_op.layer_supported(s, z, q, kv, q_pts, kv_pts, r)):
+                head_w = self.softplus(self.head_weights) * math.sqrt(1.0 / (3 * (self.no_qk_points * 9.0 / 2)))
+                return self.linear_out(ipa_op.ipa_layer(q, kv, q_pts, kv_pts, r, z, self.linear_b.weight, self.linear_b.bias, head_w, mask,
+                                                        math.sqrt(1.0 / (3 * self.c_hidden)), math.sqrt(1.0 / 3), self.inf, self.eps))
         q = q.view(q.shape[:-1] + (H, -1))
         if self.is_multimer:
             k = self.linear_k(s)
@@ -120,20 +121,16 @@ class InvariantPointAttention(nn.Module):
             k_pts = self.linear_k_points(s, r)
             v_pts = self.linear_v_points(s, r)
         else:
-            kv = self.linear_kv(s)
             kv = kv.view(kv.shape[:-1] + (H, -1))
             k, v = torch.split(kv, self.c_hidden, dim=-1)
-            q_pts = self.linear_q_points(s)
             q_pts = torch.stack(torch.split(q_pts, q_pts.shape[-1] // 3, dim=-1), dim=-1)
             q_pts = r[..., None].apply(q_pts)
             q_pts = q_pts.view(q_pts.shape[:-2] + (H, self.no_qk_points, 3))
-            kv_pts = self.linear_kv_points(s)
             kv_pts = torch.stack(torch.split(kv_pts, kv_pts.shape[-1] // 3, dim=-1), dim=-1)
             kv_pts = r[..., None].apply(kv_pts)
             kv_pts = kv_pts.view(kv_pts.shape[:-2] + (H, -1, 3))
             k_pts, v_pts = torch.split(kv_pts, [self.no_qk_points, self.no_v_points], dim=-2)
         head_w = self.softplus(self.head_weights) * math.sqrt(1.0 / (3 * (self.no_qk_points * 9.0 / 2)))
-        from ...ops import ipa as ipa_op
         if s.dim() == 2 and z.shape[-3] != s.shape[-2]:
             # Row-parallel attention over the DAP group: this rank holds rows [row0, row0 + n_local) of the pair tensor,
             # which is all that queries row0 .. need (bias b[i, j] and o_pair[i] = sum_j a[i, j] z[i, j] use row i only).

@@ -101,3 +101,23 @@ def test_ipa_layer_in_three_kernels(N, fmt, device_status):
     assert out.shape == ref.shape and out.dtype == torch.bfloat16
     assert ((out.float() - ref).norm() / ref.norm()).item() < 4e-3
     assert (out.float() - ref).abs().max().item() < 2.0 ** -8 * ref.abs().max().item() + 1e-3
+
+
+@pytest.mark.parametrize("case", ["layer", "fp32", "batched"])
+def test_ipa_module_projects_once(case, device_status):
+    """Each input projection is evaluated once, whichever path the rest of the layer takes."""
+    from fastfold_b200.models.nn.structure_module import InvariantPointAttention
+    from fastfold_b200.utils.rigid_utils import Rigid, Rotation
+    torch.manual_seed(0)
+    dt = torch.float32 if case == "fp32" else torch.bfloat16
+    lead = (1,) if case == "batched" else ()
+    mod = InvariantPointAttention(384, 128, 16, 12, 4, 8).to(DEV, dt)
+    calls = []
+    for name in ("linear_q", "linear_kv", "linear_q_points", "linear_kv_points"):
+        getattr(mod, name).register_forward_hook(lambda m, x, y, name=name: calls.append(name))
+    N = 24
+    frames = Rigid(Rotation(quats=torch.randn(*lead, N, 4, device=DEV), normalize_quats=True), torch.randn(*lead, N, 3, device=DEV))
+    with torch.no_grad():
+        mod(torch.randn(*lead, N, 384, device=DEV, dtype=dt), torch.randn(*lead, N, N, 128, device=DEV, dtype=dt), frames,
+            torch.ones(*lead, N, device=DEV, dtype=dt))
+    assert sorted(calls) == ["linear_kv", "linear_kv_points", "linear_q", "linear_q_points"]
