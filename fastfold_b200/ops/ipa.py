@@ -97,6 +97,8 @@ def ipa_core(q, k, v, q_pts, k_pts, v_pts, z, wb, bb, gamma, mask, w_c, w_b, inf
         return ipa_core_ref(q, k, v, q_pts, k_pts, v_pts, z, wb, bb, gamma, mask, w_c, w_b, inf, row0)
     f32 = lambda t: t.float().contiguous()
     q, k, v, q_pts, k_pts, v_pts, wb, bb, gamma, mask = (f32(t) for t in (q, k, v, q_pts, k_pts, v_pts, wb, bb, gamma, mask))
+    if k_pts.data_ptr() % 16:
+        k_pts = k_pts.clone()                    # a view off a 16-byte boundary: the kernel reads four coordinates at a time
     N, H, C = q.shape
     rows = z.shape[0]
     o = torch.empty(rows, H, C, device=z.device, dtype=torch.float32)

@@ -121,3 +121,15 @@ def test_ipa_module_projects_once(case, device_status):
         mod(torch.randn(*lead, N, 384, device=DEV, dtype=dt), torch.randn(*lead, N, N, 128, device=DEV, dtype=dt), frames,
             torch.ones(*lead, N, device=DEV, dtype=dt))
     assert sorted(calls) == ["linear_kv", "linear_kv_points", "linear_q", "linear_q_points"]
+
+
+def test_ipa_core_takes_key_points_off_a_16_byte_boundary(device_status):
+    from fastfold_b200.ops.ipa import ipa_core
+    args = _inputs(70, seed=5)
+    w = (math.sqrt(1.0 / 48), math.sqrt(1.0 / 3), 1e5)
+    with torch.no_grad():
+        want = ipa_core(*args, *w)
+        flat = torch.empty(args[4].numel() + 1, device=DEV)
+        args[4] = flat[1:].view(args[4].shape).copy_(args[4])
+        got = ipa_core(*args, *w)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
