@@ -94,7 +94,7 @@ Tensor gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, double alpha, OptTensor bi
   if (block_out) {
     const auto& q = *block_out;      // [shape ..., mdiv, sr2, sr1, sc1]
     const size_t n = q.size() - 4;
-    expect(!out && M % 32 == 0 && n_out % 32 == 0 && (M / 32) % q[n] == 0 && !out_f32, "block-permuted output");
+    expect(!out && M % 32 == 0 && n_out % 32 == 0 && q[n] > 0 && (M / 32) % q[n] == 0 && !out_f32, "block-permuted output");
     result = at::empty(at::IntArrayRef(q.data(), n), a.options());
     expect(result.numel() == M * n_out, "block-permuted output");
     g.cq = 1;
@@ -192,6 +192,12 @@ std::tuple<OptTensor, OptTensor, OptTensor> linear_bwd(const Tensor& dy, const T
   return {dx, dw, db};
 }
 
+// An extent that lengths are divided by; integers do not raise by themselves here.
+int64_t divisor(int64_t extent) {
+  expect(extent > 0, "empty last dimension");
+  return extent;
+}
+
 int dtype_code(const Tensor& t) {
   return t.scalar_type() == at::kFloat ? 0 : (t.scalar_type() == at::kHalf ? 1 : 2);
 }
@@ -199,7 +205,7 @@ int dtype_code(const Tensor& t) {
 // y, and mean / rstd when `stats`
 std::tuple<Tensor, OptTensor, OptTensor> layer_norm_fwd(const Tensor& x, const Tensor& weight, const Tensor& bias, double eps, bool stats) {
   const Tensor w = weight.contiguous(), b = bias.contiguous();
-  const int64_t C = x.size(-1), rows = x.numel() / C;
+  const int64_t C = divisor(x.size(-1)), rows = x.numel() / C;
   Tensor y = at::empty_like(x);
   OptTensor mean, rstd;
   if (stats) {
@@ -214,7 +220,7 @@ std::tuple<Tensor, OptTensor, OptTensor> layer_norm_fwd(const Tensor& x, const T
 
 std::tuple<Tensor, Tensor, Tensor> layer_norm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd,
                                                   int64_t nblocks) {
-  const int64_t C = x.size(-1), rows = x.numel() / C;
+  const int64_t C = divisor(x.size(-1)), rows = x.numel() / C;
   Tensor dx = at::empty_like(x), dg = at::empty_like(w), db = at::empty_like(w), part = f32({nblocks * 2 * C}, x);
   check(ffb_layernorm_bwd(ptr(dy), ptr(x), ptr(w), static_cast<const float*>(ptr(mean)), static_cast<const float*>(ptr(rstd)), ptr(dx),
                           static_cast<float*>(ptr(part)), (int)nblocks, ptr(dg), ptr(db), rows, (int)C, dtype_code(x), stream()),
@@ -259,7 +265,7 @@ std::tuple<Tensor, OptTensor> attention_packed_fwd(const Tensor& qkv, const OptT
   return {out, lse};
 }
 
-int64_t rows_of(const Tensor& x) { return x.numel() / x.size(-1); }
+int64_t rows_of(const Tensor& x) { return x.numel() / divisor(x.size(-1)); }
 
 Tensor bias_sigmoid_mul_fwd(const Tensor& g, const Tensor& b, const Tensor& o) {
   Tensor y = at::empty_like(g);

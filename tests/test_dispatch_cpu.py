@@ -21,3 +21,16 @@ def test_gemm_refuses_fewer_row_factors_than_rows(batch, shape, dtype):
     a = torch.zeros(*([batch] if batch else []), 128, 64, dtype=torch.bfloat16)
     with pytest.raises(AssertionError, match="fewer row factors than rows"):
         _gemm(a, torch.zeros(64, 64, dtype=torch.bfloat16), torch.ones(shape, dtype=dtype))
+
+
+def test_empty_extents_raise():
+    """Integer division by an extent of 0 ends the process in native code; it raised in Python."""
+    n, w = _lib.native(), torch.ones(0, dtype=torch.bfloat16)
+    x = torch.empty(3, 0, dtype=torch.bfloat16)
+    calls = [lambda: n.layer_norm_fwd(x, w, w, 1e-5, False), lambda: n.layer_norm_bwd(x, x, w, w.float(), w.float(), 1),
+             lambda: n.bias_sigmoid_mul_fwd(x, w, x), lambda: n.bias_dropout_add_fwd(x, None, None, x, 1, 1), lambda: n.act_bwd(x, x, 1),
+             lambda: n.gemm(torch.empty(32, 64).bfloat16(), torch.empty(32, 64).bfloat16(), False, False, 1.0, None, 0, False, None, None, None,
+                            1, 1, None, False, None, False, 1, False, 0, [32, 32, 0, 1024, 1024, 1024])]
+    for call in calls:
+        with pytest.raises((AssertionError, RuntimeError)):        # RuntimeError: the stream, asked for first, needs a GPU
+            call()
