@@ -267,40 +267,60 @@ std::tuple<Tensor, OptTensor> attention_packed_fwd(const Tensor& qkv, const OptT
 
 int64_t rows_of(const Tensor& x) { return x.numel() / divisor(x.size(-1)); }
 
-Tensor bias_sigmoid_mul_fwd(const Tensor& g, const Tensor& b, const Tensor& o) {
+// The elementwise kernels move 16 bytes per thread and operand and do not look at the pointers: a view that starts off a
+// 16-byte boundary is copied.
+void dense16(Tensor& t) {
+  t = t.contiguous();
+  if (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) t = t.clone();
+}
+void dense16(OptTensor& t) {
+  if (t) dense16(*t);
+}
+template <class... T>
+void dense16(T&... ts) {
+  (dense16(ts), ...);
+}
+
+Tensor bias_sigmoid_mul_fwd(Tensor g, Tensor b, Tensor o) {
+  dense16(g, b, o);
   Tensor y = at::empty_like(g);
   check(ffb_bias_sigmoid_mul_fwd(ptr(g), ptr(b), ptr(o), ptr(y), rows_of(g), (int)g.size(-1), stream()), "bias_sigmoid_mul_fwd");
   return y;
 }
 
-std::tuple<Tensor, Tensor> bias_sigmoid_mul_bwd(const Tensor& dy, const Tensor& g, const Tensor& b, const Tensor& o) {
+std::tuple<Tensor, Tensor> bias_sigmoid_mul_bwd(Tensor dy, Tensor g, Tensor b, Tensor o) {
+  dense16(dy, g, b, o);
   Tensor dg = at::empty_like(g), dob = at::empty_like(o);
   check(ffb_bias_sigmoid_mul_bwd(ptr(dy), ptr(g), ptr(b), ptr(o), ptr(dg), ptr(dob), rows_of(g), (int)g.size(-1), stream()), "bias_sigmoid_mul_bwd");
   return {dg, dob};
 }
 
-Tensor bias_dropout_add_fwd(const Tensor& x, const OptTensor& b, const OptTensor& m, const Tensor& r, int64_t div, int64_t mod) {
+Tensor bias_dropout_add_fwd(Tensor x, OptTensor b, OptTensor m, Tensor r, int64_t div, int64_t mod) {
+  dense16(x, b, m, r);
   Tensor y = at::empty_like(x);
   check(ffb_bias_dropout_add_fwd(ptr(x), ptr(b), ptr(m), ptr(r), ptr(y), rows_of(x), (int)x.size(-1), (int)div, (int)mod, stream()),
         "bias_dropout_add_fwd");
   return y;
 }
 
-Tensor mask_mul(const Tensor& dy, const Tensor& m, int64_t div, int64_t mod) {
+Tensor mask_mul(Tensor dy, Tensor m, int64_t div, int64_t mod) {
+  dense16(dy, m);
   Tensor dx = at::empty_like(dy);
   check(ffb_mask_mul(ptr(dy), ptr(m), ptr(dx), rows_of(dy), (int)dy.size(-1), (int)div, (int)mod, stream()), "mask_mul");
   return dx;
 }
 
-Tensor bias_ele_dropout_res_fwd(const Tensor& ab, const Tensor& b, const Tensor& g, const OptTensor& m, const Tensor& r, int64_t div, int64_t mod) {
+Tensor bias_ele_dropout_res_fwd(Tensor ab, Tensor b, Tensor g, OptTensor m, Tensor r, int64_t div, int64_t mod) {
+  dense16(ab, b, g, m, r);
   Tensor y = at::empty_like(ab);
   check(ffb_bias_ele_dropout_res_fwd(ptr(ab), ptr(b), ptr(g), ptr(m), ptr(r), ptr(y), rows_of(ab), (int)ab.size(-1), (int)div, (int)mod, stream()),
         "bias_ele_dropout_res_fwd");
   return y;
 }
 
-std::tuple<Tensor, Tensor> bias_ele_dropout_res_bwd(const Tensor& dy, const Tensor& ab, const Tensor& b, const Tensor& g, const OptTensor& m,
+std::tuple<Tensor, Tensor> bias_ele_dropout_res_bwd(Tensor dy, Tensor ab, Tensor b, Tensor g, OptTensor m,
                                                     int64_t div, int64_t mod) {
+  dense16(dy, ab, b, g, m);
   Tensor dab = at::empty_like(ab), dg = at::empty_like(g);
   check(ffb_bias_ele_dropout_res_bwd(ptr(dy), ptr(ab), ptr(b), ptr(g), ptr(m), ptr(dab), ptr(dg), rows_of(ab), (int)ab.size(-1), (int)div, (int)mod,
                                      stream()),
@@ -308,20 +328,23 @@ std::tuple<Tensor, Tensor> bias_ele_dropout_res_bwd(const Tensor& dy, const Tens
   return {dab, dg};
 }
 
-Tensor glu_mask_t_fwd(const Tensor& pre, const Tensor& mask) {
+Tensor glu_mask_t_fwd(Tensor pre, Tensor mask) {
+  dense16(pre, mask);
   const int64_t C2 = pre.size(0) / 2, R = pre.size(1);
   Tensor out = at::empty({C2, R}, pre.options());
   check(ffb_glu_mask_t_fwd(ptr(pre), ptr(mask), ptr(out), (int)C2, R, stream()), "glu_mask_t_fwd");
   return out;
 }
 
-Tensor glu_mask_t_bwd(const Tensor& dout, const Tensor& pre, const Tensor& mask) {
+Tensor glu_mask_t_bwd(Tensor dout, Tensor pre, Tensor mask) {
+  dense16(dout, pre, mask);
   Tensor dpre = at::empty_like(pre);
   check(ffb_glu_mask_t_bwd(ptr(dout), ptr(pre), ptr(mask), ptr(dpre), (int)(pre.size(0) / 2), pre.size(1), stream()), "glu_mask_t_bwd");
   return dpre;
 }
 
-Tensor act_bwd(const Tensor& dy, const Tensor& y, int mode) {
+Tensor act_bwd(Tensor dy, Tensor y, int mode) {
+  dense16(dy, y);
   Tensor dx = at::empty_like(dy);
   check(ffb_act_bwd(ptr(dy), ptr(y), ptr(dx), rows_of(dy), (int)dy.size(-1), mode, stream()), "act_bwd");
   return dx;

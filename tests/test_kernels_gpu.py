@@ -294,3 +294,29 @@ def test_recycling_embedder_module_uses_fused_pair_update(device_status):
     assert torch.equal(m1, m2.detach())
     err = (z1.float() - z2.detach().float()).abs().amax(dim=-1)
     assert (err > 8e-2).float().mean().item() < 1e-3, err.max().item()
+
+
+def test_elementwise_operands_off_a_16_byte_boundary(device_status):
+    """Views that start at an odd element (into a flat buffer): the bits of aligned operands, forward and backward."""
+    torch.manual_seed(0)
+    shape, C = (1, 6, 10, 64), 64
+
+    def run(place):
+        def leaf(t):
+            return place(t).detach().requires_grad_(True)
+        g = torch.Generator(device=DEV).manual_seed(1)
+        r = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+        x, y, z, res, b, up = r(*shape), r(*shape), r(*shape), r(*shape), r(C), r(*shape)
+        drop = (torch.rand(1, 1, 10, C, device=DEV, generator=g) > 0.25).bfloat16() / 0.75
+        x, y, z, res, b = (leaf(t) for t in (x, y, z, res, b))
+        outs = [ops.bias_sigmod_ele(x, b, z), ops.bias_dropout_add(x, b, place(drop), res, prob=0.0, training=True),
+                ops.bias_ele_dropout_residual(x, b, y, place(drop), res, prob=0.0, training=True)]
+        grads = [torch.autograd.grad(o, [t for t in (x, y, z, res, b)], place(up), allow_unused=True) for o in outs]
+        return outs + [t for gs in grads for t in gs if t is not None]
+
+    def off(t):
+        flat = torch.empty(t.numel() + 1, device=DEV, dtype=t.dtype)
+        return flat[1:].view(t.shape).copy_(t)
+
+    for a, b in zip(run(lambda t: t.clone()), run(off)):
+        assert torch.equal(a, b)
