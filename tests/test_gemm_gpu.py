@@ -208,3 +208,22 @@ def test_pair_bias_hqk_matches_permuted_projection(device_status):
     ref = torch.einsum("bqkc,hc->bhqk", zn.float(), w.float())
     assert b is not None and b.shape == (1, 8, 64, 64)
     _close(b, ref, 128)
+
+
+@pytest.mark.parametrize("N", [16, 24, 32, 40, 64, 72, 200])
+@pytest.mark.parametrize("M", [1, 33, 64, 201, 1000])
+def test_bf16_row_factors_and_narrow_outputs(M, N, device_status):
+    """One bf16 factor per row, each its own value, on every epilogue that reads one; outputs narrower than a 64-column tile."""
+    torch.manual_seed(M + N)
+    K, batch = 72, 3
+    a, b = torch.randn(batch, M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    bias, rs = torch.randn(N, device=DEV).bfloat16(), (torch.rand(batch, M, device=DEV) + 0.5).bfloat16()
+    resid, mul = torch.randn(batch, M, N, device=DEV).bfloat16(), torch.randn(batch, M, N, device=DEV).bfloat16()
+    ref = lambda x, **kw: gemm_ref(x, b, out_dtype=torch.float32, **kw)
+    _close(gemm(a[0], b, bias=bias, rowscale=rs[0]), ref(a[0], bias=bias, rowscale=rs[0]), K)
+    _close(gemm(a, b, bias=bias, rowscale=rs), ref(a, bias=bias, rowscale=rs), K)
+    _close(gemm(a, b, bias=bias, rowscale=rs[1]), ref(a, bias=bias, rowscale=rs[1]), K)          # shared by the batch
+    _close(gemm(a, b, bias=bias, rowscale=rs, resid=resid, mul=mul), ref(a, bias=bias, rowscale=rs, resid=resid, mul=mul), K)
+    _close(gemm(a[0], b, bias=bias, rowscale=rs[0], trans_out=True), ref(a[0], bias=bias, rowscale=rs[0], trans_out=True), K)
+    _close(gemm(a[0], b, bias=bias, glu=True, rowscale=rs[0], trans_out=True), ref(a[0], bias=bias, glu=True, rowscale=rs[0], trans_out=True), K)
+    _close(gemm(a[0], b, bias=bias), ref(a[0], bias=bias), K)

@@ -133,3 +133,17 @@ def test_ipa_core_takes_key_points_off_a_16_byte_boundary(device_status):
         args[4] = flat[1:].view(args[4].shape).copy_(args[4])
         got = ipa_core(*args, *w)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("N,row0,rows", [(1024, 0, 1024), (1027, 0, 1027), (1101, 50, 1026)])
+def test_ipa_core_from_1024_rows_on(N, row0, rows, device_status):
+    """The instance with four query rows per CTA: whole and partial last groups, and a block of rows.  Bounds as above."""
+    from fastfold_b200.ops.ipa import ipa_core, ipa_core_ref
+    args = _inputs(N, seed=N)
+    args[6] = args[6][row0:row0 + rows].contiguous()
+    w = (math.sqrt(1.0 / 48), math.sqrt(1.0 / 3), 1e5)
+    with torch.no_grad():
+        got, want = ipa_core(*args, *w, row0=row0), ipa_core_ref(*args, *w, row0=row0)
+    for a, b, tol in zip(got, want, (2e-3, 2e-2, 2e-3)):
+        assert a.shape == b.shape
+        assert (a - b).abs().max().item() <= tol * max(1.0, b.abs().max().item())

@@ -237,3 +237,18 @@ def test_outer_product_mean_with_only_its_bias_trainable(n, device_status):
     (grad,) = torch.autograd.grad(mod(m, mask.bfloat16(), z), [mod.o_linear.bias], up)
     want = up.float().sum((0, 1, 2)) / (8 + 1e-3)                  # 1 / (sequences + 1e-3) for every pair
     assert ((grad.float() - want).norm() / want.norm()).item() < 2e-2
+
+
+@pytest.mark.parametrize("s,n", [(7, 33), (40, 77), (64, 64), (128, 100)])
+def test_outer_product_mean_with_masks(s, n, device_status):
+    """Whole sequences, whole residues and single positions masked: every row of both projections has its own mask value.
+    Pairs without a common sequence are divided by 1e-3, so their update is that of the bias."""
+    torch.manual_seed(s * n)
+    mod = _random_parameters(fops.OutProductMean(256, 128, 32)).eval()
+    mask = (torch.rand(1, s, n) > 0.3).float()
+    mask[:, s // 2] = 0
+    mask[:, :, n // 3] = 0
+    m, z = torch.randn(1, s, n, 256).bfloat16(), torch.randn(1, n, n, 128).bfloat16()
+    _check(mod, [m, mask, z], lambda f, x: f(*x))
+    both = mask[0].t() @ mask[0] > 0                              # and the pairs that have one, where the operands matter
+    _check(mod, [m, mask, z], lambda f, x: (f(*x) - x[2])[0][both.to(x[0].device)])
