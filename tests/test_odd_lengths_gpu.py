@@ -252,3 +252,19 @@ def test_outer_product_mean_with_masks(s, n, device_status):
     _check(mod, [m, mask, z], lambda f, x: f(*x))
     both = mask[0].t() @ mask[0] > 0                              # and the pairs that have one, where the operands matter
     _check(mod, [m, mask, z], lambda f, x: (f(*x) - x[2])[0][both.to(x[0].device)])
+
+
+@pytest.mark.parametrize("n", [1, 2, 5, 9, 17])
+def test_a_few_residues(n, device_status):
+    """The smallest lengths of every pair and MSA module: extents below a tile, a vector and a warp."""
+    torch.manual_seed(n)
+    pm, mm = torch.ones(1, n, n), torch.ones(1, 3, n)
+    z, m = torch.randn(1, n, n, 128).bfloat16(), torch.randn(1, 3, n, 256).bfloat16()
+    for cls in (TriangleAttentionStartingNode, TriangleAttentionEndingNode, TriangleMultiplicationOutgoing, TriangleMultiplicationIncoming):
+        att = cls in (TriangleAttentionStartingNode, TriangleAttentionEndingNode)
+        mod = _random_parameters(cls(128, p_drop=0.25, c=32 if att else 128, **({"n_head": 4} if att else {}))).eval()
+        _check(mod, [z, pm], lambda f, x: f(*x))
+    _check(_random_parameters(MSARowAttentionWithPairBias(256, 128)).eval(), [m, z, mm], lambda f, x: f(*x))
+    _check(_random_parameters(MSAColumnAttention(256)).eval(), [m, mm], lambda f, x: f(*x))
+    _check(_random_parameters(ExtraMSACore(64, 128)).eval(), [m[..., :64], z, mm], lambda f, x: f(*x))
+    _check(_random_parameters(fops.OutProductMean(256, 128, 32)).eval(), [m, mm, z], lambda f, x: f(*x))
