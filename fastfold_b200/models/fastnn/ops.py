@@ -199,7 +199,10 @@ class OutProductMean(nn.Module):
         """``proj(M) * mask`` with one mask value per row; without gradients in the projection's epilogue."""
         if not (_fusable(M) and proj.weight.dtype == M.dtype):
             return proj(M) * mask
-        return K.gemm(M.reshape(-1, M.shape[-1]), proj.weight, bias=proj.bias, rowscale=mask.expand(*M.shape[:-1], 1).reshape(-1)).view(*M.shape[:-1], -1)
+        M2 = M.reshape(-1, M.shape[-1])
+        if mask.numel() != M2.shape[0]:                           # a mask that broadcasts
+            mask = mask.expand(*M.shape[:-1], 1)
+        return K.gemm(M2, proj.weight, bias=proj.bias, rowscale=mask.reshape(-1)).view(*M.shape[:-1], -1)
 
     def _outer(self, left, right_all, inv_norm, Z_raw):
         """left [1,S,ni,d], right_all [1,S,N,e] -> Z_raw + o_linear(outer) * inv_norm."""
@@ -276,7 +279,8 @@ class OutProductMean(nn.Module):
         left_act = self._masked(self.linear_a, M, mask_col_a)
         inv_norm = memo.cached("opm_inv_norm", (src,), lambda: 1.0 / (torch.einsum("bsid,bsjd->bijd", M_mask_col.float(), M_mask.float()) + 1e-3))
         right_act_all = gather_async_opp(right_act_all, work, dim=2)
-        inv_norm = inv_norm.expand(-1, left_act.shape[2], right_act_all.shape[2], -1)      # of a mask that broadcasts
+        if inv_norm.shape[1:3] != (left_act.shape[2], right_act_all.shape[2]):             # of a mask that broadcasts
+            inv_norm = inv_norm.expand(-1, left_act.shape[2], right_act_all.shape[2], -1)
         if CHUNK_SIZE is None:
             return self._outer(left_act, right_act_all, inv_norm, Z_raw)
         out = Z_raw if INPLACE else torch.empty_like(Z_raw)

@@ -36,7 +36,7 @@ def supported(q, k, v, mask, bias):
     n_k = k.shape[3]
     if n_k % 8:
         return False
-    if bias is not None and (bias.dtype != q.dtype or tuple(bias.shape) != (1, 1, q.shape[2], q.shape[3], n_k)):
+    if bias is not None and (bias.dtype != q.dtype or bias.shape != (1, 1, q.shape[2], q.shape[3], n_k)):
         return False
     return True
 
@@ -141,7 +141,7 @@ def packed_supported(qkv, mask, bias, transposed=False):
     if n % 8 and bias is not None and need_grad:
         return False            # the backward kernel stores the logit gradient in 16-byte pieces of un-padded rows
     # the kernels read the bias as bf16 ``[H, n, n]``; another type or one that broadcasts is the composite's
-    if bias is not None and (bias.dtype != qkv.dtype or tuple(bias.shape) != (1, 1, qkv.shape[4], n, n)):
+    if bias is not None and (bias.dtype != qkv.dtype or bias.shape != (1, 1, qkv.shape[4], n, n)):
         return False
     return True
 
