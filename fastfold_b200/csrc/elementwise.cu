@@ -11,8 +11,9 @@
 // The dropout mask m is shared along one axis of the activation, so it is a
 // small [mod, C] tensor indexed by (row / div) % mod; it already contains the
 // 1/(1-p) scale.  All kernels move 16 bytes per thread per tensor; C must be a
-// multiple of 8 and pointers 16-byte aligned (the Python wrappers route other
-// shapes to a composite implementation).
+// multiple of 8 (the Python wrappers route other shapes to a composite
+// implementation) and pointers 16-byte aligned (the callers copy operands that
+// are not).
 //
 // These are the reference's TorchScript fusions
 // (fastfold/model/fastnn/kernel/jit/fused_ops.py:5-22) written as explicit

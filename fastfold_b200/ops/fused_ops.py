@@ -155,11 +155,17 @@ def bias_ele_dropout_residual(ab, b, g, dropout_mask, Z_raw, prob, training=True
 
 
 # ---------------------------------------------------------------------------
+def _dense16(t):
+    """``t`` dense and on a 16-byte boundary, as the kernels load it."""
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
+
+
 class _GluMask(torch.autograd.Function):
     @staticmethod
     def forward(ctx, p, q, rowmask):
         lib = _lib.get()
-        pc, qc = p.contiguous(), q.contiguous()
+        pc, qc = _dense16(p), _dense16(q)
         rows, C = _rows_c(pc)
         y = torch.empty_like(pc)
         rm = rowmask.to(torch.bfloat16).contiguous() if rowmask is not None else None
@@ -172,7 +178,7 @@ class _GluMask(torch.autograd.Function):
         lib = _lib.get()
         pc, qc, rm = ctx.saved_tensors
         rows, C = _rows_c(pc)
-        dyc = dy.contiguous()
+        dyc = _dense16(dy)
         dp = torch.empty_like(pc)
         dq = torch.empty_like(qc)
         _lib.check(lib.ffb_glu_mask_bwd(_lib.ptr(dyc), _lib.ptr(pc), _lib.ptr(qc), _lib.ptr(rm), _lib.ptr(dp), _lib.ptr(dq), rows, C,

@@ -310,7 +310,8 @@ def test_elementwise_operands_off_a_16_byte_boundary(device_status):
         drop = (torch.rand(1, 1, 10, C, device=DEV, generator=g) > 0.25).bfloat16() / 0.75
         x, y, z, res, b = (leaf(t) for t in (x, y, z, res, b))
         outs = [ops.bias_sigmod_ele(x, b, z), ops.bias_dropout_add(x, b, place(drop), res, prob=0.0, training=True),
-                ops.bias_ele_dropout_residual(x, b, y, place(drop), res, prob=0.0, training=True)]
+                ops.bias_ele_dropout_residual(x, b, y, place(drop), res, prob=0.0, training=True),
+                ops.glu_mask(x, y, place(drop[..., 0].expand(1, 6, 10).contiguous()))]
         grads = [torch.autograd.grad(o, [t for t in (x, y, z, res, b)], place(up), allow_unused=True) for o in outs]
         return outs + [t for gs in grads for t in gs if t is not None]
 
