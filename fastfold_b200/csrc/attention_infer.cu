@@ -20,15 +20,19 @@
 // rescaling of the output.  The reference point M of a row only has to keep the row sum inside the exponent range, so it
 // starts at 0 and is moved (exact block maximum, output and sum rescaled) only when the sum leaves [2^-60, 2^60] - a
 // warp-uniform side path; bf16 and fp32 have the same exponent range, so P, the sums and the output lose no precision at
-// any M in between.  Four groups, because a group waits for its S product once per block and the others fill that time.
+// any M in between, as long as P V has room too: a row whose sum is near 2^60 takes values up to 2^68, one near 2^-60 down
+// to 2^-56.  A narrower window would give them more, but the side path nearly doubles a block's time (q 4x as large,
+// n 256, B 256: 40 us with this window, 43 with 2^+-32, 69 with 2^+-24).  Rows whose logits are themselves masks (biases of
+// -1e9, the lowest bf16 value, -inf) take a general step, see FAR_LOGIT.
+// Four groups, because a group waits for its S product once per block and the others fill that time.
 // Two issuer warps with descriptors that are only added to: with one issuer that built each descriptor where it was used,
 // its instructions were the longest chain of a block and the kernel took 1.8x as long.
-//   Measured (B200, against the kernel that also serves training, which keeps a running maximum and P in shared memory;
-//   same clocks on both sides): B 128, H 4, n 1024 with bias 738 -> 444 us, with a random mask 967 -> 490 us; B 256, H 4,
-//   n 256 126 -> 71 us; B 256, H 8, n 128 without bias 80 -> 24 us; B 32, H 8, n 64 9.8 -> 6.5 us.
+//   Measured (B200 at 1965 MHz, alternating with the kernel that also serves training, which keeps a running maximum and P
+//   in shared memory): B 128, H 4, n 1024 with bias 451 -> 246 us, with a random mask 516 -> 267 us; B 256, H 4, n 256
+//   67 -> 40 us; B 256, H 8, n 128 without bias 46 -> 21 us; B 32, H 8, n 64 8.6 -> 5.8 us.
 // Masked keys get a huge negative logit (replaced, not added; -2^30 here, -1e9 in the reference's
-// softmax kernels, softmax_cuda_kernel.cu:338-423,618-706 - same weights); keys beyond the
-// sequence end get -inf.
+// softmax kernels, softmax_cuda_kernel.cu:338-423,618-706 - same weights), which is weight 0 next to any ordinary
+// key: there they are left out; keys beyond the sequence end get -inf.
 // The forward pass of training stays on the kernel of attention_tcgen05.cu, which also leaves the row statistic for the
 // backward pass: the logits' gradients are differences of nearly equal numbers (dP - rowsum(dO o O)), so rounding P at
 // another reference point moves weight gradients by up to 4% of their norm, with neither kernel closer to 64 bits (0.057

@@ -963,7 +963,8 @@ static int gemm_launch(const void* A, const void* B, int a_mn, int b_mn, long lo
   if (tma_epi && g.mul && !(al16(g.mul, g.ldmul, g.mul_bstride) && (batch == 1 || g.mul_bstride != 0))) tma_epi = 0;
   if (tma_epi && g.resid && !(al16(g.resid, g.ldres, g.res_bstride) && (batch == 1 || g.res_bstride != 0))) tma_epi = 0;
   if (g.cq) {
-    // block-permuted store: bf16, whole 32 x 64 warp tiles only, no mul / residual tiles (they would be fetched in matrix layout)
+    // block-permuted store: bf16, whole 32 x 32 blocks only (the last 32 x 64 warp tile of a row may hold one), no mul /
+    // residual tiles (they would be fetched in matrix layout)
     if (g.out_mode != OUT_BF16 || g.trans_out || g.glu || g.mul || g.resid || (g.M % 32) || (g.N % 32)) return -23;
     if ((reinterpret_cast<uintptr_t>(g.C) & 15) || (g.cq_sr1 % 8) || (g.cq_sr2 % 8) || (g.cq_sc1 % 8) || (g.c_bstride % 8) || g.cq_mdiv < 1) return -23;
     tma_epi = 1;

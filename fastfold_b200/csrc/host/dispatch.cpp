@@ -1,10 +1,10 @@
 // Host side of the operator calls: argument checks, output allocation and the launch, from tensors to the C entry points
 // of libffb200.so, without a trip through Python objects for every pointer, stride and flag.
 //
-// Why it is native: a block of the trunk is 60 - 90 launches (a training step of it 250), and with the argument block of
-// a launch filled through ctypes each cost the host 20 - 35 us, so that calls of up to 256 residues were bound by the host:
-// a block of 32 x 64 took 1.98 ms and takes 0.95 ms (65 launches), 128 x 256 the same, the training pass of the pair half at
-// 256 residues 5.3 and 3.5 ms (198 launches).
+// Why it is native: a block of the trunk is 50 - 100 launches (the training pass of its two halves 290), and with the argument
+// block of a launch filled through ctypes each cost the host 20 - 35 us, so that calls of up to 256 residues were bound by the
+// host: a block of 32 x 64 took 1.98 ms and takes 0.9 ms (57 launches), 128 x 256 the same, the training pass of the pair half
+// at 256 residues 5.3 and 3.5 ms (198 launches).
 //
 // Nothing is kept between calls.  Work goes to the caller's current stream; tensors are allocated by PyTorch's allocator
 // on that stream, exactly as the Python code did.
@@ -139,7 +139,8 @@ Tensor gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, double alpha, OptTensor bi
   }
   if (rowscale) {
     // bf16 masks are read as they are, which saves the conversion's launch; not so in the gated projection of the triangle
-    // multiplication, which is 3 % faster on the converted mask (1215 against 1250 us at 1024 residues)
+    // multiplication: with them the whole operator took 1250 us at 1024 residues, with the converted mask 1215 us (why is not
+    // known, and only that size was measured)
     g.rs_bf16 = rowscale->scalar_type() == at::kBFloat16 && !glu;
     rowscale = (g.rs_bf16 ? *rowscale : rowscale->to(at::kFloat)).contiguous();
     g.rowscale = ptr(rowscale);

@@ -55,9 +55,10 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool i
 // What bounds it: instruction issue (about 50 issue slots x SM sub-partition per (query, key) pair for all heads) and, below
 // some 150 CTAs, the number of SMs in use.  One row per CTA with one key-value read per row, which this replaces, spent its
 // time waiting for L2: every row re-read 3.2 KB of keys, values and points per key, a quarter of the warps in flight.
-// R = 2 with two CTAs per SM below 1024 rows, where R = 4 would leave SMs without a CTA; R = 4 (half the key / value traffic)
-// from there on.
-//   Measured (B200, N = 512): 349 us with one row per CTA, 200 us with R = 2.
+// R = 2 with two CTAs per SM below 1024 rows; R = 4, with half the key / value traffic, from there on.
+//   Measured (B200, the core alone, us, R = 2 / R = 4): N = 256 90 / 78, 512 192 / 171, 768 592 / 525, 1024 792 / 740,
+//   1184 966 / 869, 1536 1796 / 1659, 2048 3207 / 2967; one row per CTA took 349 at 512.  So R = 4 would be the better choice
+//   below the line too, where its fewer CTAs had been expected to leave SMs idle: 8 - 13 % of the core there.
 template <int R, int H, int C, int PQ, int PV, int CZ>
 __global__ void __launch_bounds__(IPA_THREADS, R == 2 ? 2 : 1) ipa_fwd_kernel(const IpaArgs a) {
   pdl_launch_dependents();
