@@ -197,7 +197,7 @@ class OutProductMean(nn.Module):
     @staticmethod
     def _masked(proj, M, mask):
         """``proj(M) * mask`` with one mask value per row; without gradients in the projection's epilogue."""
-        if not (_fusable(M) and proj.weight.dtype == M.dtype):
+        if not (_fusable(M) and proj.weight.dtype == M.dtype and M.shape[-1] % 8 == 0):
             return proj(M) * mask
         M2 = M.reshape(-1, M.shape[-1])
         if mask.numel() != M2.shape[0]:                           # a mask that broadcasts
@@ -461,7 +461,7 @@ class SelfAttention(nn.Module):
     def _one(self, x, mask, bias, tail, transposed=False):
         """``transposed``: ``x [b1, n, b2, c]`` and the attention runs along dim 1 (``mask [b1, b2, n]``)."""
         H, d = self.n_head, self.c
-        if d < flash.HEAD_DIM and not transposed and _fusable(x):
+        if d < flash.HEAD_DIM and not transposed and _fusable(x) and x.shape[-1] % 8 == 0:
             res = self._one_padded(x, mask, bias, tail)
             if res is not None:
                 return res

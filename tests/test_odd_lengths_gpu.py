@@ -268,3 +268,12 @@ def test_a_few_residues(n, device_status):
     _check(_random_parameters(MSAColumnAttention(256)).eval(), [m, mm], lambda f, x: f(*x))
     _check(_random_parameters(ExtraMSACore(64, 128)).eval(), [m[..., :64], z, mm], lambda f, x: f(*x))
     _check(_random_parameters(fops.OutProductMean(256, 128, 32)).eval(), [m, mm, z], lambda f, x: f(*x))
+
+
+def test_widths_that_are_no_multiple_of_8(device_status):
+    """The GEMM reads rows at a pitch of 16 bytes; layers of other widths are the library's."""
+    torch.manual_seed(0)
+    s, n = 9, 61
+    m, z, mask = torch.randn(1, s, n, 20).bfloat16(), torch.randn(1, n, n, 128).bfloat16(), torch.ones(1, s, n)
+    _check(_random_parameters(fops.OutProductMean(20, 128, 32)).eval(), [m, mask, z], lambda f, x: f(*x))
+    _check(_random_parameters(fops.SelfAttention(qkv_dim=20, c=8, n_head=4, out_dim=64, gating=False)).eval(), [m, mask], lambda f, x: f(*x)[0])
