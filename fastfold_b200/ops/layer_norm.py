@@ -70,8 +70,8 @@ def _needs_graph(*ts):
     return (torch.is_grad_enabled() and any(t.requires_grad for t in ts)) or forward_ad._current_level >= 0
 
 
-def _ln_t_supported(x_cm):
-    return x_cm.is_cuda and x_cm.dtype == torch.bfloat16 and x_cm.shape[0] <= 256
+def _ln_t_supported(x_cm, weight, bias):
+    return x_cm.is_cuda and x_cm.dtype == weight.dtype == bias.dtype == torch.bfloat16 and x_cm.shape[0] <= 256
 
 
 def _ln_t_forward(x_cm, weight, bias, eps, want_stats):
@@ -117,7 +117,7 @@ class _LayerNormTFn(torch.autograd.Function):
 def layer_norm_transposed(x_cm, weight, bias, eps=1e-5):
     """LayerNorm over dim 0 of ``x_cm [C, rows]`` returning ``[rows, C]``; differentiable (the gradient of ``x_cm`` is
     produced channel-major by its own kernel)."""
-    if not _ln_t_supported(x_cm):
+    if not _ln_t_supported(x_cm, weight, bias):
         return layer_norm(x_cm.t().contiguous(), weight, bias, eps)
     if torch.is_grad_enabled() and (x_cm.requires_grad or weight.requires_grad or bias.requires_grad):
         if _lib.has("ffb_layernorm_bwd_transposed"):

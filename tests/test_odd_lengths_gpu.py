@@ -277,3 +277,17 @@ def test_widths_that_are_no_multiple_of_8(device_status):
     m, z, mask = torch.randn(1, s, n, 20).bfloat16(), torch.randn(1, n, n, 128).bfloat16(), torch.ones(1, s, n)
     _check(_random_parameters(fops.OutProductMean(20, 128, 32)).eval(), [m, mask, z], lambda f, x: f(*x))
     _check(_random_parameters(fops.SelfAttention(qkv_dim=20, c=8, n_head=4, out_dim=64, gating=False)).eval(), [m, mask], lambda f, x: f(*x)[0])
+
+
+@pytest.mark.parametrize("n", [61, 64])
+def test_triangle_multiplication_with_fp32_norms(n, device_status):
+    """Norm parameters kept in fp32 next to bf16 activations: the kernels take one type only, other parameters are converted."""
+    torch.manual_seed(n)
+    mod = _random_parameters(TriangleMultiplicationOutgoing(128, p_drop=0.25, c=128)).eval().to(DEV, torch.bfloat16)
+    z, mask = torch.randn(1, n, n, 128, device=DEV).bfloat16(), torch.ones(1, n, n, device=DEV).bfloat16()
+    with torch.no_grad():
+        want = mod(z, mask).float()
+        mod.layernorm1.float()
+        mod.layernorm2.float()
+        got = mod(z, mask).float()
+    assert ((got - want).norm() / want.norm()).item() < 1e-2
