@@ -83,7 +83,7 @@ def _fusable(x):
 def _mask_idx(x, mask):
     from ...ops.fused_ops import _mask_index
     m2, div, mod = _mask_index(x, mask)
-    return (m2.contiguous(), div, mod)
+    return (m2.to(x.dtype).contiguous(), div, mod)
 
 
 def _apply_dropout(mask, p, training):

@@ -291,3 +291,16 @@ def test_triangle_multiplication_with_fp32_norms(n, device_status):
         mod.layernorm2.float()
         got = mod(z, mask).float()
     assert ((got - want).norm() / want.norm()).item() < 1e-2
+
+
+@pytest.mark.parametrize("n", [61, 64])
+def test_dropout_masks_in_fp32(n, device_status):
+    """The first pass of activation checkpointing with a mask of another type than the activations."""
+    torch.manual_seed(n)
+    z, mask = torch.randn(1, n, n, 128, device=DEV).bfloat16(), torch.ones(1, n, n, device=DEV).bfloat16()
+    for mod, shape in ((TriangleMultiplicationOutgoing(128, p_drop=0.25, c=128), (1, 1, n, 128)),
+                       (TriangleAttentionEndingNode(128, p_drop=0.25, c=32, n_head=4), (1, n, 1, 128))):
+        mod = _random_parameters(mod).train().to(DEV, torch.bfloat16)
+        drop = (torch.rand(shape, device=DEV) > 0.25).float() * 1.25             # 1.25 is a bf16 value
+        with torch.no_grad():
+            assert torch.equal(mod(z, mask, drop), mod(z, mask, drop.bfloat16()))
