@@ -212,7 +212,7 @@ class OutProductMean(nn.Module):
         r2 = right_all.reshape(S, N * e)
         need_grad = torch.is_grad_enabled() and any(t is not None and t.requires_grad
                                                     for t in (l2, r2, Z_raw, self.o_linear.weight, self.o_linear.bias))
-        if (Z_raw.is_cuda and Z_raw.dtype == torch.bfloat16 and d == 32 and e == 32 and (N % 32 == 0 or not need_grad) and ni * d >= 64
+        if (Z_raw.is_cuda and Z_raw.dtype == l2.dtype == r2.dtype == torch.bfloat16 and d == 32 and e == 32 and (N % 32 == 0 or not need_grad) and ni * d >= 64
                 and N * e >= 64 and self.o_linear.bias is not None):
             # the product [(i d), (j e)] leaves the GEMM epilogue already laid out as [i, j, d, e], the operand layout of
             # the output projection; its gradient comes back the other way through the same block-permuting store, which

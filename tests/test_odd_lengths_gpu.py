@@ -304,3 +304,15 @@ def test_dropout_masks_in_fp32(n, device_status):
         drop = (torch.rand(shape, device=DEV) > 0.25).float() * 1.25             # 1.25 is a bf16 value
         with torch.no_grad():
             assert torch.equal(mod(z, mask, drop), mod(z, mask, drop.bfloat16()))
+
+
+@pytest.mark.parametrize("n", [40, 64])
+def test_outer_product_mean_of_an_fp32_msa(n, device_status):
+    """An fp32 module and MSA next to a bf16 pair tensor."""
+    torch.manual_seed(n)
+    mod = _random_parameters(fops.OutProductMean(256, 128, 32)).eval().to(DEV)
+    m, z, mask = torch.randn(1, 9, n, 256, device=DEV), torch.randn(1, n, n, 128, device=DEV).bfloat16(), torch.ones(1, 9, n, device=DEV)
+    with torch.no_grad():
+        want = mod(m, mask, z.float())
+        got = mod(m, mask, z).float()
+    assert ((got - want).norm() / want.norm()).item() < 1e-2
