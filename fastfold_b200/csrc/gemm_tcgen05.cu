@@ -17,7 +17,7 @@
 //   warp 0      : TMA producer (one elected lane) - fills a STAGES-deep ring of
 //                 128B-swizzled operand tiles, completion via mbarrier tx-count;
 //                 the ring keeps running across tile boundaries
-//   warp 1      : MMA issuer (one lane) - tcgen05.mma, 128 x BN x 16 per
+//   warp 1      : MMA issuer - tcgen05.mma, 128 x BN x 16 per
 //                 instruction, into one of TWO accumulator stages in TMEM;
 //                 tcgen05.commit releases ring slots and signals "stage full"
 //   warps 2..5  : epilogue - tcgen05.ld of their 32-lane TMEM quadrant, a
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_kernel(const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* s_bias = reinterpret_cast<float*>(smem_al + STAGES * Cfg::STAGE_BYTES + Cfg::STG_BYTES + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);    // the same in all lanes, and known to be
   const int lane = threadIdx.x & 31;
   const int kb_total = (g.K + BK - 1) / BK;
   if (threadIdx.x == 0) {
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_kernel(const __grid
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   GEMM_TRACE_CTA(1);   // barriers initialised, tensor memory allocated
   // everything above touches only this CTA's shared and tensor memory; from here on global memory is read
   pdl_wait();
@@ -315,47 +315,50 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_kernel(const __grid
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---------------- MMA issuer ----------------
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      uint32_t it = 0, lt = 0;   // k-block counter, local tile counter
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++lt) {
-        const TileCoord tc = tile_coord(tile, tiles_n, tiles_m, g.splits);
-        const int kb_begin = tc.split * g.kblocks_per_split;
-        int kb_end = kb_begin + g.kblocks_per_split;
-        if (kb_end > kb_total) kb_end = kb_total;
-        const uint32_t as = lt & 1;
-        if (!mbar_wait(bar_acce + 8 * as, ((lt >> 1) & 1) ^ 1)) {
-          report(ST_TIMEOUT_EPI, 1);
+    // ---------------- MMA issuer (the whole warp, see umma_bf16_by) ----------------
+    // Against one lane issuing (us, alternating on one box): 128 x 1024^3, both operands K-major 253 -> 245, both MN-major 261 -> 251;
+    // 12288 x 12288 x 512 block-permuted 145 -> 136; 65536 x 512 x 128 with B MN-major 18.4 -> 15.9; 32768 x 256 x 1024 21.5 -> 20.5.
+    constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    const uint32_t lead = elect_one();
+    // descriptors of ring slot 0; the address field counts 16 bytes, so slots and steps along K are additions
+    const uint64_t ad0 = A_MN ? make_smem_desc(smem_base, BK * 128, 1024) : make_smem_desc(smem_base, 16, 1024);
+    const uint64_t bd0 = B_MN ? make_smem_desc(smem_base + Cfg::A_BYTES, BK * 128, 1024) : make_smem_desc(smem_base + Cfg::A_BYTES, 16, 1024);
+    uint32_t s = 0, phase = 0, lt = 0;   // ring slot and its parity, local tile counter
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++lt) {
+      const TileCoord tc = tile_coord(tile, tiles_n, tiles_m, g.splits);
+      const int kb_begin = tc.split * g.kblocks_per_split;
+      int kb_end = kb_begin + g.kblocks_per_split;
+      if (kb_end > kb_total) kb_end = kb_total;
+      const uint32_t as = lt & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(bar_acce + 8 * as, ((lt >> 1) & 1) ^ 1))) {
+        if (lead) report(ST_TIMEOUT_EPI, 1);
+        *abort_flag = 1;
+        break;
+      }
+      tc_fence_after();
+      const uint32_t tmem_acc = tmem_base + as * BN;
+      for (int kb = kb_begin; kb < kb_end; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait(bar_full + 8 * s, phase))) {
+          if (lead) report(ST_TIMEOUT_TMA, kb);
           *abort_flag = 1;
+          ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t tmem_acc = tmem_base + as * BN;
-        for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
-          const int s = it % STAGES;
-          if (!mbar_wait(bar_full + 8 * s, (it / STAGES) & 1)) {
-            report(ST_TIMEOUT_TMA, kb);
-            *abort_flag = 1;
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          if (kb == kb_begin) GEMM_TRACE(lt, 1);       // issuer: first operand tile landed
-          const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES;
-          const uint32_t sb = sa + Cfg::A_BYTES;
+        if (kb == kb_begin && lead) GEMM_TRACE(lt, 1);       // issuer: first operand tile landed
+        const uint64_t ad = ad0 + s * (Cfg::STAGE_BYTES >> 4), bd = bd0 + s * (Cfg::STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t ad = A_MN ? make_smem_desc(sa + k * 2048, BK * 128, 1024) : make_smem_desc(sa + k * 32, 16, 1024);
-            const uint64_t bd = B_MN ? make_smem_desc(sb + k * 2048, BK * 128, 1024) : make_smem_desc(sb + k * 32, 16, 1024);
-            umma_bf16(tmem_acc, ad, bd, idesc, (kb > kb_begin || k > 0) ? 1u : 0u);
-          }
-          umma_commit(bar_empty + 8 * s);   // slot reusable once these MMAs retire
+        for (int k = 0; k < BK / 16; ++k)
+          umma_bf16_by(lead, tmem_acc, ad + k * ((A_MN ? 2048 : 32) >> 4), bd + k * ((B_MN ? 2048 : 32) >> 4), idesc, (kb > kb_begin || k > 0) ? 1u : 0u);
+        umma_commit_by(lead, bar_empty + 8 * s);   // slot reusable once these MMAs retire
+        if (++s == STAGES) {
+          s = 0;
+          phase ^= 1;
         }
-        if (ok) umma_commit(bar_accf + 8 * as);   // accumulator stage complete
-        GEMM_TRACE(lt, 2);                         // issuer: all MMAs of the tile issued
       }
+      if (ok) umma_commit_by(lead, bar_accf + 8 * as);   // accumulator stage complete
+      if (lead) GEMM_TRACE(lt, 2);                       // issuer: all MMAs of the tile issued
     }
     __syncwarp();
   } else {
