@@ -171,14 +171,211 @@ __global__ void __launch_bounds__(GA_THREADS) global_attention_kernel(const bf16
   }
 }
 
+constexpr int GC_H = 8, GC_C = 8, GC_HC = GC_H * GC_C;
+constexpr int GC_REC = 2 + GC_C;          // per head: max, sum, C weighted values
+
+// Online softmax state of a thread: half of the heads, every second key of its CTA's share.
+struct GcState {
+  float m[GC_H / 2], l[GC_H / 2], acc[GC_H / 2][GC_C];
+};
+__device__ __forceinline__ void gc_init(GcState& t) {
+#pragma unroll
+  for (int h = 0; h < GC_H / 2; ++h) {
+    t.m[h] = -INFINITY;
+    t.l[h] = 0.f;
+#pragma unroll
+    for (int i = 0; i < GC_C; ++i) t.acc[h][i] = 0.f;
+  }
+}
+__device__ __forceinline__ void gc_key(GcState& t, uint4 kraw, uint4 vraw, bool masked, const float* q) {
+  float kf[GC_C], vf[GC_C];
+  const bf162* kh = reinterpret_cast<const bf162*>(&kraw);
+  const bf162* vh = reinterpret_cast<const bf162*>(&vraw);
+#pragma unroll
+  for (int i = 0; i < GC_C / 2; ++i) {
+    const float2 a = __bfloat1622float2(kh[i]), b = __bfloat1622float2(vh[i]);
+    kf[2 * i] = a.x; kf[2 * i + 1] = a.y;
+    vf[2 * i] = b.x; vf[2 * i + 1] = b.y;
+  }
+#pragma unroll
+  for (int h = 0; h < GC_H / 2; ++h) {
+    float d = 0.f;
+#pragma unroll
+    for (int i = 0; i < GC_C; ++i) d = fmaf(q[h * GC_C + i], kf[i], d);
+    if (masked) d = GA_MASKED;
+    if (d > t.m[h]) {                         // the running maximum settles after a few keys: the rescale is rare
+      const float a = __expf(t.m[h] - d);     // m = -inf on the first key: a = 0
+      t.l[h] *= a;
+#pragma unroll
+      for (int i = 0; i < GC_C; ++i) t.acc[h][i] *= a;
+      t.m[h] = d;
+    }
+    const float pw = __expf(d - t.m[h]);
+    t.l[h] += pw;
+#pragma unroll
+    for (int i = 0; i < GC_C; ++i) t.acc[h][i] = fmaf(pw, vf[i], t.acc[h][i]);
+  }
+}
+// over the 16 lanes of each head group (even / odd lanes): common maximum, rescaled sums
+__device__ __forceinline__ void gc_fold_warp(const GcState& t, int lane, int hg, float (*rec)[GC_REC]) {
+#pragma unroll
+  for (int h = 0; h < GC_H / 2; ++h) {
+    float wm = t.m[h];
+#pragma unroll
+    for (int o = 16; o > 1; o >>= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
+    const float sc = (t.m[h] == -INFINITY) ? 0.f : __expf(t.m[h] - wm);
+    float v = t.l[h] * sc;
+#pragma unroll
+    for (int o = 16; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane < 2) {
+      rec[hg * (GC_H / 2) + h][0] = wm;
+      rec[hg * (GC_H / 2) + h][1] = v;
+    }
+#pragma unroll
+    for (int i = 0; i < GC_C; ++i) {
+      float a = t.acc[h][i] * sc;
+#pragma unroll
+      for (int o = 16; o > 1; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane < 2) rec[hg * (GC_H / 2) + h][2 + i] = a;
+    }
+  }
+}
+// thread (h, i): maximum, sum and i-th weighted value of head h over the warps of the CTA
+__device__ __forceinline__ void gc_fold_warps(const float (*rec)[GC_H][GC_REC], int h, int i, float& mx, float& lt, float& at) {
+  mx = -INFINITY;
+  for (int w = 0; w < GA_THREADS / 32; ++w) mx = fmaxf(mx, rec[w][h][0]);
+  lt = at = 0.f;
+  for (int w = 0; w < GA_THREADS / 32; ++w) {
+    const float mw = rec[w][h][0];
+    const float sc = (mw == -INFINITY) ? 0.f : __expf(mw - mx);
+    lt = fmaf(rec[w][h][1], sc, lt);
+    at = fmaf(rec[w][h][2 + i], sc, at);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The whole column up to its value vector, from the MSA as it is stored ([S][N][64], no transposed copy): masked mean of the
+// normalised rows, projected to the column's eight queries, online softmax over the sequences, o[n][64] in 32 bits.  The gate, which is
+// per row, belongs to the output projection (ln_gemm.cu).  One CTA per column; the rows of a column are 128-byte pieces N rows
+// apart and its keys 32-byte ones, so neighbouring CTAs share cache lines of the keys only.
+// Replaces transposing the MSA, normalising it, the mask product, two reductions, the query projection and the core kernel below:
+// 14 launches of the layer become 3.
+__global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma,
+                                                                      const bf16* __restrict__ beta, float eps, const bf16* __restrict__ wq,
+                                                                      const bf16* __restrict__ kv, const bf16* __restrict__ mask,
+                                                                      float* __restrict__ out, int S, int N, float scaling) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int WARPS = GA_THREADS / 32;
+  __shared__ float s_sum[WARPS][GC_HC + 1];
+  __shared__ float s_mean[GC_HC], s_q[GC_HC];
+  __shared__ float s_warp[WARPS][GC_H][GC_REC];
+  const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // masked sum of the normalised rows (rounded to bf16, as a LayerNorm kernel stores them): eight lanes a row, four rows a warp
+  {
+    const int li = lane & 7;
+    float g[8], b[8], acc[8], cnt = 0.f;
+    auto unpack = [](uint4 u, float (&v)[8]) {
+      const bf162* h = reinterpret_cast<const bf162*>(&u);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(h[i]);
+        v[2 * i] = f.x;
+        v[2 * i + 1] = f.y;
+      }
+    };
+    unpack(*reinterpret_cast<const uint4*>(gamma + li * 8), g);
+    unpack(*reinterpret_cast<const uint4*>(beta + li * 8), b);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+    constexpr int U = 4;
+    for (int s0 = warp * 4; s0 < S; s0 += U * WARPS * 4) {      // all lanes of a warp together (shuffles below)
+      uint4 raw[U];
+      float mk[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int s = s0 + (lane >> 3) + u * WARPS * 4;
+        const bool in = s < S;
+        raw[u] = in ? *reinterpret_cast<const uint4*>(x + ((long long)s * N + n) * GC_HC + li * 8) : make_uint4(0, 0, 0, 0);
+        mk[u] = in ? __bfloat162float(mask[(long long)s * N + n]) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float v[8], t = 0.f, q = 0.f;
+        unpack(raw[u], v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t += v[i];
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        const float mean = t * (1.f / GC_HC);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          v[i] -= mean;
+          q = fmaf(v[i], v[i], q);
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+        const float rstd = rsqrtf(q * (1.f / GC_HC) + eps);
+        cnt += mk[u];
+        if (s0 + (lane >> 3) + u * WARPS * 4 < S) {             // an unnormalisable masked row counts as it would in a product with its mask
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i] = fmaf(mk[u], __bfloat162float(__float2bfloat16(v[i] * rstd * g[i] + b[i])), acc[i]);
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {
+      cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+    }
+    if (lane < 8) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s_sum[warp][li * 8 + i] = acc[i];
+      if (lane == 0) s_sum[warp][GC_HC] = cnt;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < GC_HC) {
+    float t = 0.f, c = 0.f;
+    for (int w = 0; w < WARPS; ++w) {
+      t += s_sum[w][threadIdx.x];
+      c += s_sum[w][GC_HC];
+    }
+    s_mean[threadIdx.x] = t / (c + 1e-10f);
+  }
+  __syncthreads();
+  if (threadIdx.x < GC_HC) {
+    float d = 0.f;
+    for (int c = 0; c < GC_HC; ++c) d = fmaf(s_mean[c], __bfloat162float(wq[threadIdx.x * GC_HC + c]), d);
+    s_q[threadIdx.x] = d * scaling;
+  }
+  __syncthreads();
+  // softmax over the sequences, as in the kernel below: two threads per key, four heads each
+  GcState st;
+  gc_init(st);
+  const int hg = threadIdx.x & 1;
+  for (int s = threadIdx.x >> 1; s < S; s += GA_THREADS / 2) {
+    const bf16* at = kv + ((long long)s * N + n) * 2 * GC_C;
+    gc_key(st, *reinterpret_cast<const uint4*>(at), *reinterpret_cast<const uint4*>(at + GC_C), __bfloat162float(mask[(long long)s * N + n]) == 0.f,
+           s_q + hg * (GC_H / 2) * GC_C);
+  }
+  gc_fold_warp(st, lane, hg, s_warp[warp]);
+  __syncthreads();
+  if (threadIdx.x < GC_HC) {
+    const int h = threadIdx.x / GC_C, i = threadIdx.x - h * GC_C;
+    float mx, lt, at;
+    gc_fold_warps(s_warp, h, i, mx, lt, at);
+    out[(long long)n * GC_HC + threadIdx.x] = lt > 0.f ? at / lt : 0.f;
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // Cluster version for the model's shape (H = 8 heads of C = 8 channels).  The CTAs of a thread-block cluster share one
 // column: each runs the online softmax over ITS slice of the sequences with two threads per key (four heads each; the
 // version above converts k and v once per head), the partial (max, sum, weighted values) of
 // every CTA are merged through distributed shared memory, and each CTA gates its slice.  No part of the column is read
 // twice and nothing but the result reaches global memory.
-constexpr int GC_H = 8, GC_C = 8, GC_HC = GC_H * GC_C;
-constexpr int GC_REC = 2 + GC_C;          // per head: max, sum, C weighted values
 
 __global__ void __launch_bounds__(GA_THREADS, 2) global_attention_cluster_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv,
                                                                                  const bf16* __restrict__ mask, const bf16* __restrict__ gate,
@@ -204,87 +401,23 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_attention_cluster_kernel
   const int s_lo = part * s_per, s_hi = min(S, s_lo + s_per);
   // two threads per key, four heads each: k and v are converted twice instead of eight times, and the running state
   // (4 x (max, sum, 8 values)) fits the registers of two CTAs per SM
-  constexpr int HG = GC_H / 2;
+  GcState st;
+  gc_init(st);
   const int hg = threadIdx.x & 1;
-  float m[HG], l[HG], acc[HG][GC_C];
-#pragma unroll
-  for (int h = 0; h < HG; ++h) {
-    m[h] = -INFINITY;
-    l[h] = 0.f;
-#pragma unroll
-    for (int i = 0; i < GC_C; ++i) acc[h][i] = 0.f;
-  }
   const bf16* kvr = kv + r * (long long)S * 2 * GC_C;
   const bf16* mr = mask + r * (long long)S;
   for (int s = s_lo + (threadIdx.x >> 1); s < s_hi; s += GA_THREADS / 2) {
-    const uint4 kraw = *reinterpret_cast<const uint4*>(kvr + (long long)s * 2 * GC_C);
-    const uint4 vraw = *reinterpret_cast<const uint4*>(kvr + (long long)s * 2 * GC_C + GC_C);
-    const bool masked = __bfloat162float(mr[s]) == 0.f;
-    float kf[GC_C], vf[GC_C];
-    {
-      const bf162* kh = reinterpret_cast<const bf162*>(&kraw);
-      const bf162* vh = reinterpret_cast<const bf162*>(&vraw);
-#pragma unroll
-      for (int i = 0; i < GC_C / 2; ++i) {
-        const float2 a = __bfloat1622float2(kh[i]), b = __bfloat1622float2(vh[i]);
-        kf[2 * i] = a.x; kf[2 * i + 1] = a.y;
-        vf[2 * i] = b.x; vf[2 * i + 1] = b.y;
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < HG; ++h) {
-      float d = 0.f;
-#pragma unroll
-      for (int i = 0; i < GC_C; ++i) d = fmaf(s_q[(hg * HG + h) * GC_C + i], kf[i], d);
-      if (masked) d = GA_MASKED;
-      if (d > m[h]) {                         // the running maximum settles after a few keys: the rescale is rare
-        const float a = __expf(m[h] - d);     // m = -inf on the first key: a = 0
-        l[h] *= a;
-#pragma unroll
-        for (int i = 0; i < GC_C; ++i) acc[h][i] *= a;
-        m[h] = d;
-      }
-      const float pw = __expf(d - m[h]);
-      l[h] += pw;
-#pragma unroll
-      for (int i = 0; i < GC_C; ++i) acc[h][i] = fmaf(pw, vf[i], acc[h][i]);
-    }
+    const bf16* at = kvr + (long long)s * 2 * GC_C;
+    gc_key(st, *reinterpret_cast<const uint4*>(at), *reinterpret_cast<const uint4*>(at + GC_C), __bfloat162float(mr[s]) == 0.f,
+           s_q + hg * (GC_H / 2) * GC_C);
   }
-  // warp level, over the 16 lanes of each head group (even / odd lanes): common maximum, rescaled sums
-#pragma unroll
-  for (int h = 0; h < HG; ++h) {
-    float wm = m[h];
-#pragma unroll
-    for (int o = 16; o > 1; o >>= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-    const float sc = (m[h] == -INFINITY) ? 0.f : __expf(m[h] - wm);
-    float v = l[h] * sc;
-#pragma unroll
-    for (int o = 16; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane < 2) {
-      s_warp[warp][hg * HG + h][0] = wm;
-      s_warp[warp][hg * HG + h][1] = v;
-    }
-#pragma unroll
-    for (int i = 0; i < GC_C; ++i) {
-      float a = acc[h][i] * sc;
-#pragma unroll
-      for (int o = 16; o > 1; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (lane < 2) s_warp[warp][hg * HG + h][2 + i] = a;
-    }
-  }
+  gc_fold_warp(st, lane, hg, s_warp[warp]);
   __syncthreads();
   // CTA level: thread (h, i) folds the eight warps
   if (threadIdx.x < GC_HC) {
     const int h = threadIdx.x / GC_C, i = threadIdx.x - h * GC_C;
-    float mx = -INFINITY;
-    for (int w = 0; w < GA_THREADS / 32; ++w) mx = fmaxf(mx, s_warp[w][h][0]);
-    float lt = 0.f, at = 0.f;
-    for (int w = 0; w < GA_THREADS / 32; ++w) {
-      const float mw = s_warp[w][h][0];
-      const float sc = (mw == -INFINITY) ? 0.f : __expf(mw - mx);
-      lt = fmaf(s_warp[w][h][1], sc, lt);
-      at = fmaf(s_warp[w][h][2 + i], sc, at);
-    }
+    float mx, lt, at;
+    gc_fold_warps(s_warp, h, i, mx, lt, at);
     if (i == 0) {
       s_part[h][0] = mx;
       s_part[h][1] = lt;
@@ -522,6 +655,15 @@ __global__ void __launch_bounds__(GA_THREADS) global_attention_bwd_kernel(const 
 }
 
 }  // namespace ffb
+
+extern "C" int ffb_global_column(const void* x, const void* gamma, const void* beta, float eps, const void* wq, const void* kv, const void* mask,
+                                 float* out, long long S, long long N, float scaling, void* stream) {
+  using namespace ffb;
+  if (S < 1 || N < 1 || S > 0x7fffffffLL || N > 0x7fffffffLL) return -1;
+  launch_light(global_column_kernel, (unsigned)N, GA_THREADS, 0, reinterpret_cast<cudaStream_t>(stream), (const bf16*)x, (const bf16*)gamma,
+               (const bf16*)beta, eps, (const bf16*)wq, (const bf16*)kv, (const bf16*)mask, out, (int)S, (int)N, scaling);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
 
 extern "C" {
 

@@ -13,6 +13,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include "gemm_api.h"
+#include "ln_gemm_api.h"
 
 extern "C" {
 int ffb_gemm_bf16(const void* A, const void* B, int a_mn, int b_mn, long long lda, long long ldb, long long a_bstride, long long b_bstride,
@@ -41,6 +42,9 @@ int ffb_glu_mask_t_fwd(const void* pre, const void* mask, void* out, int C2, lon
 int ffb_glu_mask_t_bwd(const void* dout, const void* pre, const void* mask, void* dpre, int C2, long long R, void* stream);
 int ffb_act_bwd(const void* dy, const void* y, void* dx, long long rows, int C, int mode, void* stream);
 int ffb_colsum(const void* x, float* out, long long rows, int C, void* stream);
+int ffb_ln_gemm(const LnGemmArgs* p, void* stream);
+int ffb_global_column(const void* x, const void* gamma, const void* beta, float eps, const void* wq, const void* kv, const void* mask, float* out,
+                      long long S, long long N, float scaling, void* stream);
 }
 
 namespace {
@@ -357,6 +361,221 @@ Tensor colsum(const Tensor& x, OptTensor out) {
   return *out;
 }
 
+// ---- LayerNorm + GEMM kernels (ln_gemm.cu) ----
+// Rows [.., C] as [batch][rows][C]; weights, norm parameters and biases contiguous bf16 (the callers in ops/ln_gemm.py see to it).
+struct Rows {
+  int64_t batch, rows, rstride, bstride;
+};
+Rows rows3(const Tensor& t) {
+  expect(t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1 && (t.dim() == 2 || t.dim() == 3), "rows of adjacent bf16 channels");
+  if (t.dim() == 2) return {1, t.size(0), t.stride(0), 0};
+  return {t.size(0), t.size(1), t.stride(1), t.size(0) > 1 ? t.stride(0) : 0};
+}
+LnGemmArgs ln_args(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, int mode) {
+  LnGemmArgs g = {};
+  const Rows r = rows3(x);
+  g.x = ptr(x);
+  g.C = (int)x.size(-1);
+  g.rows = r.rows;
+  g.batch = r.batch;
+  g.x_rstride = r.rstride;
+  g.x_bstride = r.bstride;
+  expect(gamma.numel() == g.C && beta.numel() == g.C, "norm parameters");
+  g.gamma = ptr(gamma);
+  g.beta = ptr(beta);
+  g.eps = (float)eps;
+  g.mode = mode;
+  return g;
+}
+void ln_run(const LnGemmArgs& g, const char* what) {
+  if (g.rows * g.batch == 0) return;
+  check(ffb_ln_gemm(&g, stream()), what);
+}
+void same_rows(const Rows& a, const LnGemmArgs& g) { expect(a.batch == g.batch && a.rows == g.rows, "operands with other rows than the input"); }
+void same_shape(const Tensor& t, const LnGemmArgs& g, int64_t n) {
+  same_rows(rows3(t), g);
+  expect(t.size(-1) == n, "operands with other columns than the result");
+}
+
+// resid + b2 + f(LN(x) w1^T + b1) w2^T; f = relu, or sigmoid(.) * mul (fp32 `mul`: one row of factors for every mul.size(0)-th row)
+Tensor ln_chain(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& w1, const OptTensor& b1, const Tensor& w2,
+                const OptTensor& b2, const OptTensor& mul, const Tensor& resid, OptTensor out) {
+  LnGemmArgs g = ln_args(x, gamma, beta, eps, mul ? LN_GATE_CHAIN : LN_RELU_CHAIN);
+  g.hidden = (int)w1.size(0);
+  expect(w1.size(1) == g.C && w2.size(0) == g.C && w2.size(1) == g.hidden && (!b1 || b1->numel() == g.hidden) && (!b2 || b2->numel() == g.C), "weights");
+  g.w1 = ptr(w1);
+  g.b1 = ptr(b1);
+  g.w2 = ptr(w2);
+  g.b2 = ptr(b2);
+  if (mul && mul->scalar_type() == at::kFloat) {
+    expect(mul->dim() == 2 && mul->is_contiguous() && mul->size(1) == g.hidden && mul->size(0) > 0, "gated operand");
+    g.mul_f32 = static_cast<const float*>(ptr(mul));
+    g.mul_mod = (int)mul->size(0);
+  } else if (mul) {
+    const Rows r = rows3(*mul);
+    same_shape(*mul, g, g.hidden);
+    g.mul = ptr(mul);
+    g.m_rstride = r.rstride;
+    g.m_bstride = r.bstride;
+  }
+  const Rows r = rows3(resid);
+  same_shape(resid, g, g.C);
+  g.resid = ptr(resid);
+  g.r_rstride = r.rstride;
+  g.r_bstride = r.bstride;
+  Tensor y = out ? *out : at::empty(resid.sizes(), resid.options());
+  const Rows o = rows3(y);
+  same_shape(y, g, g.C);
+  g.out = ptr(y);
+  g.o_rstride = o.rstride;
+  g.o_bstride = o.bstride;
+  ln_run(g, "ln_chain");
+  return y;
+}
+
+LnSegment ln_rows(const LnGemmArgs& g, const Tensor& w, const OptTensor& bias, int act, bool scaled, const Tensor& out) {
+  const Rows o = rows3(out);
+  expect(w.size(1) == g.C && (!bias || bias->numel() == w.size(0)), "weights");
+  same_shape(out, g, w.size(0));
+  LnSegment s = {};
+  s.w = ptr(w);
+  s.bias = ptr(bias);
+  s.n = (int)w.size(0);
+  s.kind = LN_ROWS;
+  s.act = act;
+  s.scaled = scaled;
+  s.out = ptr(out);
+  s.o_rstride = o.rstride;
+  s.o_bstride = o.bstride;
+  return s;
+}
+Tensor like_rows(const Tensor& x, int64_t n) {
+  auto shape = x.sizes().vec();
+  shape.back() = n;
+  return at::empty(shape, x.options());
+}
+
+// LN(x) w^T of rows [.., C], and / or the pair bias LN(x) wb^T of a pair tensor's rows (i j): bias [H, q, k] with q = i and k = j,
+// or q = j and k = i (`transposed`), into `bias`, whose last two axes may have any pitch
+OptTensor ln_qkv(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, const OptTensor& w, const OptTensor& wb, const OptTensor& bias,
+                 bool transposed) {
+  LnGemmArgs g = ln_args(x, gamma, beta, eps, LN_PROJECT);
+  OptTensor y;
+  if (w) {
+    y = like_rows(x, w->size(0));
+    g.seg[g.nseg++] = ln_rows(g, *w, std::nullopt, ACT_NONE, false, *y);
+  }
+  if (wb) {
+    expect(bias && bias->dim() == 3 && wb->size(1) == g.C, "pair bias");
+    const int64_t ni = bias->size(transposed ? 2 : 1), nj = bias->size(transposed ? 1 : 2);
+    expect(bias->scalar_type() == at::kBFloat16 && bias->size(0) == wb->size(0) && ni * nj == g.rows * g.batch, "pair bias");
+    LnSegment& s = g.seg[g.nseg++];
+    s.w = ptr(wb);
+    s.n = (int)wb->size(0);
+    s.kind = LN_PAIR_BIAS;
+    s.out = ptr(bias);
+    g.pb_n = (int)nj;
+    g.pb_h = bias->stride(0);
+    g.pb_i = bias->stride(transposed ? 2 : 1);
+    g.pb_j = bias->stride(transposed ? 1 : 2);
+  }
+  ln_run(g, "ln_qkv");
+  return y;
+}
+
+// Value vectors [N, 64] (fp32) of the global column attention over x [S, N, 64] with keys and values kv [S * N, 16]
+Tensor global_column(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& wq, const Tensor& kv, Tensor mask, double scaling) {
+  const int64_t S = x.size(0), N = x.size(1);
+  mask = mask.to(at::kBFloat16).contiguous();
+  expect(x.dim() == 3 && x.is_contiguous() && x.size(2) == 64 && gamma.numel() == 64 && beta.numel() == 64 && wq.is_contiguous() && wq.size(0) == 64 &&
+             wq.size(1) == 64 && kv.is_contiguous() && kv.numel() == S * N * 16 && mask.numel() == S * N,
+         "global column attention");
+  const Tensor out = f32({N, 64}, x);
+  if (x.numel() == 0) return out;
+  check(ffb_global_column(ptr(x), ptr(gamma), ptr(beta), (float)eps, ptr(wq), ptr(kv), ptr(mask), static_cast<float*>(ptr(out)), S, N, (float)scaling,
+                          stream()),
+        "global_column");
+  return out;
+}
+
+void ln_scale(LnGemmArgs& g, Tensor& scale) {
+  g.rs_bf16 = scale.scalar_type() == at::kBFloat16;
+  scale = (g.rs_bf16 ? scale : scale.to(at::kFloat)).contiguous();
+  expect(scale.numel() >= g.rows * g.batch, "fewer row factors than rows");
+  g.rowscale = ptr(scale);
+}
+
+// Operands of the triangle multiplication: the gated projections, channels first, into lr [2c, batch, rows] (any pitch), times one
+// factor per row; returns the output gate sigmoid(LN(x) wg^T + bg)
+Tensor ln_tri_in(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& w, const Tensor& b, const Tensor& wg,
+                 const Tensor& bg, Tensor scale, const Tensor& lr) {
+  LnGemmArgs g = ln_args(x, gamma, beta, eps, LN_PROJECT);
+  ln_scale(g, scale);
+  expect(lr.dim() == 3 && lr.scalar_type() == at::kBFloat16 && lr.size(0) * 2 == w.size(0) && lr.size(1) == g.batch && lr.size(2) == g.rows &&
+             lr.stride(2) == 1 && w.size(1) == g.C && b.numel() == w.size(0),
+         "gated operands");
+  LnSegment& s = g.seg[0];
+  s.w = ptr(w);
+  s.bias = ptr(b);
+  s.n = (int)w.size(0);
+  s.kind = LN_GLU_T;
+  s.scaled = 1;
+  s.out = ptr(lr);
+  s.o_rstride = lr.stride(0);
+  s.o_bstride = g.batch > 1 ? lr.stride(1) : 0;
+  const Tensor y = like_rows(x, wg.size(0));
+  g.seg[1] = ln_rows(g, wg, bg, ACT_SIGMOID, false, y);
+  g.nseg = 2;
+  ln_run(g, "ln_tri_in");
+  return y;
+}
+
+// Output of the triangle multiplication: resid + mul * (LN(p) w^T + b) of a channels-first p [c, batch, rows] (any pitch)
+Tensor ln_tri_out(const Tensor& p, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& w, const Tensor& b, const Tensor& mul,
+                  const Tensor& resid, OptTensor out) {
+  LnGemmArgs g = {};
+  expect(p.scalar_type() == at::kBFloat16 && p.dim() == 3 && p.stride(2) == 1, "channels-first operand");
+  g.x = ptr(p);
+  g.channels_first = 1;
+  g.C = (int)p.size(0);
+  g.batch = p.size(1);
+  g.rows = p.size(2);
+  g.x_rstride = p.stride(0);
+  g.x_bstride = g.batch > 1 ? p.stride(1) : 0;
+  expect(gamma.numel() == g.C && beta.numel() == g.C, "norm parameters");
+  g.gamma = ptr(gamma);
+  g.beta = ptr(beta);
+  g.eps = (float)eps;
+  g.mode = LN_PROJECT;
+  const Rows m = rows3(mul), r = rows3(resid);
+  same_shape(mul, g, w.size(0));
+  same_shape(resid, g, w.size(0));
+  g.mul = ptr(mul);
+  g.m_rstride = m.rstride;
+  g.m_bstride = m.bstride;
+  g.resid = ptr(resid);
+  g.r_rstride = r.rstride;
+  g.r_bstride = r.bstride;
+  Tensor y = out ? *out : at::empty(resid.sizes(), resid.options());
+  g.seg[0] = ln_rows(g, w, b, ACT_NONE, false, y);
+  g.nseg = 1;
+  ln_run(g, "ln_tri_out");
+  return y;
+}
+
+// (LN(x) wa^T + ba) * scale and (LN(x) wb^T + bb) * scale
+std::tuple<Tensor, Tensor> ln_pair(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& wa, const OptTensor& ba,
+                                   const Tensor& wb, const OptTensor& bb, Tensor scale) {
+  LnGemmArgs g = ln_args(x, gamma, beta, eps, LN_PROJECT);
+  ln_scale(g, scale);
+  const Tensor ya = like_rows(x, wa.size(0)), yb = like_rows(x, wb.size(0));
+  g.seg[0] = ln_rows(g, wa, ba, ACT_NONE, true, ya);
+  g.seg[1] = ln_rows(g, wb, bb, ACT_NONE, true, yb);
+  g.nseg = 2;
+  ln_run(g, "ln_pair");
+  return {ya, yb};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_ffb_dispatch, m) {
@@ -376,5 +595,11 @@ PYBIND11_MODULE(_ffb_dispatch, m) {
   m.def("glu_mask_t_bwd", &glu_mask_t_bwd);
   m.def("act_bwd", &act_bwd);
   m.def("colsum", &colsum);
+  m.def("ln_chain", &ln_chain);
+  m.def("ln_qkv", &ln_qkv);
+  m.def("ln_tri_in", &ln_tri_in);
+  m.def("ln_tri_out", &ln_tri_out);
+  m.def("ln_pair", &ln_pair);
+  m.def("global_column", &global_column);
   m.def("launches", []() { return g_launches; });
 }

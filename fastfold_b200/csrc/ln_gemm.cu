@@ -1,0 +1,848 @@
+// LayerNorm of the rows of an activation and the small GEMMs that follow it, in one kernel:
+//
+//   chains       out = resid + b2 + f(LN(x) W1^T + b1) W2^T      f = relu (transition) or sigmoid(.) * o (gated attention output)
+//   projections  y_s = act(LN(x) W_s^T + b_s) ...                up to three weights that read the same rows (QKV and pair bias;
+//                                                                gated operands and output gate of the triangle multiplication)
+//
+// The modules of the trunk are made of these: a LayerNorm over 64, 128 or 256 channels and one or two products with weights of a
+// few hundred kilobytes.  As single kernels each wrote its result to memory and the next one read it back, the hidden
+// activation of a transition (four times its input) among them, and on short inputs each was a launch.  Here a tile of 128 rows is
+// read once; its normalised form (rounded to bf16, as the LayerNorm kernel stores it) and the hidden activation never leave the SM.
+//
+// Persistent, one CTA per SM, 448 threads, tiles of 128 rows:
+//   warps 0-3    LayerNorm, a thread per row (channels-first input: per pair of rows and half of the channels), in place in the
+//                shared-memory tile that becomes the A operand.  The 128-byte swizzle makes a thread's 16-byte accesses to its own row
+//                free of conflicts, so no shuffles are needed
+//   warps 4-11   epilogues, two warps per tensor-memory quadrant, 64 columns each
+//   warp 12      TMA: rows of the next tile, weights through a ring of 16 KB boxes (128 rows x 64 columns; out of L2 for all but the
+//                first CTA)
+//   warp 13      MMA issue, 128 x 128 x 16
+// Weights come in chunks of 128 rows.  Of a chain, chunk h of the hidden activation goes through tensor memory: the epilogue
+// reads the accumulator, applies f and writes bf16 pairs over it, and the second product takes them from there as its A operand.
+// The products of chunk h + 1 are issued before the second product of chunk h, which hides the epilogue.
+//
+// What bounds it: the weights, which every tile of 128 rows streams from L2 again (1 MB a tile for the transition of 256 channels, which
+// runs at 0.44 of the tensor cores' rate), the output bytes of the wide projections, and below some 20 tiles the chain of a single tile.
+//   Measured (B200, against LayerNorm and GEMM kernels in the same order, us): transition 262144 x 64 89 -> 46, 65536 x 128
+//   47 -> 32, 589824 x 128 341 -> 208, 32768 x 256 54 -> 48, 2048 x 256 16 -> 26 (three launches fewer by two: the host side gains more
+//   than that); gated output with the norm (left side without it) 589824 x 128 192 -> 139, 32768 x 256 30 -> 24; QKV 589824 x 128
+//   181 -> 130; operands and gate of the triangle multiplication at 1024 residues 539 -> 480, its output 293 -> 177.
+//
+// Stands for the nn.LayerNorm / nn.Linear / elementwise chains of the reference (fastfold/model/fastnn/ops.py:85-106, 143-160,
+// 275-324, 393-404).
+#include "common.cuh"
+#include "gemm_api.h"
+#include "ln_gemm_api.h"
+#include "tmap.h"
+
+namespace ffb {
+
+constexpr int LG_THREADS = 448;
+constexpr int LG_EPI = 8;                 // epilogue warps
+constexpr int LG_BOX = 16384;             // weight box: 128 rows x 64 columns
+constexpr int LG_MAX_N = 1280;            // columns of all weights (biases in shared memory)
+
+struct LgMaps {
+  CUtensorMap x, w[3], mul, resid, out[3];
+};
+
+struct LgSeg {
+  int kind, act, scaled, n;
+  bf16* out;
+};
+
+struct LgArgs {
+  int rows, batch, tiles_m, num_tiles;
+  int bpt;                                // batches per tile: 128 / rows where that is 2 or 4, else 1
+  const bf16 *gamma, *beta;
+  float eps;
+  int hidden, has_mul;
+  const float* mul_f32;
+  int mul_mod;
+  const bf16 *b1, *b2;
+  int nseg, chunks;                       // projections: segments, chunks of 128 weight rows in all
+  LgSeg seg[3];
+  const bf16* seg_bias[3];
+  const void* rowscale;
+  int rs_bf16;
+  long long pb_h, pb_i, pb_j;
+  int pb_n;
+};
+
+template <int C, int MODE>
+struct LgCfg {
+  static constexpr int KB = C / 64;
+  static constexpr int A_BYTES = KB * 16384;
+  static constexpr int TILES = C == 256 ? 1 : 2;                     // 4 KB staging tiles per epilogue warp
+  static constexpr int NA = C == 256 ? 1 : 2;                        // tiles of rows: one less, and the ring holds four boxes more
+  static constexpr int RING = C == 256 ? 7 : 5;
+  static constexpr int NB2 = C < 128 ? C : 128;                      // columns of one second product
+  static constexpr int NACC = MODE == LN_PROJECT ? 4 : (C == 256 ? 2 : 3);      // 128-column accumulators of the first product
+  static constexpr int ACC2 = NACC * 128;                            // tensor-memory column of the second product's accumulator
+  static constexpr int A0 = 0, W0 = NA * A_BYTES, STG = W0 + RING * LG_BOX, VEC = STG + LG_EPI * TILES * 4096;
+  static constexpr int VEC_FLOATS = 2 * C + LG_MAX_N + 256 + (MODE == LN_PROJECT ? 512 : 0);     // gamma, beta, biases, channel sums
+  static constexpr int BARS = VEC + VEC_FLOATS * 4;
+  static constexpr int SMEM = BARS + 512 + 1024;
+  static_assert(SMEM <= 232448, "shared memory");
+};
+
+__device__ __forceinline__ void lg_unpack(uint4 u, float (&v)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ uint32_t lg_pack2(float a, float b) {
+  const bf162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ uint4 lg_pack(const float* v) { return make_uint4(lg_pack2(v[0], v[1]), lg_pack2(v[2], v[3]), lg_pack2(v[4], v[5]), lg_pack2(v[6], v[7])); }
+
+// Two floats in one 64-bit register pair: the FMA pipe does both in one instruction.
+__device__ __forceinline__ uint64_t lg_pair(float a, float b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t lg_bf2(uint32_t w) { return lg_pair(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ float2 lg_split(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t lg_add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t lg_mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t lg_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint32_t lg_pack2v(uint64_t v) {
+  const float2 f = lg_split(v);
+  return lg_pack2(f.x, f.y);
+}
+
+// One row of a [kb][128 rows][64] swizzled tile, in place.  A warp per scheduler does this, so what counts are its instructions and
+// the independent ones among them: two-wide arithmetic and four partial sums.  64 channels stay in registers (packed) between the
+// mean, the variance and the result; with more they would be spilled, and the three sweeps read shared memory.
+template <int C>
+__device__ __forceinline__ void lg_norm_row(uint8_t* tile, int row, const float* gamma, const float* beta, float eps) {
+  constexpr int KB = C / 64;
+  constexpr bool KEEP = C <= 64;
+  uint8_t* p = tile + row * 128;
+  const int x = row & 7;
+  uint4 raw[8];
+  auto load = [&](int kb) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) raw[u] = *reinterpret_cast<const uint4*>(p + kb * 16384 + ((u ^ x) << 4));
+  };
+  // keeps the compiler from holding the unpacked row (twice the registers) from one sweep to the next
+  auto sweep = [&]() {
+    if (KEEP) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) asm volatile("" : "+r"(raw[i].x), "+r"(raw[i].y), "+r"(raw[i].z), "+r"(raw[i].w));
+    } else {
+      asm volatile("" ::: "memory");
+    }
+  };
+  uint64_t s[4], q[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) s[i] = q[i] = lg_pair(0.f, 0.f);
+#pragma unroll 1
+  for (int kb = 0; kb < KB; ++kb) {
+    load(kb);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      s[0] = lg_add2(s[0], lg_bf2(raw[u].x));
+      s[1] = lg_add2(s[1], lg_bf2(raw[u].y));
+      s[2] = lg_add2(s[2], lg_bf2(raw[u].z));
+      s[3] = lg_add2(s[3], lg_bf2(raw[u].w));
+    }
+  }
+  const float2 st = lg_split(lg_add2(lg_add2(s[0], s[1]), lg_add2(s[2], s[3])));
+  const float mean = (st.x + st.y) * (1.f / C);
+  const uint64_t m2 = lg_pair(-mean, -mean);
+  sweep();
+#pragma unroll 1
+  for (int kb = 0; kb < KB; ++kb) {
+    if (!KEEP) load(kb);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t e[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint64_t d = lg_add2(lg_bf2(e[i]), m2);
+        q[i] = lg_fma2(d, d, q[i]);
+      }
+    }
+  }
+  const float2 qt = lg_split(lg_add2(lg_add2(q[0], q[1]), lg_add2(q[2], q[3])));
+  const float rstd = rsqrtf((qt.x + qt.y) * (1.f / C) + eps);
+  const uint64_t r2 = lg_pair(rstd, rstd);
+  sweep();
+#pragma unroll 1
+  for (int kb = 0; kb < KB; ++kb) {
+    if (!KEEP) load(kb);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const ulonglong2* g = reinterpret_cast<const ulonglong2*>(gamma + kb * 64 + u * 8);       // the same in every lane
+      const ulonglong2* b = reinterpret_cast<const ulonglong2*>(beta + kb * 64 + u * 8);
+      const ulonglong2 g0 = g[0], g1 = g[1], b0 = b[0], b1 = b[1];
+      uint4 o;
+      o.x = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[u].x), m2), r2), g0.x, b0.x));
+      o.y = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[u].y), m2), r2), g0.y, b0.y));
+      o.z = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[u].z), m2), r2), g1.x, b1.x));
+      o.w = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[u].w), m2), r2), g1.y, b1.y));
+      *reinterpret_cast<uint4*>(p + kb * 16384 + ((u ^ x) << 4)) = o;
+    }
+  }
+}
+
+// Channels-first tile [kb][2 chunks of 64 rows][64 channels][64 rows], in place: thread t holds rows 2 (t % 64) and the next for
+// the 64 channels of block t / 64; the two threads of a pair of rows add their sums through `part` ([2][128] float2).
+__device__ __forceinline__ void lg_norm_columns(uint8_t* tile, int t, float2* part, const float* gamma, const float* beta, float eps) {
+  const int pr = t & 63, kb = t >> 6;
+  uint8_t* p = tile + kb * 16384 + (pr >> 5) * 8192 + ((pr & 3) << 2);
+  const int u = (pr & 31) >> 2;
+  uint64_t s[4];
+  auto sweep = [&](auto&& each) {         // 16 channels at a time
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[i] = lg_pair(0.f, 0.f);
+#pragma unroll 1
+    for (int k0 = 0; k0 < 64; k0 += 16) {
+      uint32_t raw[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) raw[k] = *reinterpret_cast<const uint32_t*>(p + (k0 + k) * 128 + ((u ^ (k & 7)) << 4));
+      each(k0, raw);
+    }
+  };
+  auto total = [&]() { return lg_split(lg_add2(lg_add2(s[0], s[1]), lg_add2(s[2], s[3]))); };
+  sweep([&](int, const uint32_t (&raw)[16]) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) s[k & 3] = lg_add2(s[k & 3], lg_bf2(raw[k]));
+  });
+  const float2 ms = total();
+  part[t] = ms;
+  asm volatile("bar.sync 2, 128;" ::: "memory");
+  const float2 os = part[t ^ 64];
+  const uint64_t m2 = lg_pair(-(ms.x + os.x) * (1.f / 128), -(ms.y + os.y) * (1.f / 128));
+  sweep([&](int, const uint32_t (&raw)[16]) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const uint64_t d = lg_add2(lg_bf2(raw[k]), m2);
+      s[k & 3] = lg_fma2(d, d, s[k & 3]);
+    }
+  });
+  const float2 mq = total();
+  part[128 + t] = mq;
+  asm volatile("bar.sync 2, 128;" ::: "memory");
+  const float2 oq = part[128 + (t ^ 64)];
+  const uint64_t r2 = lg_pair(rsqrtf((mq.x + oq.x) * (1.f / 128) + eps), rsqrtf((mq.y + oq.y) * (1.f / 128) + eps));
+  sweep([&](int k0, const uint32_t (&raw)[16]) {
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) {
+      const float4 g = *reinterpret_cast<const float4*>(gamma + kb * 64 + k0 + k), b = *reinterpret_cast<const float4*>(beta + kb * 64 + k0 + k);
+      const float gv[4] = {g.x, g.y, g.z, g.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint64_t y = lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[k + i]), m2), r2), lg_pair(gv[i], gv[i]), lg_pair(bv[i], bv[i]));
+        *reinterpret_cast<uint32_t*>(p + (k0 + k + i) * 128 + ((u ^ ((k + i) & 7)) << 4)) = lg_pack2v(y);
+      }
+    }
+  });
+}
+
+__device__ __forceinline__ void lg_store_tile(const CUtensorMap* map, uint32_t smem, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(smem), "r"(x), "r"(y), "r"(z) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
+template <int C, int MODE, bool CF>
+__global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_constant__ LgMaps maps, const __grid_constant__ LgArgs a) {
+  pdl_launch_dependents();
+  using Cfg = LgCfg<C, MODE>;
+  constexpr int KB = Cfg::KB, RING = Cfg::RING, NACC = Cfg::NACC, NB2 = Cfg::NB2, NA = Cfg::NA;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
+  float* gamma = reinterpret_cast<float*>(sm + Cfg::VEC);
+  float* beta = gamma + C;
+  float* bias1 = beta + C;                  // [LG_MAX_N]
+  float* bias2 = bias1 + LG_MAX_N;          // [256]
+  float2* part = reinterpret_cast<float2*>(bias2 + 256);
+  const uint32_t b0 = base + Cfg::BARS;
+  const uint32_t x_full = b0, a_full = b0 + 16, a_empty = b0 + 32, acc_full = b0 + 48, acc_free = b0 + 80, h_full = b0 + 112;
+  const uint32_t acc2_full = b0 + 144, acc2_empty = b0 + 152, w_full = b0 + 160, w_empty = b0 + 216, ld_bar = b0 + 272;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + Cfg::BARS + 336);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(x_full + 8 * i, 1);
+      mbar_init(a_full + 8 * i, 4);
+      mbar_init(a_empty + 8 * i, 1);
+    }
+    for (int i = 0; i < NACC; ++i) {
+      mbar_init(acc_full + 8 * i, 1);
+      mbar_init(acc_free + 8 * i, MODE == LN_PROJECT ? LG_EPI : 1);
+      mbar_init(h_full + 8 * i, LG_EPI);
+    }
+    mbar_init(acc2_full, 1);
+    mbar_init(acc2_empty, LG_EPI);
+    for (int i = 0; i < RING; ++i) {
+      mbar_init(w_full + 8 * i, 1);
+      mbar_init(w_empty + 8 * i, 1);
+    }
+    for (int i = 0; i < LG_EPI; ++i) mbar_init(ld_bar + 8 * i, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    prefetch_tmap(&maps.x);
+    prefetch_tmap(&maps.w[0]);
+  }
+  if (warp == 0) {
+    __syncwarp();
+    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_relinquish();
+  }
+  pdl_wait();
+  // gamma, beta and all biases as fp32; read back as broadcasts
+  for (int i = threadIdx.x; i < C; i += LG_THREADS) {
+    gamma[i] = __bfloat162float(a.gamma[i]);
+    beta[i] = __bfloat162float(a.beta[i]);
+  }
+  if (MODE != LN_PROJECT) {
+    for (int i = threadIdx.x; i < ((a.hidden + 127) & ~127); i += LG_THREADS) bias1[i] = (a.b1 && i < a.hidden) ? __bfloat162float(a.b1[i]) : 0.f;
+    for (int i = threadIdx.x; i < C; i += LG_THREADS) bias2[i] = a.b2 ? __bfloat162float(a.b2[i]) : 0.f;
+  } else {
+    int off = 0;
+    for (int s = 0; s < a.nseg; ++s) {
+      const int n = a.seg[s].n, nc = (n + 127) & ~127;
+      for (int i = threadIdx.x; i < nc; i += LG_THREADS) bias1[off + i] = (a.seg_bias[s] && i < n) ? __bfloat162float(a.seg_bias[s][i]) : 0.f;
+      off += nc;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const int chunks = MODE == LN_PROJECT ? a.chunks : (a.hidden + 127) / 128;
+
+  if (warp < 4) {
+    // ---------------- LayerNorm ----------------
+    bool ok = true;
+    uint32_t t = 0;
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < a.num_tiles; tile += gridDim.x, ++t) {
+      const uint32_t s = t % NA;
+      ok = __all_sync(0xffffffffu, mbar_wait(x_full + 8 * s, (t / NA) & 1));
+      if (!ok) break;
+      uint8_t* At = sm + Cfg::A0 + s * Cfg::A_BYTES;
+      if (CF) lg_norm_columns(At, threadIdx.x, part, gamma, beta, a.eps);
+      else lg_norm_row<C>(At, threadIdx.x, gamma, beta, a.eps);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(a_full + 8 * s);
+    }
+    if (!ok && lane == 0) {
+      if (*abort_flag == 0) report(ST_TIMEOUT_TMA, 50);
+      *abort_flag = 1;
+    }
+  } else if (warp == 12) {
+    // ---------------- TMA: rows and weights ----------------
+    if (lane == 0) {
+      bool ok = true;
+      uint32_t wi = 0, t = 0;
+      auto load_x = [&](int tile, uint32_t n) {
+        const uint32_t s = n % NA, dst = base + Cfg::A0 + s * Cfg::A_BYTES, bar = x_full + 8 * s;
+        if (!mbar_wait(a_empty + 8 * s, ((n / NA) & 1) ^ 1)) {
+          ok = false;
+          return;
+        }
+        const int m0 = (tile % a.tiles_m) * 128, b = tile / a.tiles_m * a.bpt;
+        mbar_expect_tx(bar, Cfg::A_BYTES);
+#pragma unroll 1
+        for (int kb = 0; kb < KB; ++kb) {
+          if (CF) {
+            tma_load_3d(dst + kb * 16384, &maps.x, bar, m0, kb * 64, b);
+            tma_load_3d(dst + kb * 16384 + 8192, &maps.x, bar, m0 + 64, kb * 64, b);
+          } else {
+            tma_load_3d(dst + kb * 16384, &maps.x, bar, kb * 64, m0, b);
+          }
+        }
+      };
+      auto load_w = [&](const CUtensorMap* map, int x, int y, uint32_t bytes) {
+        const uint32_t s = wi % RING;
+        if (!ok) return;
+        ok = mbar_wait(w_empty + 8 * s, ((wi / RING) & 1) ^ 1);
+        if (!ok) return;
+        mbar_expect_tx(w_full + 8 * s, bytes);
+        tma_load_3d(base + Cfg::W0 + s * LG_BOX, map, w_full + 8 * s, x, y, 0);
+        ++wi;
+      };
+      load_x(blockIdx.x, 0);
+#pragma unroll 1
+      for (int tile = blockIdx.x; tile < a.num_tiles && ok; tile += gridDim.x, ++t) {
+        const bool more = tile + gridDim.x < a.num_tiles;       // with one tile of rows its place is free after the last first product
+        if (MODE == LN_PROJECT) {
+          int seg = 0, row = 0;
+#pragma unroll 1
+          for (int h = 0; h < chunks && ok; ++h) {
+#pragma unroll 1
+            for (int kb = 0; kb < KB; ++kb) load_w(&maps.w[seg], kb * 64, row, LG_BOX);
+            row += 128;
+            if (row >= a.seg[seg].n) {
+              ++seg;
+              row = 0;
+            }
+            if (h == (NA == 1 ? chunks - 1 : 0) && more) load_x(tile + gridDim.x, t + 1);
+          }
+        } else {
+#pragma unroll 1
+          for (int h = 0; h <= chunks && ok; ++h) {
+#pragma unroll 1
+            for (int kb = 0; kb < KB && h < chunks; ++kb) load_w(&maps.w[0], kb * 64, h * 128, LG_BOX);
+            if (h > 0) {
+#pragma unroll 1
+              for (int kk = 0; kk < 2; ++kk)
+#pragma unroll 1
+                for (int n = 0; n < C; n += NB2) load_w(&maps.w[1], (h - 1) * 128 + kk * 64, n, NB2 * 128);
+            }
+            if (h == (NA == 1 ? chunks : 0) && more) load_x(tile + gridDim.x, t + 1);
+          }
+        }
+      }
+      if (!ok) {
+        if (*abort_flag == 0) report(ST_TIMEOUT_MMA, 51);
+        *abort_flag = 1;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 13) {
+    // ---------------- MMA issue (the whole warp, see umma_bf16_by) ----------------
+    constexpr uint32_t idesc1 = make_idesc_bf16(128, 128, CF ? 1 : 0, 0), idesc2 = make_idesc_bf16(128, NB2, 0, 0);
+    const uint32_t lead = elect_one();
+    // descriptors of the first row tile and ring slot; the address field counts 16 bytes, so slots and steps are additions
+    const uint64_t ad0 = CF ? make_smem_desc(base + Cfg::A0, 8192, 1024) : make_smem_desc(base + Cfg::A0, 16, 1024);
+    const uint64_t wd0 = make_smem_desc(base + Cfg::W0, 16, 1024);
+    bool ok = true;
+    uint32_t ws = 0, wphase = 0, t = 0, c1 = 0, c2 = 0;          // ring slot and parity, tiles, chunks of the first and second products so far
+    auto await = [&](uint32_t bar, uint32_t parity, int code) {
+      if (!ok) return;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+      if (!ok && lead && *abort_flag == 0) report(code, 52);
+    };
+    auto box_done = [&]() {
+      umma_commit_by(lead, w_empty + 8 * ws);
+      if (++ws == RING) {
+        ws = 0;
+        wphase ^= 1;
+      }
+    };
+    auto first = [&](uint64_t ad) {                    // chunk of the first product
+      const uint32_t b = c1 % NACC;
+      await(acc_free + 8 * b, ((c1 / NACC) & 1) ^ 1, ST_TIMEOUT_EPI);
+#pragma unroll 1
+      for (int kb = 0; kb < KB && ok; ++kb) {
+        await(w_full + 8 * ws, wphase, ST_TIMEOUT_TMA);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t wd = wd0 + ws * (LG_BOX >> 4);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_bf16_by(lead, tmem + b * 128, ad + kb * (16384 >> 4) + k * ((CF ? 2048 : 32) >> 4), wd + k * (32 >> 4), idesc1, (kb > 0 || k > 0) ? 1u : 0u);
+        box_done();
+      }
+      if (ok) umma_commit_by(lead, acc_full + 8 * b);
+      ++c1;
+    };
+    auto second = [&](int h) {                         // chunk of the second product
+      const uint32_t b = c2 % NACC;
+      await(h_full + 8 * b, (c2 / NACC) & 1, ST_TIMEOUT_EPI);
+      if (h == 0) await(acc2_empty, (t & 1) ^ 1, ST_TIMEOUT_EPI);
+#pragma unroll 1
+      for (int kk = 0; kk < 2; ++kk)
+#pragma unroll 1
+        for (int n = 0; n < C && ok; n += NB2) {
+          await(w_full + 8 * ws, wphase, ST_TIMEOUT_TMA);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t wd = wd0 + ws * (LG_BOX >> 4);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)                  // columns 0-31 and 64-95 of the accumulator hold the two halves
+            umma_bf16_ts_by(lead, tmem + Cfg::ACC2 + n, tmem + b * 128 + kk * 64 + k * 8, wd + k * (32 >> 4), idesc2, (h > 0 || kk > 0 || k > 0) ? 1u : 0u);
+          box_done();
+        }
+      if (!ok) return;
+      umma_commit_by(lead, acc_free + 8 * b);
+      if (h + 1 == chunks) umma_commit_by(lead, acc2_full);
+      ++c2;
+    };
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < a.num_tiles && ok; tile += gridDim.x, ++t) {
+      const uint32_t s = t % NA;
+      await(a_full + 8 * s, (t / NA) & 1, ST_TIMEOUT_EPI);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll 1
+      for (int h = 0; h <= chunks && ok; ++h) {
+        if (h < chunks) first(ad0 + s * (Cfg::A_BYTES >> 4));
+        if (h + 1 == chunks && ok) umma_commit_by(lead, a_empty + 8 * s);        // the last product that reads the rows is in
+        if (MODE != LN_PROJECT && h > 0 && ok) second(h - 1);
+      }
+    }
+    if (!ok && lead) *abort_flag = 1;
+    __syncwarp();
+  } else {
+    // ---------------- epilogues (warps 4..11) ----------------
+    const int quad = warp & 3, half = (warp - 4) >> 2;
+    uint8_t* stg = sm + Cfg::STG + (warp - 4) * (Cfg::TILES * 4096);
+    const uint32_t stg_u = smem_u32(stg), my_ld = ld_bar + 8 * (warp - 4);
+    const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
+    uint32_t c1 = 0, t = 0, ld_phase = 0;
+    bool ok = true;
+    auto wait = [&](uint32_t bar, uint32_t parity, int code) -> bool {
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+      if (!ok && lane == 0 && *abort_flag == 0) report(code, 53);
+      return ok;
+    };
+    // 64 columns of this thread's row of an accumulator, bias added
+    auto read64 = [&](uint32_t col, const float* bias, float (&v)[64]) {
+      tmem_ld_32x32(lane_base + col, v);
+      tmem_ld_32x32(lane_base + col + 32, v + 32);
+      tmem_ld_wait();
+      const float4* bp = reinterpret_cast<const float4*>(bias);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        const float4 f = bp[q];
+        v[4 * q] += f.x;
+        v[4 * q + 1] += f.y;
+        v[4 * q + 2] += f.z;
+        v[4 * q + 3] += f.w;
+      }
+    };
+    auto mul_tile = [&](const uint8_t* buf, float (&v)[64]) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        float m[8];
+        lg_unpack(*reinterpret_cast<const uint4*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4)), m);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[u * 8 + j] *= m[j];
+      }
+    };
+    // the tile that leaves, with the residual tile in the same place added where there is one
+    auto write_tile = [&](uint8_t* buf, float (&v)[64], bool resid) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        uint4* at = reinterpret_cast<uint4*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4));
+        if (resid) {
+          float m[8];
+          lg_unpack(*at, m);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[u * 8 + j] += m[j];
+        }
+        *at = lg_pack(v + u * 8);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+    };
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < a.num_tiles && ok; tile += gridDim.x, ++t) {
+      int row0 = (tile % a.tiles_m) * 128 + quad * 32, batch = tile / a.tiles_m;
+      if (a.bpt > 1) {
+        batch = tile * a.bpt + row0 / a.rows;
+        row0 %= a.rows;
+      }
+      const bool valid = row0 < a.rows && batch < a.batch;
+      if (MODE != LN_PROJECT) {
+        uint8_t* obuf = stg + (Cfg::TILES - 1) * 4096;          // residual and result; the other one (or the same) takes the mul tiles
+        const uint32_t obuf_u = stg_u + (Cfg::TILES - 1) * 4096;
+        auto fetch_mul = [&](int h) {
+          if (lane == 0) {
+            if (Cfg::TILES == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            mbar_expect_tx(my_ld, 4096);
+            tma_load_3d(stg_u, &maps.mul, my_ld, h * 128 + half * 64, row0, batch);
+          }
+        };
+        if (MODE == LN_GATE_CHAIN && !a.mul_f32) fetch_mul(0);
+#pragma unroll 1
+        for (int h = 0; h < chunks; ++h, ++c1) {
+          const uint32_t b = c1 % NACC;
+          if (!wait(acc_full + 8 * b, (c1 / NACC) & 1, ST_TIMEOUT_MMA)) break;
+          tc_fence_after();
+          float v[64];
+          read64(b * 128 + half * 64, bias1 + h * 128 + half * 64, v);
+          if (MODE == LN_RELU_CHAIN) {
+#pragma unroll
+            for (int j = 0; j < 64; ++j) v[j] = fmaxf(v[j], 0.f);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 64; ++j) v[j] = sigmoidf_(v[j]);
+            if (a.mul_f32) {
+              // one row of 32-bit factors for all rows of a column: a few ten kilobytes that stay in L1
+              const int col = h * 128 + half * 64;
+              const float4* m = reinterpret_cast<const float4*>(a.mul_f32 + ((long long)batch * a.rows + row0 + lane) % a.mul_mod * a.hidden + col);
+#pragma unroll
+              for (int q = 0; q < 16; ++q) {
+                const float4 f = col + 4 * q < a.hidden ? m[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[4 * q] *= f.x;
+                v[4 * q + 1] *= f.y;
+                v[4 * q + 2] *= f.z;
+                v[4 * q + 3] *= f.w;
+              }
+            } else {
+              if (!wait(my_ld, ld_phase, ST_TIMEOUT_TMA)) break;
+              ld_phase ^= 1;
+              mul_tile(stg, v);
+              __syncwarp();
+              if (h + 1 < chunks) fetch_mul(h + 1);
+            }
+          }
+          float p[32];                                          // bf16 pairs
+#pragma unroll
+          for (int j = 0; j < 32; ++j) p[j] = __uint_as_float(lg_pack2(v[2 * j], v[2 * j + 1]));
+          tmem_st_32x32(lane_base + b * 128 + half * 64, p);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(h_full + 8 * b);
+        }
+        if (!ok) break;
+        bool waited = false;
+#pragma unroll 1
+        for (int c = half; c < C / 64; c += 2) {
+          if (lane == 0) {
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            mbar_expect_tx(my_ld, 4096);
+            tma_load_3d(obuf_u, &maps.resid, my_ld, c * 64, row0, batch);
+          }
+          __syncwarp();
+          if (!waited && !wait(acc2_full, t & 1, ST_TIMEOUT_MMA)) break;
+          waited = true;
+          tc_fence_after();
+          float v[64];
+          read64(Cfg::ACC2 + c * 64, bias2 + c * 64, v);
+          if (!wait(my_ld, ld_phase, ST_TIMEOUT_TMA)) break;
+          ld_phase ^= 1;
+          write_tile(obuf, v, true);
+          if (lane == 0 && valid) lg_store_tile(&maps.out[0], obuf_u, c * 64, row0, batch);
+        }
+        if (!ok) break;
+        if (!waited && !wait(acc2_full, t & 1, ST_TIMEOUT_MMA)) break;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc2_empty);
+      } else {
+        const int row = row0 + lane;
+        float rs = 1.f;
+        if (a.rowscale && valid && row < a.rows) {
+          const long long i = (long long)batch * a.rows + row;
+          rs = a.rs_bf16 ? __bfloat162float(reinterpret_cast<const bf16*>(a.rowscale)[i]) : reinterpret_cast<const float*>(a.rowscale)[i];
+        }
+        int seg = 0, col = 0;                                   // segment and first column of the chunk
+#pragma unroll 1
+        for (int h = 0; h < chunks; ++h, ++c1) {
+          const LgSeg sg = a.seg[seg];
+          const int mycol = col + half * 64, b = c1 % NACC;
+          const bool work = mycol < sg.n && valid;
+          const uint32_t ob = Cfg::TILES == 2 ? (c1 & 1) : 0;
+          uint8_t* obuf = stg + ob * 4096;
+          const uint32_t obuf_u = stg_u + ob * 4096;
+          const bool fused = a.has_mul != 0 && seg == 0;        // mul and residual tiles (two staging tiles; first segment)
+          if (work && lane == 0) {
+            if (fused || Cfg::TILES == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            if (fused) {
+              mbar_expect_tx(my_ld, 8192);
+              tma_load_3d(obuf_u, &maps.resid, my_ld, mycol, row0, batch);
+              tma_load_3d(stg_u + (ob ^ 1) * 4096, &maps.mul, my_ld, mycol, row0, batch);
+            }
+          }
+          __syncwarp();
+          if (!wait(acc_full + 8 * b, (c1 / NACC) & 1, ST_TIMEOUT_MMA)) break;
+          tc_fence_after();
+          if (work) {
+            if (sg.kind == LN_PAIR_BIAS) {
+              float v[32];
+              tmem_ld_32x32(lane_base + b * 128 + half * 64, v);
+              tmem_ld_wait();
+              if (row < a.rows) {
+                const long long r = (long long)batch * a.rows + row;
+                bf16* dst = sg.out + (r / a.pb_n) * a.pb_i + (r % a.pb_n) * a.pb_j;
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                  if (j < sg.n) dst[j * a.pb_h] = __float2bfloat16(v[j]);
+              }
+            } else {
+              float v[64];
+              read64(b * 128 + half * 64, bias1 + h * 128 + half * 64, v);
+              if (sg.kind == LN_GLU_T) {
+                bf16* o = reinterpret_cast<bf16*>(obuf) + lane;       // [32 columns][32 rows]
+#pragma unroll
+                for (int j = 0; j < 32; ++j) o[j * 32] = __float2bfloat16(v[2 * j] * sigmoidf_(v[2 * j + 1]) * rs);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) lg_store_tile(&maps.out[seg], obuf_u, row0, mycol >> 1, batch);
+              } else {
+                if (sg.act == ACT_SIGMOID) {
+#pragma unroll
+                  for (int j = 0; j < 64; ++j) v[j] = sigmoidf_(v[j]);
+                }
+                if (sg.scaled) {
+#pragma unroll
+                  for (int j = 0; j < 64; ++j) v[j] *= rs;
+                }
+                if (fused) {
+                  if (!wait(my_ld, ld_phase, ST_TIMEOUT_TMA)) break;
+                  ld_phase ^= 1;
+                  mul_tile(stg + (ob ^ 1) * 4096, v);
+                }
+                write_tile(obuf, v, fused);
+                if (lane == 0) lg_store_tile(&maps.out[seg], obuf_u, mycol, row0, batch);
+              }
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_free + 8 * b);
+          col += 128;
+          if (col >= sg.n) {
+            ++seg;
+            col = 0;
+          }
+        }
+      }
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    if (!ok && lane == 0) *abort_flag = 1;
+    __syncwarp();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+template <int C, int MODE, bool CF>
+static int lg_launch(const LgMaps& maps, const LgArgs& a, cudaStream_t st) {
+  auto kern = ln_gemm_kernel<C, MODE, CF>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LgCfg<C, MODE>::SMEM) != cudaSuccess) return -30;
+    attr_set = true;
+  }
+  static int sm_count = 0;
+  if (!sm_count) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0) sm_count = 148;
+  }
+  const int grid = a.num_tiles < sm_count ? a.num_tiles : sm_count;
+  launch_k(kern, grid, LG_THREADS, LgCfg<C, MODE>::SMEM, st, maps, a);
+  return cudaGetLastError() == cudaSuccess ? 0 : -31;
+}
+
+}  // namespace ffb
+
+using namespace ffb;
+
+extern "C" int ffb_ln_gemm(const LnGemmArgs* p, void* stream) {
+  const LnGemmArgs& q = *p;
+  if ((q.C != 64 && q.C != 128 && q.C != 256) || q.rows < 1 || q.batch < 1 || (q.channels_first && (q.C != 128 || q.mode != LN_PROJECT))) return -1;
+  // short rows of many batches (a slice of columns of the pair or MSA tensor): several batches share a tile
+  const int bpt = (!q.channels_first && q.batch > 1 && (q.rows == 32 || q.rows == 64)) ? (int)(128 / q.rows) : 1;
+  const long long tiles_m = (q.rows + 127) / 128, tiles = tiles_m * ((q.batch + bpt - 1) / bpt);
+  if (tiles > 0x7fffffffLL || q.rows > 0x7fffffffLL || q.batch > 0x7fffffffLL) return -2;
+  auto bad = [](const void* ptr, long long rs, long long bs) { return !ptr || (reinterpret_cast<uintptr_t>(ptr) & 15) || (rs % 8) || (bs % 8); };
+  if (bad(q.x, q.x_rstride, q.x_bstride)) return -3;
+  LgMaps m;
+  LgArgs a = {};
+  a.rows = (int)q.rows;
+  a.batch = (int)q.batch;
+  a.tiles_m = (int)tiles_m;
+  a.num_tiles = (int)tiles;
+  a.bpt = bpt;
+  a.gamma = (const bf16*)q.gamma;
+  a.beta = (const bf16*)q.beta;
+  a.eps = q.eps;
+  a.rowscale = q.rowscale;
+  a.rs_bf16 = q.rs_bf16;
+  a.pb_h = q.pb_h;
+  a.pb_i = q.pb_i;
+  a.pb_j = q.pb_j;
+  a.pb_n = q.pb_n > 0 ? q.pb_n : 1;
+  // d0 is the contiguous extent
+  auto map = [&](CUtensorMap* t, const void* ptr, long long d0, long long d1, long long d2, long long s1, long long s2, int b0, int b1, int swizzle, int b2 = 1) {
+    return encode_tmap3_bf16(t, ptr, d0, d1, d2, s1, s2, b0, b1, swizzle, b2);
+  };
+  int r = q.channels_first ? map(&m.x, q.x, q.rows, q.C, q.batch, q.x_rstride, q.x_bstride, 64, 64, 128)
+                           : map(&m.x, q.x, q.C, q.rows, q.batch, q.x_rstride, q.x_bstride, 64, 128 / bpt, 128, bpt);
+  if (r) return 1000 + r;
+  m.mul = m.resid = m.out[0] = m.out[1] = m.out[2] = m.w[0] = m.w[1] = m.w[2] = m.x;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (q.mode != LN_PROJECT) {
+    const bool f32 = q.mode == LN_GATE_CHAIN && q.mul_f32;
+    if (f32 && (q.mul_mod < 1 || (reinterpret_cast<uintptr_t>(q.mul_f32) & 15))) return -4;
+    if (q.hidden < 8 || q.hidden % 8 || q.hidden > LG_MAX_N || bad(q.w1, 0, 0) || bad(q.w2, 0, 0) || bad(q.resid, q.r_rstride, q.r_bstride) ||
+        bad(q.out, q.o_rstride, q.o_bstride) || (q.mode == LN_GATE_CHAIN && !f32 && bad(q.mul, q.m_rstride, q.m_bstride)))
+      return -4;
+    a.hidden = q.hidden;
+    a.mul_f32 = f32 ? q.mul_f32 : nullptr;
+    a.mul_mod = f32 ? q.mul_mod : 1;
+    a.b1 = (const bf16*)q.b1;
+    a.b2 = (const bf16*)q.b2;
+    r = map(&m.w[0], q.w1, q.C, q.hidden, 1, q.C, 0, 64, 128, 128);
+    if (!r) r = map(&m.w[1], q.w2, q.hidden, q.C, 1, q.hidden, 0, 64, q.C < 128 ? q.C : 128, 128);
+    if (!r) r = map(&m.resid, q.resid, q.C, q.rows, q.batch, q.r_rstride, q.r_bstride, 64, 32, 128);
+    if (!r) r = map(&m.out[0], q.out, q.C, q.rows, q.batch, q.o_rstride, q.o_bstride, 64, 32, 128);
+    if (!r && q.mode == LN_GATE_CHAIN && !f32) r = map(&m.mul, q.mul, q.hidden, q.rows, q.batch, q.m_rstride, q.m_bstride, 64, 32, 128);
+    if (r) return 2000 + r;
+    if (q.mode == LN_RELU_CHAIN) {
+      if (q.C == 64) return lg_launch<64, LN_RELU_CHAIN, false>(m, a, st);
+      if (q.C == 128) return lg_launch<128, LN_RELU_CHAIN, false>(m, a, st);
+      return lg_launch<256, LN_RELU_CHAIN, false>(m, a, st);
+    }
+    if (q.C == 64) return lg_launch<64, LN_GATE_CHAIN, false>(m, a, st);
+    if (q.C == 128) return lg_launch<128, LN_GATE_CHAIN, false>(m, a, st);
+    return lg_launch<256, LN_GATE_CHAIN, false>(m, a, st);
+  }
+  if (q.nseg < 1 || q.nseg > 3) return -5;
+  a.nseg = q.nseg;
+  for (int s = 0; s < q.nseg; ++s) {
+    const LnSegment& g = q.seg[s];
+    if (g.n < 1 || bad(g.w, 0, 0) || !g.out) return -6;
+    if (g.kind != LN_PAIR_BIAS && bad(g.out, g.o_rstride, g.o_bstride)) return -7;
+    if ((g.kind == LN_PAIR_BIAS && g.n > 32) || (g.kind == LN_GLU_T && (g.n & 1))) return -8;
+    a.seg[s] = {g.kind, g.act, g.scaled, g.n, (bf16*)g.out};
+    a.seg_bias[s] = (const bf16*)g.bias;
+    a.chunks += (g.n + 127) / 128;
+    r = map(&m.w[s], g.w, q.C, g.n, 1, q.C, 0, 64, 128, 128);
+    if (!r && g.kind == LN_ROWS) r = map(&m.out[s], g.out, g.n, q.rows, q.batch, g.o_rstride, g.o_bstride, 64, 32, 128);
+    if (!r && g.kind == LN_GLU_T) r = map(&m.out[s], g.out, q.rows, g.n / 2, q.batch, g.o_rstride, g.o_bstride, 32, 32, 0);
+    if (r) return 3000 + r;
+  }
+  if (a.chunks * 128 > LG_MAX_N) return -9;
+  if (q.mul || q.resid) {
+    if (q.C == 256 || bad(q.mul, q.m_rstride, q.m_bstride) || bad(q.resid, q.r_rstride, q.r_bstride) || q.seg[0].kind != LN_ROWS) return -10;
+    a.has_mul = 1;
+    r = map(&m.mul, q.mul, q.seg[0].n, q.rows, q.batch, q.m_rstride, q.m_bstride, 64, 32, 128);
+    if (!r) r = map(&m.resid, q.resid, q.seg[0].n, q.rows, q.batch, q.r_rstride, q.r_bstride, 64, 32, 128);
+    if (r) return 4000 + r;
+  }
+  if (q.channels_first) return lg_launch<128, LN_PROJECT, true>(m, a, st);
+  if (q.C == 64) return lg_launch<64, LN_PROJECT, false>(m, a, st);
+  if (q.C == 128) return lg_launch<128, LN_PROJECT, false>(m, a, st);
+  return lg_launch<256, LN_PROJECT, false>(m, a, st);
+}

@@ -39,13 +39,13 @@ static void bind_primary_context() {
 }
 
 int encode_tmap3_bf16(CUtensorMap* map, const void* ptr, long long d0, long long d1, long long d2, long long s1, long long s2,
-                      int b0, int b1, int swizzle_bytes) {
+                      int b0, int b1, int swizzle_bytes, int b2) {
   static EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(entry("cuTensorMapEncodeTiled"));
   if (!enc) return -1;
   cuuint64_t dims[3] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)(d2 > 0 ? d2 : 1)};
   cuuint64_t strides[2] = {(cuuint64_t)s1 * 2, (cuuint64_t)(d2 > 1 ? s2 : d1 * s1) * 2};
   if (strides[1] == 0) strides[1] = (cuuint64_t)s1 * 2 * (cuuint64_t)d1;
-  cuuint32_t box[3] = {(cuuint32_t)b0, (cuuint32_t)b1, 1};
+  cuuint32_t box[3] = {(cuuint32_t)b0, (cuuint32_t)b1, (cuuint32_t)b2};
   cuuint32_t estr[3] = {1, 1, 1};
   const CUtensorMapSwizzle sw = swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                                 : (swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B

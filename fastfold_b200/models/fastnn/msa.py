@@ -7,7 +7,7 @@ from ... import ops as K
 from ...parallel import core
 from ...parallel.comm import gather, scatter, scatter_mask, row_to_col, col_to_row
 from ...parallel.comm_async import all_to_all_async, all_to_all_async_opp
-from ...parallel.fused import a2a_layer_norm
+from ...parallel.fused import a2a_layer_norm, norm_later
 from ...utils import memo
 from ...utils.checkpointing import checkpoint_blocks
 from .ops import (ChunkMSARowAttentionWithPairBias, ChunkMSAColumnGlobalAttention, ChunkTransition, GlobalAttention,
@@ -46,15 +46,18 @@ class MSAColumnAttention(nn.Module):
         ``strided`` (then in the layout of ``M_raw``); ``strided=None`` decides here."""
         if strided is None:
             strided = M_norm_t is None and self.strided_for(M_raw.shape[1], M_raw)
+        mask_t = memo.cached("mask_t", (M_mask,), lambda: M_mask.transpose(-1, -2).contiguous())
+        if strided and M_norm_t is None and self.attention.takes_raw(M_raw, self.layernormM, None):
+            return self.attention(M_raw, mask_t, tail=(None, None, M_raw), transposed=True, norm=self.layernormM)[0]
         if strided:
             M = self.layernormM(M_raw) if M_norm_t is None else M_norm_t
             tail = (None, None, _residual(M_raw)) if _fusable(M_raw) else None          # the residual joins in the output projection
-            out, done = self.attention(M, memo.cached("mask_t", (M_mask,), lambda: M_mask.transpose(-1, -2).contiguous()), tail=tail, transposed=True)
+            out, done = self.attention(M, mask_t, tail=tail, transposed=True)
             if done:
                 return out
             return M_raw.add_(out) if fops.INPLACE else M_raw + out
         M = self.layernormM(M_raw.transpose(-2, -3).contiguous()) if M_norm_t is None else M_norm_t
-        out, _ = self.attention(M, memo.cached("mask_t", (M_mask,), lambda: M_mask.transpose(-1, -2).contiguous()))
+        out, _ = self.attention(M, mask_t)
         return M_raw.add_(out.transpose(-2, -3)) if fops.INPLACE else M_raw + out.transpose(-2, -3)
 
 
@@ -74,7 +77,10 @@ class MSACore(nn.Module):
         node = self.MSARowAttentionWithPairBias(node, pair, node_mask_row, dropmask)
         # row -> column switch fused with the transpose + LayerNorm of the column attention
         strided = self.MSAColumnAttention.strided_for(node.shape[1] * core.get_dap_size(), node)     # full sequence count after the switch
-        node, node_nt = a2a_layer_norm(node, self.MSAColumnAttention.layernormM, 0, transpose_norm=not strided)
+        if strided and norm_later(node):
+            node_nt = None
+        else:
+            node, node_nt = a2a_layer_norm(node, self.MSAColumnAttention.layernormM, 0, transpose_norm=not strided)
         node_mask_col = scatter_mask(node_mask, dim=2)
         node = self.MSAColumnAttention(node, node_mask_col, M_norm_t=node_nt, strided=strided)
         node = self.MSATransition(node)

@@ -4,7 +4,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ...parallel.comm import scatter, scatter_mask, row_to_col, col_to_row
-from ...parallel.fused import a2a_layer_norm
+from ...parallel.fused import a2a_layer_norm, norm_later
 from ...utils.tensor_utils import permute_final_dims  # noqa: F401
 from .ops import (AsyncChunkTriangleMultiplicationOutgoing, AsyncChunkTriangleMultiplicationIncoming,
                   ChunkTriangleAttentionStartingNode, ChunkTriangleAttentionEndingNode, ChunkTransition)
@@ -65,6 +65,11 @@ class PairCore(nn.Module):
         pair_mask_col = scatter_mask(pair_mask, dim=2)
         # each axis switch is fused with the LayerNorm (and transpose) of the module that consumes its result
         pair = self.TriangleMultiplicationOutgoing(pair, pair_mask_row, d.get("tri_mul_out"))
+        if norm_later(pair):                     # nothing to switch and no gradients: every module sees to its norm itself
+            pair = self.TriangleMultiplicationIncoming(pair, pair_mask_col, d.get("tri_mul_in"))
+            pair = self.TriangleAttentionStartingNode(pair, pair_mask_row, d.get("tri_att_start"))
+            pair = self.TriangleAttentionEndingNode(pair, pair_mask_col, d.get("tri_att_end"))
+            return self.PairTransition(pair)
         pair, pn = a2a_layer_norm(pair, self.TriangleMultiplicationIncoming.layernorm1, 0)
         dm = d.get("tri_mul_in")
         if dm is not None:

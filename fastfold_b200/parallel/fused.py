@@ -59,6 +59,11 @@ class _A2ALayerNorm(torch.autograd.Function):
         return dx.squeeze(0), dg, db, None, None, None
 
 
+def norm_later(x):
+    """One rank, no gradients: there is no axis switch to fuse the norm into, so the consumer fuses it into its projections."""
+    return core.get_dap_size() == 1 and x.is_cuda and not torch.is_grad_enabled()
+
+
 def a2a_layer_norm(x, ln, mode, transpose_norm=False):
     """``x`` is ``[1, a, b, C]``; returns ``(raw, norm)`` as ``[1, ., ., C]`` tensors in the switched sharding.
 

@@ -1,0 +1,173 @@
+"""LayerNorm + GEMM kernels (csrc/ln_gemm.cu) and the column kernel of global_attention.cu against the same mathematics in 64 bits,
+with the roundings to bf16 that the kernels make (normalised rows, hidden activation) made there too.  Bound: what is left are the fp32
+sums and the rounding of the result, 2^-9 of each value at most, so 2^-9 in the 2-norm; a normalised or hidden value that rounds the
+other way adds less than that again."""
+import pytest
+import torch
+
+from fastfold_b200.models.fastnn import ops as fops
+from fastfold_b200.ops import LayerNorm, ln_gemm
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+TOL = 2.0 ** -8
+
+
+def _randn(*shape, scale=1.0):
+    return (torch.randn(*shape, device=DEV) * scale).to(torch.bfloat16)
+
+
+def _norm(C):
+    norm = LayerNorm(C).to(DEV, torch.bfloat16).requires_grad_(False)
+    norm.weight.copy_(1 + 0.1 * torch.randn(C, device=DEV))
+    norm.bias.copy_(0.1 * torch.randn(C, device=DEV))
+    return norm
+
+
+def _ln(x, norm):
+    y = torch.nn.functional.layer_norm(x.double(), (x.shape[-1],), norm.weight.double(), norm.bias.double(), norm.eps)
+    return y.bfloat16().double()
+
+
+def _close(a, ref):
+    assert a.shape == ref.shape
+    assert torch.isfinite(a.float()).all()
+    assert (a.double() - ref).norm() <= TOL * ref.norm()
+
+
+def _lin(x, w, b=None):
+    y = x @ w.double().t()
+    return y if b is None else y + b.double()
+
+
+@pytest.mark.parametrize("C", [64, 128, 256])
+@pytest.mark.parametrize("M", [1, 31, 128, 129, 19000])
+def test_chains(C, M, device_status):
+    """Transition and gated output: less than a tile, a whole one, a remainder of one row, more tiles than CTAs; one and two chunks
+    of gated columns; the result over the residual."""
+    torch.manual_seed(C + M)
+    with torch.no_grad():
+        x, norm, H = _randn(M, C), _norm(C), 4 * C
+        w1, b1, w2, b2 = _randn(H, C, scale=C ** -0.5), _randn(H, scale=0.1), _randn(C, H, scale=H ** -0.5), _randn(C, scale=0.1)
+        assert ln_gemm.ready(x, norm, (), (w1, b1, w2, b2))
+        X = _ln(x, norm)
+        _close(ln_gemm.chain(x, norm, w1, b1, w2, b2, x), x.double() + _lin(torch.relu(_lin(X, w1, b1)).bfloat16().double(), w2, b2))
+        for G in (128, 256):
+            o, wg, bg, wo = _randn(M, G), _randn(G, C, scale=C ** -0.5), _randn(G, scale=0.1), _randn(C, G, scale=G ** -0.5)
+            ref = x.double() + _lin((torch.sigmoid(_lin(X, wg, bg)) * o.double()).bfloat16().double(), wo)
+            _close(ln_gemm.chain(x, norm, wg, bg, wo, None, x, mul=o), ref)
+        y = x.clone()
+        assert ln_gemm.chain(y, norm, wg, bg, wo, None, y, mul=o, out=y).data_ptr() == y.data_ptr()
+        _close(y, ref)
+
+
+@pytest.mark.parametrize("batch,rows", [(5, 64), (7, 32), (3, 16), (6, 96), (4, 200), (2, 1)])
+def test_rows_in_batches(batch, rows, device_status):
+    """Slices of columns: two or four batches share a tile (64 and 32 rows), one otherwise; nothing outside the slice is written."""
+    torch.manual_seed(batch * rows)
+    with torch.no_grad():
+        whole, norm = _randn(batch, rows + 24, 128), _norm(128)
+        x = whole[:, 8:8 + rows]
+        w, b, wo, o = _randn(128, 128, scale=0.09), _randn(128, scale=0.1), _randn(128, 128, scale=0.09), _randn(batch, rows, 128)
+        out = torch.zeros_like(whole)
+        X = _ln(x, norm)
+        ln_gemm.chain(x, norm, w, b, wo, b, x, mul=o, out=out[:, 8:8 + rows])
+        _close(out[:, 8:8 + rows], x.double() + _lin((torch.sigmoid(_lin(X, w, b)) * o.double()).bfloat16().double(), wo, b))
+        assert not out[:, :8].any() and not out[:, 8 + rows:].any()
+        _close(ln_gemm.qkv(x, norm, w), _lin(X, w))
+
+
+@pytest.mark.parametrize("C,n", [(128, 5), (128, 16), (128, 77), (128, 130), (64, 33), (256, 40)])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_qkv_and_pair_bias(C, n, transposed, device_status):
+    torch.manual_seed(n)
+    with torch.no_grad():
+        z, norm, w, wb = _randn(n, n, C), _norm(C), _randn(384, C, scale=C ** -0.5), _randn(8, C, scale=C ** -0.5)
+        buf = torch.full((8, n, (n + 7) // 8 * 8), 7.0, device=DEV, dtype=torch.bfloat16)
+        y = ln_gemm.qkv(z.view(-1, C), norm, w, wb, buf[:, :, :n], transposed)
+        X = _ln(z, norm)
+        _close(y.view(n, n, -1), _lin(X, w))
+        _close(buf[:, :, :n], _lin(X, wb).permute(2, 1, 0) if transposed else _lin(X, wb).permute(2, 0, 1))
+        assert (buf[:, :, n:] == 7.0).all()
+
+
+@pytest.mark.parametrize("M,dtype", [(3, torch.bfloat16), (300, torch.float32), (5000, torch.bfloat16)])
+@pytest.mark.parametrize("C", [64, 256])
+def test_pair_of_projections(C, M, dtype, device_status):
+    torch.manual_seed(M)
+    with torch.no_grad():
+        x, norm, s = _randn(M, C), _norm(C), torch.rand(M, device=DEV).to(dtype)
+        ws = [_randn(32, C, scale=C ** -0.5) for _ in range(2)]
+        bs = [_randn(32, scale=0.1) for _ in range(2)]
+        for y, w, b in zip(ln_gemm.pair(x, norm, ws[0], bs[0], ws[1], bs[1], s), ws, bs):
+            _close(y, _lin(_ln(x, norm), w, b) * s.double()[:, None])
+
+
+def _randomise(net):
+    for p in net.parameters():
+        p.copy_(torch.randn_like(p) * (p.shape[-1] ** -0.5 if p.dim() == 2 else 0.1) + (1.0 if p.dim() == 1 and p.float().mean() > 0.5 else 0.0))
+
+
+@pytest.mark.parametrize("n", [1, 8, 27, 64, 131, 200])
+@pytest.mark.parametrize("cls", [fops.AsyncChunkTriangleMultiplicationOutgoing, fops.AsyncChunkTriangleMultiplicationIncoming])
+def test_triangle_multiplication(cls, n, device_status):
+    """The three-kernel path against the layer in 64 bits (its roundings are not restated here: operands, their product, its norm and
+    the gate are rounded to bf16, 2^-9 each, and the update is added to a residual of about its size)."""
+    torch.manual_seed(n)
+    net = cls(128, p_drop=0.25).to(DEV, torch.bfloat16).eval().requires_grad_(False)
+    with torch.no_grad():
+        _randomise(net)
+        z, mask = _randn(1, n, n, 128), (torch.rand(1, n, n, device=DEV) > 0.2).to(torch.bfloat16)
+        assert net._takes_raw(z, None)
+        P = {k: v.double() for k, v in net.named_parameters()}
+        lin = lambda x, name: torch.nn.functional.linear(x, P[name + ".weight"], P.get(name + ".bias"))  # noqa: E731
+        ln = lambda x, name: torch.nn.functional.layer_norm(x, (128,), P[name + ".weight"], P[name + ".bias"], 1e-5)  # noqa: E731
+        x = ln(z[0].double(), "layernorm1")
+        a, b = (lin(x, "left_right_projection") * torch.sigmoid(lin(x, "left_right_gate")) * mask[0].double()[..., None]).chunk(2, -1)
+        p = torch.einsum("ikc,jkc->ijc", a, b) if net.outgoing else torch.einsum("kic,kjc->ijc", a, b)
+        ref = z.double() + torch.sigmoid(lin(x, "output_gate")) * (lin(ln(p, "layernorm2"), "output_projection") + P["output_bias"])
+        out = net(z, mask)
+        assert (out.double() - ref).norm() <= 4 * TOL * ref.norm()
+
+
+@pytest.mark.parametrize("S,N", [(1, 3), (5, 40), (31, 8), (130, 33), (700, 17)])
+def test_global_column_attention(S, N, device_status):
+    """The layer against the same in 64 bits, with masked sequences and a wholly masked column.  Bound as above, once for the gated
+    product that is rounded before the output projection."""
+    torch.manual_seed(S)
+    net = fops.ChunkMSAColumnGlobalAttention(64, c=8, n_head=8).to(DEV, torch.bfloat16).eval().requires_grad_(False)
+    with torch.no_grad():
+        _randomise(net)
+        m, mask = _randn(1, S, N, 64), (torch.rand(1, S, N, device=DEV) > 0.2).to(torch.bfloat16)
+        mask[0, :, 1] = 0
+        assert net._from_raw(m, mask) is not None
+        ga = net.global_attention
+        x, mk = _ln(m[0], net.layernormM).transpose(0, 1), mask[0].double().t()                       # [N, S, c]
+        q = (x * mk[..., None]).sum(1) / (mk.sum(-1, keepdim=True) + 1e-10)
+        q = (_lin(q, ga.to_q.weight) * ga.scaling).view(N, 8, 8)
+        k, v = _lin(x, ga.to_kv.weight).bfloat16().double().chunk(2, -1)
+        a = (q @ k.transpose(1, 2)).masked_fill(mk[:, None] == 0, -1e9).softmax(-1)
+        o = (a @ v).reshape(N, 1, 64) * torch.sigmoid(_lin(x, ga.gating_linear.weight, ga.gating_bias))
+        ref = m[0].double() + _lin(o, ga.o_linear.weight, ga.o_linear.bias).transpose(0, 1)
+        _close(net(m, mask)[0], ref)
+
+
+def test_calls_that_stay_with_the_composition():
+    norm = _norm(128)
+    x = _randn(64, 128)
+    with torch.no_grad():
+        assert ln_gemm.ready(x, norm)
+        assert not ln_gemm.ready(x.float(), norm)
+        assert not ln_gemm.ready(x[:0], norm)
+        for odd in (x.t().contiguous().t(), _randn(64 * 128 + 4)[4:].view(64, 128)):  # channels not adjacent, off a 16-byte boundary
+            d = ln_gemm.dense(odd)
+            assert d.is_contiguous() and d.data_ptr() % 16 == 0 and torch.equal(d, odd)
+        assert not ln_gemm.ready(x, norm, (), (_randn(256, 128)[::2],))
+        assert not ln_gemm.ready(x, norm, (), (torch.ones(128, device=DEV),))
+        handle = norm.register_forward_hook(lambda *a: None)
+        assert not ln_gemm.ready(x, norm)
+        handle.remove()
+        assert ln_gemm.ready(x, norm)
+        with torch.autograd.forward_ad.dual_level():
+            assert not ln_gemm.ready(x, norm)
+    assert not ln_gemm.ready(x, norm)                                                # gradients
