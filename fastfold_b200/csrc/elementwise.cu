@@ -280,6 +280,46 @@ __global__ void adam_k(float* w, float* m, float* v, const bf16* grad, bf16* w16
   w16[i] = __float2bfloat16(ww);
 }
 
+// out[i][j] = 1 / (sum_s mask[s][i] * mask[s][j] + eps): the normaliser of the outer product mean, from a mask [S][N].  64 x 64 outputs
+// per CTA, 4 x 4 per thread; one launch for the conversions, the product, the sum and the reciprocal, which as tensor operations are six.
+template <typename T>
+__global__ void __launch_bounds__(256) mask_norm_k(const T* __restrict__ mask, float* __restrict__ out, int S, int N, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int KS = 32;
+  __shared__ __align__(16) float a[KS][64], b[KS][64];
+  const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  for (int s0 = 0; s0 < S; s0 += KS) {
+#pragma unroll
+    for (int u = 0; u < KS * 64 / 256; ++u) {
+      const int t = threadIdx.x + u * 256, s = s0 + (t >> 6), c = t & 63;
+      a[t >> 6][c] = (s < S && i0 + c < N) ? to_f(mask[(long long)s * N + i0 + c]) : 0.f;
+      b[t >> 6][c] = (s < S && j0 + c < N) ? to_f(mask[(long long)s * N + j0 + c]) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < KS; ++k) {
+      const float4 u = *reinterpret_cast<const float4*>(&a[k][ty * 4]), v = *reinterpret_cast<const float4*>(&b[k][tx * 4]);
+      const float x[4] = {u.x, u.y, u.z, u.w}, y[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + ty * 4 + i < N && j0 + tx * 4 + j < N) out[(long long)(i0 + ty * 4 + i) * N + j0 + tx * 4 + j] = 1.f / (acc[i][j] + eps);
+}
+
 }  // namespace ffb
 
 using namespace ffb;
@@ -348,6 +388,16 @@ int ffb_colsum(const void* x, float* out, long long rows, int C, void* stream) {
   dim3 grid((C / 2 + 127) / 128, (unsigned)((rows + rpb - 1) / rpb));
   launch_light(colsum_k, grid, 128, 0, reinterpret_cast<cudaStream_t>(stream), (const bf16*)x, out, rows, C, rpb);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// mask [S][N], bf16 or fp32; out [N][N] fp32
+int ffb_mask_norm(const void* mask, float* out, int S, int N, float eps, int is_bf16, void* stream) {
+  if (S < 1 || N < 1 || (N + 63) / 64 > 65535) return -1;
+  const dim3 grid((unsigned)((N + 63) / 64), (unsigned)((N + 63) / 64));
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (is_bf16) launch_light(mask_norm_k<bf16>, grid, 256, 0, st, (const bf16*)mask, out, S, N, eps);
+  else launch_light(mask_norm_k<float>, grid, 256, 0, st, (const float*)mask, out, S, N, eps);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 int ffb_adam(float* w, float* m, float* v, const void* grad, void* w16, long long n, const float* hp, float b1, float b2,

@@ -43,6 +43,7 @@ int ffb_glu_mask_t_bwd(const void* dout, const void* pre, const void* mask, void
 int ffb_act_bwd(const void* dy, const void* y, void* dx, long long rows, int C, int mode, void* stream);
 int ffb_colsum(const void* x, float* out, long long rows, int C, void* stream);
 int ffb_ln_gemm(const LnGemmArgs* p, void* stream);
+int ffb_mask_norm(const void* mask, float* out, int S, int N, float eps, int is_bf16, void* stream);
 int ffb_global_column(const void* x, const void* gamma, const void* beta, float eps, const void* wq, const void* kv, const void* mask, float* out,
                       long long S, long long N, float scaling, void* stream);
 }
@@ -576,6 +577,167 @@ std::tuple<Tensor, Tensor> ln_pair(const Tensor& x, const Tensor& gamma, const T
   return {ya, yb};
 }
 
+// ---- whole modules without gradients, from their input to their result ----
+// A module is two to four launches, and checks, views and calls made one by one from Python took three times as long as the
+// launches: a block of 32 x 64 was 830 us of host time for 265 us of kernels.  Each returns None where the kernels do not cover the
+// call; the caller then composes the module from its parts.
+bool plain(const Tensor& t) {
+  return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
+bool plain(const OptTensor& t) { return !t || plain(*t); }
+template <class... T>
+bool all_plain(const T&... ts) {
+  return (plain(ts) && ...);
+}
+bool rows_of_channels(const Tensor& x) {
+  const int64_t C = x.dim() > 0 ? x.size(-1) : 0;
+  return x.is_cuda() && x.scalar_type() == at::kBFloat16 && (C == 64 || C == 128 || C == 256) && x.numel() > 0;
+}
+bool matrix(const Tensor& w, int64_t rows, int64_t cols) { return w.dim() == 2 && w.size(0) == rows && w.size(1) == cols; }
+bool vector(const OptTensor& b, int64_t n) { return !b || b->numel() == n; }
+constexpr int64_t LN_MAX_COLUMNS = 1280;      // weight rows of one call of the LayerNorm + GEMM kernels
+
+// x as the kernels address it: contiguous rows on a 16-byte boundary
+Tensor dense_rows(Tensor x) {
+  dense16(x);
+  return x;
+}
+
+OptTensor transition_module(const Tensor& x0, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& w1, const OptTensor& b1, const Tensor& w2,
+                            const OptTensor& b2, bool inplace) {
+  if (!rows_of_channels(x0) || !all_plain(gamma, beta, w1, b1, w2, b2)) return std::nullopt;
+  const int64_t C = x0.size(-1), hidden = w1.size(0);
+  if (hidden % 128 || hidden > LN_MAX_COLUMNS || !matrix(w1, hidden, C) || !matrix(w2, C, hidden) || !vector(b1, hidden) || !vector(b2, C) ||
+      gamma.numel() != C || beta.numel() != C)
+    return std::nullopt;
+  const Tensor x = dense_rows(x0), x2 = x.view({-1, C});
+  return ln_chain(x2, gamma, beta, eps, w1, b1, w2, b2, std::nullopt, x2, inplace ? OptTensor(x2) : std::nullopt).view(x.sizes());
+}
+
+// A pair bias [H, n, n] with rows at an 8-element pitch
+Tensor pitched(int64_t H, int64_t n, const Tensor& like) { return at::empty({H, n, (n + 7) / 8 * 8}, like.options()).narrow(2, 0, n); }
+
+// x [1, A, B, C] plus the gated attention over norm(x) along its second axis (first with `transposed`), `chunk` rows (columns) at a
+// time where that is > 0.  Pair bias: none, or pair_w applied to norm(x), or to norm_z(z) where z is given.
+OptTensor attention_module(const Tensor& x0, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& wq, const Tensor& wg, const Tensor& bg,
+                           const Tensor& wo, const OptTensor& bo, const OptTensor& mask, const OptTensor& pair_w, const OptTensor& z0,
+                           const OptTensor& z_gamma, const OptTensor& z_beta, double z_eps, int64_t H, int64_t D, double scale, bool transposed,
+                           int64_t chunk, bool inplace) {
+  if (!rows_of_channels(x0) || x0.dim() != 4 || x0.size(0) != 1 || !all_plain(gamma, beta, wq, wg, bg, wo, bo, pair_w, z_gamma, z_beta)) return std::nullopt;
+  const int64_t A = x0.size(1), B = x0.size(2), C = x0.size(3), HD = H * D;
+  const int64_t n = transposed ? A : B, rows = transposed ? B : A;
+  if ((D != 16 && D != 32) || HD % 128 || 3 * HD + 128 > LN_MAX_COLUMNS || !matrix(wq, 3 * HD, C) || !matrix(wg, HD, C) || bg.numel() != HD || !matrix(wo, C, HD) ||
+      !vector(bo, C) || gamma.numel() != C || beta.numel() != C)
+    return std::nullopt;
+  if (mask && mask->numel() != rows * n) return std::nullopt;
+  if (pair_w) {
+    const Tensor& src = z0 ? *z0 : x0;
+    if (H > 32 || !rows_of_channels(src) || src.dim() != 4 || src.size(0) != 1 || src.size(1) != n || src.size(2) != n || !matrix(*pair_w, H, src.size(3)))
+      return std::nullopt;
+    if (z0 && (!z_gamma || !z_beta || z_gamma->numel() != src.size(3) || z_beta->numel() != src.size(3))) return std::nullopt;
+  }
+  const Tensor x = dense_rows(x0), x3 = x.view({A, B, C}), x2 = x.view({-1, C});
+  const Tensor out = inplace ? x3 : at::empty_like(x3);
+  OptTensor m2, bias;
+  if (mask) m2 = mask->reshape({rows, n}).to(at::kBFloat16).contiguous();
+  const bool whole = chunk <= 0 || chunk >= rows;
+  OptTensor own_w;                                    // pair weight that rides along with QKV
+  if (pair_w) {
+    bias = pitched(H, n, x);
+    if (z0) ln_qkv(dense_rows(*z0).view({n * n, -1}), *z_gamma, *z_beta, z_eps, std::nullopt, pair_w, bias, false);
+    else if (whole) own_w = pair_w;
+    else ln_qkv(x2, gamma, beta, eps, std::nullopt, pair_w, bias, transposed);
+  }
+  const int64_t pitch = bias ? bias->stride(1) : n;
+  for (int64_t at = 0; at < rows; at += whole ? rows : chunk) {
+    const int64_t len = whole ? rows : std::min(chunk, rows - at);
+    Tensor part = x2, dst = out.view({-1, C});
+    if (!whole) {
+      // rows are contiguous: one matrix; columns are not: a batch of them, one per position along the attention
+      part = x3.narrow(transposed ? 1 : 0, at, len);
+      dst = out.narrow(transposed ? 1 : 0, at, len);
+      if (!transposed) {
+        part = part.view({-1, C});
+        dst = dst.view({-1, C});
+      }
+    }
+    const Tensor qkv = *ln_qkv(part, gamma, beta, eps, wq, own_w, own_w ? bias : OptTensor(), transposed);
+    const OptTensor m = m2 ? OptTensor(whole ? *m2 : m2->narrow(0, at, len)) : std::nullopt;
+    const Tensor o = std::get<0>(attention_packed_fwd(transposed ? qkv.view({1, n, len, 3, H, D}) : qkv.view({1, len, n, 3, H, D}), m, bias, pitch, scale,
+                                                      false, transposed));
+    ln_chain(part, gamma, beta, eps, wg, bg, wo, bo, part.dim() == 3 ? o.view({part.size(0), part.size(1), HD}) : o.view({-1, HD}), part, dst);
+  }
+  return out.unsqueeze(0);
+}
+
+// Triangle multiplication of a square pair tensor [1, n, n, 128].  w / b: projection and gate weights interleaved by rows.  Extents
+// that are no multiple of 8 make the first axis the batch, so that the channels-first tensors get rows at an 8-element pitch (TMA
+// wants 16-byte strides); the padding is neither written nor read.
+OptTensor triangle_module(const Tensor& z0, const Tensor& g1, const Tensor& b1, double eps1, const Tensor& w, const Tensor& b, const Tensor& wg, const Tensor& bg,
+                          const Tensor& g2, const Tensor& b2, double eps2, const Tensor& wo, const Tensor& bo, const Tensor& mask, bool outgoing, bool inplace) {
+  if (!rows_of_channels(z0) || z0.dim() != 4 || z0.size(0) != 1 || z0.size(1) != z0.size(2) || z0.size(3) != 128 ||
+      !all_plain(g1, b1, w, b, wg, bg, g2, b2, wo, bo))
+    return std::nullopt;
+  constexpr int64_t c = 128;
+  const int64_t n = z0.size(1), pitch = (n + 7) / 8 * 8;
+  if (!matrix(w, 4 * c, c) || b.numel() != 4 * c || !matrix(wg, c, c) || bg.numel() != c || !matrix(wo, c, c) || bo.numel() != c || g1.numel() != c ||
+      b1.numel() != c || g2.numel() != c || b2.numel() != c)
+    return std::nullopt;
+  const Tensor z = dense_rows(z0), scale = mask.expand({1, n, n}).reshape({-1});
+  const Tensor lr = at::empty({2 * c, n, pitch}, z.options()), p = at::empty({c, n, pitch}, z.options());
+  const bool flat = pitch == n;
+  const Tensor z3 = flat ? z.view({1, n * n, c}) : z.view({n, n, c});
+  auto cut = [&](const Tensor& t) { return flat ? t.view({t.size(0), 1, n * n}) : t.narrow(2, 0, n); };
+  const Tensor gate = ln_tri_in(z3, g1, b1, eps1, w, b, wg, bg, scale, cut(lr));
+  const Tensor lr_n = lr.narrow(2, 0, n), p_n = p.narrow(2, 0, n);
+  const OptTensor none;
+  gemm(lr_n.narrow(0, 0, c), lr_n.narrow(0, c, c), !outgoing, !outgoing, 1.0, none, ACT_NONE, false, none, none, none, 1, 1, none, false, p_n, false, 1,
+       false, 0, std::nullopt);
+  return ln_tri_out(cut(p), g2, b2, eps2, wo, bo, gate, z3, inplace ? OptTensor(z3) : std::nullopt).view(z.sizes());
+}
+
+// Global column attention of the extra-MSA stack over x [1, S, N, 64], 8 heads of 8 channels
+OptTensor global_column_module(const Tensor& x0, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& wq, const Tensor& wkv, const Tensor& wg,
+                               const Tensor& bg, const Tensor& wo, const OptTensor& bo, const Tensor& mask, double scale, bool inplace) {
+  if (!rows_of_channels(x0) || x0.dim() != 4 || x0.size(0) != 1 || x0.size(3) != 64 || !all_plain(gamma, beta, wq, wkv, wg, bg, wo, bo)) return std::nullopt;
+  if (!matrix(wq, 64, 64) || !matrix(wkv, 16, 64) || !matrix(wg, 64, 64) || bg.numel() != 64 || !matrix(wo, 64, 64) || !vector(bo, 64) || gamma.numel() != 64 ||
+      beta.numel() != 64 || mask.numel() != x0.size(1) * x0.size(2))
+    return std::nullopt;
+  const Tensor x = dense_rows(x0), x2 = x.view({-1, 64});
+  const Tensor kv = *ln_qkv(x2, gamma, beta, eps, wkv, std::nullopt, std::nullopt, false);
+  const Tensor o = global_column(x.view({x.size(1), x.size(2), 64}), gamma, beta, eps, wq, kv, mask, scale);
+  return ln_chain(x2, gamma, beta, eps, wg, bg, wo, bo, o, x2, inplace ? OptTensor(x2) : std::nullopt).view(x.sizes());
+}
+
+// Masked projections of the outer product mean
+std::optional<std::tuple<Tensor, Tensor>> masked_pair(const Tensor& x0, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& wa,
+                                                      const OptTensor& ba, const Tensor& wb, const OptTensor& bb, const Tensor& mask) {
+  if (!rows_of_channels(x0) || !all_plain(gamma, beta, wa, ba, wb, bb)) return std::nullopt;
+  const int64_t C = x0.size(-1);
+  if (!matrix(wa, wa.size(0), C) || !matrix(wb, wb.size(0), C) || !vector(ba, wa.size(0)) || !vector(bb, wb.size(0)) || wa.size(0) % 8 || wb.size(0) % 8 ||
+      wa.size(0) + wb.size(0) + 256 > LN_MAX_COLUMNS || gamma.numel() != C || beta.numel() != C)
+    return std::nullopt;
+  const Tensor x = dense_rows(x0);
+  auto shape = x.sizes().vec();
+  shape.back() = 1;
+  auto [a, b] = ln_pair(x.view({-1, C}), gamma, beta, eps, wa, ba, wb, bb, mask.expand(shape).reshape({-1}));
+  shape.back() = wa.size(0);
+  const Tensor a4 = a.view(shape);
+  shape.back() = wb.size(0);
+  return std::make_tuple(a4, b.view(shape));
+}
+
+// 1 / (mask^T mask + eps) of a mask [1, S, N], as [1, N, N, 1] in fp32; None for other shapes and types
+OptTensor mask_norm(const Tensor& mask, double eps) {
+  const bool half = mask.scalar_type() == at::kBFloat16;
+  if (!mask.is_cuda() || (!half && mask.scalar_type() != at::kFloat) || mask.dim() != 3 || mask.size(0) != 1 || mask.numel() == 0) return std::nullopt;
+  const Tensor m = mask.contiguous();
+  const int64_t S = m.size(1), N = m.size(2);
+  const Tensor out = f32({1, N, N, 1}, m);
+  check(ffb_mask_norm(ptr(m), static_cast<float*>(ptr(out)), (int)S, (int)N, (float)eps, half, stream()), "mask_norm");
+  return out;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_ffb_dispatch, m) {
@@ -601,5 +763,11 @@ PYBIND11_MODULE(_ffb_dispatch, m) {
   m.def("ln_tri_out", &ln_tri_out);
   m.def("ln_pair", &ln_pair);
   m.def("global_column", &global_column);
+  m.def("transition_module", &transition_module);
+  m.def("attention_module", &attention_module);
+  m.def("triangle_module", &triangle_module);
+  m.def("global_column_module", &global_column_module);
+  m.def("masked_pair", &masked_pair);
+  m.def("mask_norm", &mask_norm);
   m.def("launches", []() { return g_launches; });
 }

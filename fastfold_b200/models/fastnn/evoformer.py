@@ -66,9 +66,9 @@ class Evoformer(nn.Module):
 
     def forward(self, m, z, msa_mask, pair_mask, chunk_size=None, _mask_trans=True, _drop=None, _memo=None):
         with memo.use(_memo):
-            return self._forward(m, z, msa_mask, pair_mask, chunk_size, _mask_trans, _drop)
+            return self._forward(m, z, msa_mask, pair_mask, chunk_size, _mask_trans, _drop, _memo)
 
-    def _forward(self, m, z, msa_mask, pair_mask, chunk_size=None, _mask_trans=True, _drop=None):
+    def _forward(self, m, z, msa_mask, pair_mask, chunk_size=None, _mask_trans=True, _drop=None, _memo=None):
         P = core.get_dap_size()
         seq_length = pair_mask.size(-1)
         pad = pad_amount(seq_length, P)
@@ -80,8 +80,10 @@ class Evoformer(nn.Module):
             else:
                 z = pad_or_pass(z.unsqueeze(0), (0, 0, 0, pad, 0, pad))
                 z = scatter(z, dim=1)
-        msa_mask = memo.cached(("pad_msa", pad), (msa_mask,), lambda: F.pad(msa_mask.unsqueeze(0), (0, pad)))
-        pair_mask = memo.cached(("pad_pair", pad), (pair_mask,), lambda: F.pad(pair_mask.unsqueeze(0), (0, pad, 0, pad)))
+        # a block by itself takes masks as they are where there is nothing to add; a stack keeps its own for all blocks
+        pad_mask = pad_or_pass if _memo is None else F.pad
+        msa_mask = memo.cached(("pad_msa", pad), (msa_mask,), lambda: pad_mask(msa_mask.unsqueeze(0), (0, pad)))
+        pair_mask = memo.cached(("pad_pair", pad), (pair_mask,), lambda: pad_mask(pair_mask.unsqueeze(0), (0, pad, 0, pad)))
         if _drop is None and self.training:
             _drop = draw_block_dropout(seq_length + pad, self.c_m, self.c_z, m.device, m.dtype, n_res=seq_length)
         d_msa = None if _drop is None else _drop.get("msa_row")

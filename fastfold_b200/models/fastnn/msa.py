@@ -48,7 +48,9 @@ class MSAColumnAttention(nn.Module):
             strided = M_norm_t is None and self.strided_for(M_raw.shape[1], M_raw)
         mask_t = memo.cached("mask_t", (M_mask,), lambda: M_mask.transpose(-1, -2).contiguous())
         if strided and M_norm_t is None and self.attention.takes_raw(M_raw, self.layernormM, None):
-            return self.attention(M_raw, mask_t, tail=(None, None, M_raw), transposed=True, norm=self.layernormM)[0]
+            out, done = self.attention(M_raw, mask_t, tail=(None, None, M_raw), transposed=True, norm=self.layernormM)
+            if done:
+                return out
         if strided:
             M = self.layernormM(M_raw) if M_norm_t is None else M_norm_t
             tail = (None, None, _residual(M_raw)) if _fusable(M_raw) else None          # the residual joins in the output projection

@@ -149,12 +149,10 @@ class Transition(nn.Module):
 
     def _one_kernel(self, src):
         """Without gradients: LayerNorm, both products and the residual in one kernel (None where it does not apply)."""
-        l1, l2 = self.linear1, self.linear2
-        hidden = l1.weight.shape[0]
-        if hidden % 128 or hidden > ln_gemm.MAX_COLUMNS or not ln_gemm.ready(src, self.norm, (l1, l2), (l1.weight, l1.bias, l2.weight, l2.bias)):
+        norm, l1, l2 = self.norm, self.linear1, self.linear2
+        if not (src.is_cuda and ln_gemm.ready(norm, l1, l2)):
             return None
-        s2 = ln_gemm.dense(src).view(-1, src.shape[-1])
-        return ln_gemm.chain(s2, self.norm, l1.weight, l1.bias, l2.weight, l2.bias, s2, out=_res_out(s2)).view(src.shape)
+        return ln_gemm.transition(src, norm, l1, l2, INPLACE and src.is_contiguous())
 
     def _one(self, src):
         x = self.norm(src)
@@ -277,26 +275,33 @@ class OutProductMean(nn.Module):
 
     def forward(self, M, M_mask, Z_raw):
         la, lb = self.linear_a, self.linear_b
-        both = core.get_dap_size() == 1 and ln_gemm.ready(M, self.layernormM, (la, lb), (la.weight, la.bias, lb.weight, lb.bias))
-        M = ln_gemm.dense(M) if both else self.layernormM(M)
+        single = M.is_cuda and core.get_dap_size() == 1 and ln_gemm.ready(self.layernormM, la, lb)
+        M_norm = None if single else self.layernormM(M)
         src = M_mask                                     # the tensors below depend on the mask only: once per stack call
         M_mask = memo.cached("opm_mask", (src,), lambda: src.unsqueeze(-1))
         M_mask_col = memo.cached("opm_mask_col", (src,), lambda: scatter_mask(M_mask, dim=2))
-        if _OPM_FUSED_GATHER:
-            out = self._fused_gather(M, M_mask, M_mask_col, Z_raw, src)
+        if _OPM_FUSED_GATHER and not single:
+            out = self._fused_gather(M_norm, M_mask, M_mask_col, Z_raw, src)
             if out is not None:
                 return out
         mask_col_a = memo.cached(("opm_mask_col_as", M.dtype), (src,), lambda: M_mask_col.to(M.dtype))
-        if both:                                         # norm, both projections and the mask in one kernel
-            left_act, right_act = ln_gemm.pair(M.view(-1, M.shape[-1]), self.layernormM, la.weight, la.bias, lb.weight, lb.bias,
-                                               mask_col_a.expand(*M.shape[:-1], 1).reshape(-1))
-            left_act, right_act_all, work = left_act.view(*M.shape[:-1], -1), right_act.view(*M.shape[:-1], -1), None
+        # norm, both projections and the mask in one kernel
+        pair = ln_gemm.masked_pair(M, self.layernormM, la, lb, mask_col_a) if single else None
+        if pair is not None:
+            left_act, right_act_all, work = pair[0], pair[1], None
         else:
+            if M_norm is None:
+                M_norm = self.layernormM(M)
             # mask before the gather: identical result, and the gathered operand is ready to use
-            right_act = self._masked(lb, M, mask_col_a)
+            right_act = self._masked(lb, M_norm, mask_col_a)
             right_act_all, work = gather_async(right_act, dim=2)
-            left_act = self._masked(la, M, mask_col_a)
-        inv_norm = memo.cached("opm_inv_norm", (src,), lambda: 1.0 / (torch.einsum("bsid,bsjd->bijd", M_mask_col.float(), M_mask.float()) + 1e-3))
+            left_act = self._masked(la, M_norm, mask_col_a)
+
+        def normaliser():
+            norm = ln_gemm.mask_norm(src, 1e-3) if single else None
+            return norm if norm is not None else 1.0 / (torch.einsum("bsid,bsjd->bijd", M_mask_col.float(), M_mask.float()) + 1e-3)
+
+        inv_norm = memo.cached("opm_inv_norm", (src,), normaliser)
         right_act_all = gather_async_opp(right_act_all, work, dim=2)
         if inv_norm.shape[1:3] != (left_act.shape[2], right_act_all.shape[2]):             # of a mask that broadcasts
             inv_norm = inv_norm.expand(-1, left_act.shape[2], right_act_all.shape[2], -1)
@@ -524,64 +529,32 @@ class SelfAttention(nn.Module):
             return out.reshape(resid.shape), True
         return self.o_linear(o), False
 
-    def takes_raw(self, x, norm, dropmask, *weights):
-        """True when ``forward`` may be given ``x`` and the ``norm`` that it has not been through yet (``norm=``)."""
-        if not (dropmask is None and self.gating and x.dim() == 4 and x.shape[0] == 1 and self.c <= max(flash.FWD_HEAD_DIMS)
-                and self.out_dim == self.qkv_dim == x.shape[-1] and core.get_dap_size() == 1):
-            return False
-        heads = self.n_head * self._padded_dim()
-        if heads % 128 or 3 * heads + 128 > ln_gemm.MAX_COLUMNS:
-            return False
-        mods = (self.to_qkv, self.gating_linear, self.o_linear)
-        return ln_gemm.ready(x, norm, mods, (self.to_qkv.weight, self.gating_linear.weight, self.gating_bias, self.o_linear.weight,
-                                             self.o_linear.bias, *weights))
+    def takes_raw(self, x, norm, dropmask):
+        """True when ``forward`` may be given ``x`` and the ``norm`` that it has not been through yet (``norm=``); it may still
+        turn out that the kernels do not cover the tensors."""
+        return (dropmask is None and x.is_cuda and self.gating and self.c <= 32 and core.get_dap_size() == 1
+                and ln_gemm.ready(norm, self, self.to_qkv, self.gating_linear, self.o_linear))
 
-    def _from_raw(self, x, norm, mask, bias, pair_weight, out_bias, transposed):
-        """``x`` plus the attention over ``norm(x)``, without gradients: one kernel from the rows to QKV (and the pair bias of
-        ``pair_weight``), the attention, and one kernel from the rows and its output to the result.  ``CHUNK_SIZE`` rows
-        (columns with ``transposed``) at a time where that is set."""
-        H, D = self.n_head, self._padded_dim()
+    def _from_raw(self, x, norm, mask, out_bias, transposed, pair_weight, pair):
+        D = self._padded_dim()
         if D == self.c:
-            wq, wg, bg, wo = self.to_qkv.weight, self.gating_linear.weight, self.gating_bias, self.o_linear.weight
+            wq, wo, wg, bg = self.to_qkv.weight, self.o_linear.weight, self.gating_linear.weight, self.gating_bias
         else:
             wq, wg, bg, wo = self._padded_heads(D)
-        x = ln_gemm.dense(x)
-        x3, x2 = x[0], x.view(-1, x.shape[-1])
-        out = x3 if INPLACE else torch.empty_like(x3)
-        n, rows = (x.shape[1], x.shape[2]) if transposed else (x.shape[2], x.shape[1])
-        step = rows if CHUNK_SIZE is None else min(CHUNK_SIZE, rows)
-        buf = None
-        if pair_weight is not None:
-            buf = torch.empty(H, n, (n + 7) // 8 * 8, device=x.device, dtype=x.dtype)[:, :, :n]
-            if step < rows:
-                ln_gemm.qkv(x2, norm, None, pair_weight, buf, transposed)
-            bias = buf.unsqueeze(0)
-        bias5 = None if bias is None else bias.unsqueeze(1)
-        for ax in range(0, rows, step):
-            if step == rows:
-                part, dst, m, shape = x2, out.view(x2.shape), mask, x3.shape[:2]
-                qkv = ln_gemm.qkv(x2, norm, wq, pair_weight, buf, transposed)
-            else:
-                # rows are contiguous: one matrix; columns are not: a batch of them, one per position along the attention
-                sl = (slice(None), slice(ax, ax + step)) if transposed else (slice(ax, ax + step),)
-                part, dst, m = x3[sl], out[sl], None if mask is None else mask[:, ax:ax + step]
-                shape = part.shape[:2]
-                if not transposed:
-                    part, dst = part.view(-1, x.shape[-1]), dst.view(-1, x.shape[-1])
-                qkv = ln_gemm.qkv(part, norm, wq)
-            o = flash.flash_attention_packed(qkv.view(1, *shape, 3, H, D), m, bias5, self.scaling, transposed=transposed)
-            ln_gemm.chain(part, norm, wg, bg, wo, out_bias if out_bias is not None else self.o_linear.bias, part,
-                          mul=o.view(*part.shape[:-1], H * D), out=dst)
-        return out.unsqueeze(0)
+        z, norm_z = (None, None) if pair is None else pair
+        return ln_gemm.attention(x, norm, wq, wg, bg, wo, self.o_linear.bias if out_bias is None else out_bias, mask, self.n_head, D, self.scaling, transposed,
+                                 CHUNK_SIZE, INPLACE and x.is_contiguous(), pair_weight, z, norm_z)
 
-    def forward(self, in_data, mask, nonbatched_bias=None, tail=None, transposed=False, norm=None, pair_weight=None):
+    def forward(self, in_data, mask, nonbatched_bias=None, tail=None, transposed=False, norm=None, pair_weight=None, pair=None):
         """``tail=(out_bias, (mask2d, div, mod) or None, residual)`` lets the output projection absorb the
         bias / dropout / residual that follow it; the second return value says whether it did.
         ``transposed``: attend along dim 1 of ``in_data`` instead of dim 2.
         ``norm``: the LayerNorm that ``in_data``, which is also the residual, still has to go through (``takes_raw`` says whether
-        it may be left to this module); ``pair_weight``: the pair bias is ``norm(in_data) . pair_weight``."""
+        it may be left to this module); ``pair_weight``: the pair bias is ``norm(in_data) . pair_weight``, or with ``pair=(z, norm_z)``
+        ``norm_z(z) . pair_weight``.  The result is then None where the kernels do not cover the tensors."""
         if norm is not None:
-            return self._from_raw(in_data, norm, mask, self._bias(nonbatched_bias), pair_weight, tail[0], transposed), True
+            out = self._from_raw(in_data, norm, mask, tail[0], transposed, pair_weight, pair)
+            return out, out is not None
         bias = self._bias(nonbatched_bias, transposed)
         if CHUNK_SIZE is None or CHUNK_SIZE >= in_data.shape[2 if transposed else 1]:
             return self._one(in_data, mask, bias, tail, transposed)
@@ -664,17 +637,6 @@ def pair_bias_rows(Zn, weight, transposed):
     n_q, n_k, H = a.shape[0], a.shape[1], weight.shape[0]
     buf = torch.empty(H, n_q, (n_k + 7) // 8 * 8, device=Zn.device, dtype=Zn.dtype)[:, :, :n_k]
     K.gemm(a, weight, trans_out=True, out=buf.permute(1, 0, 2))
-    return buf.unsqueeze(0)
-
-
-def pair_bias_raw(Z, norm, weight):
-    """The pair bias ``[1, H, q, k]`` of ``norm(Z)`` for attention over the second axis of ``Z``, in one kernel without gradients;
-    None where that does not apply."""
-    if not (Z.dim() == 4 and Z.shape[0] == 1 and weight.shape[0] <= 32 and core.get_dap_size() == 1 and ln_gemm.ready(Z, norm, (), (weight,))):
-        return None
-    n_q, n_k = Z.shape[1], Z.shape[2]
-    buf = torch.empty(weight.shape[0], n_q, (n_k + 7) // 8 * 8, device=Z.device, dtype=Z.dtype)[:, :, :n_k]
-    ln_gemm.qkv(ln_gemm.dense(Z).view(-1, Z.shape[-1]), norm, None, weight, buf)
     return buf.unsqueeze(0)
 
 
@@ -861,39 +823,14 @@ class _TriangleMultiplication(nn.Module):
                      dmask=None if dropmask is None else _mask_idx(Z_raw, dropmask), resid=zr2, out=_res_out(zr2))
         return out.reshape(Z_raw.shape)
 
-    def _takes_raw(self, Z_raw, dropmask):
-        """True when ``_from_raw`` applies: one GPU, a square pair tensor of 128 channels, no gradients and no dropout mask."""
-        p, g, o = self.left_right_projection, self.left_right_gate, self.output_gate
-        if not (dropmask is None and self.c == self.d_pair == 128 and Z_raw.shape[0] == 1 and Z_raw.shape[1] == Z_raw.shape[2]
-                and core.get_dap_size() == 1):
-            return False
-        n2 = self.layernorm2
-        return ln_gemm.ready(Z_raw, self.layernorm1, (p, g, o, self.output_projection, n2),
-                             (o.weight, o.bias, self.output_projection.weight, self.output_bias, n2.weight, n2.bias, p.weight, g.weight,
-                              p.bias, g.bias))
-
     def _from_raw(self, Z_raw, Z_mask):
-        """Without gradients, from the pair tensor to its update in three kernels: the norm with the gated operands (channels
-        first) and the output gate, the contraction, and the norm over its channels with the output projection, gate and
-        residual.  Extents that are no multiple of 8 make the first axis the batch, so that the channels-first tensors get rows
-        at an 8-element pitch (TMA wants 16-byte strides); the padding is neither written nor read."""
-        c, n = self.c, Z_raw.shape[1]
-        Z_raw = ln_gemm.dense(Z_raw)
+        """Without gradients, from the pair tensor to its update in three kernels (None where they do not apply)."""
+        n1, n2, gate, o = self.layernorm1, self.layernorm2, self.output_gate, self.output_projection
+        if not (self.c == self.d_pair == 128 and core.get_dap_size() == 1
+                and ln_gemm.ready(n1, n2, gate, o, self.left_right_projection, self.left_right_gate)):
+            return None
         w, b = self._glu_weights()
-        mask = Z_mask.expand(1, n, n).reshape(-1)
-        pitch = (n + 7) // 8 * 8
-        lr = torch.empty(2 * c, n, pitch, device=Z_raw.device, dtype=Z_raw.dtype)
-        p = torch.empty(c, n, pitch, device=Z_raw.device, dtype=Z_raw.dtype)
-        z3 = Z_raw.view(1, n * n, -1) if pitch == n else Z_raw.view(n, n, -1)
-        cut = (lambda t: t.view(t.shape[0], 1, n * n)) if pitch == n else (lambda t: t[:, :, :n])
-        g = ln_gemm.tri_in(z3, self.layernorm1, w, b, self.output_gate.weight, self.output_gate.bias, mask, cut(lr))
-        left, right = lr[:c, :, :n], lr[c:, :, :n]
-        if self.outgoing:
-            K.gemm(left, right, out=p[:, :, :n])
-        else:
-            K.gemm(left, right, a_mn=True, b_mn=True, out=p[:, :, :n])
-        out = ln_gemm.tri_out(cut(p), self.layernorm2, self.output_projection.weight, self.output_bias, g, z3, out=_res_out(z3))
-        return out.view(Z_raw.shape)
+        return ln_gemm.triangle(Z_raw, n1, w, b, gate, n2, o.weight, self.output_bias, Z_mask, self.outgoing, INPLACE and Z_raw.is_contiguous())
 
     def _chunked(self, Z_raw, Z_mask):
         """Slab-by-slab evaluation for long sequences: the gathered operand is never materialised.
@@ -957,8 +894,10 @@ class _TriangleMultiplication(nn.Module):
             # taken whenever that is a small part of the GPU's memory.
             if not ((can_fuse or can_fuse_any) and _dense_fits(Z_raw)):
                 return self._chunked(Z_raw, Z_mask)
-        if (can_fuse or can_fuse_any) and Z_norm is None and self._takes_raw(Z_raw, dropmask):
-            return self._from_raw(Z_raw, Z_mask)
+        if (can_fuse or can_fuse_any) and Z_norm is None and dropmask is None and A == B and Z_raw.shape[0] == 1:
+            out = self._from_raw(Z_raw, Z_mask)
+            if out is not None:
+                return out
         if can_fuse_any:
             return self._fused_nograd_any(Z_raw, Z_mask, dropmask, Z_norm)
         if can_fuse:
@@ -1082,11 +1021,11 @@ class _TriangleAttention(nn.Module):
             dropmask = None
         if strided is None:
             strided = self.strided(Z_raw)
-        if (Z_norm is None and (self.starting or strided) and Z_raw.dim() == 4 and Z_raw.shape[1] == Z_raw.shape[2]
-                and not ln_gemm.hooked(self.linear_b) and self.n_head <= 32
-                and self.attention.takes_raw(Z_raw, self.layernorm1, dropmask, self.linear_b.weight, self.out_bias)):
-            return self.attention(Z_raw, mask, None, tail=(self.out_bias, None, Z_raw), transposed=strided, norm=self.layernorm1,
-                                  pair_weight=self.linear_b.weight)[0]
+        if Z_norm is None and (self.starting or strided) and self.attention.takes_raw(Z_raw, self.layernorm1, dropmask) and not ln_gemm.hooked(self.linear_b):
+            out, done = self.attention(Z_raw, mask, tail=(self.out_bias, None, Z_raw), transposed=strided, norm=self.layernorm1,
+                                       pair_weight=self.linear_b.weight)
+            if done:
+                return out
         if Z_norm is not None:
             Z = Z_norm
         else:
@@ -1157,10 +1096,11 @@ class ChunkMSARowAttentionWithPairBias(nn.Module):
             dropmask = F.dropout(torch.ones_like(M_raw[:, 0:1, :, :]), p=self.p_drop, training=True)
         if not training:
             dropmask = None
-        if self.attention.takes_raw(M_raw, self.layernormM, dropmask, self.out_bias):
-            b = pair_bias_raw(Z, self.layernormZ, self.linear_b_weights)
-            if b is not None:
-                return self.attention(M_raw, M_mask, (b, -1), tail=(self.out_bias, None, M_raw), norm=self.layernormM)[0]
+        if self.attention.takes_raw(M_raw, self.layernormM, dropmask) and not ln_gemm.hooked(self.layernormZ):
+            out, done = self.attention(M_raw, M_mask, tail=(self.out_bias, None, M_raw), norm=self.layernormM, pair_weight=self.linear_b_weights,
+                                       pair=(Z, self.layernormZ))
+            if done:
+                return out
         M = self.layernormM(M_raw)
         Zn = self.layernormZ(Z)
         b = pair_bias_hqk(Zn, self.linear_b_weights)
@@ -1195,20 +1135,11 @@ class ChunkMSAColumnGlobalAttention(nn.Module):
     def _from_raw(self, M_raw, M_mask):
         """Without gradients, on the MSA as it is stored: keys and values from the rows, a kernel per column up to its value vector, and
         gate, output projection and residual from the rows again.  None where the kernels do not apply."""
-        ga, (c, h) = self.global_attention, (self.c, self.n_head)
-        if not (c == h == 8 and M_raw.dim() == 4 and M_raw.shape[0] == 1 and M_raw.shape[-1] == 64 and M_mask.shape == M_raw.shape[:-1]
-                and core.get_dap_size() == 1):
+        ga = self.global_attention
+        if not (self.c == self.n_head == 8 and M_raw.is_cuda and M_mask.shape == M_raw.shape[:-1] and core.get_dap_size() == 1
+                and ln_gemm.ready(self.layernormM, ga, ga.to_q, ga.to_kv, ga.gating_linear, ga.o_linear)):
             return None
-        mods = (ga, ga.to_q, ga.to_kv, ga.gating_linear, ga.o_linear)
-        if not ln_gemm.ready(M_raw, self.layernormM, mods, (ga.to_q.weight, ga.to_kv.weight, ga.gating_linear.weight, ga.gating_bias,
-                                                            ga.o_linear.weight, ga.o_linear.bias)):
-            return None
-        M_raw = ln_gemm.dense(M_raw)
-        x2 = M_raw.view(-1, M_raw.shape[-1])
-        kv = ln_gemm.qkv(x2, self.layernormM, ga.to_kv.weight)
-        o = ln_gemm.global_column(M_raw[0], self.layernormM, ga.to_q.weight, kv, M_mask[0], ga.scaling)
-        return ln_gemm.chain(x2, self.layernormM, ga.gating_linear.weight, ga.gating_bias, ga.o_linear.weight, ga.o_linear.bias, x2, mul=o,
-                             out=_res_out(x2)).view(M_raw.shape)
+        return ln_gemm.global_column_attention(M_raw, self.layernormM, ga, M_mask, INPLACE and M_raw.is_contiguous())
 
     def forward(self, M_raw, M_mask):
         out = self._from_raw(M_raw, M_mask)

@@ -1,7 +1,7 @@
 """LayerNorm and the GEMMs that read its rows, in one kernel each (csrc/ln_gemm.cu), without gradients.
 
-The callers (``models/fastnn``) ask ``ready`` first and otherwise compose LayerNorm and GEMM; the two agree up to
-the rounding of the LayerNorm's sums.
+``models/fastnn`` calls whole modules through the native functions below, which return None for tensors that the
+kernels do not cover, and otherwise composes LayerNorm and GEMM; the two agree up to the rounding of the LayerNorm's sums.
 """
 import torch
 from torch.autograd import forward_ad
@@ -9,31 +9,19 @@ from torch.nn.modules import module as _nn_module
 
 from . import _lib
 
-CHANNELS = (64, 128, 256)
-MAX_COLUMNS = 1280          # weight rows of one call (their biases are kept in shared memory)
-
-
 def hooked(mod):
     return bool(mod._forward_hooks or mod._forward_pre_hooks)
 
 
-def ready(x, norm, modules=(), tensors=()):
-    """True when the kernels may stand for ``norm(x)`` and what follows: bf16 activations in GPU memory, contiguous bf16
-    parameters, no gradients or forward-mode level, and no hook on a module that would be passed by."""
-    if torch.is_grad_enabled() or not (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[-1] in CHANNELS and x.numel() > 0):
+def ready(*modules):
+    """True when the kernels may stand for calls of ``modules``: no gradients or forward-mode level, and no hook on a module that
+    would be passed by.  Whether they cover the tensors is checked by the native functions, which return None where not."""
+    if torch.is_grad_enabled() or forward_ad._current_level >= 0 or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
         return False
-    if forward_ad._current_level >= 0 or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
-        return False
-    if hooked(norm) or any(hooked(m) for m in modules):
-        return False
-    return all(t is None or (t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 and t.is_cuda)
-               for t in (norm.weight, norm.bias, *tensors))
-
-
-def dense(x):
-    """``x`` as the kernels address it: contiguous rows on a 16-byte boundary (a copy of anything else)."""
-    x = x.contiguous()
-    return x.clone() if x.data_ptr() % 16 else x
+    for m in modules:
+        if m._forward_hooks or m._forward_pre_hooks:
+            return False
+    return True
 
 
 def chain(x, norm, w1, b1, w2, b2, resid, mul=None, out=None):
@@ -66,3 +54,38 @@ def pair(x, norm, wa, ba, wb, bb, scale):
 def global_column(x, norm, wq, kv, mask, scaling):
     """Value vectors ``[N, 64]`` (fp32) of the global column attention over ``x [S, N, 64]``: one mean query per column and head."""
     return _lib.native().global_column(x, norm.weight, norm.bias, norm.eps, wq, kv, mask, scaling)
+
+
+def transition(x, norm, l1, l2, inplace):
+    return _lib.native().transition_module(x, norm.weight, norm.bias, norm.eps, l1.weight, l1.bias, l2.weight, l2.bias, inplace)
+
+
+def attention(x, norm, wq, wg, bg, wo, bo, mask, H, D, scaling, transposed=False, chunk=None, inplace=False, pair_w=None, z=None, norm_z=None):
+    """``x [1, A, B, C]`` plus the gated attention over ``norm(x)``: one kernel from the rows to QKV (and the pair bias
+    ``pair_w . norm(x)``), the attention, and one kernel from the rows and its output to the result.  With ``z`` the pair bias is
+    ``pair_w . norm_z(z)``."""
+    zg, zb, ze = (None, None, 0.0) if z is None else (norm_z.weight, norm_z.bias, norm_z.eps)
+    return _lib.native().attention_module(x, norm.weight, norm.bias, norm.eps, wq, wg, bg, wo, bo, mask, pair_w, z, zg, zb, ze, H, D, scaling, transposed,
+                                          chunk or 0, inplace)
+
+
+def triangle(z, norm1, w, b, gate, norm2, wo, bo, mask, outgoing, inplace):
+    """Triangle multiplication in three kernels: the norm with the gated operands (channels first) and the output gate, the
+    contraction, and the norm over its channels with the output projection, gate and residual."""
+    return _lib.native().triangle_module(z, norm1.weight, norm1.bias, norm1.eps, w, b, gate.weight, gate.bias, norm2.weight, norm2.bias, norm2.eps, wo, bo,
+                                         mask, outgoing, inplace)
+
+
+def global_column_attention(x, norm, ga, mask, inplace):
+    return _lib.native().global_column_module(x, norm.weight, norm.bias, norm.eps, ga.to_q.weight, ga.to_kv.weight, ga.gating_linear.weight, ga.gating_bias,
+                                              ga.o_linear.weight, ga.o_linear.bias, mask, ga.scaling, inplace)
+
+
+def masked_pair(x, norm, la, lb, mask):
+    """``la(norm(x)) * mask`` and ``lb(norm(x)) * mask`` with one mask value per row, or None."""
+    return _lib.native().masked_pair(x, norm.weight, norm.bias, norm.eps, la.weight, la.bias, lb.weight, lb.bias, mask)
+
+
+def mask_norm(mask, eps):
+    """``1 / (mask^T mask + eps)`` of ``mask [1, S, N]`` as ``[1, N, N, 1]`` in fp32, or None."""
+    return _lib.native().mask_norm(mask, eps)

@@ -49,7 +49,6 @@ def test_chains(C, M, device_status):
     with torch.no_grad():
         x, norm, H = _randn(M, C), _norm(C), 4 * C
         w1, b1, w2, b2 = _randn(H, C, scale=C ** -0.5), _randn(H, scale=0.1), _randn(C, H, scale=H ** -0.5), _randn(C, scale=0.1)
-        assert ln_gemm.ready(x, norm, (), (w1, b1, w2, b2))
         X = _ln(x, norm)
         _close(ln_gemm.chain(x, norm, w1, b1, w2, b2, x), x.double() + _lin(torch.relu(_lin(X, w1, b1)).bfloat16().double(), w2, b2))
         for G in (128, 256):
@@ -103,6 +102,19 @@ def test_pair_of_projections(C, M, dtype, device_status):
             _close(y, _lin(_ln(x, norm), w, b) * s.double()[:, None])
 
 
+@pytest.mark.parametrize("S,N", [(1, 1), (7, 64), (32, 65), (33, 130), (100, 200)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_mask_normaliser(S, N, dtype, device_status):
+    """fp32 sums of at most 100 products of values in [0, 1], one reciprocal: 100 x 2^-24 relative, and 2 ulp."""
+    torch.manual_seed(N)
+    mask = torch.rand(1, S, N, device=DEV).to(dtype)
+    ref = 1.0 / (mask[0].double().t() @ mask[0].double() + 1e-3)
+    out = ln_gemm.mask_norm(mask, 1e-3)
+    assert out.shape == (1, N, N, 1)
+    assert ((out[0, :, :, 0].double() - ref).abs() <= 1e-5 * ref).all()
+    assert ln_gemm.mask_norm(mask[0], 1e-3) is None and ln_gemm.mask_norm(mask.double(), 1e-3) is None
+
+
 def _randomise(net):
     for p in net.parameters():
         p.copy_(torch.randn_like(p) * (p.shape[-1] ** -0.5 if p.dim() == 2 else 0.1) + (1.0 if p.dim() == 1 and p.float().mean() > 0.5 else 0.0))
@@ -118,7 +130,7 @@ def test_triangle_multiplication(cls, n, device_status):
     with torch.no_grad():
         _randomise(net)
         z, mask = _randn(1, n, n, 128), (torch.rand(1, n, n, device=DEV) > 0.2).to(torch.bfloat16)
-        assert net._takes_raw(z, None)
+        assert net._from_raw(z, mask) is not None
         P = {k: v.double() for k, v in net.named_parameters()}
         lin = lambda x, name: torch.nn.functional.linear(x, P[name + ".weight"], P.get(name + ".bias"))  # noqa: E731
         ln = lambda x, name: torch.nn.functional.layer_norm(x, (128,), P[name + ".weight"], P[name + ".bias"], 1e-5)  # noqa: E731
@@ -153,21 +165,46 @@ def test_global_column_attention(S, N, device_status):
 
 
 def test_calls_that_stay_with_the_composition():
-    norm = _norm(128)
-    x = _randn(64, 128)
+    """What the kernels do not cover goes the way of the separate kernels: None from the native functions, or `ready` says no."""
     with torch.no_grad():
-        assert ln_gemm.ready(x, norm)
-        assert not ln_gemm.ready(x.float(), norm)
-        assert not ln_gemm.ready(x[:0], norm)
-        for odd in (x.t().contiguous().t(), _randn(64 * 128 + 4)[4:].view(64, 128)):  # channels not adjacent, off a 16-byte boundary
-            d = ln_gemm.dense(odd)
-            assert d.is_contiguous() and d.data_ptr() % 16 == 0 and torch.equal(d, odd)
-        assert not ln_gemm.ready(x, norm, (), (_randn(256, 128)[::2],))
-        assert not ln_gemm.ready(x, norm, (), (torch.ones(128, device=DEV),))
-        handle = norm.register_forward_hook(lambda *a: None)
-        assert not ln_gemm.ready(x, norm)
+        net = fops.Transition(128).to(DEV, torch.bfloat16)
+        x = _randn(1, 6, 7, 128)
+        assert net._one_kernel(x) is not None
+        assert net._one_kernel(x.float()) is None
+        assert net._one_kernel(x[:0]) is None
+        assert net._one_kernel(x[..., :96]) is None
+        assert ln_gemm.transition(x, LayerNorm(128).to(DEV), net.linear1, net.linear2, False) is None            # fp32 norm
+        for odd in (x.transpose(1, 3).contiguous().transpose(1, 3), _randn(6 * 7 * 128 + 4)[4:].view(1, 6, 7, 128)):
+            assert torch.equal(net(odd), net(odd.clone(memory_format=torch.contiguous_format)))
+        handle = net.linear1.register_forward_hook(lambda *a: None)
+        assert net._one_kernel(x) is None
         handle.remove()
-        assert ln_gemm.ready(x, norm)
+        assert net._one_kernel(x) is not None
         with torch.autograd.forward_ad.dual_level():
-            assert not ln_gemm.ready(x, norm)
-    assert not ln_gemm.ready(x, norm)                                                # gradients
+            assert net._one_kernel(x) is None
+    assert net._one_kernel(x) is None                                                # gradients
+
+
+@pytest.mark.parametrize("n", [24, 100])
+@pytest.mark.parametrize("chunk", [None, 16, 64])
+@pytest.mark.parametrize("cls", [fops.ChunkTriangleAttentionStartingNode, fops.ChunkTriangleAttentionEndingNode])
+def test_triangle_attention(cls, chunk, n, device_status):
+    """Whole and in chunks of rows / columns, in place and not, against the composition from separate kernels: roundings of a
+    different LayerNorm sum only (2^-9 of a normalised value) on an update of about the residual's size."""
+    torch.manual_seed(n)
+    net = cls(128, p_drop=0.25, c=32, n_head=4).to(DEV, torch.bfloat16).eval().requires_grad_(False)
+    z, mask = _randn(1, n, n, 128), (torch.rand(1, n, n, device=DEV) > 0.2).to(torch.bfloat16)
+    with torch.no_grad():
+        _randomise(net)
+        handle = net.linear_b.register_forward_hook(lambda *a: None)
+        ref = net(z, mask)
+        handle.remove()
+        fops.set_chunk_size(chunk)
+        try:
+            _close(net(z, mask), ref.double())
+            held = z.clone()
+            out = net.inplace([held], mask)[0]
+            assert out.data_ptr() == held.data_ptr()
+            _close(out, ref.double())
+        finally:
+            fops.set_chunk_size(None)
