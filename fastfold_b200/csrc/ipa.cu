@@ -1,6 +1,6 @@
 // Invariant point attention core (AlphaFold Algorithm 22, lines 7-11) as one flash-style kernel.
 //
-// For every query residue i (two or four per CTA) the kernel streams the keys j in chunks and keeps, per head h,
+// For every query residue i (four per CTA) the kernel streams the keys j in chunks and keeps, per head h,
 // an online softmax over
 //     logit[h][j] = w_C * q_i.k_j  +  sqrt(1/3) * (z[i][j] . W_b[h] + b_b[h])
 //                   - 0.5 * gamma_h * sum_p |q_pt[i][h][p] - k_pt[j][h][p]|^2  +  inf * (mask_i * mask_j - 1)
@@ -55,12 +55,12 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool i
 // What bounds it: instruction issue (about 50 issue slots x SM sub-partition per (query, key) pair for all heads) and, below
 // some 150 CTAs, the number of SMs in use.  One row per CTA with one key-value read per row, which this replaces, spent its
 // time waiting for L2: every row re-read 3.2 KB of keys, values and points per key, a quarter of the warps in flight.
-// R = 2 with two CTAs per SM below 1024 rows; R = 4, with half the key / value traffic, from there on.
+// Four rows at every length: a CTA with two, and two of those per SM, read keys and values twice as often and were slower even
+// where four rows leave SMs idle.
 //   Measured (B200, the core alone, us, R = 2 / R = 4): N = 256 90 / 78, 512 192 / 171, 768 592 / 525, 1024 792 / 740,
-//   1184 966 / 869, 1536 1796 / 1659, 2048 3207 / 2967; one row per CTA took 349 at 512.  So R = 4 would be the better choice
-//   below the line too, where its fewer CTAs had been expected to leave SMs idle: 8 - 13 % of the core there.
+//   1184 966 / 869, 1536 1796 / 1659, 2048 3207 / 2967; one row per CTA took 349 at 512.
 template <int R, int H, int C, int PQ, int PV, int CZ>
-__global__ void __launch_bounds__(IPA_THREADS, R == 2 ? 2 : 1) ipa_fwd_kernel(const IpaArgs a) {
+__global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   static_assert(H * 32 == IPA_THREADS && CZ == 128, "one warp per head");
@@ -443,7 +443,7 @@ int ffb_ipa_fwd(const float* q, const float* k, const float* v, const float* q_p
   a.N = N; a.H = H; a.C = C; a.Pq = Pq; a.Pv = Pv; a.CZ = CZ; a.row0 = row0; a.rows = rows;
   a.w_c = w_c; a.w_b = w_b; a.inf = inf;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  return rows >= 1024 ? ipa_launch<4>(a, st) : ipa_launch<2>(a, st);
+  return ipa_launch<4>(a, st);
 }
 
 }  // extern "C"
