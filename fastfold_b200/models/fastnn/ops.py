@@ -214,8 +214,9 @@ class OutProductMean(nn.Module):
             mask = mask.expand(*M.shape[:-1], 1)
         return K.gemm(M2, proj.weight, bias=proj.bias, rowscale=mask.reshape(-1)).view(*M.shape[:-1], -1)
 
-    def _outer(self, left, right_all, inv_norm, Z_raw):
-        """left [1,S,ni,d], right_all [1,S,N,e] -> Z_raw + o_linear(outer) * inv_norm."""
+    def _outer(self, left, right_all, inv_norm, Z_raw, out=None):
+        """left [1,S,ni,d], right_all [1,S,N,e] -> Z_raw + o_linear(outer) * inv_norm; without gradients into ``out`` where that is
+        given and the kernels apply."""
         S, ni, d = left.shape[1], left.shape[2], left.shape[3]
         N, e = right_all.shape[2], right_all.shape[3]
         l2 = left.reshape(S, ni * d)
@@ -230,7 +231,8 @@ class OutProductMean(nn.Module):
             if need_grad:
                 out = _OpmCore.apply(l2, r2, self.o_linear.weight, self.o_linear.bias, inv_norm.reshape(-1), Z_raw.reshape(ni * N, -1))
             else:
-                out = _opm_forward(l2, r2, self.o_linear.weight, self.o_linear.bias, inv_norm.reshape(-1), _residual(Z_raw).reshape(ni * N, -1))[0]
+                out = _opm_forward(l2, r2, self.o_linear.weight, self.o_linear.bias, inv_norm.reshape(-1), _residual(Z_raw).reshape(ni * N, -1),
+                                   None if out is None else out.view(ni * N, -1))[0]
             return out.reshape(Z_raw.shape)
         if left.is_cuda and left.dtype == torch.bfloat16 and (ni * d) % 8 == 0 and (N * e) % 64 == 0 and ni * d >= 64:
             o = K.gemm(l2, r2, a_mn=True, b_mn=True) if not torch.is_grad_enabled() else _bmm_tn(l2, r2)
@@ -309,9 +311,11 @@ class OutProductMean(nn.Module):
             return self._outer(left_act, right_act_all, inv_norm, Z_raw)
         out = Z_raw if INPLACE else torch.empty_like(Z_raw)
         for ax in range(0, left_act.shape[2], CHUNK_SIZE):
-            zpart = Z_raw[:, ax:ax + CHUNK_SIZE]
-            res = self._outer(left_act[:, :, ax:ax + CHUNK_SIZE].contiguous(), right_act_all, inv_norm[:, ax:ax + CHUNK_SIZE], zpart)
-            if res.data_ptr() != zpart.data_ptr():
+            # the GEMM reads its columns of the left factor through their strides and writes its rows of the result
+            zpart, opart = Z_raw[:, ax:ax + CHUNK_SIZE], out[:, ax:ax + CHUNK_SIZE]
+            res = self._outer(left_act[:, :, ax:ax + CHUNK_SIZE], right_act_all, inv_norm[:, ax:ax + CHUNK_SIZE], zpart,
+                              opart if opart.is_contiguous() and not torch.is_grad_enabled() else None)
+            if res.data_ptr() != opart.data_ptr():
                 out[:, ax:ax + CHUNK_SIZE] = res
         return out
 
@@ -321,12 +325,14 @@ class OutProductMean(nn.Module):
         return Z_raw
 
 
-def _opm_forward(l2, r2, w, bias, inv_norm, z2):
+def _opm_forward(l2, r2, w, bias, inv_norm, z2, out=None):
     """o4 [i, j, d, e] = sum_s l2[s, (i d)] r2[s, (j e)];  out = z2 + inv_norm * (o4 W^T + bias)."""
     S = l2.shape[0]
     ni, N = l2.shape[1] // 32, r2.shape[1] // 32
     o4 = K.gemm(l2, r2, a_mn=True, b_mn=True, block_out=((ni * N, 1024), 1, N * 1024, 0, 1024))
-    out = K.gemm(o4, w, bias=bias, rowscale=inv_norm, resid=z2, out=_res_out(z2) if not torch.is_grad_enabled() else None)
+    if out is None and not torch.is_grad_enabled():
+        out = _res_out(z2)
+    out = K.gemm(o4, w, bias=bias, rowscale=inv_norm, resid=z2, out=out)
     return out, o4
 
 
