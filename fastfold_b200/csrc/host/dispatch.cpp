@@ -683,7 +683,7 @@ OptTensor triangle_module(const Tensor& z0, const Tensor& g1, const Tensor& b1, 
   if (!matrix(w, 4 * c, c) || b.numel() != 4 * c || !matrix(wg, c, c) || bg.numel() != c || !matrix(wo, c, c) || bo.numel() != c || g1.numel() != c ||
       b1.numel() != c || g2.numel() != c || b2.numel() != c)
     return std::nullopt;
-  const Tensor z = dense_rows(z0), scale = mask.expand({1, n, n}).reshape({-1});
+  const Tensor z = dense_rows(z0), scale = mask.numel() == n * n ? mask.reshape({-1}) : mask.expand({1, n, n}).reshape({-1});
   const Tensor lr = at::empty({2 * c, n, pitch}, z.options()), p = at::empty({c, n, pitch}, z.options());
   const bool flat = pitch == n;
   const Tensor z3 = flat ? z.view({1, n * n, c}) : z.view({n, n, c});
@@ -720,7 +720,8 @@ std::optional<std::tuple<Tensor, Tensor>> masked_pair(const Tensor& x0, const Te
   const Tensor x = dense_rows(x0);
   auto shape = x.sizes().vec();
   shape.back() = 1;
-  auto [a, b] = ln_pair(x.view({-1, C}), gamma, beta, eps, wa, ba, wb, bb, mask.expand(shape).reshape({-1}));
+  const Tensor factors = mask.numel() == x.numel() / C ? mask.reshape({-1}) : mask.expand(shape).reshape({-1});
+  auto [a, b] = ln_pair(x.view({-1, C}), gamma, beta, eps, wa, ba, wb, bb, factors);
   shape.back() = wa.size(0);
   const Tensor a4 = a.view(shape);
   shape.back() = wb.size(0);

@@ -117,6 +117,7 @@ class DropoutColumnwise(nn.Module):
         return x * F.dropout(torch.ones_like(x[:, :, 0:1, :]), p=self.p, training=self.training)
 
 
+@ln_gemm.stands_for
 class Linear(nn.Linear):
     """nn.Linear with AlphaFold initialisers, evaluated by the tcgen05 GEMM on CUDA bf16 tensors."""
 
@@ -382,6 +383,7 @@ def _key_contiguous(b):
     return buf.copy_(b)
 
 
+@ln_gemm.stands_for
 class SelfAttention(nn.Module):
     """Multi-head gated self attention on ``[b1, b2, n, c]`` (attention along ``n``)."""
 
@@ -646,6 +648,7 @@ def pair_bias_rows(Zn, weight, transposed):
     return buf.unsqueeze(0)
 
 
+@ln_gemm.stands_for
 class GlobalAttention(nn.Module):
     """Column-wise global attention of the extra-MSA stack: one mean-pooled query per column."""
 

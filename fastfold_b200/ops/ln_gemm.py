@@ -8,18 +8,28 @@ from torch.autograd import forward_ad
 from torch.nn.modules import module as _nn_module
 
 from . import _lib
+from .layer_norm import LayerNorm
+
+_known = {LayerNorm}
+
+
+def stands_for(cls):
+    """Class decorator: ``ready`` takes modules of exactly this class for what their parameters say."""
+    _known.add(cls)
+    return cls
 
 def hooked(mod):
     return bool(mod._forward_hooks or mod._forward_pre_hooks)
 
 
 def ready(*modules):
-    """True when the kernels may stand for calls of ``modules``: no gradients or forward-mode level, and no hook on a module that
-    would be passed by.  Whether they cover the tensors is checked by the native functions, which return None where not."""
+    """True when the kernels may stand for calls of ``modules``: no gradients or forward-mode level, and each of the modules that
+    would be passed by is one of this package's own, unchanged - no subclass, parametrisation, replaced ``forward`` or hook.
+    Whether the kernels cover the tensors is checked by the native functions, which return None where not."""
     if torch.is_grad_enabled() or forward_ad._current_level >= 0 or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
         return False
     for m in modules:
-        if m._forward_hooks or m._forward_pre_hooks:
+        if type(m) not in _known or m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
             return False
     return True
 

@@ -142,6 +142,19 @@ def test_triangle_multiplication(cls, n, device_status):
         assert (out.double() - ref).norm() <= 4 * TOL * ref.norm()
 
 
+@pytest.mark.parametrize("n", [16, 27])
+def test_masks_of_other_shapes(n, device_status):
+    """A mask with an axis more, and one that broadcasts, give what the mask of the pair tensor's shape gives."""
+    torch.manual_seed(n)
+    net = fops.AsyncChunkTriangleMultiplicationOutgoing(128, p_drop=0.25).to(DEV, torch.bfloat16).eval().requires_grad_(False)
+    with torch.no_grad():
+        _randomise(net)
+        z, row = _randn(1, n, n, 128), (torch.rand(1, 1, n, device=DEV) > 0.2).to(torch.bfloat16)
+        whole = row.expand(1, n, n).contiguous()
+        ref = net._from_raw(z, whole)
+        assert torch.equal(net._from_raw(z, whole[None]), ref) and torch.equal(net._from_raw(z, row), ref)
+
+
 @pytest.mark.parametrize("S,N", [(1, 3), (5, 40), (31, 8), (130, 33), (700, 17)])
 def test_global_column_attention(S, N, device_status):
     """The layer against the same in 64 bits, with masked sequences and a wholly masked column.  Bound as above, once for the gated
@@ -182,6 +195,18 @@ def test_calls_that_stay_with_the_composition():
         assert net._one_kernel(x) is not None
         with torch.autograd.forward_ad.dual_level():
             assert net._one_kernel(x) is None
+
+        class Doubled(fops.Linear):
+            def forward(self, x, act=None):
+                return 2 * super().forward(x, act)
+
+        plain, net.linear1 = net.linear1, Doubled(128, 512).to(DEV, torch.bfloat16)                              # a module of another class
+        assert net._one_kernel(x) is None
+        net.linear1 = plain
+        net.norm.forward = lambda x: x                                               # a replaced forward
+        assert net._one_kernel(x) is None
+        del net.norm.forward
+        assert net._one_kernel(x) is not None
     assert net._one_kernel(x) is None                                                # gradients
 
 
