@@ -510,6 +510,8 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
     const uint32_t stg_u = smem_u32(stg), my_ld = ld_bar + 8 * (warp - 4);
     const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
     uint32_t c1 = 0, t = 0, ld_phase = 0;
+    uint32_t ob = 0;                            // projections: byte offset of the staging tile of the next store
+    constexpr uint32_t OTHER = Cfg::TILES == 2 ? 4096 : 0;
     bool ok = true;
     auto wait = [&](uint32_t bar, uint32_t parity, int code) -> bool {
       ok = __all_sync(0xffffffffu, mbar_wait(bar, parity));
@@ -655,17 +657,17 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
           const LgSeg sg = a.seg[seg];
           const int mycol = col + half * 64, b = c1 % NACC;
           const bool work = mycol < sg.n && valid;
-          const uint32_t ob = Cfg::TILES == 2 ? (c1 & 1) : 0;
-          uint8_t* obuf = stg + ob * 4096;
-          const uint32_t obuf_u = stg_u + ob * 4096;
+          uint8_t* obuf = stg + ob;
           const bool fused = a.has_mul != 0 && seg == 0;        // mul and residual tiles (two staging tiles; first segment)
-          if (work && lane == 0) {
+          // The tiles alternate by the stores that this warp has issued, not by chunks: with all but the newest store done reading,
+          // the other tile is free.  Chunks without a store (pair bias, columns or rows past the end) would break the alternation
+          if (work && sg.kind != LN_PAIR_BIAS && lane == 0) {
             if (fused || Cfg::TILES == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
             if (fused) {
               mbar_expect_tx(my_ld, 8192);
-              tma_load_3d(obuf_u, &maps.resid, my_ld, mycol, row0, batch);
-              tma_load_3d(stg_u + (ob ^ 1) * 4096, &maps.mul, my_ld, mycol, row0, batch);
+              tma_load_3d(stg_u + ob, &maps.resid, my_ld, mycol, row0, batch);
+              tma_load_3d(stg_u + (ob ^ OTHER), &maps.mul, my_ld, mycol, row0, batch);
             }
           }
           __syncwarp();
@@ -692,7 +694,8 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
                 for (int j = 0; j < 32; ++j) o[j * 32] = __float2bfloat16(v[2 * j] * sigmoidf_(v[2 * j + 1]) * rs);
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) lg_store_tile(&maps.out[seg], obuf_u, row0, mycol >> 1, batch);
+                if (lane == 0) lg_store_tile(&maps.out[seg], stg_u + ob, row0, mycol >> 1, batch);
+                ob ^= OTHER;
               } else {
                 if (sg.act == ACT_SIGMOID) {
 #pragma unroll
@@ -705,10 +708,11 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
                 if (fused) {
                   if (!wait(my_ld, ld_phase, ST_TIMEOUT_TMA)) break;
                   ld_phase ^= 1;
-                  mul_tile(stg + (ob ^ 1) * 4096, v);
+                  mul_tile(stg + (ob ^ OTHER), v);
                 }
                 write_tile(obuf, v, fused);
-                if (lane == 0) lg_store_tile(&maps.out[seg], obuf_u, mycol, row0, batch);
+                if (lane == 0) lg_store_tile(&maps.out[seg], stg_u + ob, mycol, row0, batch);
+                ob ^= OTHER;
               }
             }
           }

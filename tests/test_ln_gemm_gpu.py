@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from fastfold_b200.models.fastnn import ops as fops
-from fastfold_b200.ops import LayerNorm, ln_gemm
+from fastfold_b200.ops import LayerNorm, _lib, ln_gemm
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -88,6 +88,57 @@ def test_qkv_and_pair_bias(C, n, transposed, device_status):
         _close(y.view(n, n, -1), _lin(X, w))
         _close(buf[:, :, :n], _lin(X, wb).permute(2, 1, 0) if transposed else _lin(X, wb).permute(2, 0, 1))
         assert (buf[:, :, n:] == 7.0).all()
+
+
+def _close_blocks(a, ref, rows=32, cols=64):
+    """The bound in the 2-norm, for every tile that an epilogue warp stores: one that holds values of another stays far below it in the whole."""
+    pad = (0, -a.shape[1] % cols, 0, -a.shape[0] % rows)
+    cut = lambda t: torch.nn.functional.pad(t.double(), pad).unfold(0, rows, rows).unfold(1, cols, cols)  # noqa: E731
+    assert ((cut(a) - cut(ref)).norm(dim=(2, 3)) <= TOL * cut(ref).norm(dim=(2, 3))).all()
+
+
+@pytest.mark.parametrize("C,n", [(64, 203), (128, 203), (128, 256), (128, 389)])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_tiles_without_a_store(C, n, transposed, device_status):
+    """Two to eight tiles per CTA, one chunk of four without a store (the pair bias) and a last tile that ends between two warps: the
+    staging tiles are filled again in another order than one by one.  The same bits every time."""
+    torch.manual_seed(n)
+    with torch.no_grad():
+        z, norm, w, wb = _randn(n * n, C), _norm(C), _randn(384, C, scale=C ** -0.5), _randn(4, C, scale=C ** -0.5)
+        X = _ln(z, norm)
+        ref, ref_b = _lin(X, w), _lin(X, wb).view(n, n, 4)
+        first = None
+        for _ in range(6):
+            bias = torch.empty(4, n, (n + 7) // 8 * 8, device=DEV, dtype=torch.bfloat16)[:, :, :n]
+            y = ln_gemm.qkv(z, norm, w, wb, bias, transposed)
+            if first is None:
+                first = (y, bias)
+                _close_blocks(y, ref)
+                _close(bias, ref_b.permute(2, 1, 0) if transposed else ref_b.permute(2, 0, 1))
+            assert torch.equal(y, first[0]) and torch.equal(bias, first[1])
+
+
+@pytest.mark.parametrize("n", [131, 203, 301])
+def test_partial_tiles_in_batches(n, device_status):
+    """Odd lengths of the triangle multiplication: five chunks a tile, a partial tile in every row of the pair tensor whose last warps
+    store nothing, several tiles per CTA.  The gated operands against 64 bits, block by block; the same bits every time."""
+    torch.manual_seed(n)
+    with torch.no_grad():
+        z, norm, w, b = _randn(n, n, 128), _norm(128), _randn(512, 128, scale=0.09), _randn(512, scale=0.1)
+        wg, bg, mask = _randn(128, 128, scale=0.09), _randn(128, scale=0.1), (torch.rand(n * n, device=DEV) > 0.2).to(torch.bfloat16)
+        X = _ln(z, norm)
+        pre = _lin(X, w, b)
+        lr_ref = (pre[..., 0::2] * torch.sigmoid(pre[..., 1::2]) * mask.double().view(n, n, 1)).permute(2, 0, 1)
+        first = None
+        for _ in range(6):
+            lr = torch.zeros(256, n, (n + 7) // 8 * 8, device=DEV, dtype=torch.bfloat16)[:, :, :n]
+            gate = _lib.native().ln_tri_in(z, norm.weight, norm.bias, norm.eps, w, b, wg, bg, mask, lr)
+            if first is None:
+                first = (lr, gate)
+                for i in range(n):
+                    _close_blocks(lr[:, i], lr_ref[:, i], 32, 32)
+                _close_blocks(gate.view(n * n, 128), torch.sigmoid(_lin(X, wg, bg)).view(n * n, 128))
+            assert torch.equal(lr, first[0]) and torch.equal(gate, first[1])
 
 
 @pytest.mark.parametrize("M,dtype", [(3, torch.bfloat16), (300, torch.float32), (5000, torch.bfloat16)])
