@@ -262,6 +262,13 @@ __device__ __forceinline__ void lg_norm_columns(uint8_t* tile, int t, float2* pa
   });
 }
 
+// Whether `ok` holds in all four LayerNorm warps.
+__device__ __forceinline__ bool lg_norm_warps_agree(bool ok) {
+  uint32_t all;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(all) : "r"((uint32_t)ok) : "memory");
+  return all != 0;
+}
+
 __device__ __forceinline__ void lg_store_tile(const CUtensorMap* map, uint32_t smem, int x, int y, int z) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(smem), "r"(x), "r"(y), "r"(z) : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -346,6 +353,8 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
     for (int tile = blockIdx.x; tile < a.num_tiles; tile += gridDim.x, ++t) {
       const uint32_t s = t % NA;
       ok = __all_sync(0xffffffffu, mbar_wait(x_full + 8 * s, (t / NA) & 1));
+      // lg_norm_columns has barriers across the four warps: all of them take the tile, or none does and each leaves here
+      if (CF) ok = lg_norm_warps_agree(ok);
       if (!ok) break;
       uint8_t* At = sm + Cfg::A0 + s * Cfg::A_BYTES;
       if (CF) lg_norm_columns(At, threadIdx.x, part, gamma, beta, a.eps);
