@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16
 #pragma unroll
         for (int i = 0; i < 8; ++i) t += v[i];
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);           // as the LayerNorm kernel sums a row
         const float mean = t * (1.f / GC_HC);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16
           q = fmaf(v[i], v[i], q);
         }
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+        for (int o = 4; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
         const float rstd = rsqrtf(q * (1.f / GC_HC) + eps);
         cnt += mk[u];
         if (s0 + (lane >> 3) + u * WARPS * 4 < S) {             // an unnormalisable masked row counts as it would in a product with its mask

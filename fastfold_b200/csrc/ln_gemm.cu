@@ -80,7 +80,7 @@ struct LgCfg {
   static constexpr int NACC = MODE == LN_PROJECT ? 4 : (C == 256 ? 2 : 3);      // 128-column accumulators of the first product
   static constexpr int ACC2 = NACC * 128;                            // tensor-memory column of the second product's accumulator
   static constexpr int A0 = 0, W0 = NA * A_BYTES, STG = W0 + RING * LG_BOX, VEC = STG + LG_EPI * TILES * 4096;
-  static constexpr int VEC_FLOATS = 2 * C + LG_MAX_N + 256 + (MODE == LN_PROJECT ? 512 : 0);     // gamma, beta, biases, channel sums
+  static constexpr int VEC_FLOATS = 2 * C + LG_MAX_N + 256 + (MODE == LN_PROJECT ? 1280 : 0);     // gamma, beta, biases, channel sums
   static constexpr int BARS = VEC + VEC_FLOATS * 4;
   static constexpr int SMEM = BARS + 512 + 1024;
   static_assert(SMEM <= 232448, "shared memory");
@@ -133,91 +133,151 @@ __device__ __forceinline__ uint32_t lg_pack2v(uint64_t v) {
 }
 
 // One row of a [kb][128 rows][64] swizzled tile, in place.  A warp per scheduler does this, so what counts are its instructions and
-// the independent ones among them: two-wide arithmetic and four partial sums.  64 channels stay in registers (packed) between the
-// mean, the variance and the result; with more they would be spilled, and the three sweeps read shared memory.
+// the independent ones among them: two-wide arithmetic in four chains.
+// The sums are taken in the order of the LayerNorm kernel (ln_fwd_mr_kernel: eight channels per lane one by one, then lanes half a row
+// apart, a quarter apart, ...), so that both give the same bits; the two halves of a pair of floats are the same channel of two pieces of
+// eight channels.  Against sums in whatever order suits the registers (us, in a graph with the kernels around them): MSA half of a block of
+// 128 x 256 246.9 -> 248.9, pair half 376.2 -> 375.9, extra-MSA core of 1024 x 256 617 -> 619.
 template <int C>
 __device__ __forceinline__ void lg_norm_row(uint8_t* tile, int row, const float* gamma, const float* beta, float eps) {
   constexpr int KB = C / 64;
-  constexpr bool KEEP = C <= 64;
   uint8_t* p = tile + row * 128;
   const int x = row & 7;
-  uint4 raw[8];
-  auto load = [&](int kb) {
+  auto load = [&](uint4 (&raw)[8], int kb) {
 #pragma unroll
     for (int u = 0; u < 8; ++u) raw[u] = *reinterpret_cast<const uint4*>(p + kb * 16384 + ((u ^ x) << 4));
   };
-  // keeps the compiler from holding the unpacked row (twice the registers) from one sweep to the next
-  auto sweep = [&]() {
-    if (KEEP) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) asm volatile("" : "+r"(raw[i].x), "+r"(raw[i].y), "+r"(raw[i].z), "+r"(raw[i].w));
-    } else {
-      asm volatile("" ::: "memory");
-    }
+  // the first and the second channel of word w of two pieces
+  auto word = [](const uint4& v, int w) { return w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w; };
+  auto even = [&](const uint4& a, const uint4& b, int w) { return lg_pair(__uint_as_float(word(a, w) << 16), __uint_as_float(word(b, w) << 16)); };
+  auto odd = [&](const uint4& a, const uint4& b, int w) {
+    return lg_pair(__uint_as_float(word(a, w) & 0xffff0000u), __uint_as_float(word(b, w) & 0xffff0000u));
   };
-  uint64_t s[4], q[4];
+  if constexpr (KB == 1) {
+    // the row stays unpacked in registers: pieces 2 h and 2 h + 1 side by side, gamma and beta too
+    uint4 raw[8];
+    load(raw, 0);
+    uint64_t v[4][8], t[4];
+    auto fold = [&]() {
+      const float2 f = lg_split(lg_add2(lg_add2(t[0], t[2]), lg_add2(t[1], t[3])));
+      return f.x + f.y;
+    };
 #pragma unroll
-  for (int i = 0; i < 4; ++i) s[i] = q[i] = lg_pair(0.f, 0.f);
-#pragma unroll 1
-  for (int kb = 0; kb < KB; ++kb) {
-    load(kb);
+    for (int h = 0; h < 4; ++h) {
+      t[h] = lg_pair(0.f, 0.f);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      s[0] = lg_add2(s[0], lg_bf2(raw[u].x));
-      s[1] = lg_add2(s[1], lg_bf2(raw[u].y));
-      s[2] = lg_add2(s[2], lg_bf2(raw[u].z));
-      s[3] = lg_add2(s[3], lg_bf2(raw[u].w));
-    }
-  }
-  const float2 st = lg_split(lg_add2(lg_add2(s[0], s[1]), lg_add2(s[2], s[3])));
-  const float mean = (st.x + st.y) * (1.f / C);
-  const uint64_t m2 = lg_pair(-mean, -mean);
-  sweep();
-#pragma unroll 1
-  for (int kb = 0; kb < KB; ++kb) {
-    if (!KEEP) load(kb);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const uint32_t e[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint64_t d = lg_add2(lg_bf2(e[i]), m2);
-        q[i] = lg_fma2(d, d, q[i]);
+      for (int j = 0; j < 8; ++j) {
+        v[h][j] = j & 1 ? odd(raw[2 * h], raw[2 * h + 1], j >> 1) : even(raw[2 * h], raw[2 * h + 1], j >> 1);
+        t[h] = lg_add2(t[h], v[h][j]);
       }
     }
-  }
-  const float2 qt = lg_split(lg_add2(lg_add2(q[0], q[1]), lg_add2(q[2], q[3])));
-  const float rstd = rsqrtf((qt.x + qt.y) * (1.f / C) + eps);
-  const uint64_t r2 = lg_pair(rstd, rstd);
-  sweep();
-#pragma unroll 1
-  for (int kb = 0; kb < KB; ++kb) {
-    if (!KEEP) load(kb);
+    const float mean = fold() * (1.f / C);
+    const uint64_t m2 = lg_pair(-mean, -mean);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const ulonglong2* g = reinterpret_cast<const ulonglong2*>(gamma + kb * 64 + u * 8);       // the same in every lane
-      const ulonglong2* b = reinterpret_cast<const ulonglong2*>(beta + kb * 64 + u * 8);
-      const ulonglong2 g0 = g[0], g1 = g[1], b0 = b[0], b1 = b[1];
-      uint4 o;
-      o.x = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[u].x), m2), r2), g0.x, b0.x));
-      o.y = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[u].y), m2), r2), g0.y, b0.y));
-      o.z = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[u].z), m2), r2), g1.x, b1.x));
-      o.w = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[u].w), m2), r2), g1.y, b1.y));
-      *reinterpret_cast<uint4*>(p + kb * 16384 + ((u ^ x) << 4)) = o;
+    for (int h = 0; h < 4; ++h) {
+      t[h] = lg_pair(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[h][j] = lg_add2(v[h][j], m2);
+        t[h] = lg_fma2(v[h][j], v[h][j], t[h]);
+      }
+    }
+    const float rstd = rsqrtf(fold() * (1.f / C) + eps);
+    const uint64_t r2 = lg_pair(rstd, rstd);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      uint32_t lo[4], hi[4];
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(gamma + h * 16 + 4 * w), b = *reinterpret_cast<const ulonglong2*>(beta + h * 16 + 4 * w);
+        const float2 e = lg_split(lg_fma2(lg_mul2(v[h][2 * w], r2), g.x, b.x));
+        const float2 o = lg_split(lg_fma2(lg_mul2(v[h][2 * w + 1], r2), g.y, b.y));
+        lo[w] = lg_pack2(e.x, o.x);
+        hi[w] = lg_pack2(e.y, o.y);
+      }
+      *reinterpret_cast<uint4*>(p + (((2 * h) ^ x) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      *reinterpret_cast<uint4*>(p + (((2 * h + 1) ^ x) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    }
+  } else {
+    // Four chains at a time: a pair of neighbouring pieces (2 i and 2 i + 1) of each of four blocks, or of two blocks and then also the pair
+    // half a block on.  Pairs half a block apart are added first
+    auto total = [&](auto&& add) {
+      uint64_t s[4], half, t;
+      auto combine = [&](int n) {
+        const uint64_t u = lg_add2(KB == 4 ? lg_add2(s[0], s[2]) : lg_add2(s[0], s[1]), KB == 4 ? lg_add2(s[1], s[3]) : lg_add2(s[2], s[3]));
+        if (KB == 4) {
+          const uint64_t w = lg_add2(half, u);
+          if (n & 1) t = n > 1 ? lg_add2(t, w) : w;
+          half = u;
+        } else {
+          t = n ? lg_add2(t, u) : u;
+        }
+      };
+      half = t = 0;
+#pragma unroll 1
+      for (int n = 0; n < KB; ++n) {
+        uint4 ra[4], rb[4];
+        const int i = KB == 4 ? (n >> 1) + 2 * (n & 1) : n;
+        const int oa = ((2 * i) ^ x) << 4, ob = oa ^ 16;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int at = KB == 4 ? c * 16384 : (c & 1) * 16384, off = KB == 4 ? 0 : (c >> 1) * 64;       // 64: four pieces on
+          ra[c] = *reinterpret_cast<const uint4*>(p + at + (oa ^ off));
+          rb[c] = *reinterpret_cast<const uint4*>(p + at + (ob ^ off));
+        }
+        if (n) combine(n - 1);          // here, with the loads under way, and not at the end of the pass, where it would wait for the sums
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s[c] = lg_pair(0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) s[c] = add(s[c], even(ra[c], rb[c], w));
+#pragma unroll
+          for (int c = 0; c < 4; ++c) s[c] = add(s[c], odd(ra[c], rb[c], w));
+        }
+      }
+      combine(KB - 1);
+      asm volatile("" ::: "memory");
+      const float2 f = lg_split(t);
+      return f.x + f.y;
+    };
+    const float mean = total([](uint64_t s, uint64_t v) { return lg_add2(s, v); }) * (1.f / C);
+    const uint64_t m2 = lg_pair(-mean, -mean);
+    const float var = total([&](uint64_t s, uint64_t v) {
+      const uint64_t d = lg_add2(v, m2);
+      return lg_fma2(d, d, s);
+    });
+    const float rstd = rsqrtf(var * (1.f / C) + eps);
+    const uint64_t r2 = lg_pair(rstd, rstd);
+#pragma unroll 1
+    for (int kb = 0; kb < KB; ++kb) {
+      uint4 ra[8];
+      load(ra, kb);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const ulonglong2* g = reinterpret_cast<const ulonglong2*>(gamma + kb * 64 + u * 8);       // the same in every lane
+        const ulonglong2* b = reinterpret_cast<const ulonglong2*>(beta + kb * 64 + u * 8);
+        const ulonglong2 g0 = g[0], g1 = g[1], b0 = b[0], b1 = b[1];
+        uint4 o;
+        o.x = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(ra[u].x), m2), r2), g0.x, b0.x));
+        o.y = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(ra[u].y), m2), r2), g0.y, b0.y));
+        o.z = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(ra[u].z), m2), r2), g1.x, b1.x));
+        o.w = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(ra[u].w), m2), r2), g1.y, b1.y));
+        *reinterpret_cast<uint4*>(p + kb * 16384 + ((u ^ x) << 4)) = o;
+      }
     }
   }
 }
 
 // Channels-first tile [kb][2 chunks of 64 rows][64 channels][64 rows], in place: thread t holds rows 2 (t % 64) and the next for
-// the 64 channels of block t / 64; the two threads of a pair of rows add their sums through `part` ([2][128] float2).
+// the 64 channels of block t / 64.  Sums in the order of ln_fwd_transposed128_kernel, so that both give the same bits: four
+// channels, four such quads, then the eight groups of 16 channels one by one; the two threads of a pair of rows exchange theirs through
+// `part` ([2][5][64] float2: the first four groups added up, the other four each).
 __device__ __forceinline__ void lg_norm_columns(uint8_t* tile, int t, float2* part, const float* gamma, const float* beta, float eps) {
   const int pr = t & 63, kb = t >> 6;
   uint8_t* p = tile + kb * 16384 + (pr >> 5) * 8192 + ((pr & 3) << 2);
   const int u = (pr & 31) >> 2;
-  uint64_t s[4];
   auto sweep = [&](auto&& each) {         // 16 channels at a time
-#pragma unroll
-    for (int i = 0; i < 4; ++i) s[i] = lg_pair(0.f, 0.f);
 #pragma unroll 1
     for (int k0 = 0; k0 < 64; k0 += 16) {
       uint32_t raw[16];
@@ -226,28 +286,36 @@ __device__ __forceinline__ void lg_norm_columns(uint8_t* tile, int t, float2* pa
       each(k0, raw);
     }
   };
-  auto total = [&]() { return lg_split(lg_add2(lg_add2(s[0], s[1]), lg_add2(s[2], s[3]))); };
-  sweep([&](int, const uint32_t (&raw)[16]) {
+  auto total = [&](float2* at, auto&& quad) {
+    uint64_t first = lg_pair(0.f, 0.f);
+    sweep([&](int k0, const uint32_t (&raw)[16]) {
+      const uint64_t g = lg_add2(lg_add2(quad(raw), quad(raw + 4)), lg_add2(quad(raw + 8), quad(raw + 12)));
+      if (kb == 0) first = lg_add2(first, g);
+      else at[(1 + (k0 >> 4)) * 64 + pr] = lg_split(g);
+    });
+    if (kb == 0) at[pr] = lg_split(first);
+    asm volatile("bar.sync 2, 128;" ::: "memory");
+    float2 sum = at[pr];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) s[k & 3] = lg_add2(s[k & 3], lg_bf2(raw[k]));
-  });
-  const float2 ms = total();
-  part[t] = ms;
-  asm volatile("bar.sync 2, 128;" ::: "memory");
-  const float2 os = part[t ^ 64];
-  const uint64_t m2 = lg_pair(-(ms.x + os.x) * (1.f / 128), -(ms.y + os.y) * (1.f / 128));
-  sweep([&](int, const uint32_t (&raw)[16]) {
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const uint64_t d = lg_add2(lg_bf2(raw[k]), m2);
-      s[k & 3] = lg_fma2(d, d, s[k & 3]);
+    for (int i = 1; i < 5; ++i) {
+      const float2 g = at[i * 64 + pr];
+      sum.x += g.x;
+      sum.y += g.y;
     }
+    return sum;
+  };
+  const float2 ms = total(part, [&](const uint32_t* r) { return lg_add2(lg_add2(lg_bf2(r[0]), lg_bf2(r[1])), lg_add2(lg_bf2(r[2]), lg_bf2(r[3]))); });
+  const uint64_t m2 = lg_pair(-ms.x * (1.f / 128), -ms.y * (1.f / 128));
+  const float2 qs = total(part + 320, [&](const uint32_t* r) {
+    uint64_t q = lg_pair(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint64_t d = lg_add2(lg_bf2(r[k]), m2);
+      q = lg_fma2(d, d, q);
+    }
+    return q;
   });
-  const float2 mq = total();
-  part[128 + t] = mq;
-  asm volatile("bar.sync 2, 128;" ::: "memory");
-  const float2 oq = part[128 + (t ^ 64)];
-  const uint64_t r2 = lg_pair(rsqrtf((mq.x + oq.x) * (1.f / 128) + eps), rsqrtf((mq.y + oq.y) * (1.f / 128) + eps));
+  const uint64_t r2 = lg_pair(rsqrtf(qs.x * (1.f / 128) + eps), rsqrtf(qs.y * (1.f / 128) + eps));
   sweep([&](int k0, const uint32_t (&raw)[16]) {
 #pragma unroll
     for (int k = 0; k < 16; k += 4) {
@@ -325,8 +393,9 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
   pdl_wait();
   // gamma, beta and all biases as fp32; read back as broadcasts
   for (int i = threadIdx.x; i < C; i += LG_THREADS) {
-    gamma[i] = __bfloat162float(a.gamma[i]);
-    beta[i] = __bfloat162float(a.beta[i]);
+    const int at = C == 64 ? (i & 48) + (i & 7) * 2 + ((i >> 3) & 1) : i;       // for lg_norm_row<64>: the same channel of two pieces side by side
+    gamma[at] = __bfloat162float(a.gamma[i]);
+    beta[at] = __bfloat162float(a.beta[i]);
   }
   if (MODE != LN_PROJECT) {
     for (int i = threadIdx.x; i < ((a.hidden + 127) & ~127); i += LG_THREADS) bias1[i] = (a.b1 && i < a.hidden) ? __bfloat162float(a.b1[i]) : 0.f;

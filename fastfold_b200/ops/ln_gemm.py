@@ -1,7 +1,8 @@
 """LayerNorm and the GEMMs that read its rows, in one kernel each (csrc/ln_gemm.cu), without gradients.
 
 ``models/fastnn`` calls whole modules through the native functions below, which return None for tensors that the
-kernels do not cover, and otherwise composes LayerNorm and GEMM; the two agree up to the rounding of the LayerNorm's sums.
+kernels do not cover, and otherwise composes LayerNorm and GEMM; both give the same bits.  (The global column attention does not: its
+mean query, which the composition rounds to bf16 three times, stays in 32 bits.)
 """
 import torch
 from torch.autograd import forward_ad

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from fastfold_b200.models.fastnn import ops as fops
+from fastfold_b200.models.fastnn.msa import MSAColumnAttention
 from fastfold_b200.ops import LayerNorm, _lib, ln_gemm
 
 pytestmark = pytest.mark.gpu
@@ -265,8 +266,7 @@ def test_calls_that_stay_with_the_composition():
 @pytest.mark.parametrize("chunk", [None, 16, 64])
 @pytest.mark.parametrize("cls", [fops.ChunkTriangleAttentionStartingNode, fops.ChunkTriangleAttentionEndingNode])
 def test_triangle_attention(cls, chunk, n, device_status):
-    """Whole and in chunks of rows / columns, in place and not, against the composition from separate kernels: roundings of a
-    different LayerNorm sum only (2^-9 of a normalised value) on an update of about the residual's size."""
+    """Whole and in chunks of rows / columns, in place and not, against the composition from separate kernels."""
     torch.manual_seed(n)
     net = cls(128, p_drop=0.25, c=32, n_head=4).to(DEV, torch.bfloat16).eval().requires_grad_(False)
     z, mask = _randn(1, n, n, 128), (torch.rand(1, n, n, device=DEV) > 0.2).to(torch.bfloat16)
@@ -282,5 +282,78 @@ def test_triangle_attention(cls, chunk, n, device_status):
             out = net.inplace([held], mask)[0]
             assert out.data_ptr() == held.data_ptr()
             _close(out, ref.double())
+        finally:
+            fops.set_chunk_size(None)
+
+
+class _composed:
+    """Inside, the module runs as separate kernels: one of the modules that would be passed by has a hook."""
+
+    def __init__(self, mod):
+        self.mod = mod
+
+    def __enter__(self):
+        self.handle = self.mod.register_forward_hook(lambda *a: None)
+
+    def __exit__(self, *exc):
+        self.handle.remove()
+
+
+def _net(cls, *args, **kw):
+    net = cls(*args, **kw).to(DEV, torch.bfloat16).eval().requires_grad_(False)
+    _randomise(net)
+    return net
+
+
+@pytest.mark.parametrize("C", [64, 128, 256])
+@pytest.mark.parametrize("shape", [(1, 1), (1, 31), (3, 43), (100, 203)])
+def test_transition_same_bits(C, shape, device_status):
+    """The sums of the LayerNorm and the roundings are those of the separate kernels, so nothing may differ."""
+    torch.manual_seed(C)
+    with torch.no_grad():
+        net, x = _net(fops.Transition, C), _randn(1, *shape, C) * 3 + 0.5
+        fused = net(x)
+        with _composed(net.linear1):
+            assert torch.equal(net(x), fused)
+
+
+@pytest.mark.parametrize("n", [8, 27, 64, 203])
+@pytest.mark.parametrize("chunk", [None, 16, 64])
+def test_pair_modules_same_bits(chunk, n, device_status):
+    torch.manual_seed(n)
+    with torch.no_grad():
+        z, mask = _randn(1, n, n, 128) * 2 + 0.25, (torch.rand(1, n, n, device=DEV) > 0.2).to(torch.bfloat16)
+        fops.set_chunk_size(chunk)
+        try:
+            for cls in (fops.AsyncChunkTriangleMultiplicationOutgoing, fops.AsyncChunkTriangleMultiplicationIncoming):
+                net = _net(cls, 128, p_drop=0.25)
+                fused = net(z, mask)
+                with _composed(net.output_projection):
+                    assert torch.equal(net(z, mask), fused), cls
+            for cls in (fops.ChunkTriangleAttentionStartingNode, fops.ChunkTriangleAttentionEndingNode):
+                net = _net(cls, 128, p_drop=0.25, c=32, n_head=4)
+                fused = net(z, mask)
+                with _composed(net.attention.o_linear):
+                    assert torch.equal(net(z, mask), fused), cls
+        finally:
+            fops.set_chunk_size(None)
+
+
+@pytest.mark.parametrize("S,n", [(5, 8), (33, 27), (64, 64), (40, 203)])
+@pytest.mark.parametrize("chunk", [None, 16])
+def test_msa_modules_same_bits(chunk, S, n, device_status):
+    torch.manual_seed(n)
+    with torch.no_grad():
+        m, e, z = _randn(1, S, n, 256) * 2 + 0.25, _randn(1, S, n, 64), _randn(1, n, n, 128)
+        mask = (torch.rand(1, S, n, device=DEV) > 0.2).to(torch.bfloat16)
+        row, extra = _net(fops.ChunkMSARowAttentionWithPairBias, 256, 128), _net(fops.ChunkMSARowAttentionWithPairBias, 64, 128, c=8)
+        col, opm = _net(MSAColumnAttention, 256), _net(fops.OutProductMean, 256, 128, 32)
+        fops.set_chunk_size(chunk)
+        try:
+            for call, inner in ((lambda: row(m, z, mask), row.attention.o_linear), (lambda: extra(e, z, mask), extra.attention.o_linear),
+                                (lambda: col(m, mask), col.attention.o_linear), (lambda: opm(m, mask, z), opm.linear_a)):
+                fused = call()
+                with _composed(inner):
+                    assert torch.equal(call(), fused)
         finally:
             fops.set_chunk_size(None)
