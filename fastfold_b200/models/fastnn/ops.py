@@ -1030,7 +1030,7 @@ class _TriangleAttention(nn.Module):
             dropmask = None
         if strided is None:
             strided = self.strided(Z_raw)
-        if Z_norm is None and (self.starting or strided) and self.attention.takes_raw(Z_raw, self.layernorm1, dropmask) and not ln_gemm.hooked(self.linear_b):
+        if Z_norm is None and (self.starting or strided) and self.attention.takes_raw(Z_raw, self.layernorm1, dropmask) and ln_gemm.ready(self.linear_b):
             out, done = self.attention(Z_raw, mask, tail=(self.out_bias, None, Z_raw), transposed=strided, norm=self.layernorm1,
                                        pair_weight=self.linear_b.weight)
             if done:
@@ -1105,7 +1105,7 @@ class ChunkMSARowAttentionWithPairBias(nn.Module):
             dropmask = F.dropout(torch.ones_like(M_raw[:, 0:1, :, :]), p=self.p_drop, training=True)
         if not training:
             dropmask = None
-        if self.attention.takes_raw(M_raw, self.layernormM, dropmask) and not ln_gemm.hooked(self.layernormZ):
+        if self.attention.takes_raw(M_raw, self.layernormM, dropmask) and ln_gemm.ready(self.layernormZ):
             out, done = self.attention(M_raw, M_mask, tail=(self.out_bias, None, M_raw), norm=self.layernormM, pair_weight=self.linear_b_weights,
                                        pair=(Z, self.layernormZ))
             if done:

@@ -19,9 +19,6 @@ def stands_for(cls):
     _known.add(cls)
     return cls
 
-def hooked(mod):
-    return bool(mod._forward_hooks or mod._forward_pre_hooks)
-
 
 def ready(*modules):
     """True when the kernels may stand for calls of ``modules``: no gradients or forward-mode level, and each of the modules that

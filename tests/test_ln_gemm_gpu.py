@@ -357,3 +357,30 @@ def test_msa_modules_same_bits(chunk, S, n, device_status):
                     assert torch.equal(call(), fused)
         finally:
             fops.set_chunk_size(None)
+
+
+class _DoubledNorm(LayerNorm):
+    def forward(self, x):
+        return 2 * super().forward(x)
+
+
+@pytest.mark.parametrize("how", ["subclass", "forward", "identity", "hook"])
+def test_replaced_pair_norm(how, device_status):
+    """The norm of the pair tensor in the row attention is evaluated from its parameters only where it is the package's own, unchanged."""
+    torch.manual_seed(5)
+    with torch.no_grad():
+        net = _net(fops.ChunkMSARowAttentionWithPairBias, 256, 128)
+        m, z, mask = _randn(1, 9, 24, 256), _randn(1, 24, 24, 128), torch.ones(1, 9, 24, device=DEV, dtype=torch.bfloat16)
+        plain = net(m, z, mask)
+        if how == "subclass":
+            net.layernormZ = _DoubledNorm(128).to(DEV, torch.bfloat16)
+        elif how == "forward":
+            net.layernormZ.forward = lambda x: 2 * x
+        elif how == "identity":
+            net.layernormZ = torch.nn.Identity()
+        else:
+            net.layernormZ.register_forward_hook(lambda mod, args, out: 2 * out)
+        out = net(m, z, mask)
+        assert not torch.equal(out, plain)
+        with _composed(net.attention.o_linear):
+            assert torch.equal(net(m, z, mask), out)
