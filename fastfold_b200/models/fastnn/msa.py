@@ -11,7 +11,7 @@ from ...parallel.fused import a2a_layer_norm, norm_later
 from ...utils import memo
 from ...utils.checkpointing import checkpoint_blocks
 from .ops import (ChunkMSARowAttentionWithPairBias, ChunkMSAColumnGlobalAttention, ChunkTransition, GlobalAttention,
-                  OutProductMean, SelfAttention, Transition, _fusable, _residual)
+                  OutProductMean, SelfAttention, Transition, _fusable, _residual, attention_takes_raw)
 from .triangle import PairCore, pad_amount, pad_or_pass as _pad
 from . import ops as fops
 
@@ -47,7 +47,7 @@ class MSAColumnAttention(nn.Module):
         if strided is None:
             strided = M_norm_t is None and self.strided_for(M_raw.shape[1], M_raw)
         mask_t = memo.cached("mask_t", (M_mask,), lambda: M_mask.transpose(-1, -2).contiguous())
-        if strided and M_norm_t is None and self.attention.takes_raw(M_raw, self.layernormM, None):
+        if strided and M_norm_t is None and attention_takes_raw(self.attention, M_raw, self.layernormM, None):
             out, done = self.attention(M_raw, mask_t, tail=(None, None, M_raw), transposed=True, norm=self.layernormM)
             if done:
                 return out

@@ -537,12 +537,6 @@ class SelfAttention(nn.Module):
             return out.reshape(resid.shape), True
         return self.o_linear(o), False
 
-    def takes_raw(self, x, norm, dropmask):
-        """True when ``forward`` may be given ``x`` and the ``norm`` that it has not been through yet (``norm=``); it may still
-        turn out that the kernels do not cover the tensors."""
-        return (dropmask is None and x.is_cuda and self.gating and self.c <= 32 and core.get_dap_size() == 1
-                and ln_gemm.ready(norm, self, self.to_qkv, self.gating_linear, self.o_linear))
-
     def _from_raw(self, x, norm, mask, out_bias, transposed, pair_weight, pair):
         D = self._padded_dim()
         if D == self.c:
@@ -557,8 +551,8 @@ class SelfAttention(nn.Module):
         """``tail=(out_bias, (mask2d, div, mod) or None, residual)`` lets the output projection absorb the
         bias / dropout / residual that follow it; the second return value says whether it did.
         ``transposed``: attend along dim 1 of ``in_data`` instead of dim 2.
-        ``norm``: the LayerNorm that ``in_data``, which is also the residual, still has to go through (``takes_raw`` says whether
-        it may be left to this module); ``pair_weight``: the pair bias is ``norm(in_data) . pair_weight``, or with ``pair=(z, norm_z)``
+        ``norm``: the LayerNorm that ``in_data``, which is also the residual, still has to go through (``attention_takes_raw`` says
+        whether it may be left to this module); ``pair_weight``: the pair bias is ``norm(in_data) . pair_weight``, or with ``pair=(z, norm_z)``
         ``norm_z(z) . pair_weight``.  The result is then None where the kernels do not cover the tensors."""
         if norm is not None:
             out = self._from_raw(in_data, norm, mask, tail[0], transposed, pair_weight, pair)
@@ -611,6 +605,15 @@ class SelfAttention(nn.Module):
                 o = K.gemm(mat(part), wg, bias=bg, act="sigmoid", mul=mat(o))
             K.gemm(mat(o), wo, bias=out_bias, dmask=dmask, resid=None if resid is None else mat(resid[0][sl]), out=mat(out[0][sl]))
         return out
+
+
+def attention_takes_raw(attention, x, norm, dropmask, *others):
+    """True when ``attention`` may be given ``x`` and the ``norm`` that it has not been through yet (``norm=``), and ``others`` be passed by;
+    it may still turn out that the kernels do not cover the tensors.  ``attention`` may be any module: only this package's own
+    has what is asked for behind the first line."""
+    return (dropmask is None and x.is_cuda and type(attention) is SelfAttention and attention.gating and attention.c <= 32
+            and core.get_dap_size() == 1
+            and ln_gemm.ready(norm, attention, attention.to_qkv, attention.gating_linear, attention.o_linear, *others))
 
 
 def pair_bias_hqk(Zn, weight):
@@ -1030,7 +1033,7 @@ class _TriangleAttention(nn.Module):
             dropmask = None
         if strided is None:
             strided = self.strided(Z_raw)
-        if Z_norm is None and (self.starting or strided) and self.attention.takes_raw(Z_raw, self.layernorm1, dropmask) and ln_gemm.ready(self.linear_b):
+        if Z_norm is None and (self.starting or strided) and attention_takes_raw(self.attention, Z_raw, self.layernorm1, dropmask, self.linear_b):
             out, done = self.attention(Z_raw, mask, tail=(self.out_bias, None, Z_raw), transposed=strided, norm=self.layernorm1,
                                        pair_weight=self.linear_b.weight)
             if done:
@@ -1105,7 +1108,7 @@ class ChunkMSARowAttentionWithPairBias(nn.Module):
             dropmask = F.dropout(torch.ones_like(M_raw[:, 0:1, :, :]), p=self.p_drop, training=True)
         if not training:
             dropmask = None
-        if self.attention.takes_raw(M_raw, self.layernormM, dropmask) and ln_gemm.ready(self.layernormZ):
+        if attention_takes_raw(self.attention, M_raw, self.layernormM, dropmask, self.layernormZ):
             out, done = self.attention(M_raw, M_mask, tail=(self.out_bias, None, M_raw), norm=self.layernormM, pair_weight=self.linear_b_weights,
                                        pair=(Z, self.layernormZ))
             if done:
@@ -1145,8 +1148,8 @@ class ChunkMSAColumnGlobalAttention(nn.Module):
         """Without gradients, on the MSA as it is stored: keys and values from the rows, a kernel per column up to its value vector, and
         gate, output projection and residual from the rows again.  None where the kernels do not apply."""
         ga = self.global_attention
-        if not (self.c == self.n_head == 8 and M_raw.is_cuda and M_mask.shape == M_raw.shape[:-1] and core.get_dap_size() == 1
-                and ln_gemm.ready(self.layernormM, ga, ga.to_q, ga.to_kv, ga.gating_linear, ga.o_linear)):
+        if not (type(ga) is GlobalAttention and ga.c == ga.n_head == 8 and ga.eps == 1e-10 and M_raw.is_cuda and M_mask.shape == M_raw.shape[:-1]
+                and core.get_dap_size() == 1 and ln_gemm.ready(self.layernormM, ga, ga.to_q, ga.to_kv, ga.gating_linear, ga.o_linear)):
             return None
         return ln_gemm.global_column_attention(M_raw, self.layernormM, ga, M_mask, INPLACE and M_raw.is_contiguous())
 

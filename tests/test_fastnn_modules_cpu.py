@@ -175,3 +175,33 @@ def test_stack_entry_passes_on_only_what_needs_no_copy():
             assert pad_or_pass(dense, (0, 0, 0, 0)).data_ptr() != dense.data_ptr()
     kept = dense.detach().requires_grad_(True)
     assert pad_or_pass(kept, (0, 0, 0, 0)).data_ptr() != dense.data_ptr()
+
+
+class _Forwarding(torch.nn.Module):
+    """A module around another that only passes the call on."""
+
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def forward(self, *args, **kw):
+        return self.inner(*args, **kw)
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("which", ["row", "column", "start", "end"])
+def test_wrapped_attention(which, grad):
+    """The attention of a module may be any module: nothing but the call is asked of it."""
+    m, z, msa_mask, pair_mask = _inputs(3)
+    if which == "row":
+        net = _randomize(fastnn.msa.MSARowAttentionWithPairBias(d_node=C_M, d_pair=C_Z, c=8, n_head=4), 1)
+        args = (m[None], z[None], msa_mask[None])
+    elif which == "column":
+        net, args = _randomize(fastnn.msa.MSAColumnAttention(d_node=C_M, c=8, n_head=4), 1), (m[None], msa_mask[None])
+    else:
+        cls = fops.ChunkTriangleAttentionStartingNode if which == "start" else fops.ChunkTriangleAttentionEndingNode
+        net, args = _randomize(cls(C_Z, p_drop=0.0, c=8, n_head=2), 1), (z[None], pair_mask[None])
+    with torch.set_grad_enabled(grad):
+        want = net(*args)
+        net.attention = _Forwarding(net.attention)
+        assert torch.equal(net(*args), want)

@@ -384,3 +384,34 @@ def test_replaced_pair_norm(how, device_status):
         assert not torch.equal(out, plain)
         with _composed(net.attention.o_linear):
             assert torch.equal(net(m, z, mask), out)
+
+
+class _Forwarding(torch.nn.Module):
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def forward(self, *args, **kw):
+        return self.inner(*args, **kw)
+
+
+def test_wrapped_attention(device_status):
+    """An attention inside a module that only passes the call on gives what the attention itself gives (the global one from separate
+    kernels, whose mean query is rounded to bf16)."""
+    torch.manual_seed(6)
+    with torch.no_grad():
+        m, z = _randn(1, 9, 24, 256), _randn(1, 24, 24, 128)
+        mask, zmask = torch.ones(1, 9, 24, device=DEV, dtype=torch.bfloat16), torch.ones(1, 24, 24, device=DEV, dtype=torch.bfloat16)
+        row, col = _net(fops.ChunkMSARowAttentionWithPairBias, 256, 128), _net(MSAColumnAttention, 256)
+        start, end = _net(fops.ChunkTriangleAttentionStartingNode, 128, p_drop=0.0), _net(fops.ChunkTriangleAttentionEndingNode, 128, p_drop=0.0)
+        for net, args in ((row, (m, z, mask)), (col, (m, mask)), (start, (z, zmask)), (end, (z, zmask))):
+            want = net(*args)
+            net.attention = _Forwarding(net.attention)
+            assert torch.equal(net(*args), want), type(net)
+        e, net = _randn(1, 40, 24, 64), _net(fops.ChunkMSAColumnGlobalAttention, 64)
+        emask = torch.ones(1, 40, 24, device=DEV, dtype=torch.bfloat16)
+        assert net._from_raw(e, emask) is not None
+        with _composed(net.layernormM):
+            want = net(e, emask)
+        net.global_attention = _Forwarding(net.global_attention)
+        assert torch.equal(net(e, emask), want)
