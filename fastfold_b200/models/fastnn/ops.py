@@ -383,6 +383,16 @@ def _key_contiguous(b):
     return buf.copy_(b)
 
 
+def _state_of(tensors):
+    """What tells whether something built from ``tensors`` is still current: memory, type and in-place changes of each."""
+    return tuple((t.data_ptr(), t.dtype, t._version) for t in tensors)
+
+
+def _held(tensors):
+    """Kept next to what was built from ``tensors``: their memory cannot come back as another tensor's while it is compared with."""
+    return [t.detach() for t in tensors]
+
+
 @ln_gemm.stands_for
 class SelfAttention(nn.Module):
     """Multi-head gated self attention on ``[b1, b2, n, c]`` (attention along ``n``)."""
@@ -421,8 +431,8 @@ class SelfAttention(nn.Module):
         H, d = self.n_head, self.c
         # Cached in eval mode only: an optimiser that updates the parameters through raw pointers (the flat fused Adam)
         # changes neither ``_version`` nor ``data_ptr``, so in training the widened copies are rebuilt on every call.
-        key = (D, self.to_qkv.weight.data_ptr(), self.to_qkv.weight._version, self.o_linear.weight._version,
-               self.gating_linear.weight._version if self.gating else 0)
+        parts = [self.to_qkv.weight, self.o_linear.weight] + ([self.gating_linear.weight, self.gating_bias] if self.gating else [])
+        key = (D, _state_of(parts))
         if self.training or getattr(self, "_pad_cache", None) is None or self._pad_cache[0] != key:
             def rows(w, groups):                      # [groups * H * d, ...] -> [groups * H * D, ...]
                 w = w.detach().reshape(groups, H, d, *w.shape[1:])
@@ -438,8 +448,8 @@ class SelfAttention(nn.Module):
                 # being captured live in the graph's memory pool, whose contents later eager code must not rely on
                 self._pad_cache = None
                 return wq, wg, bg, wo
-            self._pad_cache = (key, wq, wg, bg, wo)
-        return self._pad_cache[1:]
+            self._pad_cache = (key, wq, wg, bg, wo, _held(parts))
+        return self._pad_cache[1:5]
 
     def _padded_heads_differentiable(self):
         """The widened weights of ``_padded_heads`` built with differentiable ops (training): gradients flow back to the
@@ -736,15 +746,15 @@ class _TriangleMultiplication(nn.Module):
         wp, wg = self.left_right_projection.weight, self.left_right_gate.weight
         # Cached in eval mode only (see ``SelfAttention._padded_heads``): under the flat fused Adam the parameters change
         # without a version bump, and a CUDA graph must capture the rebuild so that replays see the current weights.
-        key = (wp._version, wg._version, wp.data_ptr(), wg.data_ptr(), wp.dtype,
-               self.left_right_projection.bias._version, self.left_right_gate.bias._version)
+        parts = [wp, wg, self.left_right_projection.bias, self.left_right_gate.bias]
+        key = _state_of(parts)
         if self.training or self._glu_cache is None or self._glu_cache[0] != key:
             w = torch.stack([wp.detach(), wg.detach()], dim=1).reshape(-1, wp.shape[1]).contiguous()
             b = torch.stack([self.left_right_projection.bias.detach(), self.left_right_gate.bias.detach()], dim=1).reshape(-1).contiguous()
             if self.training:
                 self._glu_cache = None          # see ``SelfAttention._padded_heads``
                 return w, b
-            self._glu_cache = (key, w, b)
+            self._glu_cache = (key, w, b, _held(parts))
         return self._glu_cache[1], self._glu_cache[2]
 
     def _contract(self, left, right):

@@ -205,3 +205,46 @@ def test_wrapped_attention(which, grad):
         want = net(*args)
         net.attention = _Forwarding(net.attention)
         assert torch.equal(net(*args), want)
+
+
+def _change(module, name, how):
+    """Other values in one parameter of a module in evaluation."""
+    with torch.no_grad():
+        old = getattr(module, name)
+        if how == "in place":
+            old.add_(1.0)
+        elif how == "data":
+            old.data = old.data + 1.0
+        else:                                    # another tensor with the same version count
+            setattr(module, name, torch.nn.Parameter(old + 1.0))
+
+
+@pytest.mark.parametrize("how", ["in place", "data", "replaced"])
+@pytest.mark.parametrize("which", ["to_qkv.weight", "gating_linear.weight", "gating_bias", "o_linear.weight"])
+def test_widened_heads_follow_their_parameters(which, how):
+    """The widened weights of narrow heads, kept in evaluation, are built again when any of the parameters changes."""
+    torch.manual_seed(0)
+    net = fops.SelfAttention(qkv_dim=64, c=8, n_head=4, out_dim=64).eval()
+    first = net._padded_heads(16)
+    assert all(a is b for a, b in zip(net._padded_heads(16), first))
+    owner = net if "." not in which else getattr(net, which.split(".")[0])
+    _change(owner, which.split(".")[-1], how)
+    got = net._padded_heads(16)
+    net._pad_cache = None
+    for a, b in zip(got, net._padded_heads(16)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("how", ["in place", "data", "replaced"])
+@pytest.mark.parametrize("name", ["weight", "bias"])
+@pytest.mark.parametrize("which", ["left_right_projection", "left_right_gate"])
+def test_gated_weights_follow_their_parameters(which, name, how):
+    torch.manual_seed(0)
+    net = fops.AsyncChunkTriangleMultiplicationOutgoing(16, p_drop=0.0, c=16).eval()
+    first = net._glu_weights()
+    assert all(a is b for a, b in zip(net._glu_weights(), first))
+    _change(getattr(net, which), name, how)
+    got = net._glu_weights()
+    net._glu_cache = None
+    for a, b in zip(got, net._glu_weights()):
+        assert torch.equal(a, b)
