@@ -603,6 +603,13 @@ Tensor dense_rows(Tensor x) {
   return x;
 }
 
+// `inplace`: the caller's tensor receives the result, also where the kernels worked on a dense copy of it
+Tensor settle(const Tensor& x0, const Tensor& out, bool inplace) {
+  if (!inplace || out.data_ptr() == x0.data_ptr()) return out;
+  x0.copy_(out);
+  return x0;
+}
+
 OptTensor transition_module(const Tensor& x0, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& w1, const OptTensor& b1, const Tensor& w2,
                             const OptTensor& b2, bool inplace) {
   if (!rows_of_channels(x0) || !all_plain(gamma, beta, w1, b1, w2, b2)) return std::nullopt;
@@ -611,7 +618,7 @@ OptTensor transition_module(const Tensor& x0, const Tensor& gamma, const Tensor&
       gamma.numel() != C || beta.numel() != C)
     return std::nullopt;
   const Tensor x = dense_rows(x0), x2 = x.view({-1, C});
-  return ln_chain(x2, gamma, beta, eps, w1, b1, w2, b2, std::nullopt, x2, inplace ? OptTensor(x2) : std::nullopt).view(x.sizes());
+  return settle(x0, ln_chain(x2, gamma, beta, eps, w1, b1, w2, b2, std::nullopt, x2, inplace ? OptTensor(x2) : std::nullopt).view(x.sizes()), inplace);
 }
 
 // A pair bias [H, n, n] with rows at an 8-element pitch
@@ -667,7 +674,7 @@ OptTensor attention_module(const Tensor& x0, const Tensor& gamma, const Tensor& 
                                                       false, transposed));
     ln_chain(part, gamma, beta, eps, wg, bg, wo, bo, part.dim() == 3 ? o.view({part.size(0), part.size(1), HD}) : o.view({-1, HD}), part, dst);
   }
-  return out.unsqueeze(0);
+  return settle(x0, out.unsqueeze(0), inplace);
 }
 
 // Triangle multiplication of a square pair tensor [1, n, n, 128].  w / b: projection and gate weights interleaved by rows.  Extents
@@ -693,7 +700,7 @@ OptTensor triangle_module(const Tensor& z0, const Tensor& g1, const Tensor& b1, 
   const OptTensor none;
   gemm(lr_n.narrow(0, 0, c), lr_n.narrow(0, c, c), !outgoing, !outgoing, 1.0, none, ACT_NONE, false, none, none, none, 1, 1, none, false, p_n, false, 1,
        false, 0, std::nullopt);
-  return ln_tri_out(cut(p), g2, b2, eps2, wo, bo, gate, z3, inplace ? OptTensor(z3) : std::nullopt).view(z.sizes());
+  return settle(z0, ln_tri_out(cut(p), g2, b2, eps2, wo, bo, gate, z3, inplace ? OptTensor(z3) : std::nullopt).view(z.sizes()), inplace);
 }
 
 // Global column attention of the extra-MSA stack over x [1, S, N, 64], 8 heads of 8 channels
@@ -706,7 +713,7 @@ OptTensor global_column_module(const Tensor& x0, const Tensor& gamma, const Tens
   const Tensor x = dense_rows(x0), x2 = x.view({-1, 64});
   const Tensor kv = *ln_qkv(x2, gamma, beta, eps, wkv, std::nullopt, std::nullopt, false);
   const Tensor o = global_column(x.view({x.size(1), x.size(2), 64}), gamma, beta, eps, wq, kv, mask, scale);
-  return ln_chain(x2, gamma, beta, eps, wg, bg, wo, bo, o, x2, inplace ? OptTensor(x2) : std::nullopt).view(x.sizes());
+  return settle(x0, ln_chain(x2, gamma, beta, eps, wg, bg, wo, bo, o, x2, inplace ? OptTensor(x2) : std::nullopt).view(x.sizes()), inplace);
 }
 
 // Masked projections of the outer product mean

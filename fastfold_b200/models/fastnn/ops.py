@@ -153,7 +153,8 @@ class Transition(nn.Module):
         norm, l1, l2 = self.norm, self.linear1, self.linear2
         if not (src.is_cuda and ln_gemm.ready(norm, l1, l2)):
             return None
-        return ln_gemm.transition(src, norm, l1, l2, INPLACE and src.is_contiguous())
+        # in place as the composition: dense tensors, and in chunks tensors of any layout
+        return ln_gemm.transition(src, norm, l1, l2, INPLACE and (src.is_contiguous() or CHUNK_SIZE is not None))
 
     def _one(self, src):
         x = self.norm(src)
@@ -1161,7 +1162,7 @@ class ChunkMSAColumnGlobalAttention(nn.Module):
         if not (type(ga) is GlobalAttention and ga.c == ga.n_head == 8 and ga.eps == 1e-10 and M_raw.is_cuda and M_mask.shape == M_raw.shape[:-1]
                 and core.get_dap_size() == 1 and ln_gemm.ready(self.layernormM, ga, ga.to_q, ga.to_kv, ga.gating_linear, ga.o_linear)):
             return None
-        return ln_gemm.global_column_attention(M_raw, self.layernormM, ga, M_mask, INPLACE and M_raw.is_contiguous())
+        return ln_gemm.global_column_attention(M_raw, self.layernormM, ga, M_mask, INPLACE)
 
     def forward(self, M_raw, M_mask):
         out = self._from_raw(M_raw, M_mask)

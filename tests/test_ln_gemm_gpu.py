@@ -415,3 +415,37 @@ def test_wrapped_attention(device_status):
             want = net(e, emask)
         net.global_attention = _Forwarding(net.global_attention)
         assert torch.equal(net(e, emask), want)
+
+
+@pytest.mark.parametrize("layout", ["dense", "off the boundary", "channels apart"])
+@pytest.mark.parametrize("chunk", [None, 16])
+def test_in_place_calls_write_into_the_tensor_itself(chunk, layout, device_status):
+    """`inplace` leaves its result in the caller's tensor, not only in the list: dense tensors on any address, and those of another
+    layout where the separate kernels did (global column attention; transitions in chunks)."""
+    torch.manual_seed(7)
+
+    def held(*shape):
+        if layout == "dense":
+            return _randn(*shape)
+        if layout == "off the boundary":
+            n = 4 + torch.Size(shape).numel()
+            return _randn(n)[4:].view(shape)
+        return _randn(shape[0], shape[3], shape[2], shape[1]).transpose(1, 3)
+
+    with torch.no_grad():
+        mask, zmask = torch.ones(1, 40, 24, device=DEV, dtype=torch.bfloat16), torch.ones(1, 24, 24, device=DEV, dtype=torch.bfloat16)
+        cases = [(_net(fops.ChunkMSAColumnGlobalAttention, 64), held(1, 40, 24, 64), (mask,))]
+        if layout != "channels apart" or chunk:
+            cases.append((_net(fops.Transition, 128), held(1, 40, 24, 128), ()))
+        if layout != "channels apart":
+            cases += [(_net(fops.AsyncChunkTriangleMultiplicationOutgoing, 128, p_drop=0.0), held(1, 24, 24, 128), (zmask,)),
+                      (_net(fops.ChunkTriangleAttentionStartingNode, 128, p_drop=0.0), held(1, 24, 24, 128), (zmask,)),
+                      (_net(fops.ChunkTriangleAttentionEndingNode, 128, p_drop=0.0), held(1, 24, 24, 128), (zmask,))]
+        fops.set_chunk_size(chunk)
+        try:
+            for net, x, args in cases:
+                want = net(x.clone(), *args)
+                out = net.inplace([x], *args)[0]
+                assert out.data_ptr() == x.data_ptr() and torch.equal(out, want) and torch.equal(x, want), type(net)
+        finally:
+            fops.set_chunk_size(None)
