@@ -10,6 +10,8 @@
 // on that stream, exactly as the Python code did.
 #include <torch/extension.h>
 
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include "gemm_api.h"
@@ -610,6 +612,24 @@ Tensor settle(const Tensor& x0, const Tensor& out, bool inplace) {
   return x0;
 }
 
+// mul * act(x w^T + b) + resid
+Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& b, int act, const OptTensor& mul, const OptTensor& resid, const OptTensor& out) {
+  const OptTensor none;
+  return gemm(x, w, false, false, 1.0, b, act, false, none, mul, none, 1, 1, resid, false, out, false, 1, false, 0, std::nullopt);
+}
+
+// Few rows of 256 channels under stream capture.  A tile of 128 rows walks all weights on one SM, 25 us for a transition whether there are
+// 64 rows or 16384, where LayerNorm and two GEMMs, whose tiles spread over the SMs, take less.  In a graph (B200, us, one kernel / separate
+// ones): transition 64 rows 24 / 13, 2048 25 / 15, 4096 25 / 16, 8192 26 / 21, 12288 26 / 28, 16384 26 / 30; column attention 32 x 64 37 / 28,
+// 128 x 64 40 / 35, 128 x 96 45 / 45, 128 x 128 48 / 51; row attention 32 x 64 47 / 35, 128 x 64 54 / 45, 128 x 96 60 / 57, 128 x 128 60 / 63;
+// the MSA half of a block of 32 x 64 110 / 77.  So up to a tile for every second SM.  Calls that are not captured are bound by the host there and
+// keep the fewer launches: a block of 32 x 64 356 / 388, 128 x 64 358 / 394, 64 x 100 359 / 394.  With 64 and 128 channels the one kernel is
+// the faster one at every length.  Both give the same bits.
+bool few_rows_captured(int64_t C, int64_t rows) {
+  return C == 256 && (rows + 127) / 128 * 2 <= at::cuda::getCurrentDeviceProperties()->multiProcessorCount &&
+         c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+}
+
 OptTensor transition_module(const Tensor& x0, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& w1, const OptTensor& b1, const Tensor& w2,
                             const OptTensor& b2, bool inplace) {
   if (!rows_of_channels(x0) || !all_plain(gamma, beta, w1, b1, w2, b2)) return std::nullopt;
@@ -618,7 +638,12 @@ OptTensor transition_module(const Tensor& x0, const Tensor& gamma, const Tensor&
       gamma.numel() != C || beta.numel() != C)
     return std::nullopt;
   const Tensor x = dense_rows(x0), x2 = x.view({-1, C});
-  return settle(x0, ln_chain(x2, gamma, beta, eps, w1, b1, w2, b2, std::nullopt, x2, inplace ? OptTensor(x2) : std::nullopt).view(x.sizes()), inplace);
+  const OptTensor dst = inplace ? OptTensor(x2) : std::nullopt;
+  if (few_rows_captured(C, x2.size(0))) {
+    const Tensor h = linear(std::get<0>(layer_norm_fwd(x2, gamma, beta, eps, false)), w1, b1, ACT_RELU, std::nullopt, std::nullopt, std::nullopt);
+    return settle(x0, linear(h, w2, b2, ACT_NONE, std::nullopt, x2, dst).view(x.sizes()), inplace);
+  }
+  return settle(x0, ln_chain(x2, gamma, beta, eps, w1, b1, w2, b2, std::nullopt, x2, dst).view(x.sizes()), inplace);
 }
 
 // A pair bias [H, n, n] with rows at an 8-element pitch
@@ -656,23 +681,28 @@ OptTensor attention_module(const Tensor& x0, const Tensor& gamma, const Tensor& 
     else ln_qkv(x2, gamma, beta, eps, std::nullopt, pair_w, bias, transposed);
   }
   const int64_t pitch = bias ? bias->stride(1) : n;
+  OptTensor norm;                                     // of the whole input, where its projections are kernels of their own
+  if (few_rows_captured(C, n * (whole ? rows : std::min(chunk, rows)))) {
+    norm = std::get<0>(layer_norm_fwd(x2, gamma, beta, eps, false)).view(x3.sizes());
+    if (own_w) ln_qkv(x2, gamma, beta, eps, std::nullopt, own_w, bias, transposed);
+  }
   for (int64_t at = 0; at < rows; at += whole ? rows : chunk) {
     const int64_t len = whole ? rows : std::min(chunk, rows - at);
-    Tensor part = x2, dst = out.view({-1, C});
-    if (!whole) {
-      // rows are contiguous: one matrix; columns are not: a batch of them, one per position along the attention
-      part = x3.narrow(transposed ? 1 : 0, at, len);
-      dst = out.narrow(transposed ? 1 : 0, at, len);
-      if (!transposed) {
-        part = part.view({-1, C});
-        dst = dst.view({-1, C});
-      }
-    }
-    const Tensor qkv = *ln_qkv(part, gamma, beta, eps, wq, own_w, own_w ? bias : OptTensor(), transposed);
+    // rows are contiguous: one matrix; columns are not: a batch of them, one per position along the attention
+    auto cut = [&](const Tensor& t) {
+      if (whole) return t.view({-1, t.size(2)});
+      const Tensor slice = t.narrow(transposed ? 1 : 0, at, len);
+      return transposed ? slice : slice.view({-1, t.size(2)});
+    };
+    const Tensor part = cut(x3), dst = cut(out);
+    const Tensor qkv = norm ? linear(cut(*norm), wq, std::nullopt, ACT_NONE, std::nullopt, std::nullopt, std::nullopt)
+                            : *ln_qkv(part, gamma, beta, eps, wq, own_w, own_w ? bias : OptTensor(), transposed);
     const OptTensor m = m2 ? OptTensor(whole ? *m2 : m2->narrow(0, at, len)) : std::nullopt;
-    const Tensor o = std::get<0>(attention_packed_fwd(transposed ? qkv.view({1, n, len, 3, H, D}) : qkv.view({1, len, n, 3, H, D}), m, bias, pitch, scale,
-                                                      false, transposed));
-    ln_chain(part, gamma, beta, eps, wg, bg, wo, bo, part.dim() == 3 ? o.view({part.size(0), part.size(1), HD}) : o.view({-1, HD}), part, dst);
+    const Tensor o4 = std::get<0>(attention_packed_fwd(transposed ? qkv.view({1, n, len, 3, H, D}) : qkv.view({1, len, n, 3, H, D}), m, bias, pitch, scale,
+                                                       false, transposed));
+    const Tensor o = part.dim() == 3 ? o4.view({part.size(0), part.size(1), HD}) : o4.view({-1, HD});
+    if (norm) linear(linear(cut(*norm), wg, bg, ACT_SIGMOID, o, std::nullopt, std::nullopt), wo, bo, ACT_NONE, std::nullopt, part, dst);
+    else ln_chain(part, gamma, beta, eps, wg, bg, wo, bo, o, part, dst);
   }
   return settle(x0, out.unsqueeze(0), inplace);
 }

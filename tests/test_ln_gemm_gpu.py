@@ -306,7 +306,7 @@ def _net(cls, *args, **kw):
 
 
 @pytest.mark.parametrize("C", [64, 128, 256])
-@pytest.mark.parametrize("shape", [(1, 1), (1, 31), (3, 43), (100, 203)])
+@pytest.mark.parametrize("shape", [(1, 1), (1, 31), (3, 43), (74, 128), (1, 9473), (100, 203)])
 def test_transition_same_bits(C, shape, device_status):
     """The sums of the LayerNorm and the roundings are those of the separate kernels, so nothing may differ."""
     torch.manual_seed(C)
@@ -339,7 +339,7 @@ def test_pair_modules_same_bits(chunk, n, device_status):
             fops.set_chunk_size(None)
 
 
-@pytest.mark.parametrize("S,n", [(5, 8), (33, 27), (64, 64), (40, 203)])
+@pytest.mark.parametrize("S,n", [(5, 8), (33, 27), (64, 64), (40, 203), (74, 128), (130, 150)])
 @pytest.mark.parametrize("chunk", [None, 16])
 def test_msa_modules_same_bits(chunk, S, n, device_status):
     torch.manual_seed(n)
@@ -447,5 +447,26 @@ def test_in_place_calls_write_into_the_tensor_itself(chunk, layout, device_statu
                 want = net(x.clone(), *args)
                 out = net.inplace([x], *args)[0]
                 assert out.data_ptr() == x.data_ptr() and torch.equal(out, want) and torch.equal(x, want), type(net)
+        finally:
+            fops.set_chunk_size(None)
+
+
+@pytest.mark.parametrize("S,n", [(3, 40), (74, 128), (75, 128)])
+@pytest.mark.parametrize("chunk", [None, 16])
+def test_captured_calls_same_bits(chunk, S, n, device_status):
+    """Few rows of 256 channels run as separate kernels under stream capture, up to 9472 rows on 148 SMs."""
+    torch.manual_seed(S)
+    with torch.no_grad():
+        m, z, mask = _randn(1, S, n, 256), _randn(1, n, n, 128), (torch.rand(1, S, n, device=DEV) > 0.2).to(torch.bfloat16)
+        row, col, tr = _net(fops.ChunkMSARowAttentionWithPairBias, 256, 128), _net(MSAColumnAttention, 256), _net(fops.Transition, 256)
+        fops.set_chunk_size(chunk)
+        try:
+            for call in (lambda x: row(x, z, mask), lambda x: col(x, mask), tr, lambda x: tr.inplace([x.clone()])[0]):
+                want = call(m)
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph):
+                    got = call(m)
+                graph.replay()
+                assert torch.equal(got, want)
         finally:
             fops.set_chunk_size(None)
