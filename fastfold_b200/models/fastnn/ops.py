@@ -385,8 +385,8 @@ def _key_contiguous(b):
 
 
 def _state_of(tensors):
-    """What tells whether something built from ``tensors`` is still current: memory, type and in-place changes of each."""
-    return tuple((t.data_ptr(), t.dtype, t._version) for t in tensors)
+    """What tells whether something built from ``tensors`` is still current: the memory of each, which is ``_held``, and its in-place changes."""
+    return [(t.data_ptr(), t._version) for t in tensors]
 
 
 def _held(tensors):
