@@ -253,11 +253,28 @@ __device__ __forceinline__ void gc_fold_warps(const float (*rec)[GC_H][GC_REC], 
   }
 }
 
+// thread (h, i): i-th value of head h from the partial states of all CTAs of a cluster
+__device__ __forceinline__ float gc_merge(cooperative_groups::cluster_group& cluster, float* part, int parts) {
+  const int h = threadIdx.x / GC_C, i = threadIdx.x - h * GC_C;
+  float mx = -INFINITY;
+  for (int p = 0; p < parts; ++p) mx = fmaxf(mx, cluster.map_shared_rank(part, p)[h * GC_REC]);
+  float lt = 0.f, at = 0.f;
+  for (int p = 0; p < parts; ++p) {
+    const float* rp = cluster.map_shared_rank(part, p) + h * GC_REC;
+    const float mp = rp[0];
+    const float sc = (mp == -INFINITY) ? 0.f : __expf(mp - mx);
+    lt = fmaf(rp[1], sc, lt);
+    at = fmaf(rp[2 + i], sc, at);
+  }
+  return lt > 0.f ? at / lt : 0.f;
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // The whole column up to its value vector, from the MSA as it is stored ([S][N][64], no transposed copy): masked mean of the
 // normalised rows, projected to the column's eight queries, online softmax over the sequences, o[n][64] in 32 bits.  The gate, which is
-// per row, belongs to the output projection (ln_gemm.cu).  One CTA per column; the rows of a column are 128-byte pieces N rows
-// apart and its keys 32-byte ones, so neighbouring CTAs share cache lines of the keys only.
+// per row, belongs to the output projection (ln_gemm.cu).  One CTA per column, or a cluster of `gridDim.y` CTAs with a slice of the
+// sequences each, whose sums and softmax states are merged through distributed shared memory; the rows of a column are 128-byte pieces
+// N rows apart and its keys 32-byte ones, so neighbouring CTAs share cache lines of the keys only.
 // Replaces transposing the MSA, normalising it, the mask product, two reductions, the query projection and the core kernel below:
 // 14 launches of the layer become 3.
 __global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma,
@@ -266,11 +283,14 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16
                                                                       float* __restrict__ out, int S, int N, float scaling) {
   pdl_launch_dependents();
   pdl_wait();
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
   constexpr int WARPS = GA_THREADS / 32;
-  __shared__ float s_sum[WARPS][GC_HC + 1];
+  __shared__ float s_sum[WARPS][GC_HC + 1], s_total[GC_HC + 1], s_part[GC_H][GC_REC];
   __shared__ float s_mean[GC_HC], s_q[GC_HC];
   __shared__ float s_warp[WARPS][GC_H][GC_REC];
   const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int parts = gridDim.y, s_per = (S + parts - 1) / parts, s_lo = blockIdx.y * s_per, s_hi = min(S, s_lo + s_per);
   // masked sum of the normalised rows (rounded to bf16, as a LayerNorm kernel stores them): eight lanes a row, four rows a warp
   {
     const int li = lane & 7;
@@ -289,13 +309,13 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.f;
     constexpr int U = 4;
-    for (int s0 = warp * 4; s0 < S; s0 += U * WARPS * 4) {      // all lanes of a warp together (shuffles below)
+    for (int s0 = s_lo + warp * 4; s0 < s_hi; s0 += U * WARPS * 4) {      // all lanes of a warp together (shuffles below)
       uint4 raw[U];
       float mk[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int s = s0 + (lane >> 3) + u * WARPS * 4;
-        const bool in = s < S;
+        const bool in = s < s_hi;
         raw[u] = in ? *reinterpret_cast<const uint4*>(x + ((long long)s * N + n) * GC_HC + li * 8) : make_uint4(0, 0, 0, 0);
         mk[u] = in ? __bfloat162float(mask[(long long)s * N + n]) : 0.f;
       }
@@ -317,7 +337,7 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16
         for (int o = 4; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
         const float rstd = rsqrtf(q * (1.f / GC_HC) + eps);
         cnt += mk[u];
-        if (s0 + (lane >> 3) + u * WARPS * 4 < S) {             // an unnormalisable masked row counts as it would in a product with its mask
+        if (s0 + (lane >> 3) + u * WARPS * 4 < s_hi) {             // an unnormalisable masked row counts as it would in a product with its mask
 #pragma unroll
           for (int i = 0; i < 8; ++i) acc[i] = fmaf(mk[u], __bfloat162float(__float2bfloat16(v[i] * rstd * g[i] + b[i])), acc[i]);
         }
@@ -336,11 +356,19 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16
     }
   }
   __syncthreads();
+  if (threadIdx.x <= GC_HC) {
+    float t = 0.f;
+    for (int w = 0; w < WARPS; ++w) t += s_sum[w][threadIdx.x];
+    s_total[threadIdx.x] = t;
+  }
+  if (parts > 1) cluster.sync();
+  else __syncthreads();
   if (threadIdx.x < GC_HC) {
     float t = 0.f, c = 0.f;
-    for (int w = 0; w < WARPS; ++w) {
-      t += s_sum[w][threadIdx.x];
-      c += s_sum[w][GC_HC];
+    for (int p = 0; p < parts; ++p) {
+      const float* r = parts > 1 ? cluster.map_shared_rank(s_total, p) : s_total;
+      t += r[threadIdx.x];
+      c += r[GC_HC];
     }
     s_mean[threadIdx.x] = t / (c + 1e-10f);
   }
@@ -355,7 +383,7 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16
   GcState st;
   gc_init(st);
   const int hg = threadIdx.x & 1;
-  for (int s = threadIdx.x >> 1; s < S; s += GA_THREADS / 2) {
+  for (int s = s_lo + (threadIdx.x >> 1); s < s_hi; s += GA_THREADS / 2) {
     const bf16* at = kv + ((long long)s * N + n) * 2 * GC_C;
     gc_key(st, *reinterpret_cast<const uint4*>(at), *reinterpret_cast<const uint4*>(at + GC_C), __bfloat162float(mask[(long long)s * N + n]) == 0.f,
            s_q + hg * (GC_H / 2) * GC_C);
@@ -366,8 +394,20 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_column_kernel(const bf16
     const int h = threadIdx.x / GC_C, i = threadIdx.x - h * GC_C;
     float mx, lt, at;
     gc_fold_warps(s_warp, h, i, mx, lt, at);
-    out[(long long)n * GC_HC + threadIdx.x] = lt > 0.f ? at / lt : 0.f;
+    if (parts == 1) {
+      out[(long long)n * GC_HC + threadIdx.x] = lt > 0.f ? at / lt : 0.f;
+    } else {
+      if (i == 0) {
+        s_part[h][0] = mx;
+        s_part[h][1] = lt;
+      }
+      s_part[h][2 + i] = at;
+    }
   }
+  if (parts == 1) return;
+  cluster.sync();                              // every CTA's partial is in its shared memory
+  if (blockIdx.y == 0 && threadIdx.x < GC_HC) out[(long long)n * GC_HC + threadIdx.x] = gc_merge(cluster, &s_part[0][0], parts);
+  cluster.sync();                              // nobody leaves while its partial may still be read
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -425,20 +465,7 @@ __global__ void __launch_bounds__(GA_THREADS, 2) global_attention_cluster_kernel
     s_part[h][2 + i] = at;
   }
   cluster.sync();                              // every CTA's partial is in its shared memory
-  if (threadIdx.x < GC_HC) {
-    const int h = threadIdx.x / GC_C, i = threadIdx.x - h * GC_C;
-    float mx = -INFINITY;
-    for (int p = 0; p < parts; ++p) mx = fmaxf(mx, cluster.map_shared_rank(&s_part[0][0], p)[h * GC_REC]);
-    float lt = 0.f, at = 0.f;
-    for (int p = 0; p < parts; ++p) {
-      const float* rp = cluster.map_shared_rank(&s_part[0][0], p) + h * GC_REC;
-      const float mp = rp[0];
-      const float sc = (mp == -INFINITY) ? 0.f : __expf(mp - mx);
-      lt = fmaf(rp[1], sc, lt);
-      at = fmaf(rp[2 + i], sc, at);
-    }
-    s_o[threadIdx.x] = lt > 0.f ? at / lt : 0.f;
-  }
+  if (threadIdx.x < GC_HC) s_o[threadIdx.x] = gc_merge(cluster, &s_part[0][0], parts);
   cluster.sync();                              // nobody leaves (or goes on) while its partial may still be read
   // gate this CTA's slice
   const bf16* gr = gate + r * (long long)S * GC_HC;
@@ -660,9 +687,33 @@ extern "C" int ffb_global_column(const void* x, const void* gamma, const void* b
                                  float* out, long long S, long long N, float scaling, void* stream) {
   using namespace ffb;
   if (S < 1 || N < 1 || S > 0x7fffffffLL || N > 0x7fffffffLL) return -1;
-  launch_light(global_column_kernel, (unsigned)N, GA_THREADS, 0, reinterpret_cast<cudaStream_t>(stream), (const bf16*)x, (const bf16*)gamma,
-               (const bf16*)beta, eps, (const bf16*)wq, (const bf16*)kv, (const bf16*)mask, out, (int)S, (int)N, scaling);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  // Two CTAs per SM are resident; with fewer columns than that a column is split over at most 8 CTAs (the portable cluster size) of 256
+  // sequences or more.  The whole layer in a graph (B200, us, one CTA per column / split): 5120 sequences x 8 residues 118 / 44, 16 132 / 61,
+  // 32 159 / 85, 64 222 / 151, 128 349 / 286, 148 378 / 316; 1024 x 16 38 / 28, 64 60 / 48, 128 78 / 71; 512 x 8 27 / 28, 64 39 / 33.
+  int parts = (int)(2 * 148 / N);
+  parts = parts < 1 ? 1 : (parts > 8 ? 8 : parts);
+  while (parts > 1 && S / parts < 256) --parts;
+  if (parts == 1) {
+    launch_light(global_column_kernel, (unsigned)N, GA_THREADS, 0, st, (const bf16*)x, (const bf16*)gamma, (const bf16*)beta, eps, (const bf16*)wq,
+                 (const bf16*)kv, (const bf16*)mask, out, (int)S, (int)N, scaling);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)N, (unsigned)parts);
+  cfg.blockDim = dim3(GA_THREADS);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = (unsigned)parts;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, global_column_kernel, (const bf16*)x, (const bf16*)gamma, (const bf16*)beta, eps, (const bf16*)wq, (const bf16*)kv,
+                            (const bf16*)mask, out, (int)S, (int)N, scaling) == cudaSuccess
+             ? 0
+             : -2;
 }
 
 extern "C" {

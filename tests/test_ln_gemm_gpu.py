@@ -207,7 +207,7 @@ def test_masks_of_other_shapes(n, device_status):
         assert torch.equal(net._from_raw(z, whole[None]), ref) and torch.equal(net._from_raw(z, row), ref)
 
 
-@pytest.mark.parametrize("S,N", [(1, 3), (5, 40), (31, 8), (130, 33), (700, 17)])
+@pytest.mark.parametrize("S,N", [(1, 3), (5, 40), (31, 8), (130, 33), (700, 17), (512, 3), (2049, 37), (5120, 5), (1030, 148), (600, 149)])
 def test_global_column_attention(S, N, device_status):
     """The layer against the same in 64 bits, with masked sequences and a wholly masked column.  Bound as above, once for the gated
     product that is rounded before the output projection."""
