@@ -153,6 +153,7 @@ Tensor gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, double alpha, OptTensor bi
     g.rowscale = ptr(rowscale);
     g.rs_bstride = (batched && rowscale->dim() == 2) ? M : 0;
     expect(rowscale->numel() >= (g.rs_bstride ? batch : 1) * M, "fewer row factors than rows");
+    expect(rowscale->device() == a.device(), "row factors on another device");
   }
   if (mul) {
     expect(mul->scalar_type() == at::kBFloat16 && mul->stride(-1) == 1, "mul operand");
@@ -256,6 +257,7 @@ std::tuple<Tensor, OptTensor, OptTensor> layer_norm_transposed_fwd(const Tensor&
 std::tuple<Tensor, OptTensor> attention_packed_fwd(const Tensor& qkv, const OptTensor& mask, const OptTensor& bias, int64_t pitch, double scale,
                                                    bool want_lse, bool transposed) {
   const int64_t B = qkv.size(transposed ? 2 : 1), n = qkv.size(transposed ? 1 : 2), H = qkv.size(4), d = qkv.size(5), HD = H * d;
+  expect(!mask || mask->device() == qkv.device(), "mask on another device");
   Tensor out = transposed ? at::empty({1, n, B, HD}, qkv.options()) : at::empty({1, B, n, HD}, qkv.options());
   OptTensor lse;
   if (want_lse) lse = f32({B, H, n}, qkv);
@@ -661,7 +663,7 @@ OptTensor attention_module(const Tensor& x0, const Tensor& gamma, const Tensor& 
   if ((D != 16 && D != 32) || HD % 128 || 3 * HD + 128 > LN_MAX_COLUMNS || !matrix(wq, 3 * HD, C) || !matrix(wg, HD, C) || bg.numel() != HD || !matrix(wo, C, HD) ||
       !vector(bo, C) || gamma.numel() != C || beta.numel() != C)
     return std::nullopt;
-  if (mask && mask->numel() != rows * n) return std::nullopt;
+  if (mask && (mask->numel() != rows * n || mask->device() != x0.device())) return std::nullopt;
   if (pair_w) {
     const Tensor& src = z0 ? *z0 : x0;
     if (H > 32 || !rows_of_channels(src) || src.dim() != 4 || src.size(0) != 1 || src.size(1) != n || src.size(2) != n || !matrix(*pair_w, H, src.size(3)))
@@ -712,7 +714,7 @@ OptTensor attention_module(const Tensor& x0, const Tensor& gamma, const Tensor& 
 // wants 16-byte strides); the padding is neither written nor read.
 OptTensor triangle_module(const Tensor& z0, const Tensor& g1, const Tensor& b1, double eps1, const Tensor& w, const Tensor& b, const Tensor& wg, const Tensor& bg,
                           const Tensor& g2, const Tensor& b2, double eps2, const Tensor& wo, const Tensor& bo, const Tensor& mask, bool outgoing, bool inplace) {
-  if (!rows_of_channels(z0) || z0.dim() != 4 || z0.size(0) != 1 || z0.size(1) != z0.size(2) || z0.size(3) != 128 ||
+  if (!rows_of_channels(z0) || z0.dim() != 4 || z0.size(0) != 1 || z0.size(1) != z0.size(2) || z0.size(3) != 128 || mask.device() != z0.device() ||
       !all_plain(g1, b1, w, b, wg, bg, g2, b2, wo, bo))
     return std::nullopt;
   constexpr int64_t c = 128;
@@ -738,7 +740,7 @@ OptTensor global_column_module(const Tensor& x0, const Tensor& gamma, const Tens
                                const Tensor& bg, const Tensor& wo, const OptTensor& bo, const Tensor& mask, double scale, bool inplace) {
   if (!rows_of_channels(x0) || x0.dim() != 4 || x0.size(0) != 1 || x0.size(3) != 64 || !all_plain(gamma, beta, wq, wkv, wg, bg, wo, bo)) return std::nullopt;
   if (!matrix(wq, 64, 64) || !matrix(wkv, 16, 64) || !matrix(wg, 64, 64) || bg.numel() != 64 || !matrix(wo, 64, 64) || !vector(bo, 64) || gamma.numel() != 64 ||
-      beta.numel() != 64 || mask.numel() != x0.size(1) * x0.size(2))
+      beta.numel() != 64 || mask.numel() != x0.size(1) * x0.size(2) || mask.device() != x0.device())
     return std::nullopt;
   const Tensor x = dense_rows(x0), x2 = x.view({-1, 64});
   const Tensor kv = *ln_qkv(x2, gamma, beta, eps, wkv, std::nullopt, std::nullopt, false);
@@ -749,7 +751,7 @@ OptTensor global_column_module(const Tensor& x0, const Tensor& gamma, const Tens
 // Masked projections of the outer product mean
 std::optional<std::tuple<Tensor, Tensor>> masked_pair(const Tensor& x0, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& wa,
                                                       const OptTensor& ba, const Tensor& wb, const OptTensor& bb, const Tensor& mask) {
-  if (!rows_of_channels(x0) || !all_plain(gamma, beta, wa, ba, wb, bb)) return std::nullopt;
+  if (!rows_of_channels(x0) || !all_plain(gamma, beta, wa, ba, wb, bb) || mask.device() != x0.device()) return std::nullopt;
   const int64_t C = x0.size(-1);
   if (!matrix(wa, wa.size(0), C) || !matrix(wb, wb.size(0), C) || !vector(ba, wa.size(0)) || !vector(bb, wb.size(0)) || wa.size(0) % 8 || wb.size(0) % 8 ||
       wa.size(0) + wb.size(0) + 256 > LN_MAX_COLUMNS || gamma.numel() != C || beta.numel() != C)

@@ -23,6 +23,16 @@ def test_gemm_refuses_fewer_row_factors_than_rows(batch, shape, dtype):
         _gemm(a, torch.zeros(64, 64, dtype=torch.bfloat16), torch.ones(shape, dtype=dtype))
 
 
+def test_factors_and_masks_on_another_device_raise():
+    """Their pointers would be read by a kernel of the other operands' device."""
+    x = torch.zeros(128, 64, dtype=torch.bfloat16)
+    with pytest.raises(AssertionError, match="another device"):
+        _gemm(x, x[:64], torch.ones(128, device="meta"))
+    qkv = torch.zeros(1, 4, 8, 3, 2, 16, dtype=torch.bfloat16)
+    with pytest.raises(AssertionError, match="another device"):
+        _lib.native().attention_packed_fwd(qkv, torch.ones(4, 8, dtype=torch.bfloat16, device="meta"), None, 8, 0.25, False, False)
+
+
 def test_empty_extents_raise():
     """Integer division by an extent of 0 ends the process in native code; it raised in Python."""
     n, w = _lib.native(), torch.ones(0, dtype=torch.bfloat16)

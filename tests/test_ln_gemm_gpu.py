@@ -470,3 +470,17 @@ def test_captured_calls_same_bits(chunk, S, n, device_status):
                 assert torch.equal(got, want)
         finally:
             fops.set_chunk_size(None)
+
+
+def test_masks_in_host_memory_raise(device_status):
+    """No kernel is launched with them: the native calls leave them to the composition, which refuses them."""
+    with torch.no_grad():
+        m, e, z = _randn(1, 9, 24, 256), _randn(1, 9, 24, 64), _randn(1, 24, 24, 128)
+        mask, zmask = torch.ones(1, 9, 24, dtype=torch.bfloat16), torch.ones(1, 24, 24, dtype=torch.bfloat16)
+        row, col, opm = _net(fops.ChunkMSARowAttentionWithPairBias, 256, 128), _net(MSAColumnAttention, 256), _net(fops.OutProductMean, 256, 128, 32)
+        glob, start = _net(fops.ChunkMSAColumnGlobalAttention, 64), _net(fops.ChunkTriangleAttentionStartingNode, 128, p_drop=0.0)
+        mul = _net(fops.AsyncChunkTriangleMultiplicationOutgoing, 128, p_drop=0.0)
+        for call in (lambda: row(m, z, mask), lambda: col(m, mask), lambda: opm(m, mask, z), lambda: glob(e, mask), lambda: start(z, zmask),
+                     lambda: mul(z, zmask)):
+            with pytest.raises((AssertionError, RuntimeError)):
+                call()
