@@ -800,9 +800,7 @@ PYBIND11_MODULE(_ffb_dispatch, m) {
   m.def("ln_chain", &ln_chain);
   m.def("ln_qkv", &ln_qkv);
   m.def("ln_tri_in", &ln_tri_in);
-  m.def("ln_tri_out", &ln_tri_out);
   m.def("ln_pair", &ln_pair);
-  m.def("global_column", &global_column);
   m.def("transition_module", &transition_module);
   m.def("attention_module", &attention_module);
   m.def("triangle_module", &triangle_module);

@@ -22,10 +22,10 @@
 // The products of chunk h + 1 are issued before the second product of chunk h, which hides the epilogue.
 //
 // What bounds it: the weights, which every tile of 128 rows streams from L2 again (1 MB a tile for the transition of 256 channels, which
-// runs at 0.44 of the tensor cores' rate), the output bytes of the wide projections, and below some 20 tiles the chain of a single tile.
+// at 32768 rows runs at 0.44 of the tensor cores' rate), the output bytes of the wide projections, and with few tiles the chain of one.
 //   Measured (B200, against LayerNorm and GEMM kernels in the same order, us): transition 262144 x 64 89 -> 46, 65536 x 128
-//   47 -> 32, 589824 x 128 341 -> 208, 32768 x 256 54 -> 48, 2048 x 256 16 -> 26 (three launches fewer by two: the host side gains more
-//   than that); gated output with the norm (left side without it) 589824 x 128 192 -> 139, 32768 x 256 30 -> 24; QKV 589824 x 128
+//   47 -> 32, 589824 x 128 341 -> 208, 32768 x 256 54 -> 48, 2048 x 256 16 -> 26 (one launch in place of three: host/dispatch.cpp, which chooses,
+//   has the line between the two); gated output with the norm (left side without it) 589824 x 128 192 -> 139, 32768 x 256 30 -> 24; QKV 589824 x 128
 //   181 -> 130; operands and gate of the triangle multiplication at 1024 residues 539 -> 480, its output 293 -> 177.
 //
 // Stands for the nn.LayerNorm / nn.Linear / elementwise chains of the reference (fastfold/model/fastnn/ops.py:85-106, 143-160,

@@ -49,19 +49,9 @@ def tri_in(x, norm, w, b, wg, bg, scale, lr):
     return _lib.native().ln_tri_in(x, norm.weight, norm.bias, norm.eps, w, b, wg, bg, scale, lr)
 
 
-def tri_out(p, norm, w, b, mul, resid, out=None):
-    """``resid + mul * (LN(p) w^T + b)`` of a channels-first ``p [c, batch, rows]``."""
-    return _lib.native().ln_tri_out(p, norm.weight, norm.bias, norm.eps, w, b, mul, resid, out)
-
-
 def pair(x, norm, wa, ba, wb, bb, scale):
     """``(LN(x) wa^T + ba) * scale`` and the same with ``wb``, ``bb``; one factor per row."""
     return _lib.native().ln_pair(x, norm.weight, norm.bias, norm.eps, wa, ba, wb, bb, scale)
-
-
-def global_column(x, norm, wq, kv, mask, scaling):
-    """Value vectors ``[N, 64]`` (fp32) of the global column attention over ``x [S, N, 64]``: one mean query per column and head."""
-    return _lib.native().global_column(x, norm.weight, norm.bias, norm.eps, wq, kv, mask, scaling)
 
 
 def transition(x, norm, l1, l2, inplace):

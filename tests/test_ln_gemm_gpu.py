@@ -7,7 +7,7 @@ import torch
 
 from fastfold_b200.models.fastnn import ops as fops
 from fastfold_b200.models.fastnn.msa import MSAColumnAttention
-from fastfold_b200.ops import LayerNorm, _lib, ln_gemm
+from fastfold_b200.ops import LayerNorm, ln_gemm
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -133,7 +133,7 @@ def test_partial_tiles_in_batches(n, device_status):
         first = None
         for _ in range(6):
             lr = torch.zeros(256, n, (n + 7) // 8 * 8, device=DEV, dtype=torch.bfloat16)[:, :, :n]
-            gate = _lib.native().ln_tri_in(z, norm.weight, norm.bias, norm.eps, w, b, wg, bg, mask, lr)
+            gate = ln_gemm.tri_in(z, norm, w, b, wg, bg, mask, lr)
             if first is None:
                 first = (lr, gate)
                 for i in range(n):
