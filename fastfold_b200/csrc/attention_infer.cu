@@ -714,12 +714,8 @@ int ffb_attention_infer(const void* q, const void* k, const void* v, long long q
   }
   auto kern = D == 32 ? (bias ? attn_infer_kernel<32, true> : attn_infer_kernel<32, false>)
                       : (bias ? attn_infer_kernel<16, true> : attn_infer_kernel<16, false>);
-  static bool attr[4];
-  const int which = (D == 32 ? 0 : 2) + (bias ? 1 : 0);
-  if (!attr[which]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnInferSmem::TOTAL) != cudaSuccess) return -14;
-    attr[which] = true;
-  }
+  static SmemLimit limit[4];
+  if (!limit[(D == 32 ? 0 : 2) + (bias ? 1 : 0)].raise(kern, AttnInferSmem::TOTAL)) return -14;
   static int sm_count = 0;
   if (!sm_count) {
     int dev = 0;

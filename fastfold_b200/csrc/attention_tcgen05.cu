@@ -507,11 +507,8 @@ int ffb_attention_fwd(const void* q, const void* k, const void* v, long long q_b
   } else {
     tb = tq;
   }
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmem::TOTAL) != cudaSuccess) return -14;
-    attr = true;
-  }
+  static SmemLimit limit;
+  if (!limit.raise(attn_fwd_kernel<32>, AttnSmem::TOTAL)) return -14;
   static int sm_count = 0;
   if (!sm_count) {
     int dev = 0;
@@ -994,11 +991,8 @@ int ffb_attention_bwd_strided(const void* q, const void* k, const void* v, long 
   } else {
     tb = tq;
   }
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(attn_bwd_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::TOTAL) != cudaSuccess) return -15;
-    attr = true;
-  }
+  static SmemLimit limit;
+  if (!limit.raise(attn_bwd_kernel<32>, BwdSmem::TOTAL)) return -15;
   static int sm_count = 0;
   if (!sm_count) {
     int dev = 0;

@@ -163,13 +163,8 @@ static int layernorm_bwd_transposed_impl(const void* dy, const void* x, const vo
   if (rows <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const size_t smem = sizeof(float) * 2 * C * (LTB_ROWS + 1);
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(ln_bwd_transposed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * 2 * 256 * (LTB_ROWS + 1))) !=
-        cudaSuccess)
-      return -3;
-    attr = true;
-  }
+  static SmemLimit limit;
+  if (!limit.raise(ln_bwd_transposed_kernel, sizeof(float) * 2 * 256 * (LTB_ROWS + 1))) return -3;
   const long long nb = (rows + LTB_ROWS - 1) / LTB_ROWS;
   if (nb > 0x7fffffffLL) return -4;
   launch_light(ln_bwd_transposed_kernel, (unsigned)nb, 256, smem, st, (const bf16*)dy, (const bf16*)x, (const bf16*)gamma, mean, rstd, (bf16*)dx, part,

@@ -10,6 +10,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 namespace ffb {
 
 typedef __nv_bfloat16 bf16;
@@ -289,6 +291,24 @@ inline int pdl_mode() {
   return mode;
 }
 inline bool pdl_enabled() { return pdl_mode() != 0; }
+
+// A kernel's limit of dynamic shared memory is an attribute of the device: one static of these beside each launch that needs more than
+// 48 KB sets it on the first launch on every device (and again on each beyond the 64th).
+class SmemLimit {
+  std::atomic<unsigned long long> set_{0};
+
+ public:
+  template <typename... KArgs>
+  bool raise(void (*kern)(KArgs...), size_t bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+    if (set_.load(std::memory_order_relaxed) & bit) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+    set_.fetch_or(bit, std::memory_order_relaxed);
+    return true;
+  }
+};
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_attr(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {

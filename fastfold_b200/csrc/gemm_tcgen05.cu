@@ -855,14 +855,11 @@ template <int BN, bool A_MN, bool B_MN, int PEER = 0>
 static int launch_cfg(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* epi, int tma_epi, const GemmArgs& g, int batch,
                       cudaStream_t st, const PeerMaps* pm = nullptr) {
   using Cfg = GemmCfg<BN>;
-  static bool attr_set = false;
+  static SmemLimit limit;
   static PeerMaps no_peers;
   if (!pm) pm = &no_peers;
   auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, PEER>;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess) return -2;
-    attr_set = true;
-  }
+  if (!limit.raise(kern, Cfg::SMEM)) return -2;
   const int tiles_n = (g.N + BN - 1) / BN, tiles_m = (g.M + BM - 1) / BM;
   const long long num_tiles = (long long)tiles_n * tiles_m * batch * g.splits;
   if (num_tiles > 0x7fffffffLL) return -5;

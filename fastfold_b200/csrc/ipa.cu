@@ -291,11 +291,8 @@ static int ipa_launch(const IpaArgs& a, cudaStream_t st) {
   constexpr int HH = 12, CC = 16, PQ = 4, PV = 8, CZZ = 128;
   constexpr size_t smem = 2 * R * IPA_J * (CZZ + IPA_ZP) * 2 + sizeof(float) * (HH * CZZ + R * HH * CC + R * HH * PQ * 3 + R * HH * IPA_J + 2 * R * HH);
   auto kern = ipa_fwd_kernel<R, HH, CC, PQ, PV, CZZ>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -4;
-    attr = true;
-  }
+  static SmemLimit limit;
+  if (!limit.raise(kern, smem)) return -4;
   launch_light(kern, (a.rows + R - 1) / R, IPA_THREADS, smem, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

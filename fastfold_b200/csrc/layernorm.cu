@@ -811,13 +811,8 @@ int ffb_layernorm_fwd_transposed(const void* x, const void* gamma, const void* b
                    (const bf16*)beta, (bf16*)y, rows, eps);
       return cudaGetLastError() == cudaSuccess ? 0 : -1;
     }
-    static bool attr = false;
-    if (!attr) {
-      if (cudaFuncSetAttribute(ln_fwd_transposed64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * 256 * (LNT64 + 1))) !=
-          cudaSuccess)
-        return -3;
-      attr = true;
-    }
+    static SmemLimit limit;
+    if (!limit.raise(ln_fwd_transposed64_kernel, sizeof(float) * 256 * (LNT64 + 1))) return -3;
     const size_t smem64 = sizeof(float) * C * (LNT64 + 1);
     launch_light(ln_fwd_transposed64_kernel, (unsigned)((rows + LNT64 - 1) / LNT64), 256, smem64, st, (const bf16*)x, (const bf16*)gamma, (const bf16*)beta, (bf16*)y, mean, rstd, rows, C, eps);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;

@@ -820,11 +820,8 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
 template <int C, int MODE, bool CF>
 static int lg_launch(const LgMaps& maps, const LgArgs& a, cudaStream_t st) {
   auto kern = ln_gemm_kernel<C, MODE, CF>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LgCfg<C, MODE>::SMEM) != cudaSuccess) return -30;
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  if (!limit.raise(kern, LgCfg<C, MODE>::SMEM)) return -30;
   static int sm_count = 0;
   if (!sm_count) {
     int dev = 0;
