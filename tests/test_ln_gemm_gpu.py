@@ -1,7 +1,7 @@
-"""LayerNorm + GEMM kernels (csrc/ln_gemm.cu) and the column kernel of global_attention.cu against the same mathematics in 64 bits,
-with the roundings to bf16 that the kernels make (normalised rows, hidden activation) made there too.  Bound: what is left are the fp32
-sums and the rounding of the result, 2^-9 of each value at most, so 2^-9 in the 2-norm; a normalised or hidden value that rounds the
-other way adds less than that again."""
+"""LayerNorm + GEMM kernels (csrc/ln_gemm.cu) and the column kernel of global_attention.cu against the separate kernels, whose bits the
+former give, and against the same mathematics in 64 bits with the roundings to bf16 that the kernels make (normalised rows, hidden
+activation) made there too.  Bound: what is left are the fp32 sums and the rounding of the result, 2^-9 of each value at most, so 2^-9 in
+the 2-norm; a normalised or hidden value that rounds the other way adds less than that again."""
 import pytest
 import torch
 
@@ -42,10 +42,10 @@ def _lin(x, w, b=None):
 
 
 @pytest.mark.parametrize("C", [64, 128, 256])
-@pytest.mark.parametrize("M", [1, 31, 128, 129, 19000])
+@pytest.mark.parametrize("M", [1, 31, 128, 129, 19000, 60007])
 def test_chains(C, M, device_status):
-    """Transition and gated output: less than a tile, a whole one, a remainder of one row, more tiles than CTAs; one and two chunks
-    of gated columns; the result over the residual."""
+    """Transition and gated output: less than a tile, a whole one, a remainder of one row, more tiles than CTAs, several per CTA; one and
+    two chunks of gated columns; the result over the residual."""
     torch.manual_seed(C + M)
     with torch.no_grad():
         x, norm, H = _randn(M, C), _norm(C), 4 * C
@@ -142,7 +142,7 @@ def test_partial_tiles_in_batches(n, device_status):
             assert torch.equal(lr, first[0]) and torch.equal(gate, first[1])
 
 
-@pytest.mark.parametrize("M,dtype", [(3, torch.bfloat16), (300, torch.float32), (5000, torch.bfloat16)])
+@pytest.mark.parametrize("M,dtype", [(3, torch.bfloat16), (300, torch.float32), (5000, torch.bfloat16), (60007, torch.float32)])
 @pytest.mark.parametrize("C", [64, 256])
 def test_pair_of_projections(C, M, dtype, device_status):
     torch.manual_seed(M)
