@@ -44,6 +44,24 @@ __device__ __forceinline__ void key_bits(const bf16* mrow, int kbase, int n_k, i
   keep_hi = __ballot_sync(0xffffffffu, on_b);
 }
 
+// The same in two steps, for entries that are loaded ahead of their use.
+struct KeyMask {
+  uint16_t a, b;                  // non-zero (but for the sign): key kbase + lane, key kbase + 32 + lane counts
+};
+__device__ __forceinline__ KeyMask load_keys(const bf16* mrow, int kbase, int n_k, int lane) {
+  KeyMask m = {0, 0};
+  const uint16_t* p = reinterpret_cast<const uint16_t*>(mrow) + kbase + lane;
+  if (kbase + lane < n_k) m.a = mrow ? p[0] : 1;
+  if (kbase + 32 + lane < n_k) m.b = mrow ? p[32] : 1;
+  return m;
+}
+struct alignas(8) Keys {
+  uint32_t lo, hi;
+};
+__device__ __forceinline__ Keys key_bits(KeyMask m) {
+  return Keys{__ballot_sync(0xffffffffu, m.a & 0x7fffu), __ballot_sync(0xffffffffu, m.b & 0x7fffu)};
+}
+
 // Masked keys take this logit (replaced, not added).  -2^30 instead of the reference's -1e9: its product with log2(e) is
 // exact in fp32, so a fully masked row still comes out as exactly uniform weights from the fused multiply-add form
 // exp2(v * log2e - m * log2e); any finite logit next to it underflows to weight 0 either way.

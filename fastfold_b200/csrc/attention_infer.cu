@@ -4,32 +4,35 @@
 //
 // in one kernel, flash style: logits never reach global memory.  The pair bias
 // is shared by every batch row b (MSA row attention: all N_seq rows; triangle
-// attention: all N_res rows), so a CTA works on FOUR batch rows of one (head,
-// 128-query tile) at a time and all four read the same bias tile in shared memory.
+// attention: all N_res rows), so a CTA works on THREE batch rows of one (head,
+// 128-query tile) at a time and all three read the same bias tile in shared memory.
 //
-// Per CTA (640 threads):
-//   warp 0      TMA producer: per group a Q tile (2 stages) and K / V blocks of 64 keys (2 stages; swizzled, straight out
+// Per CTA (512 threads):
+//   warp 0      TMA producer: per group a Q tile (2 stages) and K / V blocks of 64 keys (4 stages; swizzled, straight out
 //               of the fused QKV projection output), bias tiles of 128 x 64 (4 slots, resident for up to 256 keys)
-//   warps 1-2   MMA issuers, two groups each: S = Q K^T (128 x 64) and O += P V (128 x D x 64, P read from tensor memory);
-//               the S product of a group's next block goes out as soon as the group has read the last one
-//   warps 4-19  softmax, four groups of four warps, one batch row each, one thread per query row.  A thread streams its
+//   warps 1-3   MMA issuer of a group each: S = Q K^T (128 x 64, two blocks ahead, into two buffers) and O += P V (128 x D x 64,
+//               P read from tensor memory); these warps also work out which keys of a block count and release the bias tiles
+//   warps 4-15  softmax, three groups of four warps, one batch row each, one thread per query row.  A thread streams its
 //               row's 64 logits once: p = exp2(logit * log2e - M), row sum, P packed to bf16 into tensor memory.
 //
-// What should bound it are the exponentials, 16 per clock and SM; what does is instruction issue and the latency around a
-// block.  So the loop around the exponentials is kept short: two-wide FMA / add (fma.rn.f32x2), no running maximum and no
-// rescaling of the output.  The reference point M of a row only has to keep the row sum inside the exponent range, so it
-// starts at 0 and is moved (exact block maximum, output and sum rescaled) only when the sum leaves [2^-60, 2^60] - a
-// warp-uniform side path; bf16 and fp32 have the same exponent range, so P, the sums and the output lose no precision at
+// What should bound it are the exponentials, 16 per clock and SM: 512 cycles a block of 128 x 64.  The arithmetic around them
+// (unpacking the bias, packing P, the sum) brings three softmax warps on a scheduler to 640; the rest is what happens between two
+// blocks.  So everything that another warp can do is done there, the loop around the exponentials is kept short: two-wide
+// FMA (fma.rn.f32x2), sums of bf16 without unpacking (add.f32.bf16), no running maximum and no rescaling of the output; and the
+// warps of a scheduler are kept out of step (take_turn).  The reference point M of a row only has to keep the row sum inside the
+// exponent range, so it starts at 0 and is moved (exact block maximum, output and sum rescaled) only when the sum leaves
+// [2^-60, 2^60] - a warp-uniform side path; bf16 and fp32 have the same exponent range, so P, the sums and the output lose no precision at
 // any M in between, as long as P V has room too: a row whose sum is near 2^60 takes values up to 2^68, one near 2^-60 down
 // to 2^-56.  A narrower window would give them more, but the side path nearly doubles a block's time (q 4x as large,
 // n 256, B 256: 40 us with this window, 43 with 2^+-32, 69 with 2^+-24).  Rows whose logits are themselves masks (biases of
 // -1e9, the lowest bf16 value, -inf) take a general step, see FAR_LOGIT.
-// Four groups, because a group waits for its S product once per block and the others fill that time.
-// Two issuer warps with descriptors that are only added to: with one issuer that built each descriptor where it was used,
-// its instructions were the longest chain of a block and the kernel took 1.8x as long.
-//   Measured (B200 at 1965 MHz, alternating with the kernel that also serves training, which keeps a running maximum and P
-//   in shared memory): B 128, H 4, n 1024 with bias 451 -> 246 us, with a random mask 516 -> 267 us; B 256, H 4, n 256
-//   67 -> 40 us; B 256, H 8, n 128 without bias 46 -> 21 us; B 32, H 8, n 64 8.6 -> 5.8 us.
+// Three groups with two S buffers each (480 of the 512 columns; P takes the place of the S it was made from), not four with one:
+// a group never waits for its S product.  With four of them the products' latency, 1500 - 1900 cycles of 4400 a block, was
+// bare, since all four were in step.
+//   Measured (B200, graph replay, us; four groups with one S buffer -> this): B 384, H 4, n 1536 with bias and mask 1690 -> 1368;
+//   B 64, H 4, n 1024 130 -> 113; B 389, H 4, n 389 191 -> 140; B 256, H 4, n 256 41.6 -> 35.7; B 1024, H 8, D 16, n 256 309 -> 210;
+//   B 300, H 2, n 700 without bias 138 -> 117; B 256, H 8, n 128 without bias 22.9 -> 21.8; B 32, H 8, n 64 5.6 -> 5.0.  Random masks:
+//   1850 -> 1611, 146 -> 136, 205 -> 157, 45.0 -> 41.4, 328 -> 255, 148 -> 130, 24.2 -> 23.5, 5.9 -> 5.2.
 // Masked keys get a huge negative logit (replaced, not added; -2^30 here, -1e9 in the reference's
 // softmax kernels, softmax_cuda_kernel.cu:338-423,618-706 - same weights), which is weight 0 next to any ordinary
 // key: there they are left out; keys beyond the sequence end get -inf.
@@ -47,18 +50,23 @@
 namespace ffb {
 
 constexpr int AF_BQ = 128;      // queries per tile
-constexpr int AF_GROUPS = 4;    // batch rows in flight per CTA
+constexpr int AF_GROUPS = 3;    // batch rows in flight per CTA
 constexpr int AF_BK = 64;       // keys per block
 constexpr int AF_THREADS = 128 + AF_GROUPS * 128;
 constexpr int AF_BSLOTS = 4;    // bias tiles in shared memory
-constexpr int AF_ISSUERS = 2;   // MMA issuer warps
-// tensor memory of group g: columns g * 128 + [0, 64) S, [64, 96) P (bf16 pairs), [96, 128) O
-constexpr uint32_t AF_TM_P = 64, AF_TM_O = 96;
+constexpr int AF_KVST = 4;      // K / V stages per group
+constexpr int AF_COST = 16;     // cost of a round of a full query tile
+// tensor memory of group g: columns g * 160 + [0, 64) and [64, 128) two S buffers, each with its P (bf16 pairs) over the first 32
+// columns once it has been read, [128, 160) O
+constexpr uint32_t AF_TM_GROUP = 160, AF_TM_O = 128;
 
 struct AttnInferArgs {
   int B, H, n_q, n_k;            // batch rows, heads, query / key lengths
   int n_qt, n_kb;                // query tiles (128), key blocks (64)
-  int units;                     // H * n_qt * B (head, query tile, batch row) units
+  int rounds, few, rest;         // rounds of a (head, query tile): `few` batch rows each, one more in the first `rest`
+  int cost_last;                 // cost of a round of the last query tile, where others cost AF_COST
+  long long share;               // cost of a CTA's rounds; the first `extra` CTAs take one more
+  int extra;
   int bias_resident;             // 1: n_kb <= AF_BSLOTS, bias tiles stay in shared memory across batch rows
   float scale, scale_log2e;      // logit scale, and times log2(e)
   const bf16* mask;              // [B][n_k] or null
@@ -77,12 +85,14 @@ __device__ __forceinline__ void write_penalties(float* pen, int lane, uint32_t k
 
 struct AttnInferSmem {
   // offsets (bytes) from the 1024-aligned base
-  static constexpr int Q = 0;                                          // [group][2] x [128][64 B]          64 KB
-  static constexpr int KV = Q + AF_GROUPS * 2 * 8192;                  // [group][2] x (K 4 KB + V 4 KB)    64 KB
-  static constexpr int BIAS = KV + AF_GROUPS * 2 * 8192;               // [slot] x [128][128 B]             64 KB
-  static constexpr int KP = BIAS + AF_BSLOTS * 16384;                  // [16 warps][64] penalties            4 KB
-  static constexpr int BARS = KP + AF_GROUPS * 4 * 64 * 4;
-  static constexpr int TOTAL = BARS + 512 + 1024;
+  static constexpr int Q = 0;                                          // [group][2] x [128][64 B]          48 KB
+  static constexpr int KV = Q + AF_GROUPS * 2 * 8192;                  // [group][stage] x (K 4 KB + V 4 KB) 96 KB
+  static constexpr int BIAS = KV + AF_GROUPS * AF_KVST * 8192;         // [slot] x [128][128 B]             64 KB
+  static constexpr int KP = BIAS + AF_BSLOTS * 16384;                  // [12 warps][64] penalties            3 KB
+  static constexpr int KEYS = KP + AF_GROUPS * 4 * 64 * 4;             // [group][2] key bits of the blocks in the S buffers
+  static constexpr int TURN = KEYS + 48;                               // [scheduler] whose turn it is
+  static constexpr int BARS = TURN + 16;
+  static constexpr int TOTAL = BARS + 576 + 1024;
 };
 
 // two floats in one 64-bit register pair: the FMA pipe does both in one instruction
@@ -103,14 +113,26 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return d;
 }
 
-// 32 logits (columns c0 .. c0+31 of the block) of one row in the log2 domain, relative to the row's reference point:
+// a + the lower / upper bf16 of w
+__device__ __forceinline__ float add_lo(float a, uint32_t w) {
+  float d;
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %1;\n\t}" : "=f"(d) : "f"(a), "r"(w));
+  return d;
+}
+__device__ __forceinline__ float add_hi(float a, uint32_t w) {
+  float d;
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, h, %1;\n\t}" : "=f"(d) : "f"(a), "r"(w));
+  return d;
+}
+
+// 16 logits (columns c0 .. c0+15 of the block) of one row in the log2 domain, relative to the row's reference point:
 // s * scale * log2e + (bias * log2e + add), plus the penalty of keys that do not count unless all of the block's do.
 template <bool PLAIN, bool BIAS>
-__device__ __forceinline__ void logits32(uint64_t (&t)[16], const float (&s)[32], const uint8_t* brow, int r, int c0, const float* pen,
+__device__ __forceinline__ void logits16(uint64_t (&t)[8], const float (&s)[16], const uint8_t* brow, int r, int c0, const float* pen,
                                          float scale_log2e, float add) {
   const uint64_t sc = pk2(scale_log2e, scale_log2e), ad = pk2(add, add), l2e = pk2(LOG2E, LOG2E);
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
+  for (int u = 0; u < 2; ++u) {
     uint64_t b[4];
     if (BIAS) {
       const uint4 raw = *reinterpret_cast<const uint4*>(brow + ((((c0 >> 3) + u) ^ (r & 7)) << 4));
@@ -135,54 +157,57 @@ __device__ __forceinline__ void logits32(uint64_t (&t)[16], const float (&s)[32]
   }
 }
 
-// p = exp2(t) of 32 logits, packed to bf16 pairs, and the two-wide running sum of p as rounded to bf16 - that is what the
-// tensor core multiplies V with, so in a row that one key dominates the rounding of its p cancels.
-__device__ __forceinline__ void exp32(const uint64_t (&t)[16], uint32_t (&p)[16], uint64_t& sum) {
+// 16 columns of a row
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, float (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]),
+        "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+      : "r"(taddr));
+}
+
+// tmem_ld_wait that the loaded registers pass through: nothing that reads them moves ahead of it
+template <int N>
+__device__ __forceinline__ void tmem_ld_wait_for(float (&v)[N]) {
+  tmem_ld_wait();
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    float a, b;
-    up2(t[i], a, b);
-    a = ex2f(a);
-    b = ex2f(b);
-    const bf162 h = __floats2bfloat162_rn(a, b);
-    p[i] = *reinterpret_cast<const uint32_t*>(&h);
-    sum = add2(sum, pk2(bf_lo(p[i]), bf_hi(p[i])));
+  for (int i = 0; i < N; i += 8)
+    asm volatile("" : "+f"(v[i]), "+f"(v[i + 1]), "+f"(v[i + 2]), "+f"(v[i + 3]), "+f"(v[i + 4]), "+f"(v[i + 5]), "+f"(v[i + 6]), "+f"(v[i + 7]));
+}
+
+// The 64 logits of a row's block, 16 at a time with the next 16 on their way: p = exp2(t), packed to bf16 pairs, and the two-wide
+// running sum of p as rounded to bf16 - that is what the tensor core multiplies V with, so in a row that one key dominates the
+// rounding of its p cancels.  Not PLAIN: where none of 16 keys counts the weights are 0.
+// `after_first` is called once a quarter is done.
+template <bool PLAIN, bool BIAS, typename F>
+__device__ __forceinline__ void softmax_block(uint32_t tm_s, const uint8_t* brow, int r, const float* pen, float scale_log2e, float add,
+                                              Keys keys, uint32_t (&p)[32], float2& sum, F&& after_first) {
+  float s[2][16];
+  tmem_ld_32x16(tm_s, s[0]);
+  tmem_ld_wait_for(s[0]);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (q < 3) tmem_ld_32x16(tm_s + (q + 1) * 16, s[(q + 1) & 1]);
+    if (q == 1) after_first();
+    if (PLAIN || ((q < 2 ? keys.lo : keys.hi) & (q & 1 ? 0xffff0000u : 0xffffu))) {
+      uint64_t t[8];
+      logits16<PLAIN, BIAS>(t, s[q & 1], brow, r, q * 16, pen, scale_log2e, add);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float x, y;
+        up2(t[i], x, y);
+        const bf162 h = __floats2bfloat162_rn(ex2f(x), ex2f(y));
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(&h);
+        p[q * 8 + i] = w;
+        sum.x = add_lo(sum.x, w);
+        sum.y = add_hi(sum.y, w);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) p[q * 8 + i] = 0u;
+    }
+    if (q < 3) tmem_ld_wait_for(s[(q + 1) & 1]);
   }
-}
-
-__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
-      : "memory");
-}
-
-// One pass over the 64 logits of a row's block: probabilities into tensor memory, their sum.
-template <bool PLAIN, bool BIAS>
-__device__ __forceinline__ void softmax_block(uint32_t tm_s, uint32_t tm_p, const uint8_t* brow, int r, const float* pen, float scale_log2e,
-                                              float add, uint64_t& sum) {
-#pragma unroll 1
-  for (int c = 0; c < 2; ++c) {
-    float s[32];
-    uint64_t t[16];
-    uint32_t p[16];
-    tmem_ld_32x32(tm_s + c * 32, s);
-    tmem_ld_wait();
-    logits32<PLAIN, BIAS>(t, s, brow, r, c * 32, pen, scale_log2e, add);
-    exp32(t, p, sum);
-    tmem_st_32x16(tm_p + c * 16, p);
-  }
-}
-
-// D[tmem] (+)= A[tmem] * B[smem]: bf16 A, two elements per column
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 
 constexpr float ROW_SUM_LO = 8.673617379884035e-19f, ROW_SUM_HI = 1.152921504606847e18f;   // 2^-60, 2^60
@@ -217,15 +242,15 @@ __device__ __forceinline__ void tmem_st_32x4(uint32_t taddr, const uint32_t (&v)
 
 // A block of keys for a warp that holds a far row: the general softmax step.  Rows with `move` get a new reference point (the
 // output and the sum so far are rescaled to it), the others keep theirs.  Eight columns at a time and inlined: no row of a
-// model's own biases gets here, but the ordinary path uses all registers that five warps per scheduler leave, and a call or
-// wider pieces cost it 2 - 8 % (n 389, B 389, H 4 with bias: 192 us without this path, 193 us as it is, 205 us as a call).
+// model's own biases gets here, and the ordinary path uses all registers that four warps per scheduler leave: a call or wider
+// pieces cost it.
 template <bool BIAS>
-__device__ __forceinline__ RowState far_block(RowState st, bool move, uint32_t tm, bool has_o, const uint8_t* brow, int r, uint32_t keep_lo,
-                                           uint32_t keep_hi, int keys, float scale, float scale_log2e) {
+__device__ __forceinline__ RowState far_block(RowState st, bool move, uint32_t tm_s, uint32_t tm_o, bool has_o, const uint8_t* brow, int r,
+                                           Keys kb, int keys, float scale, float scale_log2e) {
   constexpr float LN2 = 0.6931471805599453f;
-  const uint64_t keep = keep_lo | (uint64_t)keep_hi << 32;        // `keys` of the 64 are in the sequence
+  const uint64_t keep = kb.lo | (uint64_t)kb.hi << 32;        // `keys` of the 64 are in the sequence
   auto load = [&](int c, float (&s)[8], float (&b)[8]) {
-    tmem_ld_32x8(tm + c * 8, s);
+    tmem_ld_32x8(tm_s + c * 8, s);
     tmem_ld_wait();
     if (BIAS) {
       const uint4 raw = *reinterpret_cast<const uint4*>(brow + ((c ^ (r & 7)) << 4));
@@ -239,7 +264,6 @@ __device__ __forceinline__ RowState far_block(RowState st, bool move, uint32_t t
   auto logit = [&](int key, float s, float b) -> float {          // natural units
     return (keep >> key) & 1u ? fmaf(s, scale, b) : (key < keys ? MASKED_LOGIT : -INFINITY);
   };
-  tmem_st_wait();                          // what the ordinary path stored for this block is about to be replaced
   float mx = -INFINITY, alpha = 1.f;
 #pragma unroll 1
   for (int c = 0; c < 8; ++c) {
@@ -262,11 +286,11 @@ __device__ __forceinline__ RowState far_block(RowState st, bool move, uint32_t t
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {          // heads of 16 channels: the upper columns are nobody's
       float o[8];
-      tmem_ld_32x8(tm + AF_TM_O + c * 8, o);
+      tmem_ld_32x8(tm_o + c * 8, o);
       tmem_ld_wait();
 #pragma unroll
       for (int e = 0; e < 8; ++e) o[e] *= alpha;
-      tmem_st_32x8(tm + AF_TM_O + c * 8, o);
+      tmem_st_32x8(tm_o + c * 8, o);
     }
   }
   float sum = 0.f;
@@ -286,10 +310,71 @@ __device__ __forceinline__ RowState far_block(RowState st, bool move, uint32_t t
       p[i] = *reinterpret_cast<const uint32_t*>(&h);
       sum += bf_lo(p[i]) + bf_hi(p[i]);
     }
-    tmem_st_32x4(tm + AF_TM_P + c * 4, p);
+    tmem_st_32x4(tm_s + c * 4, p);         // over columns that have been read: 4c + 3 < 8 (c + 1)
   }
   st.l = st.l * alpha + sum;
   return st;
+}
+
+// Where the rows of a (query tile, batch row) lie in the tile's 128 lanes.  The last tile of a sequence may fill only some of the
+// four warps; such a tile is loaded so that it starts at another warp's lanes from batch row to batch row, because warp q of a
+// group runs on scheduler q: the warps without a row have nothing to do, and the work stays spread over the schedulers.
+struct TileRows {
+  int first, warps;               // first warp with rows, number of warps with rows
+};
+__device__ __forceinline__ TileRows tile_rows(int n_q, int qt, int b) {
+  const int rows = n_q - qt * AF_BQ;
+  TileRows t;
+  t.warps = rows >= AF_BQ ? 4 : (rows + 31) >> 5;
+  t.first = t.warps == 1 ? (b & 3) : t.warps == 2 ? (b & 1) * 2 : t.warps == 3 ? (b & 1) : 0;
+  return t;
+}
+
+// A round is up to AF_GROUPS batch rows of one (head, query tile), spread evenly over the tile's rounds; rounds are numbered tile by
+// tile, and every role of a CTA walks the same ones.
+struct Round {
+  int i, b, cnt;                  // number, first batch row, batch rows
+  int k, qt, h;                   // number within the tile, query tile, head
+  __device__ __forceinline__ Round(const AttnInferArgs& a, int round) : i(round) {
+    const int tile = round / a.rounds;
+    k = round - tile * a.rounds;
+    h = tile / a.n_qt;
+    qt = tile - h * a.n_qt;
+    rows(a);
+  }
+  __device__ __forceinline__ void rows(const AttnInferArgs& a) {       // the first `rest` rounds have a row more than the others
+    b = k * a.few + min(k, a.rest);
+    cnt = a.few + (k < a.rest);
+  }
+  __device__ __forceinline__ void next(const AttnInferArgs& a) {
+    ++i;
+    if (++k == a.rounds) {
+      k = 0;
+      if (++qt == a.n_qt) {
+        qt = 0;
+        ++h;
+      }
+    }
+    rows(a);
+  }
+  __device__ __forceinline__ bool fresh() const { return k == 0; }     // first round of a tile
+  __device__ __forceinline__ bool last(const AttnInferArgs& a) const { return k + 1 == a.rounds; }
+};
+
+// Rounds are shared out by their cost: first round at or after position `x` of the work.
+template <typename T>
+__device__ __forceinline__ int round_at(const AttnInferArgs& a, T x) {
+  if (a.n_qt == 1) return (int)((x + a.cost_last - 1) / a.cost_last);
+  const T full = (T)AF_COST * (a.n_qt - 1) * a.rounds, head = full + (T)a.cost_last * a.rounds;
+  const int h = (int)(x / head);
+  const T rem = x - h * head;
+  const int in_head = rem <= full ? (int)((rem + AF_COST - 1) / AF_COST) : (a.n_qt - 1) * a.rounds + (int)((rem - full + a.cost_last - 1) / a.cost_last);
+  return h * a.n_qt * a.rounds + in_head;
+}
+// where the rounds of CTA `i` begin
+__device__ __forceinline__ int cta_begin(const AttnInferArgs& a, int i) {
+  const long long x = a.share * i + min(i, a.extra);
+  return a.share * gridDim.x < 0x70000000LL ? round_at<uint32_t>(a, (uint32_t)x) : round_at<long long>(a, x);
 }
 
 template <int D, bool BIAS>   // head dim: 32 (64-byte rows, 64-byte swizzle) or 16 (32-byte)
@@ -305,10 +390,11 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t b0 = base + AttnInferSmem::BARS;
-  // barrier map (8 bytes each): [group][2 stages] for Q and K / V, [slot] for the bias, [group] for the rest
-  const uint32_t q_full = b0, q_empty = b0 + 64, kv_full = b0 + 128, kv_empty = b0 + 192;
-  const uint32_t bias_full = b0 + 256, bias_empty = b0 + 288, s_full = b0 + 320, p_full = b0 + 352, o_done = b0 + 384;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + AttnInferSmem::BARS + 448);
+  // barrier map (8 bytes each): [group][2] Q stages, [group][AF_KVST] K / V stages, [slot] bias, [group][2] S buffers
+  const uint32_t q_full = b0, q_empty = b0 + 48, kv_full = b0 + 96, kv_empty = b0 + 192, bias_full = b0 + 288, bias_empty = b0 + 320;
+  const uint32_t s_full = b0 + 352, p_full = b0 + 400, o_done = b0 + 448;
+  static_assert(AF_GROUPS == 3 && AF_KVST == 4 && AF_BSLOTS == 4, "barrier map");
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + AttnInferSmem::BARS + 512);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -318,19 +404,20 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
     for (int i = 0; i < 2 * AF_GROUPS; ++i) {
       mbar_init(q_full + 8 * i, 1);
       mbar_init(q_empty + 8 * i, 1);
+      mbar_init(s_full + 8 * i, 2);               // the S product, and the block's key bits
+      mbar_init(p_full + 8 * i, 4);
+      mbar_init(o_done + 8 * i, 1);
+    }
+    for (int i = 0; i < AF_KVST * AF_GROUPS; ++i) {
       mbar_init(kv_full + 8 * i, 1);
       mbar_init(kv_empty + 8 * i, 1);
     }
     for (int i = 0; i < AF_BSLOTS; ++i) {
       mbar_init(bias_full + 8 * i, 1);
-      mbar_init(bias_empty + 8 * i, AF_GROUPS * 4);
-    }
-    for (int i = 0; i < AF_GROUPS; ++i) {
-      mbar_init(s_full + 8 * i, 1);
-      mbar_init(p_full + 8 * i, 4);
-      mbar_init(o_done + 8 * i, 1);
+      mbar_init(bias_empty + 8 * i, AF_GROUPS);
     }
     *abort_flag = 0;
+    for (int i = 0; i < 4; ++i) reinterpret_cast<int*>(sm + AttnInferSmem::TURN)[i] = 0;
     fence_mbar_init();
     prefetch_tmap(&tmQ);
     prefetch_tmap(&tmK);
@@ -342,310 +429,337 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
   }
+  // contiguous range of rounds of this CTA
+  const int r_begin = cta_begin(a, blockIdx.x), r_end = cta_begin(a, blockIdx.x + 1);
+  const Round rd0(a, r_begin);
   pdl_wait();          // the prologue above touched no global memory; everything below may
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // Contiguous range of units for this CTA; unit = (h * n_qt + qt) * B + b.  A round takes up to AF_GROUPS consecutive
-  // batch rows of one (head, query tile); every role walks the same rounds.
-  const int per = (a.units + gridDim.x - 1) / gridDim.x;
-  const int u_begin = blockIdx.x * per;
-  int u_end = u_begin + per;
-  if (u_end > a.units) u_end = a.units;
-  auto round_count = [&](int u) -> int {        // batch rows in the round that starts at unit u (0 past the end)
-    if (u >= u_end) return 0;
-    int c = a.B - u % a.B;
-    if (c > u_end - u) c = u_end - u;
-    return c < AF_GROUPS ? c : AF_GROUPS;
+  // A wait of this CTA's pipeline.  The first one that runs out reports and sets the flag, at which all others end: the kernel
+  // then runs to its end on whatever the buffers hold, and the caller sees the status.
+  auto wait = [&](uint32_t bar, uint32_t parity, int code, int detail) -> bool {
+    if (mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = globaltimer_ns();
+    for (;;) {
+#pragma unroll 1
+      for (int i = 0; i < 256; ++i)
+        if (mbar_try_wait(bar, parity)) return true;
+      if (*abort_flag) return false;
+      if (globaltimer_ns() - t0 > FFB_LOCAL_WAIT_NS) {
+        report(code, detail);
+        *abort_flag = 1;
+        return false;
+      }
+    }
   };
 
+
+  // The producer and the issuers run as whole warps (see umma_bf16_by).
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer ----------------
-      uint32_t qi[AF_GROUPS], jt[AF_GROUPS];     // items and key blocks loaded per group
+    // ---------------- TMA producer ----------------
+    const uint32_t lead = elect_one();
+    uint32_t qi[AF_GROUPS], jt[AF_GROUPS];     // items and key blocks loaded per group
 #pragma unroll
-      for (int g = 0; g < AF_GROUPS; ++g) qi[g] = jt[g] = 0;
-      uint32_t fill = 0;                         // bias: streamed tiles so far, or resident (head, tile) sets so far
-      int prev = -1;
-      bool ok = true;
-      for (int u = u_begin; u < u_end && ok;) {
-        const int cnt = round_count(u);
-        const int grp = u / a.B, bb = u % a.B;
-        const int qt = grp % a.n_qt, h = grp / a.n_qt;
-        const bool load_bias = BIAS && (!a.bias_resident || grp != prev);
-        const uint32_t set = fill;               // resident: index of the set loaded in this round
-        if (load_bias && a.bias_resident) ++fill;
-        prev = grp;
-        for (int j = 0; j < a.n_kb && ok; ++j) {
-          if (load_bias) {
-            const uint32_t slot = a.bias_resident ? (uint32_t)j : fill % AF_BSLOTS;
-            const uint32_t nth = a.bias_resident ? set : fill / AF_BSLOTS;       // fill index of this slot
-            if (!mbar_wait(bias_empty + 8 * slot, (nth & 1) ^ 1)) { report(ST_TIMEOUT_EPI, 11); ok = false; break; }
-            mbar_expect_tx(bias_full + 8 * slot, 16384);
-            tma_load_3d(base + AttnInferSmem::BIAS + slot * 16384, &tmBias, bias_full + 8 * slot, j * AF_BK, qt * AF_BQ, h);
-            if (!a.bias_resident) ++fill;
-          }
-#pragma unroll
-          for (int g = 0; g < AF_GROUPS; ++g) {
-            if (g >= cnt || !ok) continue;
-            if (j == 0) {
-              const uint32_t qs = g * 2 + (qi[g] & 1);
-              if (!mbar_wait(q_empty + 8 * qs, ((qi[g] >> 1) & 1) ^ 1)) { report(ST_TIMEOUT_MMA, 10); ok = false; continue; }
-              mbar_expect_tx(q_full + 8 * qs, Q_BYTES);
-              tma_load_3d(base + AttnInferSmem::Q + qs * 8192, &tmQ, q_full + 8 * qs, h * D, qt * AF_BQ, bb + g);
-              ++qi[g];
-            }
-            const uint32_t ks = g * 2 + (jt[g] & 1);
-            if (!mbar_wait(kv_empty + 8 * ks, ((jt[g] >> 1) & 1) ^ 1)) { report(ST_TIMEOUT_MMA, 12); ok = false; continue; }
-            mbar_expect_tx(kv_full + 8 * ks, 2 * KV_BYTES);
-            tma_load_3d(base + AttnInferSmem::KV + ks * 8192, &tmK, kv_full + 8 * ks, h * D, j * AF_BK, bb + g);
-            tma_load_3d(base + AttnInferSmem::KV + ks * 8192 + 4096, &tmV, kv_full + 8 * ks, h * D, j * AF_BK, bb + g);
-            ++jt[g];
-          }
-        }
-        u += cnt;
-      }
-      if (!ok) *abort_flag = 1;
-    }
-    __syncwarp();
-  } else if (warp <= AF_ISSUERS) {
-    if (lane == 0) {
-      // ---------------- MMA issuers: GPI groups each ----------------
-      constexpr uint32_t idesc_s = make_idesc_bf16(128, AF_BK, 0, 0);     // Q (K-major) x K (K-major)
-      constexpr uint32_t idesc_o = make_idesc_bf16(128, D, 0, 1);         // P (tensor memory) x V (MN-major)
-      constexpr int GPI = AF_GROUPS / AF_ISSUERS;
-      const int gb = (warp - 1) * GPI;
-      // descriptors of stage 0 of group gb; the address field counts 16 bytes, so stages and groups are additions
-      const uint64_t dq = make_desc(base + AttnInferSmem::Q + gb * 16384, 16, GROUP, LAYOUT), dk = make_desc(base + AttnInferSmem::KV + gb * 16384, 16, GROUP, LAYOUT),
-                     dv = make_desc(base + AttnInferSmem::KV + gb * 16384 + 4096, 16, GROUP, LAYOUT);
-      uint32_t si[GPI], qi[GPI], pi[GPI];                                 // per group: S products, items, PV products issued
-      bool ahead[GPI];                                                    // S of the group's next block already issued
-#pragma unroll
-      for (int e = 0; e < GPI; ++e) {
-        si[e] = qi[e] = pi[e] = 0;
-        ahead[e] = false;
-      }
-      bool ok = true;
-      // S product of a group's next block; `first` / `last`: position of that block in its item
-      auto issue_s = [&](int e, uint32_t& sg, uint32_t& qg, bool first, bool last) -> bool {
-        const uint32_t qs = (gb + e) * 2 + (qg & 1), ks = (gb + e) * 2 + (sg & 1);
-        if (first && !mbar_wait(q_full + 8 * qs, (qg >> 1) & 1)) { report(ST_TIMEOUT_TMA, 22); return false; }
-        if (!mbar_wait(kv_full + 8 * ks, (sg >> 1) & 1)) { report(ST_TIMEOUT_TMA, 20); return false; }
-        tc_fence_after();
-        const uint64_t q = dq + (e * 2 + (qg & 1)) * (8192 >> 4), k = dk + (e * 2 + (sg & 1)) * (8192 >> 4);
-#pragma unroll
-        for (int i = 0; i < D / 16; ++i) umma_bf16(tmem + (gb + e) * 128, q + i * (32 >> 4), k + i * (32 >> 4), idesc_s, i > 0 ? 1u : 0u);
-        umma_commit(s_full + 8 * (gb + e));
-        ++sg;
-        if (last) {
-          umma_commit(q_empty + 8 * qs);        // all S products of this item issued: the Q slot drains with them
-          ++qg;
-        }
-        return true;
-      };
-      for (int u = u_begin; u < u_end && ok;) {
-        const int cnt = round_count(u);
-        const int cnt_next = round_count(u + cnt);
-#pragma unroll
-        for (int e = 0; e < GPI; ++e) {
-          if (gb + e < cnt && !ahead[e] && ok) ok = issue_s(e, si[e], qi[e], true, a.n_kb == 1);
-          ahead[e] = false;
-        }
-        for (int j = 0; j < a.n_kb && ok; ++j) {
-          const bool last = j + 1 == a.n_kb;
-#pragma unroll
-          for (int e = 0; e < GPI; ++e) {
-            if (gb + e >= cnt || !ok) continue;
-            const int g = gb + e;
-            // the group has read S of block j and written P
-            if (!mbar_wait(p_full + 8 * g, pi[e] & 1)) { if (*abort_flag == 0) report(ST_TIMEOUT_EPI, 23); ok = false; continue; }
-            tc_fence_after();
-            const uint32_t st = pi[e] & 1;
-            if (!last) {
-              ok = issue_s(e, si[e], qi[e], false, j + 2 == a.n_kb);
-            } else if (g < cnt_next) {
-              ok = issue_s(e, si[e], qi[e], true, a.n_kb == 1);
-              ahead[e] = true;
-            }
-            if (!ok) continue;
-            const uint64_t v = dv + (e * 2 + st) * (8192 >> 4);
-#pragma unroll
-            for (int k = 0; k < AF_BK / 16; ++k)
-              umma_bf16_ts(tmem + g * 128 + AF_TM_O, tmem + g * 128 + AF_TM_P + k * 8, v + ((k * 2 * GROUP) >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-            umma_commit(o_done + 8 * g);
-            umma_commit(kv_empty + 8 * (g * 2 + st));
-            ++pi[e];
-          }
-        }
-        u += cnt;
-      }
-      if (!ok) *abort_flag = 1;
-    }
-    __syncwarp();
-  } else if (warp >= 4) {
-    // ---------------- softmax / output (warps 4..19): group = batch row of the round, thread = query row ----------------
-    const int quad = warp & 3;                      // TMEM lane quadrant this warp may read
-    const int g = (warp - 4) >> 2;
-    const int r = quad * 32 + lane;                 // row within the query tile
-    const uint32_t tm = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)g * 128;
-    float* pen = reinterpret_cast<float*>(sm + AttnInferSmem::KP) + (warp - 4) * 64;
-    uint32_t jt = 0;                                // blocks of this group so far
-    uint32_t fill = 0;                              // bias tiles (streamed) or sets (resident) this warp has waited for
-    int prev = -1;
+    for (int g = 0; g < AF_GROUPS; ++g) qi[g] = jt[g] = 0;
+    uint32_t fill = 0;                         // bias: streamed tiles so far, or resident (head, tile) sets so far
     bool ok = true;
-    for (int u = u_begin; u < u_end && ok;) {
-      const int cnt = round_count(u);
-      const int grp = u / a.B, b = u % a.B + g;
-      const int qt = grp % a.n_qt, h = grp / a.n_qt;
-      const bool active = g < cnt;
-      u += cnt;
-      const bool new_set = BIAS && grp != prev;
-      if (new_set && a.bias_resident) ++fill;
-      prev = grp;
-      // resident tiles are released in the last round that reads them, streamed ones at once
-      const bool release = BIAS && (!a.bias_resident || u >= u_end || u / a.B != grp);
-      RowState row = {0.f, 0.f, false};
-      const bf16* mrow = (a.mask && active) ? a.mask + (long long)b * a.mask_bstride : nullptr;
-      for (int j = 0; j < a.n_kb; ++j) {
-        uint32_t slot = 0, bpar = 0;
-        if (BIAS) {
-          slot = a.bias_resident ? (uint32_t)j : fill % AF_BSLOTS;
-          bpar = a.bias_resident ? (fill - 1) & 1 : (fill / AF_BSLOTS) & 1;
+    for (Round rd = rd0; rd.i < r_end && ok; rd.next(a)) {
+      const int cnt = rd.cnt, bb = rd.b, qt = rd.qt, h = rd.h;
+      const bool load_bias = BIAS && (!a.bias_resident || rd.i == r_begin || rd.fresh());
+      const uint32_t set = fill;               // resident: index of the set loaded in this round
+      if (load_bias && a.bias_resident) ++fill;
+      for (int j = 0; j < a.n_kb && ok; ++j) {
+#pragma unroll
+        for (int g = 0; g < AF_GROUPS; ++g) {
+          if (g >= cnt || !ok) continue;
+          if (j == 0) {
+            const uint32_t qs = g * 2 + (qi[g] & 1);
+            if (!(ok = wait(q_empty + 8 * qs, ((qi[g] >> 1) & 1) ^ 1, ST_TIMEOUT_MMA, 10))) continue;
+            mbar_expect_tx_by(lead, q_full + 8 * qs, Q_BYTES);
+            tma_load_3d_by(lead, base + AttnInferSmem::Q + qs * 8192, &tmQ, q_full + 8 * qs, h * D, qt * AF_BQ - 32 * tile_rows(a.n_q, qt, bb + g).first, bb + g);
+            ++qi[g];
+          }
+          const uint32_t ks = g * AF_KVST + (jt[g] % AF_KVST);
+          if (!(ok = wait(kv_empty + 8 * ks, ((jt[g] / AF_KVST) & 1) ^ 1, ST_TIMEOUT_MMA, 12))) continue;
+          mbar_expect_tx_by(lead, kv_full + 8 * ks, 2 * KV_BYTES);
+          tma_load_3d_by(lead, base + AttnInferSmem::KV + ks * 8192, &tmK, kv_full + 8 * ks, h * D, j * AF_BK, bb + g);
+          tma_load_3d_by(lead, base + AttnInferSmem::KV + ks * 8192 + 4096, &tmV, kv_full + 8 * ks, h * D, j * AF_BK, bb + g);
+          ++jt[g];
+        }
+        if (load_bias && ok) {
+          const uint32_t slot = a.bias_resident ? (uint32_t)j : fill % AF_BSLOTS;
+          const uint32_t nth = a.bias_resident ? set : fill / AF_BSLOTS;       // fill index of this slot
+          if (!(ok = wait(bias_empty + 8 * slot, (nth & 1) ^ 1, ST_TIMEOUT_EPI, 11))) break;
+          mbar_expect_tx_by(lead, bias_full + 8 * slot, 16384);
+          tma_load_3d_by(lead, base + AttnInferSmem::BIAS + slot * 16384, &tmBias, bias_full + 8 * slot, j * AF_BK, qt * AF_BQ, h);
           if (!a.bias_resident) ++fill;
         }
-        if (!active) {                              // keeps the tile accounting: one release per warp and fill
-          if (release) {
-            bool w = mbar_wait(bias_full + 8 * slot, bpar);
-            ok = __all_sync(0xffffffffu, w);
-            if (!ok) break;
-            if (lane == 0) mbar_arrive(bias_empty + 8 * slot);
-          }
-          continue;
+      }
+    }
+    if (!ok) {                                 // copies that nobody will wait for any more: they land long before this ends
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 1000000ull) {
+      }
+    }
+  } else if (warp <= AF_GROUPS) {
+    // ---------------- MMA issuer of one group ----------------
+    const uint32_t lead = elect_one();
+    constexpr uint32_t idesc_s = make_idesc_bf16(128, AF_BK, 0, 0);     // Q (K-major) x K (K-major)
+    constexpr uint32_t idesc_o = make_idesc_bf16(128, D, 0, 1);         // P (tensor memory) x V (MN-major)
+    const int g = warp - 1;
+    const uint32_t tg = tmem + (uint32_t)g * AF_TM_GROUP;
+    // descriptors of stage 0; the address field counts 16 bytes, so stages are additions
+    const uint64_t dq = make_desc(base + AttnInferSmem::Q + g * 16384, 16, GROUP, LAYOUT),
+                   dk = make_desc(base + AttnInferSmem::KV + g * AF_KVST * 8192, 16, GROUP, LAYOUT),
+                   dv = make_desc(base + AttnInferSmem::KV + g * AF_KVST * 8192 + 4096, 16, GROUP, LAYOUT);
+    uint32_t si = 0, qi = 0, pi = 0;                                    // S products, items, PV products issued
+    Round rs = rd0;                                               // block of the next S product
+    int sj = 0;
+    auto next_s = [&]() {                                               // rounds without a row for this group have none
+      while (rs.i < r_end && g >= rs.cnt) rs.next(a);
+    };
+    next_s();
+    // Two S products ahead, but not past the round after the one whose P V products are being issued: in a round without a row
+    // for this group there are still bias tiles to release.
+    int reach = r_begin;
+    uint32_t slot = 0, bpar = a.bias_resident ? 1u : 0u;                // bias tile of the block, phase of its barrier
+    // This warp has time to spare: it also works out which keys of a block count, from entries loaded a block ahead.
+    Keys* key_ring = reinterpret_cast<Keys*>(sm + AttnInferSmem::KEYS) + g * 2;
+    const bf16* mrow = nullptr;
+    KeyMask km = {0, 0};
+    auto look_ahead = [&]() {
+      if (rs.i >= r_end) return;
+      if (sj == 0) mrow = a.mask ? a.mask + (long long)(rs.b + g) * a.mask_bstride : nullptr;
+      km = load_keys(mrow, sj * AF_BK, a.n_k, lane);
+    };
+    look_ahead();
+    // S product of the next block, into the buffer whose last P V product has been issued: products execute in order
+    auto issue_s = [&]() {
+      const uint32_t qs = g * 2 + (qi & 1), ks = g * AF_KVST + si % AF_KVST;
+      const Keys keys = key_bits(km);
+      if (sj == 0) wait(q_full + 8 * qs, (qi >> 1) & 1, ST_TIMEOUT_TMA, 22);
+      wait(kv_full + 8 * ks, (si / AF_KVST) & 1, ST_TIMEOUT_TMA, 20);
+      tc_fence_after();
+      const uint64_t q = dq + (qi & 1) * (8192 >> 4), k = dk + (si % AF_KVST) * (8192 >> 4);
+#pragma unroll
+      for (int i = 0; i < D / 16; ++i) umma_bf16_by(lead, tg + (si & 1) * AF_BK, q + i * (32 >> 4), k + i * (32 >> 4), idesc_s, i > 0 ? 1u : 0u);
+      umma_commit_by(lead, s_full + 8 * (g * 2 + (si & 1)));
+      if (lead) {
+        key_ring[si & 1] = keys;
+        mbar_arrive(s_full + 8 * (g * 2 + (si & 1)));
+      }
+      ++si;
+      if (++sj == a.n_kb) {
+        umma_commit_by(lead, q_empty + 8 * qs);       // all S products of this item issued: the Q slot drains with them
+        ++qi;
+        sj = 0;
+        rs.next(a);
+        next_s();
+      }
+      look_ahead();
+    };
+    for (Round rd = rd0; rd.i < r_end; rd.next(a)) {
+      if (BIAS && a.bias_resident) {
+        slot = 0;
+        bpar ^= rd.i == r_begin || rd.fresh();
+      }
+      // resident tiles are released in the last round that reads them, streamed ones at once
+      const bool release = BIAS && (!a.bias_resident || rd.i + 1 == r_end || rd.last(a));
+      const bool active = g < rd.cnt;
+      reach = rd.i + 1;
+      while (active && si < pi + 2 && rs.i < r_end && rs.i <= reach) issue_s();
+      for (int j = 0; j < a.n_kb; ++j) {
+        if (active) {
+          const uint32_t buf = pi & 1, st = pi % AF_KVST;
+          // the group has read S of this block and written P
+          wait(p_full + 8 * (g * 2 + buf), (pi >> 1) & 1, ST_TIMEOUT_EPI, 23);
+          tc_fence_after();
+          const uint64_t v = dv + st * (8192 >> 4);
+#pragma unroll
+          for (int k = 0; k < AF_BK / 16; ++k)
+            umma_bf16_ts_by(lead, tg + AF_TM_O, tg + buf * AF_BK + k * 8, v + ((k * 2 * GROUP) >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+          umma_commit_by(lead, o_done + 8 * (g * 2 + buf));
+          umma_commit_by(lead, kv_empty + 8 * (g * AF_KVST + st));
+          ++pi;
+        } else if (release) {
+          wait(bias_full + 8 * slot, bpar, ST_TIMEOUT_TMA, 30);
         }
-        // key bits first: their global loads overlap the wait for S
-        uint32_t keep_lo, keep_hi, valid_lo, valid_hi;
-        key_bits(mrow, j * AF_BK, a.n_k, lane, keep_lo, keep_hi, valid_lo, valid_hi);
-        const bool plain = (keep_lo & keep_hi) == 0xffffffffu;         // every key of this block in range and unmasked
-        const bool none = (keep_lo | keep_hi) == 0u;                   // no key of this block counts
-        if (!plain && !none) write_penalties(pen, lane, keep_lo, keep_hi);
-        bool w = true;
-        if (BIAS && !mbar_wait(bias_full + 8 * slot, bpar)) { if (lane == 0 && *abort_flag == 0) report(ST_TIMEOUT_TMA, 30); w = false; }
-        if (w && !mbar_wait(s_full + 8 * g, jt & 1)) { if (lane == 0 && *abort_flag == 0) report(ST_TIMEOUT_MMA, 31); w = false; }
-        ok = __all_sync(0xffffffffu, w);
-        if (!ok) break;
+        if (release) {
+          if (lead) mbar_arrive(bias_empty + 8 * slot);
+          if (++slot == AF_BSLOTS && !a.bias_resident) {
+            slot = 0;
+            bpar ^= 1;
+          }
+        }
+        if (active && rs.i < r_end && rs.i <= reach) issue_s();
+      }
+    }
+  } else {
+    // ---------------- softmax / output (warps 4..15): group = batch row of the round, thread = query row ----------------
+    const int quad = warp & 3;                      // TMEM lane quadrant this warp may read
+    const int g = (warp - 4) >> 2;
+    const uint32_t tg = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)g * AF_TM_GROUP;
+    float* pen = reinterpret_cast<float*>(sm + AttnInferSmem::KP) + (warp - 4) * 64;
+    uint32_t jt = 0;                                // blocks of this group so far
+    // Warps that share a scheduler (one of each group) begin a block one after the other: a warp takes the turn for the first
+    // quarter of its logits.  Left alone they fall into step - whoever is ahead finds fewer others and is slowed down when they
+    // come - and then all are in their exponentials at once and all between blocks at once (n 1024: 2700 cycles a block, of which
+    // 450 between blocks; n 1536, B 384: 1440 us, 1380 with turns).  Only a hint: the tries are few, and it is harmless to go on
+    // without the turn.
+    int* turn = reinterpret_cast<int*>(sm + AttnInferSmem::TURN) + quad;
+    auto take_turn = [&]() {
+      if (lane == 0)
+        for (int i = 0; i < 32 && atomicExch(turn, 1) != 0; ++i) {
+        }
+      __syncwarp();
+    };
+    auto pass_turn = [&]() {
+      if (lane == 0) *reinterpret_cast<volatile int*>(turn) = 0;
+    };
+    // P V product of block `t` of this group: O holds it
+    auto wait_o = [&](uint32_t t, int detail) {
+      wait(o_done + 8 * (g * 2 + (t & 1)), (t >> 1) & 1, ST_TIMEOUT_MMA, detail);
+      __syncwarp();
+      tc_fence_after();
+    };
+    const Keys* key_ring = reinterpret_cast<const Keys*>(sm + AttnInferSmem::KEYS) + g * 2;
+    uint32_t slot = 0, bpar = a.bias_resident ? 1u : 0u;      // bias tile of the block, phase of its barrier
+    for (Round rd = rd0; rd.i < r_end; rd.next(a)) {
+      const bool first = rd.i == r_begin || rd.fresh();
+      if (BIAS && a.bias_resident) {
+        slot = 0;
+        bpar ^= first;
+      }
+      if (g >= rd.cnt) {
+        if (BIAS && !a.bias_resident) {             // tiles of a round without a row for this group
+          slot += a.n_kb;
+          bpar ^= (slot / AF_BSLOTS) & 1;
+          slot %= AF_BSLOTS;
+        }
+        continue;
+      }
+      const int qt = rd.qt, h = rd.h, b = rd.b + g;
+      const bool look = BIAS && (!a.bias_resident || first);                        // tiles that this warp has not waited for yet
+      const TileRows rows = tile_rows(a.n_q, qt, b);
+      const bool mine = quad >= rows.first && quad < rows.first + rows.warps;       // this warp has query rows
+      const int r = (quad - rows.first) * 32 + lane;                                // row within the query tile
+      RowState row = {0.f, 0.f, false};
+      for (int j = 0; j < a.n_kb; ++j) {
+        // S first: the phase of the bias tile's barrier means something only once S is there, until then tiles of a round without a
+        // row for this group may still be on their way.  Not side by side either: the first may be suspended and end well while
+        // the second has long been answered.
+        wait(s_full + 8 * (g * 2 + (jt & 1)), (jt >> 1) & 1, ST_TIMEOUT_MMA, 31);
+        if (look) wait(bias_full + 8 * slot, bpar, ST_TIMEOUT_TMA, 32);
+        __syncwarp();
         tc_fence_after();
         const uint8_t* brow = BIAS ? sm + AttnInferSmem::BIAS + slot * 16384 + r * 128 : nullptr;
-        // P of the previous block has been read and O holds its product
-        if (j > 0) {
-          w = mbar_wait(o_done + 8 * g, (jt - 1) & 1);
-          if (!w && lane == 0 && *abort_flag == 0) report(ST_TIMEOUT_MMA, 32);
-          ok = __all_sync(0xffffffffu, w);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        uint64_t sum = pk2(0.f, 0.f);
-        if (none) {
-          // masked keys next to a real one have weight 0; where there has been no other key they all have the same logit
-          const bool alone = row.l == 0.f || (row.far && row.M == MASKED_LOGIT);
-          if (__any_sync(0xffffffffu, row.far && !alone)) {
-            row = far_block<BIAS>(row, alone || row.far, tm, j > 0, brow, r, 0u, 0u, a.n_k - j * AF_BK, a.scale, a.scale_log2e);
-          } else {
-            if (alone) {
-              row.M = MASKED_LOGIT;
-              row.far = 1;
-              row.l += (float)(__popc(valid_lo) + __popc(valid_hi));
+        const uint32_t tm_s = tg + (jt & 1) * AF_BK;
+        if (mine) {
+          const Keys kb = key_ring[jt & 1];
+          const bool plain = (kb.lo & kb.hi) == 0xffffffffu;           // every key of this block in range and unmasked
+          if (kb.lo | kb.hi) {
+            float2 sum = {0.f, 0.f};
+            uint32_t p[32];                         // stored once the sum is known to be in range: P takes the place of S
+            bool store = true;
+            if (plain) {
+              take_turn();
+              softmax_block<true, BIAS>(tm_s, brow, r, pen, a.scale_log2e, -row.M, kb, p, sum, pass_turn);
+            } else {
+              write_penalties(pen, lane, kb.lo, kb.hi);
+              softmax_block<false, BIAS>(tm_s, brow, r, pen, a.scale_log2e, -row.M, kb, p, sum, []() {});
             }
+            const float ln = row.l + (sum.x + sum.y);
+            const bool bad = row.far || !(ln > ROW_SUM_LO && ln < ROW_SUM_HI);
+            if (__any_sync(0xffffffffu, bad)) {
+              // some row's sum has left the safe range (first block of a row with large logits, only masked keys before this
+              // block, or a much larger logit in it): move that row's reference point and redo the block
+              if (plain) write_penalties(pen, lane, 0xffffffffu, 0xffffffffu);
+              float mx = -INFINITY, alpha = 1.f;
+              if (j > 0) wait_o(jt - 1, 34);
+#pragma unroll 1
+              for (int c = 0; c < 4; ++c) {
+                float s[16];
+                uint64_t t[8];
+                tmem_ld_32x16(tm_s + c * 16, s);
+                tmem_ld_wait_for(s);
+                logits16<false, BIAS>(t, s, brow, r, c * 16, pen, a.scale_log2e, 0.f);
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              uint32_t p[16];
+                for (int i = 0; i < 8; ++i) {
+                  float x, y;
+                  up2(t[i], x, y);
+                  mx = fmaxf(mx, fmaxf(x, y));
+                }
+              }
+              const float m2 = (row.l > 0.f && !row.far) ? fmaxf(mx, row.M + log2f(row.l)) : mx;
+              // a row that leaves the domain of the ordinary path, or that has not re-entered it from above
+              const bool out = bad && (!(fabsf(m2) < FAR_LOGIT) || (row.far && row.M > 0.f));
+              if (__any_sync(0xffffffffu, out)) {
+                row = far_block<BIAS>(row, bad, tm_s, tg + AF_TM_O, j > 0, brow, r, kb, a.n_k - j * AF_BK, a.scale, a.scale_log2e);
+                store = false;
+              } else {
+                if (bad) {
+                  if (row.l > 0.f) alpha = ex2f((row.far ? row.M * LOG2E : row.M) - m2);
+                  row.M = m2;
+                  row.far = 0;
+                }
+                if (j > 0) {
+                  float o[32];                      // D = 16: the upper columns are nobody's
+                  tmem_ld_32x32(tg + AF_TM_O, o);
+                  tmem_ld_wait_for(o);
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const uint32_t bits = ((c ? valid_hi : valid_lo) >> (2 * i)) & 3u;
+                  for (int c = 0; c < 32; ++c) o[c] *= alpha;
+                  tmem_st_32x32(tg + AF_TM_O, o);
+                }
+                sum = {0.f, 0.f};
+                softmax_block<false, BIAS>(tm_s, brow, r, pen, a.scale_log2e, -row.M, kb, p, sum, []() {});
+                row.l = row.l * alpha + (sum.x + sum.y);
+              }
+            } else {
+              row.l = ln;
+            }
+            if (store) tmem_st_32x32(tm_s, reinterpret_cast<const float*>(p));
+          } else {
+            // masked keys next to a real one have weight 0; where there has been no other key they all have the same logit
+            const bool alone = row.l == 0.f || (row.far && row.M == MASKED_LOGIT);
+            if (__any_sync(0xffffffffu, row.far && !alone)) {
+              if (j > 0) wait_o(jt - 1, 32);
+              row = far_block<BIAS>(row, alone || row.far, tm_s, tg + AF_TM_O, j > 0, brow, r, kb, a.n_k - j * AF_BK, a.scale, a.scale_log2e);
+            } else {
+              const Keys valid = key_bits(load_keys(nullptr, j * AF_BK, a.n_k, lane));
+              if (alone) {
+                row.M = MASKED_LOGIT;
+                row.far = 1;
+                row.l += (float)(__popc(valid.lo) + __popc(valid.hi));
+              }
+              uint32_t p[32];
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                const uint32_t bits = ((i < 16 ? valid.lo : valid.hi) >> (2 * (i & 15))) & 3u;
                 p[i] = alone ? (bits & 1u) * 0x3f80u + (bits >> 1) * 0x3f800000u : 0u;
               }
-              tmem_st_32x16(tm + AF_TM_P + c * 16, p);
+              tmem_st_32x32(tm_s, reinterpret_cast<const float*>(p));
             }
           }
-        } else {
-          if (plain) softmax_block<true, BIAS>(tm, tm + AF_TM_P, brow, r, pen, a.scale_log2e, -row.M, sum);
-          else softmax_block<false, BIAS>(tm, tm + AF_TM_P, brow, r, pen, a.scale_log2e, -row.M, sum);
-          float sx, sy;
-          up2(sum, sx, sy);
-          float ln = row.l + (sx + sy);
-          const bool bad = row.far || !(ln > ROW_SUM_LO && ln < ROW_SUM_HI);
-          if (__any_sync(0xffffffffu, bad)) {
-            // some row's sum has left the safe range (first block of a row with large logits, only masked keys before this
-            // block, or a much larger logit in it): move that row's reference point and redo the block
-            if (plain) write_penalties(pen, lane, 0xffffffffu, 0xffffffffu);
-            float mx = -INFINITY, alpha = 1.f;
-            tmem_st_wait();                         // the first attempt's P is about to be replaced
-#pragma unroll 1
-            for (int c = 0; c < 2; ++c) {
-              float s[32];
-              uint64_t t[16];
-              tmem_ld_32x32(tm + c * 32, s);
-              tmem_ld_wait();
-              logits32<false, BIAS>(t, s, brow, r, c * 32, pen, a.scale_log2e, 0.f);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                float x, y;
-                up2(t[i], x, y);
-                mx = fmaxf(mx, fmaxf(x, y));
-              }
-            }
-            const float m2 = (row.l > 0.f && !row.far) ? fmaxf(mx, row.M + log2f(row.l)) : mx;
-            // a row that leaves the domain of the ordinary path, or that has not re-entered it from above
-            const bool out = bad && (!(fabsf(m2) < FAR_LOGIT) || (row.far && row.M > 0.f));
-            if (__any_sync(0xffffffffu, out)) {
-              // the keys from the table: bits kept until here would be spilled
-              row = far_block<BIAS>(row, bad, tm, j > 0, brow, r, __ballot_sync(0xffffffffu, pen[lane] == 0.f),
-                                    __ballot_sync(0xffffffffu, pen[lane + 32] == 0.f), a.n_k - j * AF_BK, a.scale, a.scale_log2e);
-            } else {
-              if (bad) {
-                if (row.l > 0.f) alpha = ex2f((row.far ? row.M * LOG2E : row.M) - m2);
-                row.M = m2;
-                row.far = 0;
-              }
-              if (j > 0) {
-                float o[32];                        // D = 16: the upper columns are nobody's
-                tmem_ld_32x32(tm + AF_TM_O, o);
-                tmem_ld_wait();
-#pragma unroll
-                for (int c = 0; c < 32; ++c) o[c] *= alpha;
-                tmem_st_32x32(tm + AF_TM_O, o);
-              }
-              sum = pk2(0.f, 0.f);
-              softmax_block<false, BIAS>(tm, tm + AF_TM_P, brow, r, pen, a.scale_log2e, -row.M, sum);
-              up2(sum, sx, sy);
-              row.l = row.l * alpha + (sx + sy);
-            }
-          } else {
-            row.l = ln;
-          }
-        }
+        }                                           // other warps: nothing of their lanes is ever read
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(p_full + 8 * g);              // S may be overwritten, P is complete
-          if (release) mbar_arrive(bias_empty + 8 * slot);
+        if (lane == 0) mbar_arrive(p_full + 8 * (g * 2 + (jt & 1)));        // P is complete, S and the bias have been read
+        if (BIAS && ++slot == AF_BSLOTS && !a.bias_resident) {
+          slot = 0;
+          bpar ^= 1;
         }
         ++jt;
       }
-      if (!ok || !active) continue;
       // ---- the item's output row ----
-      {
-        bool w = mbar_wait(o_done + 8 * g, (jt - 1) & 1);
-        if (!w && lane == 0 && *abort_flag == 0) report(ST_TIMEOUT_MMA, 33);
-        ok = __all_sync(0xffffffffu, w);
-        if (!ok) break;
-      }
-      tc_fence_after();
-      float o[32];
-      tmem_ld_32x32(tm + AF_TM_O, o);
-      tmem_ld_wait();
+      if (!mine) continue;
+      wait_o(jt - 1, 33);
+      float o[32];                                  // D = 16: the upper columns are nobody's
+      tmem_ld_32x32(tg + AF_TM_O, o);
+      tmem_ld_wait_for(o);
       const int qrow = qt * AF_BQ + r;
       if (qrow < a.n_q) {
         const float inv = 1.f / row.l;
@@ -659,7 +773,6 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
           *reinterpret_cast<uint4*>(dst + c) = pk;
         }
       }
-      tc_fence_before();
     }
   }
   tc_fence_before();
@@ -693,7 +806,29 @@ int ffb_attention_infer(const void* q, const void* k, const void* v, long long q
   a.n_kb = (n_k + AF_BK - 1) / AF_BK;
   const long long units = (long long)H * a.n_qt * B;
   if (units <= 0 || units > 0x7fffffffLL || a.n_kb <= 0) return -6;
-  a.units = (int)units;
+  static int sm_count = 0;
+  if (!sm_count) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0) sm_count = 148;
+  }
+  // Batch rows per round: three at a time give the most per SM (blocks of 64 keys with one, two, three softmax warps on a scheduler
+  // take 1020, 1500, 2000 cycles), but a grid of few rounds is done sooner with less in each.
+  long long best = 0;
+  for (int c = AF_GROUPS; c > 0; --c) {
+    const long long per_tile = (B + c - 1) / c, time = ((long long)H * a.n_qt * per_tile + sm_count - 1) / sm_count * (c + 1);
+    if (c == AF_GROUPS || time < best) {
+      best = time;
+      a.rounds = (int)per_tile;
+    }
+  }
+  a.few = B / a.rounds;
+  a.rest = B - a.few * a.rounds;
+  // Last query tile with rows for 1 .. 4 warps of a group (n_k 512 with bias, B 3552, H 1: 69, 78, 100, 105 us; n_k 192: 31, 34, 46, 49).
+  static const int cost[4] = {10, 12, 15, AF_COST};
+  const bool one_each = (long long)H * a.n_qt * a.rounds <= sm_count;
+  a.cost_last = one_each ? AF_COST : cost[(n_q - (a.n_qt - 1) * AF_BQ + 31) / 32 - 1];
+  const long long work = (long long)H * a.rounds * (AF_COST * (a.n_qt - 1) + a.cost_last);
   a.bias_resident = (bias && a.n_kb <= AF_BSLOTS) ? 1 : 0;
   a.scale = scale;
   a.scale_log2e = scale * LOG2E;
@@ -716,13 +851,10 @@ int ffb_attention_infer(const void* q, const void* k, const void* v, long long q
                       : (bias ? attn_infer_kernel<16, true> : attn_infer_kernel<16, false>);
   static SmemLimit limit[4];
   if (!limit[(D == 32 ? 0 : 2) + (bias ? 1 : 0)].raise(kern, AttnInferSmem::TOTAL)) return -14;
-  static int sm_count = 0;
-  if (!sm_count) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0) sm_count = 148;
-  }
-  const int grid = units < sm_count ? (int)units : sm_count;
+  const long long rounds = (long long)H * a.n_qt * a.rounds;
+  const int grid = rounds < sm_count ? (int)rounds : sm_count;
+  a.share = work / grid;
+  a.extra = (int)(work % grid);
   launch_k(kern, grid, AF_THREADS, AttnInferSmem::TOTAL,
            reinterpret_cast<cudaStream_t>(stream), tq, tk, tv, tb, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -15;

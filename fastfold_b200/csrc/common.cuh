@@ -187,6 +187,21 @@ __device__ __forceinline__ void umma_bf16_ts_by(uint32_t lead, uint32_t d_tmem, 
       ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
+__device__ __forceinline__ void mbar_expect_tx_by(uint32_t lead, uint32_t bar, uint32_t bytes) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_by(uint32_t lead, uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(lead)
+      : "memory");
+}
 __device__ __forceinline__ void umma_commit_by(uint32_t lead, uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"

@@ -63,6 +63,47 @@ def test_forward_rows_that_leave_the_exponent_range(B, n, H, use_bias, device_st
     assert (out.float() - ref).abs().max().item() < 3.8e-2
 
 
+def _infer(x, bias, mask, n_q):
+    """The kernel without gradients on ``x [B, n, 3, H, d]``, the first ``n_q`` rows as queries; bias rows at a pitch of 8."""
+    from fastfold_b200.ops import _lib
+    B, n, _, H, d = x.shape
+    pitch = (n + 7) // 8 * 8
+    b = None if bias is None else torch.nn.functional.pad(bias, (0, pitch - n)).contiguous()
+    out = torch.full((B, n_q, H * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+    p, rs = x.data_ptr(), 3 * H * d
+    rc = _lib.get().ffb_attention_infer(p, p + 2 * H * d, p + 4 * H * d, n * rs, rs, n * rs, rs, _lib.ptr(b), pitch, _lib.ptr(mask), n,
+                                        out.data_ptr(), n_q * H * d, H * d, B, H, n_q, n, d, d ** -0.5, _lib.stream_ptr())
+    assert rc == 0
+    return out.view(B, n_q, H, d).transpose(1, 2)
+
+
+@pytest.mark.parametrize("B,H,n_q,n,d", [
+    (1, 1, 1, 1, 32), (3, 2, 33, 17, 32), (7, 4, 97, 64, 16),              # one round per CTA, one to four warps with rows
+    (445, 1, 129, 65, 32), (446, 1, 161, 129, 16), (447, 2, 225, 256, 32),  # several rounds per CTA, resident bias, last query tile in part
+    (100, 8, 257, 257, 32), (64, 4, 390, 390, 16), (67, 4, 520, 389, 32),   # streamed bias, rounds with fewer than three rows, key tails
+    (1000, 4, 64, 321, 32),
+])
+@pytest.mark.parametrize("use_bias", [True, False])
+def test_forward_rounds_and_tails(B, H, n_q, n, d, use_bias, device_status):
+    """Query tiles and key blocks that are filled in part, batch rows in rounds of one to three, several rounds per CTA: every
+    element, twice the same bits.  Bound: P and the output are rounded to bf16 and |v| < 5.5, as above, with logits of order 1."""
+    g = torch.Generator(device=DEV).manual_seed(B + n)
+    m = max(n, n_q)
+    x = torch.randn(B, m, 3, H, d, device=DEV, generator=g).to(torch.bfloat16)
+    bias = torch.randn(H, n_q, m, device=DEV, generator=g).to(torch.bfloat16) if use_bias else None
+    mask = (torch.rand(B, m, device=DEV, generator=g) > 0.3).to(torch.bfloat16)
+    mask[:, 0] = 1
+    mask[B // 2:] = 1
+    if m > n:                                                             # as many keys as the mask leaves
+        mask[:, n:] = 0
+    out = _infer(x, bias, mask, n_q)
+    assert torch.equal(out, _infer(x, bias, mask, n_q))
+    for i in range(0, B, 64):
+        q, k, v = (t.transpose(1, 2) for t in x[i:i + 64].float().unbind(2))
+        ref = attention_core_ref(q[:, :, :n_q], k, v, mask[i:i + 64].float(), None if bias is None else bias.float())
+        assert (out[i:i + 64].float() - ref).abs().max().item() < 2.2e-2
+
+
 @pytest.mark.parametrize("n", [128, 200, 640])
 @pytest.mark.parametrize("level", [-8e8, -1e9])
 def test_forward_masked_block_before_keys_of_a_low_bias(level, n, device_status):
