@@ -19,6 +19,7 @@ namespace ffb {
 
 constexpr int IPA_THREADS = 384;   // one warp per head
 constexpr int IPA_J = 64;          // keys per chunk
+enum { IPA_BF16_WB = 1, IPA_BF16_BB = 2, IPA_BF16_GAMMA = 4, IPA_BF16_MASK = 8 };
 constexpr int IPA_ZP = 8;          // padding (bf16) of a z row in shared memory: consecutive keys fall into different banks
 
 struct IpaArgs {
@@ -29,16 +30,43 @@ struct IpaArgs {
   const float* k_pts;   // [N][H][Pq][3]
   const float* v_pts;   // [N][H][Pv][3]
   const bf16* z;        // [rows][N][CZ]  (row r = query row0 + r)
-  const float* wb;      // [H][CZ]
-  const float* bb;      // [H]
-  const float* gamma;   // [H]  softplus(head_weights) * sqrt(1 / (3 * Pq * 9 / 2))
-  const float* mask;    // [N]
+  const void* wb;       // [H][CZ]
+  const void* bb;       // [H]
+  const void* gamma;    // [H]  softplus(head_weights) * sqrt(1 / (3 * Pq * 9 / 2))
+  const void* mask;     // [N]
   float* o;             // [rows][H][C]
   float* o_pt;          // [rows][H][Pv][3]
   float* o_pair;        // [rows][H][CZ]
   int N, H, C, Pq, Pv, CZ, row0, rows;
   float w_c, w_b, inf;
+  int bf;               // which of wb, bb, gamma, mask are bf16 (IPA_BF16_*), the others fp32
 };
+
+__device__ __forceinline__ float ipa_load(const void* p, long long i, bool half) {
+  return half ? __bfloat162float(reinterpret_cast<const bf16*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
+}
+
+// two floats in one 64-bit register pair: the FMA pipe does both in one instruction
+__device__ __forceinline__ uint64_t ipa_pair(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 ipa_split(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t ipa_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t ipa_mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in_range) {
   const int bytes = in_range ? 16 : 0;                         // 0: the 16 bytes are filled with zeros, nothing is read
@@ -52,19 +80,23 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool i
 //            rows, so that v and v_pts are read once per CTA.
 // The z chunk after next is on its way (cp.async) while this one is used; two barriers per chunk.
 //
-// What bounds it: instruction issue (about 50 issue slots x SM sub-partition per (query, key) pair for all heads) and, below
-// some 150 CTAs, the number of SMs in use.  One row per CTA with one key-value read per row, which this replaces, spent its
-// time waiting for L2: every row re-read 3.2 KB of keys, values and points per key, a quarter of the warps in flight.
+// What bounds it: instruction issue by three warps per scheduler, and, below some 150 CTAs, the number of SMs in use.  So everything
+// goes two by two (fma.rn.f32x2): even and odd pair channels in the bias, neighbouring heads in the pair sums, neighbouring rows in the
+// value sums, for which the probabilities lie in shared memory in both orders; the sums' order and so the bits are those of single FMAs.
+// One row per CTA with one key-value read per row spent its time waiting for L2: every row re-read 3.2 KB of keys, values and points
+// per key, a quarter of the warps in flight.
 // Four rows at every length: a CTA with two, and two of those per SM, read keys and values twice as often and were slower even
 // where four rows leave SMs idle.
-//   Measured (B200, the core alone, us, R = 2 / R = 4): N = 256 90 / 78, 512 192 / 171, 768 592 / 525, 1024 792 / 740,
-//   1184 966 / 869, 1536 1796 / 1659, 2048 3207 / 2967; one row per CTA took 349 at 512.
+//   Measured (B200, the core alone, us, with single FMAs, R = 2 / R = 4): N = 256 90 / 78, 512 192 / 171, 768 592 / 525, 1024 792 / 740,
+//   1184 966 / 869, 1536 1796 / 1659, 2048 3207 / 2967; one row per CTA took 349 at 512.  Two by two: 512 165 -> 150.
 template <int R, int H, int C, int PQ, int PV, int CZ>
 __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   static_assert(H * 32 == IPA_THREADS && CZ == 128, "one warp per head");
   constexpr int ZROW = CZ + IPA_ZP;
+  constexpr int PRS = H * R + 4;                             // + 4: the keys of a warp's 16-byte stores fall into different banks
+  static_assert(R == 4 && H % 4 == 0, "four rows in a 16-byte access, pairs of heads");
   constexpr int VC = H * C, VT = H * PV * 3;                 // value channels from v and from v_pts
   constexpr int ZT = R * (CZ / 2);                           // threads on the pair channels
   constexpr int NV_T = IPA_THREADS - ZT;                     // threads on the value channels
@@ -75,7 +107,8 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
   float* qs = wbs + H * CZ;                                                      // [R][H][C]
   float* qp = qs + R * H * C;                                                    // [R][H][PQ * 3]
   float* ps = qp + R * H * PQ * 3;                                               // [R][J][H] probabilities of the chunk
-  float* alph = ps + R * IPA_J * H;                                              // [R][H] rescale factor of the chunk
+  float* pr = ps + R * IPA_J * H;                                                // [J][PRS]: the same as [H][R] per key
+  float* alph = pr + IPA_J * PRS;                                                // [R][H] rescale factor of the chunk
   float* lfin = alph + R * H;                                                    // [R][H] row sums at the end
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r0 = blockIdx.x * R;
@@ -92,7 +125,7 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   load_z(0);
-  for (int t = tid; t < H * CZ; t += IPA_THREADS) wbs[t] = a.wb[t];
+  for (int t = tid; t < H * CZ; t += IPA_THREADS) wbs[t] = ipa_load(a.wb, t, a.bf & IPA_BF16_WB);
   for (int t = tid; t < R * H * C; t += IPA_THREADS) {
     const int r = t / (H * C);
     qs[t] = r0 + r < a.rows ? a.q[(long long)(a.row0 + r0 + r) * H * C + t % (H * C)] : 0.f;
@@ -106,15 +139,16 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
   for (int r = 0; r < R; ++r) {
     mrun[r] = -INFINITY;
     lrun[r] = 0.f;
-    mask_i[r] = (a.mask && r0 + r < a.rows) ? a.mask[a.row0 + r0 + r] : 1.f;
+    mask_i[r] = (a.mask && r0 + r < a.rows) ? ipa_load(a.mask, a.row0 + r0 + r, a.bf & IPA_BF16_MASK) : 1.f;
   }
-  const float bb_h = a.bb[warp], ghalf = 0.5f * a.gamma[warp];
-  // accumulators: pair channels 2 * cp, 2 * cp + 1 of one row for every head, or NVA value channels for every row
+  const float bb_h = ipa_load(a.bb, warp, a.bf & IPA_BF16_BB), ghalf = 0.5f * ipa_load(a.gamma, warp, a.bf & IPA_BF16_GAMMA);
+  // accumulators, two by two: pair channels 2 * cp, 2 * cp + 1 of one row for every pair of heads, or NVA value channels for every
+  // pair of rows
   const int zr = tid / (CZ / 2), cp = tid % (CZ / 2);
-  constexpr int NACC = 2 * H > NVA * R ? 2 * H : NVA * R;
-  float acc[NACC];
+  constexpr int NACC = H > NVA * (R / 2) ? H : NVA * (R / 2);
+  uint64_t acc[NACC];
 #pragma unroll
-  for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
+  for (int i = 0; i < NACC; ++i) acc[i] = ipa_pair(0.f, 0.f);
   int vhead[NVA], vstep[NVA];
   const float* vbase[NVA];
 #pragma unroll
@@ -139,29 +173,22 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
       const int j = half * 32 + lane;
       const bool on = j < jn;
       const long long jj = on ? j0 + j : 0;
-      float acc0[R], acc1[R];                           // even / odd pair channels
+      uint64_t zw[R];                                   // even / odd pair channels
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        acc0[r] = bb_h;
-        acc1[r] = 0.f;
-      }
+      for (int r = 0; r < R; ++r) zw[r] = ipa_pair(bb_h, 0.f);
 #pragma unroll 2
       for (int c = 0; c < CZ; c += 8) {
-        const float4 w0 = *reinterpret_cast<const float4*>(wbs + warp * CZ + c), w1 = *reinterpret_cast<const float4*>(wbs + warp * CZ + c + 4);
+        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(wbs + warp * CZ + c), w1 = *reinterpret_cast<const ulonglong2*>(wbs + warp * CZ + c + 4);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const uint4 raw = *reinterpret_cast<const uint4*>(zc + (r * IPA_J + j) * ZROW + c);
-          acc0[r] = fmaf(__uint_as_float(raw.x << 16), w0.x, acc0[r]);
-          acc1[r] = fmaf(__uint_as_float(raw.x & 0xffff0000u), w0.y, acc1[r]);
-          acc0[r] = fmaf(__uint_as_float(raw.y << 16), w0.z, acc0[r]);
-          acc1[r] = fmaf(__uint_as_float(raw.y & 0xffff0000u), w0.w, acc1[r]);
-          acc0[r] = fmaf(__uint_as_float(raw.z << 16), w1.x, acc0[r]);
-          acc1[r] = fmaf(__uint_as_float(raw.z & 0xffff0000u), w1.y, acc1[r]);
-          acc0[r] = fmaf(__uint_as_float(raw.w << 16), w1.z, acc0[r]);
-          acc1[r] = fmaf(__uint_as_float(raw.w & 0xffff0000u), w1.w, acc1[r]);
+          zw[r] = ipa_fma2(ipa_pair(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u)), w0.x, zw[r]);
+          zw[r] = ipa_fma2(ipa_pair(__uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u)), w0.y, zw[r]);
+          zw[r] = ipa_fma2(ipa_pair(__uint_as_float(raw.z << 16), __uint_as_float(raw.z & 0xffff0000u)), w1.x, zw[r]);
+          zw[r] = ipa_fma2(ipa_pair(__uint_as_float(raw.w << 16), __uint_as_float(raw.w & 0xffff0000u)), w1.y, zw[r]);
         }
       }
-      const float mj = a.mask ? a.mask[jj] : 1.f;
+      const float mj = a.mask ? ipa_load(a.mask, jj, a.bf & IPA_BF16_MASK) : 1.f;
       float qk[R], d2[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) qk[r] = d2[r] = 0.f;
@@ -188,27 +215,31 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
       }
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        lg[r][half] = on ? a.w_c * qk[r] + a.w_b * (acc0[r] + acc1[r]) - ghalf * d2[r] + a.inf * (mask_i[r] * mj - 1.f) : -INFINITY;
+        lg[r][half] = on ? a.w_c * qk[r] + a.w_b * (ipa_split(zw[r]).x + ipa_split(zw[r]).y) - ghalf * d2[r] + a.inf * (mask_i[r] * mj - 1.f) : -INFINITY;
     }
+    float p0[R], p1[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const float mnew = fmaxf(mrun[r], warp_max(fmaxf(lg[r][0], lg[r][1])));
-      const float p0 = __expf(lg[r][0] - mnew), p1 = __expf(lg[r][1] - mnew);      // -inf logits (beyond N) give 0
+      p0[r] = __expf(lg[r][0] - mnew);                                             // -inf logits (beyond N) give 0
+      p1[r] = __expf(lg[r][1] - mnew);
       const float al = __expf(mrun[r] - mnew);                                     // 0 on the first chunk (-inf)
-      ps[(r * IPA_J + lane) * H + warp] = p0;
-      ps[(r * IPA_J + 32 + lane) * H + warp] = p1;
-      lrun[r] = lrun[r] * al + warp_sum(p0 + p1);
+      ps[(r * IPA_J + lane) * H + warp] = p0[r];
+      ps[(r * IPA_J + 32 + lane) * H + warp] = p1[r];
+      lrun[r] = lrun[r] * al + warp_sum(p0[r] + p1[r]);
       mrun[r] = mnew;
       if (lane == 0) alph[r * H + warp] = al;
     }
+    *reinterpret_cast<float4*>(pr + lane * PRS + warp * R) = make_float4(p0[0], p0[1], p0[2], p0[3]);
+    *reinterpret_cast<float4*>(pr + (32 + lane) * PRS + warp * R) = make_float4(p1[0], p1[1], p1[2], p1[3]);
     __syncthreads();
     // ---- weighted sums ----
     if (tid < ZT) {
 #pragma unroll
-      for (int h = 0; h < H; ++h) {
-        const float al = alph[zr * H + h];
-        acc[2 * h] *= al;
-        acc[2 * h + 1] *= al;
+      for (int h2 = 0; h2 < H / 2; ++h2) {
+        const uint64_t al = *reinterpret_cast<const uint64_t*>(alph + zr * H + 2 * h2);
+        acc[h2] = ipa_mul2(acc[h2], al);
+        acc[H / 2 + h2] = ipa_mul2(acc[H / 2 + h2], al);
       }
       const bf16* zp = zc + zr * IPA_J * ZROW + 2 * cp;
       const float* pp = ps + zr * IPA_J * H;
@@ -216,24 +247,28 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
       for (int j = 0; j < IPA_J; ++j) {                 // rows past N: z = 0 and p = 0
         const uint32_t zz = *reinterpret_cast<const uint32_t*>(zp + j * ZROW);
         const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xffff0000u);
+        const uint64_t z00 = ipa_pair(z0, z0), z11 = ipa_pair(z1, z1);
 #pragma unroll
         for (int h4 = 0; h4 < H / 4; ++h4) {
-          const float4 p = *reinterpret_cast<const float4*>(pp + j * H + h4 * 4);  // same address in every lane
-          acc[h4 * 8 + 0] = fmaf(p.x, z0, acc[h4 * 8 + 0]);
-          acc[h4 * 8 + 1] = fmaf(p.x, z1, acc[h4 * 8 + 1]);
-          acc[h4 * 8 + 2] = fmaf(p.y, z0, acc[h4 * 8 + 2]);
-          acc[h4 * 8 + 3] = fmaf(p.y, z1, acc[h4 * 8 + 3]);
-          acc[h4 * 8 + 4] = fmaf(p.z, z0, acc[h4 * 8 + 4]);
-          acc[h4 * 8 + 5] = fmaf(p.z, z1, acc[h4 * 8 + 5]);
-          acc[h4 * 8 + 6] = fmaf(p.w, z0, acc[h4 * 8 + 6]);
-          acc[h4 * 8 + 7] = fmaf(p.w, z1, acc[h4 * 8 + 7]);
+          const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(pp + j * H + h4 * 4);  // same address in every lane
+          acc[h4 * 2] = ipa_fma2(p.x, z00, acc[h4 * 2]);
+          acc[h4 * 2 + 1] = ipa_fma2(p.y, z00, acc[h4 * 2 + 1]);
+          acc[H / 2 + h4 * 2] = ipa_fma2(p.x, z11, acc[H / 2 + h4 * 2]);
+          acc[H / 2 + h4 * 2 + 1] = ipa_fma2(p.y, z11, acc[H / 2 + h4 * 2 + 1]);
         }
       }
     } else {
 #pragma unroll
-      for (int u = 0; u < NVA; ++u)
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[u * R + r] *= alph[r * H + vhead[u]];
+      for (int u = 0; u < NVA; ++u) {
+        acc[u * 2] = ipa_mul2(acc[u * 2], ipa_pair(alph[vhead[u]], alph[H + vhead[u]]));
+        acc[u * 2 + 1] = ipa_mul2(acc[u * 2 + 1], ipa_pair(alph[2 * H + vhead[u]], alph[3 * H + vhead[u]]));
+      }
+      auto add = [&](int u, int j, float v) {
+        const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(pr + j * PRS + vhead[u] * R);
+        const uint64_t vv = ipa_pair(v, v);
+        acc[u * 2] = ipa_fma2(p.x, vv, acc[u * 2]);
+        acc[u * 2 + 1] = ipa_fma2(p.y, vv, acc[u * 2 + 1]);
+      };
       int j = 0;
 #pragma unroll 1
       for (; j + 4 <= jn; j += 4) {
@@ -243,18 +278,14 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
 #pragma unroll
           for (int e = 0; e < 4; ++e) v[u][e] = vbase[u][(j0 + j + e) * vstep[u]];
 #pragma unroll
-        for (int u = 0; u < NVA; ++u)
+        for (int e = 0; e < 4; ++e)
 #pragma unroll
-          for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[u * R + r] = fmaf(ps[(r * IPA_J + j + e) * H + vhead[u]], v[u][e], acc[u * R + r]);
+          for (int u = 0; u < NVA; ++u) add(u, j + e, v[u][e]);
       }
 #pragma unroll 1
       for (; j < jn; ++j)
 #pragma unroll
-        for (int u = 0; u < NVA; ++u)
-#pragma unroll
-          for (int r = 0; r < R; ++r) acc[u * R + r] = fmaf(ps[(r * IPA_J + j) * H + vhead[u]], vbase[u][(j0 + j) * vstep[u]], acc[u * R + r]);
+        for (int u = 0; u < NVA; ++u) add(u, j, vbase[u][(j0 + j) * vstep[u]]);
     }
   }
   // ---- normalise and store ----
@@ -267,7 +298,9 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
 #pragma unroll
       for (int h = 0; h < H; ++h) {
         const float l = lfin[zr * H + h];
-        *reinterpret_cast<float2*>(a.o_pair + ((long long)(r0 + zr) * H + h) * CZ + 2 * cp) = make_float2(acc[2 * h] / l, acc[2 * h + 1] / l);
+        const float2 lo = ipa_split(acc[h / 2]), hi = ipa_split(acc[H / 2 + h / 2]);
+        *reinterpret_cast<float2*>(a.o_pair + ((long long)(r0 + zr) * H + h) * CZ + 2 * cp) =
+            h & 1 ? make_float2(lo.y / l, hi.y / l) : make_float2(lo.x / l, hi.x / l);
       }
     }
   } else {
@@ -278,7 +311,8 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if (r0 + r >= a.rows) continue;
-        const float val = acc[u * R + r] / lfin[r * H + vhead[u]];
+        const float2 two = ipa_split(acc[u * 2 + r / 2]);
+        const float val = (r & 1 ? two.y : two.x) / lfin[r * H + vhead[u]];
         if (ch < VC) a.o[(long long)(r0 + r) * VC + ch] = val;
         else a.o_pt[(long long)(r0 + r) * VT + ch - VC] = val;
       }
@@ -289,7 +323,7 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
 template <int R>
 static int ipa_launch(const IpaArgs& a, cudaStream_t st) {
   constexpr int HH = 12, CC = 16, PQ = 4, PV = 8, CZZ = 128;
-  constexpr size_t smem = 2 * R * IPA_J * (CZZ + IPA_ZP) * 2 + sizeof(float) * (HH * CZZ + R * HH * CC + R * HH * PQ * 3 + R * HH * IPA_J + 2 * R * HH);
+  constexpr size_t smem = 2 * R * IPA_J * (CZZ + IPA_ZP) * 2 + sizeof(float) * (HH * CZZ + R * HH * CC + R * HH * PQ * 3 + R * HH * IPA_J + IPA_J * (R * HH + 4) + 2 * R * HH);
   auto kern = ipa_fwd_kernel<R, HH, CC, PQ, PV, CZZ>;
   static SmemLimit limit;
   if (!limit.raise(kern, smem)) return -4;
@@ -424,9 +458,10 @@ int ffb_ipa_cat(const float* o, const float* o_pt, const float* o_pair, const fl
 // All pointers are device memory; q / k / v / points / weights / outputs fp32, z bf16 (layouts in IpaArgs).
 // Supported configuration: H = 12 heads, C = 16 channels, 4 query / key points, 8 value points, c_z = 128 (AlphaFold's
 // structure module); anything else returns -2 and the caller uses its PyTorch composite.
-int ffb_ipa_fwd(const float* q, const float* k, const float* v, const float* q_pts, const float* k_pts, const float* v_pts, const void* z,
-                const float* wb, const float* bb, const float* gamma, const float* mask, float* o, float* o_pt, float* o_pair, int N, int H,
-                int C, int Pq, int Pv, int CZ, int row0, int rows, float w_c, float w_b, float inf, void* stream) {
+// ..._mixed: wb, bb, gamma and mask in fp32 or, as `bf` says (bits 1, 2, 4, 8), in bf16.
+int ffb_ipa_fwd_mixed(const float* q, const float* k, const float* v, const float* q_pts, const float* k_pts, const float* v_pts, const void* z,
+                      const void* wb, const void* bb, const void* gamma, const void* mask, int bf, float* o, float* o_pt, float* o_pair, int N, int H,
+                      int C, int Pq, int Pv, int CZ, int row0, int rows, float w_c, float w_b, float inf, void* stream) {
   if (H != 12 || C != 16 || Pq != 4 || Pv != 8 || CZ != 128) return -2;
   if (rows <= 0) return 0;
   if (N <= 0 || row0 < 0 || row0 + rows > N || (reinterpret_cast<uintptr_t>(z) & 15) || (reinterpret_cast<uintptr_t>(k) & 15) ||
@@ -439,8 +474,15 @@ int ffb_ipa_fwd(const float* q, const float* k, const float* v, const float* q_p
   a.o = o; a.o_pt = o_pt; a.o_pair = o_pair;
   a.N = N; a.H = H; a.C = C; a.Pq = Pq; a.Pv = Pv; a.CZ = CZ; a.row0 = row0; a.rows = rows;
   a.w_c = w_c; a.w_b = w_b; a.inf = inf;
+  a.bf = bf;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   return ipa_launch<4>(a, st);
+}
+
+int ffb_ipa_fwd(const float* q, const float* k, const float* v, const float* q_pts, const float* k_pts, const float* v_pts, const void* z,
+                const float* wb, const float* bb, const float* gamma, const float* mask, float* o, float* o_pt, float* o_pair, int N, int H,
+                int C, int Pq, int Pv, int CZ, int row0, int rows, float w_c, float w_b, float inf, void* stream) {
+  return ffb_ipa_fwd_mixed(q, k, v, q_pts, k_pts, v_pts, z, wb, bb, gamma, mask, 0, o, o_pt, o_pair, N, H, C, Pq, Pv, CZ, row0, rows, w_c, w_b, inf, stream);
 }
 
 }  // extern "C"

@@ -23,10 +23,7 @@ def _fn():
     if not _declared:
         P, I, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
         lib.ffb_ipa_fwd.argtypes = [P] * 14 + [I] * 8 + [F, F, F, P]
-        lib.ffb_ipa_prep.argtypes = [P] * 5 + [I] + [P] * 7 + [I] * 5 + [P]
-        lib.ffb_ipa_cat.argtypes = [P] * 4 + [I, P, P] + [I] * 5 + [F, P]
-        for fn in (lib.ffb_ipa_fwd, lib.ffb_ipa_prep, lib.ffb_ipa_cat):
-            fn.restype = I
+        lib.ffb_ipa_fwd.restype = I
         _declared = True
     return lib.ffb_ipa_fwd
 
@@ -35,7 +32,7 @@ def _frame(r):
     """(rotation, is_quaternion, translation) of a ``Rigid [N]`` as fp32 tensors; quaternions are used as they are held."""
     rots = r.get_rots()
     q = rots._quats
-    return (rots._rot_mats if q is None else q).float().contiguous(), 0 if q is None else 1, r.get_trans().float().contiguous()
+    return (rots._rot_mats if q is None else q).float().contiguous(), q is not None, r.get_trans().float().contiguous()
 
 
 def layer_supported(s, z, q, kv, q_pts, kv_pts, r):
@@ -50,22 +47,8 @@ def ipa_layer(q, kv, q_pts, kv_pts, r, z, wb, bb, gamma, mask, w_c, w_b, inf, ep
     """The layer between its input projections and its output projection in three kernels (points into the global frame,
     core, features back into the local frames): the bf16 projections ``[N, .]`` in, the concatenated features
     ``[N, 2112]`` in bf16 out."""
-    H, C, Pq, Pv = 12, 16, 4, 8
-    N, dev = z.shape[0], z.device
-    _fn()
-    lib = _lib.get()
     rot, is_quat, trans = _frame(r)
-    new = lambda *shape: torch.empty(*shape, device=dev, dtype=torch.float32)
-    qf, kf, vf = new(N, H, C), new(N, H, C), new(N, H, C)
-    qp, kp, vp = new(N, H, Pq, 3), new(N, H, Pq, 3), new(N, H, Pv, 3)
-    P = _lib.ptr
-    _lib.check(lib.ffb_ipa_prep(P(q), P(kv), P(q_pts), P(kv_pts), P(rot), is_quat, P(trans), P(qf), P(kf), P(vf), P(qp), P(kp), P(vp), N, H, C, Pq, Pv,
-                                _lib.stream_ptr()), "ffb_ipa_prep(N=%d)" % N)
-    o, o_pt, o_pair = ipa_core(qf, kf, vf, qp, kp, vp, z, wb, bb, gamma, mask, w_c, w_b, inf)
-    out = torch.empty(N, H * (C + 4 * Pv + z.shape[-1]), device=dev, dtype=torch.bfloat16)
-    _lib.check(lib.ffb_ipa_cat(P(o), P(o_pt), P(o_pair), P(rot), is_quat, P(trans), P(out), N, H, C, Pv, z.shape[-1], float(eps), _lib.stream_ptr()),
-               "ffb_ipa_cat(N=%d)" % N)
-    return out
+    return _lib.native().ipa_layer(q, kv, q_pts, kv_pts, rot, is_quat, trans, z, wb, bb, gamma, mask, w_c, w_b, inf, eps)
 
 
 def supported(q, q_pts, v_pts, z):

@@ -103,6 +103,23 @@ def test_ipa_layer_in_three_kernels(N, fmt, device_status):
     assert (out.float() - ref).abs().max().item() < 2.0 ** -8 * ref.abs().max().item() + 1e-3
 
 
+@pytest.mark.parametrize("half", [(0,), (1,), (2,), (3,), (0, 1, 2, 3)])
+def test_ipa_layer_takes_parameters_and_mask_as_they_come(half, device_status):
+    """Pair-bias weight and bias, point weights and mask in bf16 give the bits of the same values in fp32."""
+    from fastfold_b200.ops import ipa as ipa_op
+    from fastfold_b200.utils.rigid_utils import Rigid, Rotation
+    g = torch.Generator().manual_seed(3)
+    b = lambda *s: torch.randn(*s, generator=g).to(DEV, torch.bfloat16)
+    N = 70
+    frames = Rigid(Rotation(quats=torch.randn(N, 4, generator=g).to(DEV), normalize_quats=True), torch.randn(N, 3, generator=g).to(DEV))
+    params = [b(12, 128), b(12), b(12).abs(), (b(N) > -1).to(torch.bfloat16)]
+    args = (b(N, 192), b(N, 384), b(N, 144), b(N, 432), frames, b(N, N, 128))
+    with torch.no_grad():
+        want = ipa_op.ipa_layer(*args, *(p.float() for p in params), 0.1, 0.5, 1e5, 1e-8)
+        got = ipa_op.ipa_layer(*args, *(p if i in half else p.float() for i, p in enumerate(params)), 0.1, 0.5, 1e5, 1e-8)
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("case", ["layer", "fp32", "batched"])
 def test_ipa_module_projects_once(case, device_status):
     """Each input projection is evaluated once, whichever path the rest of the layer takes."""
