@@ -281,16 +281,18 @@ __global__ void adam_k(float* w, float* m, float* v, const bf16* grad, bf16* w16
 }
 
 // out[i][j] = 1 / (sum_s mask[s][i] * mask[s][j] + eps): the normaliser of the outer product mean, from a mask [S][N].  32 x 32 outputs
-// per CTA, 2 x 2 per thread, the next 64 rows of the mask on their way while these are summed; one launch for the conversions, the
-// product, the sum and the reciprocal, which as tensor operations are six.  Small tiles, since the chain over S is what it takes:
-// 64 x 64 outputs made 36 CTAs at 384 residues and 512 sequences, and the whole layer took 355 us with them, 334 us with these.
+// per CTA, the next 128 rows of the mask on their way while these are summed; one launch for the conversions, the product, the sum and
+// the reciprocal, which as tensor operations are six.  Small tiles, since the chain over S is what it takes: 64 x 64 outputs made 36
+// CTAs at 384 residues and 512 sequences.  Four groups of 64 threads take every fourth sequence and 4 x 4 outputs a thread: two
+// 16-byte reads for 16 FMAs, where 2 x 2 outputs took two reads for 4 (512 x 384: 22 us, the whole layer 340; with these 12 and 332).
 template <typename T>
 __global__ void __launch_bounds__(256) mask_norm_k(const T* __restrict__ mask, float* __restrict__ out, int S, int N, float eps) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int KS = 64, W = 32, U = KS * W / 256;
+  constexpr int KS = 128, W = 32, U = KS * W / 256, G = 4;
   __shared__ __align__(16) float a[KS][W], b[KS][W];
-  const int i0 = blockIdx.y * W, j0 = blockIdx.x * W, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int i0 = blockIdx.y * W, j0 = blockIdx.x * W;
+  const int g = threadIdx.x >> 6, tx = threadIdx.x & 7, ty = (threadIdx.x >> 3) & 7;       // quarter of the sequences, 4 x 4 outputs
   const int c = threadIdx.x & 31, r = threadIdx.x >> 5;
   float ra[U], rb[U];
   auto fetch = [&](int s0) {
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(256) mask_norm_k(const T* __restrict__ mask, f
       rb[u] = (s < S && j0 + c < N) ? to_f(mask[(long long)s * N + j0 + c]) : 0.f;
     }
   };
-  float acc[2][2] = {};
+  float acc[4][4] = {};
   fetch(0);
   for (int s0 = 0; s0 < S; s0 += KS) {
 #pragma unroll
@@ -311,21 +313,26 @@ __global__ void __launch_bounds__(256) mask_norm_k(const T* __restrict__ mask, f
     }
     __syncthreads();
     if (s0 + KS < S) fetch(s0 + KS);
-#pragma unroll 16
-    for (int k = 0; k < KS; ++k) {
-      const float2 u = *reinterpret_cast<const float2*>(&a[k][ty * 2]), v = *reinterpret_cast<const float2*>(&b[k][tx * 2]);
-      acc[0][0] = fmaf(u.x, v.x, acc[0][0]);
-      acc[0][1] = fmaf(u.x, v.y, acc[0][1]);
-      acc[1][0] = fmaf(u.y, v.x, acc[1][0]);
-      acc[1][1] = fmaf(u.y, v.y, acc[1][1]);
+#pragma unroll 8
+    for (int k = g; k < KS; k += G) {
+      const float4 u = *reinterpret_cast<const float4*>(&a[k][ty * 4]), v = *reinterpret_cast<const float4*>(&b[k][tx * 4]);
+      const float uu[4] = {u.x, u.y, u.z, u.w}, vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(uu[i], vv[j], acc[i][j]);
     }
     __syncthreads();
   }
+  // the four quarters, in the place of the rows
+  float* part = &a[0][0];                                   // [G][W][W]
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(part + (g * W + ty * 4 + i) * W + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
-      if (i0 + ty * 2 + i < N && j0 + tx * 2 + j < N) out[(long long)(i0 + ty * 2 + i) * N + j0 + tx * 2 + j] = 1.f / (acc[i][j] + eps);
+  for (int i = r; i < W; i += 8)
+    if (i0 + i < N && j0 + c < N)
+      out[(long long)(i0 + i) * N + j0 + c] = 1.f / (((part[i * W + c] + part[(W + i) * W + c]) + (part[(2 * W + i) * W + c] + part[(3 * W + i) * W + c])) + eps);
 }
 
 }  // namespace ffb
