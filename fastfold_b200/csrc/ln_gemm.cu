@@ -9,14 +9,16 @@
 // activation of a transition (four times its input) among them, and on short inputs each was a launch.  Here a tile of 128 rows is
 // read once; its normalised form (rounded to bf16, as the LayerNorm kernel stores it) and the hidden activation never leave the SM.
 //
-// Persistent, one CTA per SM, 448 threads, tiles of 128 rows:
+// Persistent, one CTA per SM, 448 or 704 threads, tiles of 128 rows:
 //   warps 0-3    LayerNorm, a thread per row (channels-first input: per pair of rows and half of the channels), in place in the
 //                shared-memory tile that becomes the A operand.  The 128-byte swizzle makes a thread's 16-byte accesses to its own row
 //                free of conflicts, so no shuffles are needed
-//   warps 4-11   epilogues, two warps per tensor-memory quadrant, 64 columns each
-//   warp 12      TMA: rows of the next tile, weights through a ring of 16 KB boxes (128 rows x 64 columns; out of L2 for all but the
+//   then         epilogues, a team of eight warps, two per tensor-memory quadrant with 64 columns each; projections of 64 and 128
+//                channels have two teams that take the chunks in turn: the epilogues are their longest chain, most of it latency
+//                (1600 cycles for 64 columns that are only converted), and two warps per scheduler do not hide it
+//   then a warp  TMA: rows of the next tile, weights through a ring of 16 KB boxes (128 rows x 64 columns; out of L2 for all but the
 //                first CTA)
-//   warp 13      MMA issue, 128 x 128 x 16
+//   and one      MMA issue, 128 x 128 x 16
 // Weights come in chunks of 128 rows.  Of a chain, chunk h of the hidden activation goes through tensor memory: the epilogue
 // reads the accumulator, applies f and writes bf16 pairs over it, and the second product takes them from there as its A operand.
 // The products of chunk h + 1 are issued before the second product of chunk h, which hides the epilogue.
@@ -27,6 +29,8 @@
 //   47 -> 32, 589824 x 128 341 -> 208, 32768 x 256 54 -> 48, 2048 x 256 16 -> 26 (one launch in place of three: host/dispatch.cpp, which chooses,
 //   has the line between the two); gated output with the norm (left side without it) 589824 x 128 192 -> 139, 32768 x 256 30 -> 24; QKV 589824 x 128
 //   181 -> 130; operands and gate of the triangle multiplication at 1024 residues 539 -> 480, its output 293 -> 177.
+//   Two teams instead of one: triangle multiplication 1024 1004 -> 932, a block of 128 x 256 729 -> 698, of 256 x 384 in chunks
+//   2240 -> 2182, the extra-MSA stack of 1024 x 256 531 -> 517; a block of 32 x 64 as before.
 //
 // Stands for the nn.LayerNorm / nn.Linear / elementwise chains of the reference (fastfold/model/fastnn/ops.py:85-106, 143-160,
 // 275-324, 393-404).
@@ -37,8 +41,7 @@
 
 namespace ffb {
 
-constexpr int LG_THREADS = 448;
-constexpr int LG_EPI = 8;                 // epilogue warps
+constexpr int LG_EPI = 8;                 // epilogue warps of a chunk
 constexpr int LG_BOX = 16384;             // weight box: 128 rows x 64 columns
 constexpr int LG_MAX_N = 1280;            // columns of all weights (biases in shared memory)
 
@@ -69,17 +72,19 @@ struct LgArgs {
   int pb_n;
 };
 
-template <int C, int MODE>
+// TEAMS: teams of eight epilogue warps, which take the chunks in turn
+template <int C, int MODE, int TEAMS>
 struct LgCfg {
+  static constexpr int EPI = LG_EPI * TEAMS, THREADS = (6 + EPI) * 32, TMA = 4 + EPI, MMA = 5 + EPI;       // the last two are warps
   static constexpr int KB = C / 64;
   static constexpr int A_BYTES = KB * 16384;
-  static constexpr int TILES = C == 256 ? 1 : 2;                     // 4 KB staging tiles per epilogue warp
+  static constexpr int TILES = C == 256 || TEAMS == 2 ? 1 : 2;                     // 4 KB staging tiles per epilogue warp
   static constexpr int NA = C == 256 ? 1 : 2;                        // tiles of rows: one less, and the ring holds four boxes more
   static constexpr int RING = C == 256 ? 7 : 5;
   static constexpr int NB2 = C < 128 ? C : 128;                      // columns of one second product
   static constexpr int NACC = MODE == LN_PROJECT ? 4 : (C == 256 ? 2 : 3);      // 128-column accumulators of the first product
   static constexpr int ACC2 = NACC * 128;                            // tensor-memory column of the second product's accumulator
-  static constexpr int A0 = 0, W0 = NA * A_BYTES, STG = W0 + RING * LG_BOX, VEC = STG + LG_EPI * TILES * 4096;
+  static constexpr int A0 = 0, W0 = NA * A_BYTES, STG = W0 + RING * LG_BOX, VEC = STG + EPI * TILES * 4096;
   static constexpr int VEC_FLOATS = 2 * C + LG_MAX_N + 256 + (MODE == LN_PROJECT ? 1280 : 0);     // gamma, beta, biases, channel sums
   static constexpr int BARS = VEC + VEC_FLOATS * 4;
   static constexpr int SMEM = BARS + 512 + 1024;
@@ -342,10 +347,11 @@ __device__ __forceinline__ void lg_store_tile(const CUtensorMap* map, uint32_t s
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 
-template <int C, int MODE, bool CF>
-__global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_constant__ LgMaps maps, const __grid_constant__ LgArgs a) {
+template <int C, int MODE, bool CF, int TEAMS>
+__global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(const __grid_constant__ LgMaps maps, const __grid_constant__ LgArgs a) {
   pdl_launch_dependents();
-  using Cfg = LgCfg<C, MODE>;
+  using Cfg = LgCfg<C, MODE, TEAMS>;
+  static_assert(TEAMS == 1 || (TEAMS == 2 && MODE == LN_PROJECT && !CF), "two teams: projections");
   constexpr int KB = Cfg::KB, RING = Cfg::RING, NACC = Cfg::NACC, NB2 = Cfg::NB2, NA = Cfg::NA;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -392,19 +398,19 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
   }
   pdl_wait();
   // gamma, beta and all biases as fp32; read back as broadcasts
-  for (int i = threadIdx.x; i < C; i += LG_THREADS) {
+  for (int i = threadIdx.x; i < C; i += Cfg::THREADS) {
     const int at = C == 64 ? (i & 48) + (i & 7) * 2 + ((i >> 3) & 1) : i;       // for lg_norm_row<64>: the same channel of two pieces side by side
     gamma[at] = __bfloat162float(a.gamma[i]);
     beta[at] = __bfloat162float(a.beta[i]);
   }
   if (MODE != LN_PROJECT) {
-    for (int i = threadIdx.x; i < ((a.hidden + 127) & ~127); i += LG_THREADS) bias1[i] = (a.b1 && i < a.hidden) ? __bfloat162float(a.b1[i]) : 0.f;
-    for (int i = threadIdx.x; i < C; i += LG_THREADS) bias2[i] = a.b2 ? __bfloat162float(a.b2[i]) : 0.f;
+    for (int i = threadIdx.x; i < ((a.hidden + 127) & ~127); i += Cfg::THREADS) bias1[i] = (a.b1 && i < a.hidden) ? __bfloat162float(a.b1[i]) : 0.f;
+    for (int i = threadIdx.x; i < C; i += Cfg::THREADS) bias2[i] = a.b2 ? __bfloat162float(a.b2[i]) : 0.f;
   } else {
     int off = 0;
     for (int s = 0; s < a.nseg; ++s) {
       const int n = a.seg[s].n, nc = (n + 127) & ~127;
-      for (int i = threadIdx.x; i < nc; i += LG_THREADS) bias1[off + i] = (a.seg_bias[s] && i < n) ? __bfloat162float(a.seg_bias[s][i]) : 0.f;
+      for (int i = threadIdx.x; i < nc; i += Cfg::THREADS) bias1[off + i] = (a.seg_bias[s] && i < n) ? __bfloat162float(a.seg_bias[s][i]) : 0.f;
       off += nc;
     }
   }
@@ -436,7 +442,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
       if (*abort_flag == 0) report(ST_TIMEOUT_TMA, 50);
       *abort_flag = 1;
     }
-  } else if (warp == 12) {
+  } else if (warp == Cfg::TMA) {
     // ---------------- TMA: rows and weights ----------------
     if (lane == 0) {
       bool ok = true;
@@ -506,7 +512,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
       }
     }
     __syncwarp();
-  } else if (warp == 13) {
+  } else if (warp == Cfg::MMA) {
     // ---------------- MMA issue (the whole warp, see umma_bf16_by) ----------------
     constexpr uint32_t idesc1 = make_idesc_bf16(128, 128, CF ? 1 : 0, 0), idesc2 = make_idesc_bf16(128, NB2, 0, 0);
     const uint32_t lead = elect_one();
@@ -582,8 +588,8 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
     if (!ok && lead) *abort_flag = 1;
     __syncwarp();
   } else {
-    // ---------------- epilogues (warps 4..11) ----------------
-    const int quad = warp & 3, half = (warp - 4) >> 2;
+    // ---------------- epilogues (from warp 4 on) ----------------
+    const int quad = warp & 3, half = ((warp - 4) >> 2) & 1, team = (warp - 4) >> 3;
     uint8_t* stg = sm + Cfg::STG + (warp - 4) * (Cfg::TILES * 4096);
     const uint32_t stg_u = smem_u32(stg), my_ld = ld_bar + 8 * (warp - 4);
     const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
@@ -734,6 +740,17 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
         for (int h = 0; h < chunks; ++h, ++c1) {
           const LgSeg sg = a.seg[seg];
           const int mycol = col + half * 64, b = c1 % NACC;
+          auto next = [&]() {
+            col += 128;
+            if (col >= sg.n) {
+              ++seg;
+              col = 0;
+            }
+          };
+          if (TEAMS == 2 && (c1 & 1) != team) {                 // the other team's
+            next();
+            continue;
+          }
           const bool work = mycol < sg.n && valid;
           uint8_t* obuf = stg + ob;
           const bool fused = a.has_mul != 0 && seg == 0;        // mul and residual tiles (two staging tiles; first segment)
@@ -762,6 +779,45 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
 #pragma unroll
                 for (int j = 0; j < 32; ++j)
                   if (j < sg.n) dst[j * a.pb_h] = __float2bfloat16(v[j]);
+              }
+            } else if constexpr (TEAMS == 2) {
+              // 32 columns at a time: 22 warps leave 88 registers a thread
+#pragma unroll 1
+              for (int e = 0; e < 2; ++e) {
+                float v[32];
+                tmem_ld_32x32(lane_base + b * 128 + half * 64 + e * 32, v);
+                const float4* bp = reinterpret_cast<const float4*>(bias1 + h * 128 + half * 64 + e * 32);
+                tmem_ld_wait();
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                  const float4 f = bp[q];
+                  v[4 * q] += f.x;
+                  v[4 * q + 1] += f.y;
+                  v[4 * q + 2] += f.z;
+                  v[4 * q + 3] += f.w;
+                }
+                if (sg.kind == LN_GLU_T) {
+                  bf16* o = reinterpret_cast<bf16*>(obuf) + e * 512 + lane;       // [32 columns][32 rows]
+#pragma unroll
+                  for (int j = 0; j < 16; ++j) o[j * 32] = __float2bfloat16(v[2 * j] * sigmoidf_(v[2 * j + 1]) * rs);
+                } else {
+                  if (sg.act == ACT_SIGMOID) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = sigmoidf_(v[j]);
+                  }
+                  if (sg.scaled) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] *= rs;
+                  }
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) *reinterpret_cast<uint4*>(obuf + lane * 128 + (((e * 4 + u) ^ (lane & 7)) << 4)) = lg_pack(v + u * 8);
+                }
+              }
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                if (sg.kind == LN_GLU_T) lg_store_tile(&maps.out[seg], stg_u, row0, mycol >> 1, batch);
+                else lg_store_tile(&maps.out[seg], stg_u, mycol, row0, batch);
               }
             } else {
               float v[64];
@@ -797,11 +853,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(acc_free + 8 * b);
-          col += 128;
-          if (col >= sg.n) {
-            ++seg;
-            col = 0;
-          }
+          next();
         }
       }
     }
@@ -817,11 +869,12 @@ __global__ void __launch_bounds__(LG_THREADS, 1) ln_gemm_kernel(const __grid_con
   }
 }
 
-template <int C, int MODE, bool CF>
+template <int C, int MODE, bool CF, int TEAMS = 1>
 static int lg_launch(const LgMaps& maps, const LgArgs& a, cudaStream_t st) {
-  auto kern = ln_gemm_kernel<C, MODE, CF>;
+  using Cfg = LgCfg<C, MODE, TEAMS>;
+  auto kern = ln_gemm_kernel<C, MODE, CF, TEAMS>;
   static SmemLimit limit;
-  if (!limit.raise(kern, LgCfg<C, MODE>::SMEM)) return -30;
+  if (!limit.raise(kern, Cfg::SMEM)) return -30;
   static int sm_count = 0;
   if (!sm_count) {
     int dev = 0;
@@ -829,7 +882,7 @@ static int lg_launch(const LgMaps& maps, const LgArgs& a, cudaStream_t st) {
     if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0) sm_count = 148;
   }
   const int grid = a.num_tiles < sm_count ? a.num_tiles : sm_count;
-  launch_k(kern, grid, LG_THREADS, LgCfg<C, MODE>::SMEM, st, maps, a);
+  launch_k(kern, grid, Cfg::THREADS, Cfg::SMEM, st, maps, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
 
@@ -921,7 +974,8 @@ extern "C" int ffb_ln_gemm(const LnGemmArgs* p, void* stream) {
     if (r) return 4000 + r;
   }
   if (q.channels_first) return lg_launch<128, LN_PROJECT, true>(m, a, st);
-  if (q.C == 64) return lg_launch<64, LN_PROJECT, false>(m, a, st);
-  if (q.C == 128) return lg_launch<128, LN_PROJECT, false>(m, a, st);
+  if (a.has_mul) return q.C == 64 ? lg_launch<64, LN_PROJECT, false>(m, a, st) : lg_launch<128, LN_PROJECT, false>(m, a, st);
+  if (q.C == 64) return lg_launch<64, LN_PROJECT, false, 2>(m, a, st);
+  if (q.C == 128) return lg_launch<128, LN_PROJECT, false, 2>(m, a, st);
   return lg_launch<256, LN_PROJECT, false>(m, a, st);
 }
