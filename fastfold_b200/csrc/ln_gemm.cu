@@ -13,9 +13,11 @@
 //   warps 0-3    LayerNorm, a thread per row (channels-first input: per pair of rows and half of the channels), in place in the
 //                shared-memory tile that becomes the A operand.  The 128-byte swizzle makes a thread's 16-byte accesses to its own row
 //                free of conflicts, so no shuffles are needed
-//   then         epilogues, a team of eight warps, two per tensor-memory quadrant with 64 columns each; projections of 64 and 128
-//                channels have two teams that take the chunks in turn: the epilogues are their longest chain, most of it latency
-//                (1600 cycles for 64 columns that are only converted), and two warps per scheduler do not hide it
+//   then         epilogues, a team of eight warps, two per tensor-memory quadrant with 64 columns each; 64 and 128 channels have two
+//                teams: the epilogues are the longest chain there, most of it latency (1600 cycles for 64 columns that are only
+//                converted), and two warps per scheduler do not hide it.  Of projections they take the chunks in turn, of chains one
+//                has the hidden activation and the other the result.  At 256 channels, whose staging tiles would cost two boxes of the
+//                ring, two teams are slower (block of 128 x 203 588 -> 591, of 256 x 384 in chunks 2172 -> 2183)
 //   then a warp  TMA: rows of the next tile, weights through a ring of 16 KB boxes (128 rows x 64 columns; out of L2 for all but the
 //                first CTA)
 //   and one      MMA issue, 128 x 128 x 16
@@ -29,8 +31,9 @@
 //   47 -> 32, 589824 x 128 341 -> 208, 32768 x 256 54 -> 48, 2048 x 256 16 -> 26 (one launch in place of three: host/dispatch.cpp, which chooses,
 //   has the line between the two); gated output with the norm (left side without it) 589824 x 128 192 -> 139, 32768 x 256 30 -> 24; QKV 589824 x 128
 //   181 -> 130; operands and gate of the triangle multiplication at 1024 residues 539 -> 480, its output 293 -> 177.
-//   Two teams instead of one: triangle multiplication 1024 1004 -> 932, a block of 128 x 256 729 -> 698, of 256 x 384 in chunks
-//   2240 -> 2182, the extra-MSA stack of 1024 x 256 531 -> 517; a block of 32 x 64 as before.
+//   Two teams instead of one, projections, then chains too: triangle multiplication 1024 1004 -> 932, a block of 128 x 256
+//   729 -> 698 -> 694, of 256 x 384 in chunks 2240 -> 2182 -> 2172, the extra-MSA stack of 1024 x 256 531 -> 517 -> 511; a block of 32 x 64
+//   as before.
 //
 // Stands for the nn.LayerNorm / nn.Linear / elementwise chains of the reference (fastfold/model/fastnn/ops.py:85-106, 143-160,
 // 275-324, 393-404).
@@ -80,7 +83,7 @@ struct LgCfg {
   static constexpr int A_BYTES = KB * 16384;
   static constexpr int TILES = C == 256 || TEAMS == 2 ? 1 : 2;                     // 4 KB staging tiles per epilogue warp
   static constexpr int NA = C == 256 ? 1 : 2;                        // tiles of rows: one less, and the ring holds four boxes more
-  static constexpr int RING = C == 256 ? 7 : 5;
+  static constexpr int RING = C == 256 && TEAMS == 1 ? 7 : 5;
   static constexpr int NB2 = C < 128 ? C : 128;                      // columns of one second product
   static constexpr int NACC = MODE == LN_PROJECT ? 4 : (C == 256 ? 2 : 3);      // 128-column accumulators of the first product
   static constexpr int ACC2 = NACC * 128;                            // tensor-memory column of the second product's accumulator
@@ -351,7 +354,7 @@ template <int C, int MODE, bool CF, int TEAMS>
 __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(const __grid_constant__ LgMaps maps, const __grid_constant__ LgArgs a) {
   pdl_launch_dependents();
   using Cfg = LgCfg<C, MODE, TEAMS>;
-  static_assert(TEAMS == 1 || (TEAMS == 2 && MODE == LN_PROJECT && !CF), "two teams: projections");
+  static_assert(TEAMS == 1 || (TEAMS == 2 && !CF), "channels-first rows have one team");
   constexpr int KB = Cfg::KB, RING = Cfg::RING, NACC = Cfg::NACC, NB2 = Cfg::NB2, NA = Cfg::NA;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -364,7 +367,7 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
   const uint32_t b0 = base + Cfg::BARS;
   const uint32_t x_full = b0, a_full = b0 + 16, a_empty = b0 + 32, acc_full = b0 + 48, acc_free = b0 + 80, h_full = b0 + 112;
   const uint32_t acc2_full = b0 + 144, acc2_empty = b0 + 152, w_full = b0 + 160, w_empty = b0 + 216, ld_bar = b0 + 272;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + Cfg::BARS + 336);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + Cfg::BARS + 400);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
@@ -385,7 +388,7 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
       mbar_init(w_full + 8 * i, 1);
       mbar_init(w_empty + 8 * i, 1);
     }
-    for (int i = 0; i < LG_EPI; ++i) mbar_init(ld_bar + 8 * i, 1);
+    for (int i = 0; i < Cfg::EPI; ++i) mbar_init(ld_bar + 8 * i, 1);
     *abort_flag = 0;
     fence_mbar_init();
     prefetch_tmap(&maps.x);
@@ -650,7 +653,122 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
         row0 %= a.rows;
       }
       const bool valid = row0 < a.rows && batch < a.batch;
-      if (MODE != LN_PROJECT) {
+      if constexpr (MODE != LN_PROJECT && TEAMS == 2) {
+        // One team for the hidden activation, one for the result: the result of a tile leaves while the next one's hidden activation is
+        // made.  32 columns at a time: 22 warps leave 80 registers a thread
+        auto read32 = [&](uint32_t col, const float* bias, float (&v)[32]) {
+          tmem_ld_32x32(lane_base + col, v);
+          const float4* bp = reinterpret_cast<const float4*>(bias);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const float4 f = bp[q];
+            v[4 * q] += f.x;
+            v[4 * q + 1] += f.y;
+            v[4 * q + 2] += f.z;
+            v[4 * q + 3] += f.w;
+          }
+        };
+        if (team == 0) {
+          auto fetch_mul = [&](int h) {
+            if (lane == 0) {
+              mbar_expect_tx(my_ld, 4096);
+              tma_load_3d(stg_u, &maps.mul, my_ld, h * 128 + half * 64, row0, batch);
+            }
+          };
+          if (MODE == LN_GATE_CHAIN && !a.mul_f32) fetch_mul(0);
+#pragma unroll 1
+          for (int h = 0; h < chunks; ++h, ++c1) {
+            const uint32_t b = c1 % NACC;
+            if (!wait(acc_full + 8 * b, (c1 / NACC) & 1, ST_TIMEOUT_MMA)) break;
+            tc_fence_after();
+            if (MODE == LN_GATE_CHAIN && !a.mul_f32) {
+              if (!wait(my_ld, ld_phase, ST_TIMEOUT_TMA)) break;
+              ld_phase ^= 1;
+            }
+#pragma unroll 1
+            for (int e = 0; e < 2; ++e) {
+              float v[32];
+              const int col = h * 128 + half * 64 + e * 32;
+              read32(b * 128 + half * 64 + e * 32, bias1 + col, v);
+              if (MODE == LN_RELU_CHAIN) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
+              } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = sigmoidf_(v[j]);
+                if (a.mul_f32) {
+                  // one row of 32-bit factors for all rows of a column: a few ten kilobytes that stay in L1
+                  const float4* m = reinterpret_cast<const float4*>(a.mul_f32 + ((long long)batch * a.rows + row0 + lane) % a.mul_mod * a.hidden + col);
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) {
+                    const float4 f = col + 4 * q < a.hidden ? m[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[4 * q] *= f.x;
+                    v[4 * q + 1] *= f.y;
+                    v[4 * q + 2] *= f.z;
+                    v[4 * q + 3] *= f.w;
+                  }
+                } else {
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) {
+                    float m[8];
+                    lg_unpack(*reinterpret_cast<const uint4*>(stg + lane * 128 + (((e * 4 + u) ^ (lane & 7)) << 4)), m);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[u * 8 + j] *= m[j];
+                  }
+                }
+              }
+              uint32_t p[16];                                   // bf16 pairs, over columns that have been read
+#pragma unroll
+              for (int j = 0; j < 16; ++j) p[j] = lg_pack2(v[2 * j], v[2 * j + 1]);
+              tmem_st_32x16(lane_base + b * 128 + half * 64 + e * 16, p);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(h_full + 8 * b);
+            if (MODE == LN_GATE_CHAIN && !a.mul_f32 && h + 1 < chunks) fetch_mul(h + 1);
+          }
+        } else {
+          bool waited = false;
+#pragma unroll 1
+          for (int c = half; c < C / 64; c += 2) {
+            if (lane == 0) {
+              asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+              mbar_expect_tx(my_ld, 4096);
+              tma_load_3d(stg_u, &maps.resid, my_ld, c * 64, row0, batch);
+            }
+            __syncwarp();
+            if (!waited && !wait(acc2_full, t & 1, ST_TIMEOUT_MMA)) break;
+            waited = true;
+            tc_fence_after();
+            if (!wait(my_ld, ld_phase, ST_TIMEOUT_TMA)) break;
+            ld_phase ^= 1;
+#pragma unroll 1
+            for (int e = 0; e < 2; ++e) {
+              float v[32];
+              read32(Cfg::ACC2 + c * 64 + e * 32, bias2 + c * 64 + e * 32, v);
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                uint4* at = reinterpret_cast<uint4*>(stg + lane * 128 + (((e * 4 + u) ^ (lane & 7)) << 4));
+                float m[8];
+                lg_unpack(*at, m);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[u * 8 + j] += m[j];
+                *at = lg_pack(v + u * 8);
+              }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0 && valid) lg_store_tile(&maps.out[0], stg_u, c * 64, row0, batch);
+          }
+          if (!ok) break;
+          if (!waited && !wait(acc2_full, t & 1, ST_TIMEOUT_MMA)) break;
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc2_empty);
+        }
+      } else if constexpr (MODE != LN_PROJECT) {
         uint8_t* obuf = stg + (Cfg::TILES - 1) * 4096;          // residual and result; the other one (or the same) takes the mul tiles
         const uint32_t obuf_u = stg_u + (Cfg::TILES - 1) * 4096;
         auto fetch_mul = [&](int h) {
@@ -942,12 +1060,12 @@ extern "C" int ffb_ln_gemm(const LnGemmArgs* p, void* stream) {
     if (!r && q.mode == LN_GATE_CHAIN && !f32) r = map(&m.mul, q.mul, q.hidden, q.rows, q.batch, q.m_rstride, q.m_bstride, 64, 32, 128);
     if (r) return 2000 + r;
     if (q.mode == LN_RELU_CHAIN) {
-      if (q.C == 64) return lg_launch<64, LN_RELU_CHAIN, false>(m, a, st);
-      if (q.C == 128) return lg_launch<128, LN_RELU_CHAIN, false>(m, a, st);
+      if (q.C == 64) return lg_launch<64, LN_RELU_CHAIN, false, 2>(m, a, st);
+      if (q.C == 128) return lg_launch<128, LN_RELU_CHAIN, false, 2>(m, a, st);
       return lg_launch<256, LN_RELU_CHAIN, false>(m, a, st);
     }
-    if (q.C == 64) return lg_launch<64, LN_GATE_CHAIN, false>(m, a, st);
-    if (q.C == 128) return lg_launch<128, LN_GATE_CHAIN, false>(m, a, st);
+    if (q.C == 64) return lg_launch<64, LN_GATE_CHAIN, false, 2>(m, a, st);
+    if (q.C == 128) return lg_launch<128, LN_GATE_CHAIN, false, 2>(m, a, st);
     return lg_launch<256, LN_GATE_CHAIN, false>(m, a, st);
   }
   if (q.nseg < 1 || q.nseg > 3) return -5;
