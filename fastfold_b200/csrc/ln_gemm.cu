@@ -23,7 +23,9 @@
 //   and one      MMA issue, 128 x 128 x 16
 // Weights come in chunks of 128 rows.  Of a chain, chunk h of the hidden activation goes through tensor memory: the epilogue
 // reads the accumulator, applies f and writes bf16 pairs over it, and the second product takes them from there as its A operand.
-// The products of chunk h + 1 are issued before the second product of chunk h, which hides the epilogue.
+// The products of chunk h + 1 are issued before the second product of chunk h, which hides the epilogue; at 64 and 128 channels, with
+// two tiles of rows, so are those of the next tile's first chunk (triangle attention 389 243 -> 240 us, extra-MSA stack 511 -> 498: in the
+// gated outputs, which have one chunk a tile, the epilogue had waited for the products of every tile).
 //
 // What bounds it: the weights, which every tile of 128 rows streams from L2 again (1 MB a tile for the transition of 256 channels, which
 // at 32768 rows runs at 0.44 of the tensor cores' rate), the output bytes of the wide projections, and with few tiles the chain of one.
@@ -356,6 +358,8 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
   using Cfg = LgCfg<C, MODE, TEAMS>;
   static_assert(TEAMS == 1 || (TEAMS == 2 && !CF), "channels-first rows have one team");
   constexpr int KB = Cfg::KB, RING = Cfg::RING, NACC = Cfg::NACC, NB2 = Cfg::NB2, NA = Cfg::NA;
+  // chains run a chunk ahead across tiles where there are two tiles of rows; with one that would wait for rows that wait for this tile
+  constexpr bool AHEAD = MODE != LN_PROJECT && NA == 2;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
@@ -495,17 +499,19 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
             if (h == (NA == 1 ? chunks - 1 : 0) && more) load_x(tile + gridDim.x, t + 1);
           }
         } else {
+          // the boxes in the order in which the issuer takes them
+          if (AHEAD && more) load_x(tile + gridDim.x, t + 1);
 #pragma unroll 1
-          for (int h = 0; h <= chunks && ok; ++h) {
+          for (int h = AHEAD && t > 0 ? 1 : 0; h <= chunks && ok; ++h) {
 #pragma unroll 1
-            for (int kb = 0; kb < KB && h < chunks; ++kb) load_w(&maps.w[0], kb * 64, h * 128, LG_BOX);
+            for (int kb = 0; kb < KB && (h < chunks || (AHEAD && more)); ++kb) load_w(&maps.w[0], kb * 64, h < chunks ? h * 128 : 0, LG_BOX);
             if (h > 0) {
 #pragma unroll 1
               for (int kk = 0; kk < 2; ++kk)
 #pragma unroll 1
                 for (int n = 0; n < C; n += NB2) load_w(&maps.w[1], (h - 1) * 128 + kk * 64, n, NB2 * 128);
             }
-            if (h == (NA == 1 ? chunks : 0) && more) load_x(tile + gridDim.x, t + 1);
+            if (!AHEAD && h == (NA == 1 ? chunks : 0) && more) load_x(tile + gridDim.x, t + 1);
           }
         }
       }
@@ -575,17 +581,40 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
       if (h + 1 == chunks) umma_commit_by(lead, acc2_full);
       ++c2;
     };
-#pragma unroll 1
-    for (int tile = blockIdx.x; tile < a.num_tiles && ok; tile += gridDim.x, ++t) {
-      const uint32_t s = t % NA;
-      await(a_full + 8 * s, (t / NA) & 1, ST_TIMEOUT_EPI);
-      if (!ok) break;
-      tc_fence_after();
-#pragma unroll 1
-      for (int h = 0; h <= chunks && ok; ++h) {
-        if (h < chunks) first(ad0 + s * (Cfg::A_BYTES >> 4));
+    if constexpr (AHEAD) {
+      // The next chunk's first product goes out before this one's second, which waits for the epilogue between them; the next tile's too
+      auto first_of = [&](uint32_t n, int h) {           // chunk h of the n-th tile
+        const uint32_t s = n % NA;
+        if (h == 0) {
+          await(a_full + 8 * s, (n / NA) & 1, ST_TIMEOUT_EPI);
+          if (!ok) return;
+          tc_fence_after();
+        }
+        first(ad0 + s * (Cfg::A_BYTES >> 4));
         if (h + 1 == chunks && ok) umma_commit_by(lead, a_empty + 8 * s);        // the last product that reads the rows is in
-        if (MODE != LN_PROJECT && h > 0 && ok) second(h - 1);
+      };
+      first_of(0, 0);
+#pragma unroll 1
+      for (int tile = blockIdx.x; tile < a.num_tiles && ok; tile += gridDim.x, ++t)
+#pragma unroll 1
+        for (int h = 0; h < chunks && ok; ++h) {
+          if (h + 1 < chunks) first_of(t, h + 1);
+          else if (tile + gridDim.x < a.num_tiles) first_of(t + 1, 0);
+          if (ok) second(h);
+        }
+    } else {
+#pragma unroll 1
+      for (int tile = blockIdx.x; tile < a.num_tiles && ok; tile += gridDim.x, ++t) {
+        const uint32_t s = t % NA;
+        await(a_full + 8 * s, (t / NA) & 1, ST_TIMEOUT_EPI);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll 1
+        for (int h = 0; h <= chunks && ok; ++h) {
+          if (h < chunks) first(ad0 + s * (Cfg::A_BYTES >> 4));
+          if (h + 1 == chunks && ok) umma_commit_by(lead, a_empty + 8 * s);        // the last product that reads the rows is in
+          if (MODE != LN_PROJECT && h > 0 && ok) second(h - 1);
+        }
       }
     }
     if (!ok && lead) *abort_flag = 1;
