@@ -88,7 +88,8 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool i
 // Four rows at every length: a CTA with two, and two of those per SM, read keys and values twice as often and were slower even
 // where four rows leave SMs idle.
 //   Measured (B200, the core alone, us, with single FMAs, R = 2 / R = 4): N = 256 90 / 78, 512 192 / 171, 768 592 / 525, 1024 792 / 740,
-//   1184 966 / 869, 1536 1796 / 1659, 2048 3207 / 2967; one row per CTA took 349 at 512.  Two by two: 512 165 -> 150.
+//   1184 966 / 869, 1536 1796 / 1659, 2048 3207 / 2967; one row per CTA took 349 at 512.  Two by two: 512 165 -> 149, with 16 keys' values
+//   on their way instead of 4 130.
 template <int R, int H, int C, int PQ, int PV, int CZ>
 __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a) {
   pdl_launch_dependents();
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
       uint64_t zw[R];                                   // even / odd pair channels
 #pragma unroll
       for (int r = 0; r < R; ++r) zw[r] = ipa_pair(bb_h, 0.f);
-#pragma unroll 2
+#pragma unroll 4
       for (int c = 0; c < CZ; c += 8) {
         const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(wbs + warp * CZ + c), w1 = *reinterpret_cast<const ulonglong2*>(wbs + warp * CZ + c + 4);
 #pragma unroll
@@ -269,23 +270,20 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
         acc[u * 2] = ipa_fma2(p.x, vv, acc[u * 2]);
         acc[u * 2 + 1] = ipa_fma2(p.y, vv, acc[u * 2 + 1]);
       };
-      int j = 0;
+      // 16 keys on their way at a time: the four warps that do this read from L2 and have nothing else to fill the wait with (the
+      // core at 512 residues: 2 keys 180 us, 4 149, 8 135, 16 130).  Keys past the end: probability 0, the last key's values
 #pragma unroll 1
-      for (; j + 4 <= jn; j += 4) {
-        float v[NVA][4];
+      for (int j = 0; j < jn; j += 16) {
+        float v[NVA][16];
 #pragma unroll
         for (int u = 0; u < NVA; ++u)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) v[u][e] = vbase[u][(j0 + j + e) * vstep[u]];
+          for (int e = 0; e < 16; ++e) v[u][e] = vbase[u][(j0 + min(j + e, jn - 1)) * vstep[u]];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+        for (int e = 0; e < 16; ++e)
 #pragma unroll
           for (int u = 0; u < NVA; ++u) add(u, j + e, v[u][e]);
       }
-#pragma unroll 1
-      for (; j < jn; ++j)
-#pragma unroll
-        for (int u = 0; u < NVA; ++u) add(u, j, vbase[u][(j0 + j) * vstep[u]]);
     }
   }
   // ---- normalise and store ----
