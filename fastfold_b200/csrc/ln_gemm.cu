@@ -77,15 +77,16 @@ struct LgArgs {
   int pb_n;
 };
 
-// TEAMS: teams of eight epilogue warps, which take the chunks in turn
-template <int C, int MODE, int TEAMS>
+// TEAMS: teams of eight epilogue warps.  NARROW: projections of 256 channels to few columns, which need two tiles of rows on their way
+// more than boxes of weights
+template <int C, int MODE, int TEAMS, bool NARROW>
 struct LgCfg {
   static constexpr int EPI = LG_EPI * TEAMS, THREADS = (6 + EPI) * 32, TMA = 4 + EPI, MMA = 5 + EPI;       // the last two are warps
   static constexpr int KB = C / 64;
   static constexpr int A_BYTES = KB * 16384;
   static constexpr int TILES = C == 256 || TEAMS == 2 ? 1 : 2;                     // 4 KB staging tiles per epilogue warp
-  static constexpr int NA = C == 256 ? 1 : 2;                        // tiles of rows: one less, and the ring holds four boxes more
-  static constexpr int RING = C == 256 && TEAMS == 1 ? 7 : 5;
+  static constexpr int NA = C == 256 && !NARROW ? 1 : 2;                        // tiles of rows: one less, and the ring holds four boxes more
+  static constexpr int RING = NARROW ? 3 : C == 256 && TEAMS == 1 ? 7 : 5;
   static constexpr int NB2 = C < 128 ? C : 128;                      // columns of one second product
   static constexpr int NACC = MODE == LN_PROJECT ? 4 : (C == 256 ? 2 : 3);      // 128-column accumulators of the first product
   static constexpr int ACC2 = NACC * 128;                            // tensor-memory column of the second product's accumulator
@@ -352,10 +353,10 @@ __device__ __forceinline__ void lg_store_tile(const CUtensorMap* map, uint32_t s
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 
-template <int C, int MODE, bool CF, int TEAMS>
+template <int C, int MODE, bool CF, int TEAMS, bool NARROW>
 __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(const __grid_constant__ LgMaps maps, const __grid_constant__ LgArgs a) {
   pdl_launch_dependents();
-  using Cfg = LgCfg<C, MODE, TEAMS>;
+  using Cfg = LgCfg<C, MODE, TEAMS, NARROW>;
   static_assert(TEAMS == 1 || (TEAMS == 2 && !CF), "channels-first rows have one team");
   constexpr int KB = Cfg::KB, RING = Cfg::RING, NACC = Cfg::NACC, NB2 = Cfg::NB2, NA = Cfg::NA;
   // chains run a chunk ahead across tiles where there are two tiles of rows; with one that would wait for rows that wait for this tile
@@ -1016,19 +1017,23 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
   }
 }
 
-template <int C, int MODE, bool CF, int TEAMS = 1>
-static int lg_launch(const LgMaps& maps, const LgArgs& a, cudaStream_t st) {
-  using Cfg = LgCfg<C, MODE, TEAMS>;
-  auto kern = ln_gemm_kernel<C, MODE, CF, TEAMS>;
-  static SmemLimit limit;
-  if (!limit.raise(kern, Cfg::SMEM)) return -30;
+static int lg_sm_count() {
   static int sm_count = 0;
   if (!sm_count) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0) sm_count = 148;
   }
-  const int grid = a.num_tiles < sm_count ? a.num_tiles : sm_count;
+  return sm_count;
+}
+
+template <int C, int MODE, bool CF, int TEAMS = 1, bool NARROW = false>
+static int lg_launch(const LgMaps& maps, const LgArgs& a, cudaStream_t st) {
+  using Cfg = LgCfg<C, MODE, TEAMS, NARROW>;
+  auto kern = ln_gemm_kernel<C, MODE, CF, TEAMS, NARROW>;
+  static SmemLimit limit;
+  if (!limit.raise(kern, Cfg::SMEM)) return -30;
+  const int grid = a.num_tiles < lg_sm_count() ? a.num_tiles : lg_sm_count();
   launch_k(kern, grid, Cfg::THREADS, Cfg::SMEM, st, maps, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
@@ -1124,5 +1129,10 @@ extern "C" int ffb_ln_gemm(const LnGemmArgs* p, void* stream) {
   if (a.has_mul) return q.C == 64 ? lg_launch<64, LN_PROJECT, false>(m, a, st) : lg_launch<128, LN_PROJECT, false>(m, a, st);
   if (q.C == 64) return lg_launch<64, LN_PROJECT, false, 2>(m, a, st);
   if (q.C == 128) return lg_launch<128, LN_PROJECT, false, 2>(m, a, st);
-  return lg_launch<256, LN_PROJECT, false>(m, a, st);
+  // Few columns (the masked projections of the outer product mean) of many tiles: the next tile's rows matter more than four boxes of the
+  // ring.  Outer product mean of 512 x 384, ten tiles a CTA, 326 -> 322 us; block of 256 x 384 in chunks, five, 2159 -> 2155; block of 128 x
+  // 256, not two, 688 -> 691.
+  bool narrow = a.num_tiles >= 4 * lg_sm_count();
+  for (int s = 0; s < q.nseg; ++s) narrow = narrow && q.seg[s].n <= 64;
+  return narrow ? lg_launch<256, LN_PROJECT, false, 1, true>(m, a, st) : lg_launch<256, LN_PROJECT, false>(m, a, st);
 }

@@ -496,3 +496,18 @@ def test_mask_normaliser_of_many_sequences(S, N, dtype, device_status):
         ref = 1.0 / (mask[0].double().t() @ mask[0].double() + 1e-3)
         out = ln_gemm.mask_norm(mask, 1e-3)
         assert ((out[0, :, :, 0].double() - ref).abs() <= 3.2e-5 * ref).all()
+
+
+@pytest.mark.parametrize("M", [4 * 148 * 128 - 128, 4 * 148 * 128 - 127, 90001])
+def test_pair_of_projections_of_many_rows(M, device_status):
+    """256 channels, on both sides of four tiles of 128 rows per SM: every element, the same bits as in two halves."""
+    torch.manual_seed(M)
+    with torch.no_grad():
+        x, norm, s = _randn(M, 256), _norm(256), torch.rand(M, device=DEV).to(torch.bfloat16)
+        ws, bs = [_randn(32, 256, scale=1 / 16) for _ in range(2)], [_randn(32, scale=0.1) for _ in range(2)]
+        ys = ln_gemm.pair(x, norm, ws[0], bs[0], ws[1], bs[1], s)
+        h = M // 256 * 128
+        halves = [ln_gemm.pair(x[i:j].contiguous(), norm, ws[0], bs[0], ws[1], bs[1], s[i:j].contiguous()) for i, j in ((0, h), (h, M))]
+        for y, a, b, w, c in zip(ys, *halves, ws, bs):
+            assert torch.equal(y, torch.cat([a, b]))
+            _close(y, _lin(_ln(x, norm), w, c) * s.double()[:, None])
