@@ -281,18 +281,21 @@ __global__ void adam_k(float* w, float* m, float* v, const bf16* grad, bf16* w16
 }
 
 // out[i][j] = 1 / (sum_s mask[s][i] * mask[s][j] + eps): the normaliser of the outer product mean, from a mask [S][N].  32 x 32 outputs
-// per CTA, the next 128 rows of the mask on their way while these are summed; one launch for the conversions, the product, the sum and
+// per CTA, the next KS rows of the mask on their way while these are summed; one launch for the conversions, the product, the sum and
 // the reciprocal, which as tensor operations are six.  Small tiles, since the chain over S is what it takes: 64 x 64 outputs made 36
-// CTAs at 384 residues and 512 sequences.  Four groups of 64 threads take every fourth sequence and 4 x 4 outputs a thread: two
-// 16-byte reads for 16 FMAs, where 2 x 2 outputs took two reads for 4 (512 x 384: 22 us, the whole layer 340; with these 12 and 332).
-template <typename T>
+// CTAs at 384 residues and 512 sequences.
+// G groups of 256 / G threads take every G-th sequence and F x F outputs a thread, F^2 = 4 G.  G = 4: two 16-byte reads from shared memory
+// for 16 FMAs, where G = 1 has two reads for 4, but the groups' sums are still to be added: 512 x 384 23.9 -> 16.7 us, 200 x 100 8.2 -> 6.7,
+// 128 x 256 5.5 -> 5.0, 64 x 384 the same, 16 x 32 2.6 -> 2.9 (graph replay; up to 64 sequences take G = 1).
+template <typename T, int G>
 __global__ void __launch_bounds__(256) mask_norm_k(const T* __restrict__ mask, float* __restrict__ out, int S, int N, float eps) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int KS = 128, W = 32, U = KS * W / 256, G = 4;
+  constexpr int F = G == 4 ? 4 : 2, W = 32, SIDE = W / F, KS = G == 4 ? 128 : 64, U = KS * W / 256;
+  static_assert(G == 1 || G == 4, "SIDE x SIDE threads in each of the G groups");
   __shared__ __align__(16) float a[KS][W], b[KS][W];
   const int i0 = blockIdx.y * W, j0 = blockIdx.x * W;
-  const int g = threadIdx.x >> 6, tx = threadIdx.x & 7, ty = (threadIdx.x >> 3) & 7;       // quarter of the sequences, 4 x 4 outputs
+  const int g = threadIdx.x / (SIDE * SIDE), tx = threadIdx.x % SIDE, ty = threadIdx.x / SIDE % SIDE;
   const int c = threadIdx.x & 31, r = threadIdx.x >> 5;
   float ra[U], rb[U];
   auto fetch = [&](int s0) {
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(256) mask_norm_k(const T* __restrict__ mask, f
       rb[u] = (s < S && j0 + c < N) ? to_f(mask[(long long)s * N + j0 + c]) : 0.f;
     }
   };
-  float acc[4][4] = {};
+  float acc[F][F] = {};
   fetch(0);
   for (int s0 = 0; s0 < S; s0 += KS) {
 #pragma unroll
@@ -313,26 +316,40 @@ __global__ void __launch_bounds__(256) mask_norm_k(const T* __restrict__ mask, f
     }
     __syncthreads();
     if (s0 + KS < S) fetch(s0 + KS);
-#pragma unroll 8
+#pragma unroll (G == 4 ? 8 : 16)
     for (int k = g; k < KS; k += G) {
-      const float4 u = *reinterpret_cast<const float4*>(&a[k][ty * 4]), v = *reinterpret_cast<const float4*>(&b[k][tx * 4]);
-      const float uu[4] = {u.x, u.y, u.z, u.w}, vv[4] = {v.x, v.y, v.z, v.w};
+      float u[F], v[F];
+      if constexpr (F == 4) {
+        *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(&a[k][ty * 4]);
+        *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(&b[k][tx * 4]);
+      } else {
+        *reinterpret_cast<float2*>(u) = *reinterpret_cast<const float2*>(&a[k][ty * 2]);
+        *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(&b[k][tx * 2]);
+      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < F; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(uu[i], vv[j], acc[i][j]);
+        for (int j = 0; j < F; ++j) acc[i][j] = fmaf(u[i], v[j], acc[i][j]);
     }
     __syncthreads();
   }
-  // the four quarters, in the place of the rows
-  float* part = &a[0][0];                                   // [G][W][W]
+  if constexpr (G == 4) {
+    // the groups' sums, in the place of the rows
+    float* part = &a[0][0];                                 // [G][W][W]
 #pragma unroll
-  for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(part + (g * W + ty * 4 + i) * W + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-  __syncthreads();
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(part + (g * W + ty * 4 + i) * W + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    __syncthreads();
 #pragma unroll
-  for (int i = r; i < W; i += 8)
-    if (i0 + i < N && j0 + c < N)
-      out[(long long)(i0 + i) * N + j0 + c] = 1.f / (((part[i * W + c] + part[(W + i) * W + c]) + (part[(2 * W + i) * W + c] + part[(3 * W + i) * W + c])) + eps);
+    for (int i = r; i < W; i += 8)
+      if (i0 + i < N && j0 + c < N)
+        out[(long long)(i0 + i) * N + j0 + c] = 1.f / (((part[i * W + c] + part[(W + i) * W + c]) + (part[(2 * W + i) * W + c] + part[(3 * W + i) * W + c])) + eps);
+  } else {
+#pragma unroll
+    for (int i = 0; i < F; ++i)
+#pragma unroll
+      for (int j = 0; j < F; ++j)
+        if (i0 + ty * F + i < N && j0 + tx * F + j < N) out[(long long)(i0 + ty * F + i) * N + j0 + tx * F + j] = 1.f / (acc[i][j] + eps);
+  }
 }
 
 }  // namespace ffb
@@ -410,8 +427,8 @@ int ffb_mask_norm(const void* mask, float* out, int S, int N, float eps, int is_
   if (S < 1 || N < 1 || (N + 31) / 32 > 65535) return -1;
   const dim3 grid((unsigned)((N + 31) / 32), (unsigned)((N + 31) / 32));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (is_bf16) launch_light(mask_norm_k<bf16>, grid, 256, 0, st, (const bf16*)mask, out, S, N, eps);
-  else launch_light(mask_norm_k<float>, grid, 256, 0, st, (const float*)mask, out, S, N, eps);
+  if (is_bf16) launch_light(S > 64 ? mask_norm_k<bf16, 4> : mask_norm_k<bf16, 1>, grid, 256, 0, st, (const bf16*)mask, out, S, N, eps);
+  else launch_light(S > 64 ? mask_norm_k<float, 4> : mask_norm_k<float, 1>, grid, 256, 0, st, (const float*)mask, out, S, N, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -486,7 +486,7 @@ def test_masks_in_host_memory_raise(device_status):
                 call()
 
 
-@pytest.mark.parametrize("S,N", [(128, 33), (129, 64), (515, 70)])
+@pytest.mark.parametrize("S,N", [(64, 40), (65, 40), (128, 33), (129, 64), (515, 70)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_mask_normaliser_of_many_sequences(S, N, dtype, device_status):
     """One, two and five passes of 128 sequences: fp32 sums of at most 515 products of values in [0, 1], one reciprocal:
