@@ -271,7 +271,8 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
         acc[u * 2 + 1] = ipa_fma2(p.y, vv, acc[u * 2 + 1]);
       };
       // 16 keys on their way at a time: the four warps that do this read from L2 and have nothing else to fill the wait with (the
-      // core at 512 residues: 2 keys 180 us, 4 149, 8 135, 16 130).  Keys past the end: probability 0, the last key's values
+      // core at 512 residues: 2 keys 180 us, 4 149, 8 135, 16 130).  Keys past the end have probability 0 and get the value 0: with the last
+      // key's, which is loaded in their place, an infinite one would make the sum NaN
 #pragma unroll 1
       for (int j = 0; j < jn; j += 16) {
         float v[NVA][16];
@@ -279,6 +280,13 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
         for (int u = 0; u < NVA; ++u)
 #pragma unroll
           for (int e = 0; e < 16; ++e) v[u][e] = vbase[u][(j0 + min(j + e, jn - 1)) * vstep[u]];
+        if (j + 16 > jn) {
+#pragma unroll
+          for (int e = 1; e < 16; ++e)
+#pragma unroll
+            for (int u = 0; u < NVA; ++u)
+              if (j + e >= jn) v[u][e] = 0.f;
+        }
 #pragma unroll
         for (int e = 0; e < 16; ++e)
 #pragma unroll

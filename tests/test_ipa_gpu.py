@@ -48,6 +48,25 @@ def test_ipa_core_row_block(device_status):
         assert torch.equal(a, b[64:128])
 
 
+@pytest.mark.parametrize("N", [1, 15, 16, 17, 70, 127, 130])
+def test_ipa_core_infinite_values_of_the_last_key(N, device_status):
+    """A sum that holds an infinite value is infinite, whatever the length: keys past the end must not take part.  The other
+    channels as in ``test_ipa_core_matches_reference``."""
+    from fastfold_b200.ops.ipa import ipa_core, ipa_core_ref
+    args = _inputs(N, seed=N, masked=False)
+    args[0], args[3], args[4] = args[0] * 0.1, args[3] * 0.05, args[4] * 0.05        # every probability well above 0
+    args[2][-1, 3, 5], args[2][-1, 7, 0] = math.inf, -math.inf
+    args[5][-1, 2, 6, 1], args[5][-1, 11, 7, 2] = -math.inf, math.inf
+    w = (math.sqrt(1.0 / 48), math.sqrt(1.0 / 3), 1e5)
+    with torch.no_grad():
+        out, ref = ipa_core(*args, *w), ipa_core_ref(*args, *w)
+    for i, (a, b) in enumerate(zip(out, ref)):
+        far = b.isinf()
+        assert not b.isnan().any() and far.sum().item() == (0 if i == 2 else 2 * N)
+        assert torch.equal(a[far], b[far]) and torch.isfinite(a[~far]).all()
+        assert (a[~far] - b[~far]).abs().max().item() <= (2e-2 if i == 1 else 2e-3) * max(1.0, b[~far].abs().max().item())
+
+
 def test_ipa_module_uses_kernel_and_matches_cpu(device_status):
     from fastfold_b200.models.nn.structure_module import InvariantPointAttention
     from fastfold_b200.ops import _lib
