@@ -29,10 +29,11 @@
 // Three groups with two S buffers each (480 of the 512 columns; P takes the place of the S it was made from), not four with one:
 // a group never waits for its S product.  With four of them the products' latency, 1500 - 1900 cycles of 4400 a block, was
 // bare, since all four were in step.
-//   Measured (B200, graph replay, us; four groups with one S buffer -> this): B 384, H 4, n 1536 with bias and mask 1690 -> 1368;
-//   B 64, H 4, n 1024 130 -> 113; B 389, H 4, n 389 191 -> 140; B 256, H 4, n 256 41.6 -> 35.7; B 1024, H 8, D 16, n 256 309 -> 210;
-//   B 300, H 2, n 700 without bias 138 -> 117; B 256, H 8, n 128 without bias 22.9 -> 21.8; B 32, H 8, n 64 5.6 -> 5.0.  Random masks:
-//   1850 -> 1611, 146 -> 136, 205 -> 157, 45.0 -> 41.4, 328 -> 255, 148 -> 130, 24.2 -> 23.5, 5.9 -> 5.2.
+//   Measured (B200, graph replay, us; four groups with one S buffer -> this): B 384, H 4, n 1536 with bias and mask 1685 -> 1418;
+//   B 64, H 4, n 1024 132 -> 113; B 389, H 4, n 389 192 -> 144; B 256, H 4, n 256 41.6 -> 36.2; B 1024, H 8, D 16, n 256 310 -> 213;
+//   B 300, H 2, n 700 without bias 139 -> 119; B 256, H 8, n 128 without bias 23.2 -> 21.6; B 32, H 8, n 64 5.7 -> 5.0.  Random masks:
+//   1854 -> 1605, 147 -> 136, 205 -> 159, 45.3 -> 41.6, 328 -> 255, 148 -> 131, 24.5 -> 23.9, 6.0 -> 5.1.  Of this 1 - 3 % is the price of
+//   the wait between a P V product and the S product over its P (issue_s).
 // Masked keys get a huge negative logit (replaced, not added; -2^30 here, -1e9 in the reference's
 // softmax kernels, softmax_cuda_kernel.cu:338-423,618-706 - same weights), which is weight 0 next to any ordinary
 // key: there they are left out; keys beyond the sequence end get -inf.
@@ -536,12 +537,14 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
       km = load_keys(mrow, sj * AF_BK, a.n_k, lane);
     };
     look_ahead();
-    // S product of the next block, into the buffer whose last P V product has been issued: products execute in order
+    // S product of the next block, into the buffer whose last P V product is over.  That one has been issued by then, but products with
+    // different accumulators and shapes have no order among themselves.  The wait is short and nobody needs this S for a block yet
     auto issue_s = [&]() {
       const uint32_t qs = g * 2 + (qi & 1), ks = g * AF_KVST + si % AF_KVST;
       const Keys keys = key_bits(km);
       if (sj == 0) wait(q_full + 8 * qs, (qi >> 1) & 1, ST_TIMEOUT_TMA, 22);
       wait(kv_full + 8 * ks, (si / AF_KVST) & 1, ST_TIMEOUT_TMA, 20);
+      wait(o_done + 8 * (g * 2 + (si & 1)), ((si >> 1) & 1) ^ 1, ST_TIMEOUT_MMA, 24);
       tc_fence_after();
       const uint64_t q = dq + (qi & 1) * (8192 >> 4), k = dk + (si % AF_KVST) * (8192 >> 4);
 #pragma unroll
