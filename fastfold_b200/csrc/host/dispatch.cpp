@@ -792,7 +792,12 @@ Tensor ipa_layer(const Tensor& q, const Tensor& kv, const Tensor& q_pts, const T
                  const Tensor& z, const Tensor& wb, const Tensor& bb, const Tensor& gamma, const Tensor& mask, double w_c, double w_b, double inf,
                  double eps) {
   constexpr int H = 12, C = 16, PQ = 4, PV = 8, CZ = 128;
-  const int64_t N = z.size(0);
+  const int64_t N = z.dim() == 3 ? z.size(0) : -1;
+  expect(N >= 0 && z.size(1) == N && z.size(2) == CZ && z.scalar_type() == at::kBFloat16 && z.is_contiguous(), "invariant point attention: dense bf16 pair tensor");
+  // the kernels index these by N alone
+  for (auto [t, width] : {std::pair(&q, H * C), std::pair(&kv, 2 * H * C), std::pair(&q_pts, 3 * H * PQ), std::pair(&kv_pts, 3 * H * (PQ + PV))})
+    expect(t->device() == z.device() && t->scalar_type() == at::kBFloat16 && t->is_contiguous() && t->numel() == N * width,
+           "invariant point attention: dense bf16 projections with a row for each of the pair tensor's, on its device");
   int bf = 0;
   auto operand = [&](const Tensor& t, int64_t numel, int bit) {
     expect(t.device() == z.device() && t.numel() == numel, "invariant point attention: parameters and mask on the device of the pair tensor");
@@ -806,6 +811,7 @@ Tensor ipa_layer(const Tensor& q, const Tensor& kv, const Tensor& q_pts, const T
   expect(rot.numel() == N * (is_quat ? 4 : 9) && trans.numel() == 3 * N && rot.scalar_type() == at::kFloat && trans.scalar_type() == at::kFloat &&
              rot.device() == z.device() && trans.device() == z.device() && rot.is_contiguous() && trans.is_contiguous(),
          "invariant point attention: frames");
+  expect(z.is_cuda(), "invariant point attention: operands on a CUDA device");
   // one workspace: queries, keys, values, their points, and the core's outputs (extents are multiples of 16 bytes a residue)
   const Tensor work = f32({N * H * (3 * C + 3 * (2 * PQ + PV) + C + 3 * PV + CZ)}, z);
   float* at = static_cast<float*>(ptr(work));

@@ -44,3 +44,25 @@ def test_empty_extents_raise():
     for call in calls:
         with pytest.raises((AssertionError, RuntimeError)):        # RuntimeError: the stream, asked for first, needs a GPU
             call()
+
+
+def _ipa_operands(N=6):
+    b = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    return {"q": b(N, 192), "kv": b(N, 384), "q_pts": b(N, 144), "kv_pts": b(N, 432), "rot": torch.zeros(N, 4), "is_quat": True, "trans": torch.zeros(N, 3),
+            "z": b(N, N, 128), "wb": b(12, 128), "bb": b(12), "gamma": b(12), "mask": b(N)}
+
+
+@pytest.mark.parametrize("name", ["q", "kv", "q_pts", "kv_pts", "z"])
+@pytest.mark.parametrize("change", [lambda t: t[:-1], lambda t: t.float(), lambda t: t.transpose(0, 1), lambda t: t[..., :-1].contiguous(), lambda t: t.to("meta")],
+                         ids=["rows", "type", "order", "columns", "device"])
+def test_ipa_layer_refuses_operands_that_its_kernels_would_misread(name, change):
+    """The kernels take the projections and the pair tensor as dense bf16 rows of fixed widths, as many as the pair tensor has."""
+    args = _ipa_operands()
+    args[name] = change(args[name])
+    with pytest.raises(AssertionError, match="invariant point attention"):
+        _lib.native().ipa_layer(*args.values(), 0.1, 0.5, 1e5, 1e-8)
+
+
+def test_ipa_layer_refuses_host_memory():
+    with pytest.raises(AssertionError, match="CUDA device"):
+        _lib.native().ipa_layer(*_ipa_operands().values(), 0.1, 0.5, 1e5, 1e-8)
