@@ -440,13 +440,14 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
   const uint32_t tmem = *tmem_slot;
 
   // A wait of this CTA's pipeline.  The first one that runs out reports and sets the flag, at which all others end: the kernel
-  // then runs to its end on whatever the buffers hold, and the caller sees the status.
+  // then runs to its end on whatever the buffers hold, and the caller sees the status.  A try lasts 4 us; the flag is looked at after a few
+  // of them, since a wait may still follow for every block that this CTA has left.
   auto wait = [&](uint32_t bar, uint32_t parity, int code, int detail) -> bool {
     if (mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
     for (;;) {
 #pragma unroll 1
-      for (int i = 0; i < 256; ++i)
+      for (int i = 0; i < 8; ++i)
         if (mbar_try_wait(bar, parity)) return true;
       if (*abort_flag) return false;
       if (globaltimer_ns() - t0 > FFB_LOCAL_WAIT_NS) {
@@ -598,6 +599,11 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
           }
         }
         if (active && rs.i < r_end && rs.i <= reach) issue_s();
+      }
+    }
+    if (*abort_flag) {                         // products that nobody will wait for any more: they are over long before this ends
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 1000000ull) {
       }
     }
   } else {

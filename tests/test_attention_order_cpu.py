@@ -3,7 +3,9 @@ record what it issues and waits for.
 
 P of a block lies over the logits it was made from, so the product P V that reads it and the S product two blocks later write and read
 the same columns.  Products with different accumulators and shapes have no order of their own: the second may only be issued after a
-wait that the first one's completion ended."""
+wait that the first one's completion ended.
+
+A wait that runs out ends the kernel: the waits after it, one or more for every block that is left, must be short."""
 import os
 import shutil
 import subprocess
@@ -37,6 +39,7 @@ struct KeyMask { uint16_t a, b; };
 static KeyMask load_keys(const bf16*, int, int, int) { return {1, 1}; }
 static Keys key_bits(KeyMask) { return {~0u, ~0u}; }
 enum { ST_TIMEOUT_TMA = 1, ST_TIMEOUT_MMA, ST_TIMEOUT_EPI };
+#define FFB_LOCAL_WAIT_NS 2000000000ull
 static void fail(const char* what, int a, int b) { std::printf("%%s (%%d, %%d)\n", what, a, b); std::exit(1); }
 
 constexpr uint32_t base = 0, q_full = 1000, q_empty = 1100, kv_full = 1200, kv_empty = 1300, bias_full = 1400, bias_empty = 1500, s_full = 1600,
@@ -46,6 +49,9 @@ struct Replay {
   std::map<uint32_t, int> seen;
   int issued = 0, done = 0, s = 0, pv = 0, g, releases = 0;
   int reader[2] = {0, 0};                       // last product that reads the P in either buffer
+  int waits = 0, lost = 1 << 30;                // waits so far, and the first that nothing ends (as after a copy that never lands)
+  int reports = 0, tries_after = 0, flag = 0;   // reports of a wait that ran out, tries made since then
+  uint64_t clock = 0;
   void wait(uint32_t bar, uint32_t parity) {
     const uint32_t group = bar / 100 * 100;
     if (group == q_full || group == kv_full || group == bias_full) return;
@@ -59,10 +65,11 @@ struct Replay {
 };
 
 template <int D, bool BIAS>
-static Replay issuer(const AttnInferArgs& a, int g0, int r_begin, int r_end) {
+static Replay issuer(const AttnInferArgs& a, int g0, int r_begin, int r_end, int lost) {
   constexpr uint32_t LAYOUT = D == 32 ? 4 : 6, GROUP = 8 * D * 2;
   Replay x;
   x.g = g0;
+  x.lost = lost;
   const int warp = g0 + 1, lane = 0;
   const uint32_t tmem = 0;
   std::vector<uint8_t> memory(AttnInferSmem::TOTAL);
@@ -72,12 +79,24 @@ static Replay issuer(const AttnInferArgs& a, int g0, int r_begin, int r_end) {
   auto make_idesc_bf16 = [](int, int, int, int) constexpr { return 0u; };
   auto make_desc = [](uint32_t, uint32_t, uint32_t, uint32_t) { return (uint64_t)0; };
   auto tc_fence_after = []() {};
-  auto wait = [&](uint32_t bar, uint32_t parity, int, int) { x.wait(bar, parity); return true; };
+  volatile int* abort_flag = &x.flag;
+  auto globaltimer_ns = [&]() { return x.clock += 700000000ull; };
+  auto report = [&](int, int) { ++x.reports; };
+  auto mbar_try_wait = [&](uint32_t bar, uint32_t parity) {
+    if (x.waits < x.lost) {
+      ++x.waits;
+      x.wait(bar, parity);
+      return true;
+    }
+    x.tries_after += x.flag;
+    return false;
+  };
+  %(wait)s
   auto mbar_arrive = [&](uint32_t bar) { x.releases += bar / 100 * 100 == bias_empty; };
   auto umma_commit_by = [&](uint32_t, uint32_t bar) { x.commits[bar].push_back(x.issued); };
   auto umma_bf16_by = [&](uint32_t, uint32_t d, uint64_t, uint64_t, uint32_t, uint32_t acc) {
     const int buf = (int)(d - g0 * AF_TM_GROUP) / AF_BK;
-    if (x.reader[buf] > x.done) fail("S product over a P that may still be read: S product, products known to be over", x.s, x.done);
+    if (!x.flag && x.reader[buf] > x.done) fail("S product over a P that may still be read: S product, products known to be over", x.s, x.done);
     ++x.issued;
     x.s += !acc;
   };
@@ -112,36 +131,52 @@ int main() {
       if (g < r.cnt) blocks += a.n_kb;
       if (bias && (!a.bias_resident || r.i + 1 == end || r.last(a))) tiles += a.n_kb;
     }
-    const Replay x = bias ? issuer<32, true>(a, g, begin, end) : issuer<16, false>(a, g, begin, end);
+    const Replay x = bias ? issuer<32, true>(a, g, begin, end, 1 << 30) : issuer<16, false>(a, g, begin, end, 1 << 30);
     if (x.s != blocks || x.pv != blocks) fail("blocks issued and due", x.pv, blocks);
     if (x.releases != tiles) fail("bias tiles released and due", x.releases, tiles);
+  }
+  // a wait that runs out early: at most nine tries (of 4 us each) for each of those after it, at most five waits a block
+  for (int lost = 0; lost < 20; ++lost) {
+    AttnInferArgs a = {};
+    a.H = 4;
+    a.n_qt = 8;
+    a.n_kb = 6;
+    a.n_k = a.n_kb * 64;
+    a.rounds = 100;
+    a.few = 3;
+    a.B = 300;
+    const int rounds = a.H * a.n_qt * a.rounds;
+    const Replay x = issuer<32, true>(a, 0, 0, rounds, lost);
+    if (x.reports != 1 || x.tries_after > 9 * 5 * rounds * a.n_kb) fail("reports, tries after a wait that ran out", x.reports, x.tries_after);
   }
   std::printf("ok\n");
 }
 """
 
 
-def _between(text, first, last, keep=True):
+def _between(text, first, last, head=True, tail=True):
+    """What lies from ``first`` to ``last``, with or without these two."""
     i = text.index(first)
     j = text.index(last, i)
-    return text[i:j + len(last)] if keep else text[i + len(first):j]
+    return text[i if head else i + len(first):j + len(last) if tail else j]
 
 
 def _program():
     with open(SOURCE) as f:
         text = f.read()
-    body = _between(text, "// ---------------- MMA issuer of one group ----------------", "  } else {\n    // ---------------- softmax / output", keep=False)
+    body = _between(text, "// ---------------- MMA issuer of one group ----------------", "  } else {\n    // ---------------- softmax / output", head=False, tail=False)
     return HARNESS % {
         "constants": "\n".join(line for line in text.splitlines() if line.startswith("constexpr") and " AF_" in line),
         "args": _between(text, "struct AttnInferArgs {", "\n};"),
         "smem": _between(text, "struct AttnInferSmem {", "\n};"),
         "round": _between(text, "struct Round {", "\n};"),
+        "wait": _between(text, "  auto wait = [&](uint32_t bar", "  // The producer and the issuers", tail=False),
         "issuer": body,
     }
 
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="no C++ compiler")
-def test_products_wait_for_the_readers_of_what_they_overwrite(tmp_path):
+def test_issuer_waits_for_readers_and_ends_after_a_lost_wait(tmp_path):
     src = tmp_path / "issuer.cpp"
     src.write_text(_program())
     exe = str(tmp_path / "issuer")
