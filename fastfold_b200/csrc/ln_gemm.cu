@@ -77,16 +77,19 @@ struct LgArgs {
   int pb_n;
 };
 
-// TEAMS: teams of eight epilogue warps.  NARROW: projections of 256 channels to few columns, which need two tiles of rows on their way
+// TEAMS: teams of eight epilogue warps.  Two teams make 22 warps, which leaves a thread 80 registers; the epilogues keep 32 columns of
+// their row in them then, and some bytes are spilled (gated chain of 64 channels 40, projections of 128 channels 16, projections and relu
+// chain of 64 channels 12).  NARROW: projections of 256 channels to few columns, which need two tiles of rows on their way
 // more than boxes of weights
 template <int C, int MODE, int TEAMS, bool NARROW>
 struct LgCfg {
   static constexpr int EPI = LG_EPI * TEAMS, THREADS = (6 + EPI) * 32, TMA = 4 + EPI, MMA = 5 + EPI;       // the last two are warps
+  static_assert(C != 256 || TEAMS == 1, "no room for the staging tiles of two teams");
   static constexpr int KB = C / 64;
   static constexpr int A_BYTES = KB * 16384;
-  static constexpr int TILES = C == 256 || TEAMS == 2 ? 1 : 2;                     // 4 KB staging tiles per epilogue warp
-  static constexpr int NA = C == 256 && !NARROW ? 1 : 2;                        // tiles of rows: one less, and the ring holds four boxes more
-  static constexpr int RING = NARROW ? 3 : C == 256 && TEAMS == 1 ? 7 : 5;
+  static constexpr int TILES = C == 256 || TEAMS == 2 ? 1 : 2;      // 4 KB staging tiles per epilogue warp (two: channels-first rows)
+  static constexpr int NA = C == 256 && !NARROW ? 1 : 2;             // tiles of rows: one less, and the ring holds four boxes more
+  static constexpr int RING = NARROW ? 3 : C == 256 ? 7 : 5;
   static constexpr int NB2 = C < 128 ? C : 128;                      // columns of one second product
   static constexpr int NACC = MODE == LN_PROJECT ? 4 : (C == 256 ? 2 : 3);      // 128-column accumulators of the first product
   static constexpr int ACC2 = NACC * 128;                            // tensor-memory column of the second product's accumulator
@@ -357,7 +360,7 @@ template <int C, int MODE, bool CF, int TEAMS, bool NARROW>
 __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(const __grid_constant__ LgMaps maps, const __grid_constant__ LgArgs a) {
   pdl_launch_dependents();
   using Cfg = LgCfg<C, MODE, TEAMS, NARROW>;
-  static_assert(TEAMS == 1 || (TEAMS == 2 && !CF), "channels-first rows have one team");
+  static_assert(TEAMS == (C == 256 || CF ? 1 : 2), "one team at 256 channels and for channels-first rows");
   constexpr int KB = Cfg::KB, RING = Cfg::RING, NACC = Cfg::NACC, NB2 = Cfg::NB2, NA = Cfg::NA;
   // chains run a chunk ahead across tiles where there are two tiles of rows; with one that would wait for rows that wait for this tile
   constexpr bool AHEAD = MODE != LN_PROJECT && NA == 2;
@@ -512,7 +515,7 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
 #pragma unroll 1
                 for (int n = 0; n < C; n += NB2) load_w(&maps.w[1], (h - 1) * 128 + kk * 64, n, NB2 * 128);
             }
-            if (!AHEAD && h == (NA == 1 ? chunks : 0) && more) load_x(tile + gridDim.x, t + 1);
+            if (!AHEAD && h == chunks && more) load_x(tile + gridDim.x, t + 1);
           }
         }
       }
@@ -685,7 +688,7 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
       const bool valid = row0 < a.rows && batch < a.batch;
       if constexpr (MODE != LN_PROJECT && TEAMS == 2) {
         // One team for the hidden activation, one for the result: the result of a tile leaves while the next one's hidden activation is
-        // made.  32 columns at a time: 22 warps leave 80 registers a thread
+        // made.  32 columns at a time, see LgCfg
         auto read32 = [&](uint32_t col, const float* bias, float (&v)[32]) {
           tmem_ld_32x32(lane_base + col, v);
           const float4* bp = reinterpret_cast<const float4*>(bias);
@@ -799,11 +802,10 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
           if (lane == 0) mbar_arrive(acc2_empty);
         }
       } else if constexpr (MODE != LN_PROJECT) {
-        uint8_t* obuf = stg + (Cfg::TILES - 1) * 4096;          // residual and result; the other one (or the same) takes the mul tiles
-        const uint32_t obuf_u = stg_u + (Cfg::TILES - 1) * 4096;
+        static_assert(Cfg::TILES == 1, "mul tiles, residual and result take turns in one staging tile");
         auto fetch_mul = [&](int h) {
           if (lane == 0) {
-            if (Cfg::TILES == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             mbar_expect_tx(my_ld, 4096);
             tma_load_3d(stg_u, &maps.mul, my_ld, h * 128 + half * 64, row0, batch);
           }
@@ -858,7 +860,7 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
           if (lane == 0) {
             asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             mbar_expect_tx(my_ld, 4096);
-            tma_load_3d(obuf_u, &maps.resid, my_ld, c * 64, row0, batch);
+            tma_load_3d(stg_u, &maps.resid, my_ld, c * 64, row0, batch);
           }
           __syncwarp();
           if (!waited && !wait(acc2_full, t & 1, ST_TIMEOUT_MMA)) break;
@@ -868,8 +870,8 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
           read64(Cfg::ACC2 + c * 64, bias2 + c * 64, v);
           if (!wait(my_ld, ld_phase, ST_TIMEOUT_TMA)) break;
           ld_phase ^= 1;
-          write_tile(obuf, v, true);
-          if (lane == 0 && valid) lg_store_tile(&maps.out[0], obuf_u, c * 64, row0, batch);
+          write_tile(stg, v, true);
+          if (lane == 0 && valid) lg_store_tile(&maps.out[0], stg_u, c * 64, row0, batch);
         }
         if (!ok) break;
         if (!waited && !wait(acc2_full, t & 1, ST_TIMEOUT_MMA)) break;
@@ -901,7 +903,7 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
           }
           const bool work = mycol < sg.n && valid;
           uint8_t* obuf = stg + ob;
-          const bool fused = a.has_mul != 0 && seg == 0;        // mul and residual tiles (two staging tiles; first segment)
+          const bool fused = CF && a.has_mul != 0 && seg == 0;  // mul and residual tiles (two staging tiles; first segment)
           // The tiles alternate by the stores that this warp has issued, not by chunks: with all but the newest store done reading,
           // the other tile is free.  Chunks without a store (pair bias, columns or rows past the end) would break the alternation
           if (work && sg.kind != LN_PAIR_BIAS && lane == 0) {
@@ -929,7 +931,7 @@ __global__ void __launch_bounds__((6 + LG_EPI * TEAMS) * 32, 1) ln_gemm_kernel(c
                   if (j < sg.n) dst[j * a.pb_h] = __float2bfloat16(v[j]);
               }
             } else if constexpr (TEAMS == 2) {
-              // 32 columns at a time: 22 warps leave 88 registers a thread
+              // 32 columns at a time, see LgCfg
 #pragma unroll 1
               for (int e = 0; e < 2; ++e) {
                 float v[32];
@@ -1119,19 +1121,20 @@ extern "C" int ffb_ln_gemm(const LnGemmArgs* p, void* stream) {
   }
   if (a.chunks * 128 > LG_MAX_N) return -9;
   if (q.mul || q.resid) {
-    if (q.C == 256 || bad(q.mul, q.m_rstride, q.m_bstride) || bad(q.resid, q.r_rstride, q.r_bstride) || q.seg[0].kind != LN_ROWS) return -10;
+    if (!q.channels_first || bad(q.mul, q.m_rstride, q.m_bstride) || bad(q.resid, q.r_rstride, q.r_bstride) || q.seg[0].kind != LN_ROWS) return -10;
     a.has_mul = 1;
     r = map(&m.mul, q.mul, q.seg[0].n, q.rows, q.batch, q.m_rstride, q.m_bstride, 64, 32, 128);
     if (!r) r = map(&m.resid, q.resid, q.seg[0].n, q.rows, q.batch, q.r_rstride, q.r_bstride, 64, 32, 128);
     if (r) return 4000 + r;
   }
   if (q.channels_first) return lg_launch<128, LN_PROJECT, true>(m, a, st);
-  if (a.has_mul) return q.C == 64 ? lg_launch<64, LN_PROJECT, false>(m, a, st) : lg_launch<128, LN_PROJECT, false>(m, a, st);
   if (q.C == 64) return lg_launch<64, LN_PROJECT, false, 2>(m, a, st);
   if (q.C == 128) return lg_launch<128, LN_PROJECT, false, 2>(m, a, st);
   // Few columns (the masked projections of the outer product mean) of many tiles: the next tile's rows matter more than four boxes of the
-  // ring.  Outer product mean of 512 x 384, ten tiles a CTA, 326 -> 322 us; block of 256 x 384 in chunks, five, 2159 -> 2155; block of 128 x
-  // 256, not two, 688 -> 691.
+  // ring.  Both lines are those of the three workloads that were measured: outer product mean of 512 x 384, ten tiles a CTA, 327 -> 325 us;
+  // block of 256 x 384 in chunks, five, 2159 -> 2155; block of 128 x 256, not two, 688 -> 691.  What lies between two and five tiles is not
+  // known, nor are other widths; the QKV projection of 768 columns gained too at ten tiles a CTA (138 -> 117 us), in the same layout for
+  // every projection of 256 channels, which was not kept.
   bool narrow = a.num_tiles >= 4 * lg_sm_count();
   for (int s = 0; s < q.nseg; ++s) narrow = narrow && q.seg[s].n <= 64;
   return narrow ? lg_launch<256, LN_PROJECT, false, 1, true>(m, a, st) : lg_launch<256, LN_PROJECT, false>(m, a, st);

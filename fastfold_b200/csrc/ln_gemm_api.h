@@ -29,7 +29,8 @@ struct LnGemmArgs {
   int hidden;               // multiple of 8
   const float* mul_f32;     // gated chain: [mul_mod][hidden] in 32 bits instead of mul; row r (batches counted through) takes r % mul_mod
   int mul_mod;
-  // mul: [batch][rows][hidden] (chain) or [batch][rows][n] (first segment); resid, out: [batch][rows][C] (chain) or of the first segment
+  // mul: [batch][rows][hidden] (chain) or [batch][rows][n] (first segment); resid, out: [batch][rows][C] (chain) or of the first segment.
+  // Of projections only those of channels-first rows take mul and resid, and both
   const void* mul;
   long long m_rstride, m_bstride;
   const void* resid;
