@@ -63,44 +63,49 @@ def test_forward_rows_that_leave_the_exponent_range(B, n, H, use_bias, device_st
     assert (out.float() - ref).abs().max().item() < 3.8e-2
 
 
-def _infer(x, bias, mask, n_q):
-    """The kernel without gradients on ``x [B, n, 3, H, d]``, the first ``n_q`` rows as queries; bias rows at a pitch of 8."""
+def _infer(xq, xkv, bias, mask, n_k):
+    """The kernel without gradients: queries from ``xq [B, n_q, 3, H, d]``, the first ``n_k`` rows of ``xkv [B, .., 3, H, d]`` as
+    keys and values, ``bias [H, n_q, n_k]`` in rows at a pitch of 8, ``mask [B, n_k]``."""
     from fastfold_b200.ops import _lib
-    B, n, _, H, d = x.shape
-    pitch = (n + 7) // 8 * 8
-    b = None if bias is None else torch.nn.functional.pad(bias, (0, pitch - n)).contiguous()
+    B, n_q, _, H, d = xq.shape
+    pitch = (n_k + 7) // 8 * 8
+    b = None if bias is None else torch.nn.functional.pad(bias, (0, pitch - n_k)).contiguous()
     out = torch.full((B, n_q, H * d), float("nan"), device=DEV, dtype=torch.bfloat16)
-    p, rs = x.data_ptr(), 3 * H * d
-    rc = _lib.get().ffb_attention_infer(p, p + 2 * H * d, p + 4 * H * d, n * rs, rs, n * rs, rs, _lib.ptr(b), pitch, _lib.ptr(mask), n,
-                                        out.data_ptr(), n_q * H * d, H * d, B, H, n_q, n, d, d ** -0.5, _lib.stream_ptr())
+    kv, rs = xkv.data_ptr(), 3 * H * d
+    rc = _lib.get().ffb_attention_infer(xq.data_ptr(), kv + 2 * H * d, kv + 4 * H * d, n_q * rs, rs, xkv.shape[1] * rs, rs, _lib.ptr(b), pitch,
+                                        _lib.ptr(mask), n_k, out.data_ptr(), n_q * H * d, H * d, B, H, n_q, n_k, d, d ** -0.5, _lib.stream_ptr())
     assert rc == 0
     return out.view(B, n_q, H, d).transpose(1, 2)
 
 
-@pytest.mark.parametrize("B,H,n_q,n,d", [
-    (1, 1, 1, 1, 32), (3, 2, 33, 17, 32), (7, 4, 97, 64, 16),              # one round per CTA, one to four warps with rows
+@pytest.mark.parametrize("B,H,n_q,n_k,d", [
+    (1, 1, 1, 1, 32), (3, 2, 33, 17, 32), (7, 4, 97, 64, 16), (5, 2, 64, 127, 32),      # one round per CTA, one to four warps with rows
     (445, 1, 129, 65, 32), (446, 1, 161, 129, 16), (447, 2, 225, 256, 32),  # several rounds per CTA, resident bias, last query tile in part
     (100, 8, 257, 257, 32), (64, 4, 390, 390, 16), (67, 4, 520, 389, 32),   # streamed bias, rounds with fewer than three rows, key tails
     (1000, 4, 64, 321, 32),
 ])
 @pytest.mark.parametrize("use_bias", [True, False])
-def test_forward_rounds_and_tails(B, H, n_q, n, d, use_bias, device_status):
-    """Query tiles and key blocks that are filled in part, batch rows in rounds of one to three, several rounds per CTA: every
-    element, twice the same bits.  Bound: P and the output are rounded to bf16 and |v| < 5.5, as above, with logits of order 1."""
-    g = torch.Generator(device=DEV).manual_seed(B + n)
-    m = max(n, n_q)
-    x = torch.randn(B, m, 3, H, d, device=DEV, generator=g).to(torch.bfloat16)
-    bias = torch.randn(H, n_q, m, device=DEV, generator=g).to(torch.bfloat16) if use_bias else None
-    mask = (torch.rand(B, m, device=DEV, generator=g) > 0.3).to(torch.bfloat16)
-    mask[:, 0] = 1
-    mask[B // 2:] = 1
-    if m > n:                                                             # as many keys as the mask leaves
-        mask[:, n:] = 0
-    out = _infer(x, bias, mask, n_q)
-    assert torch.equal(out, _infer(x, bias, mask, n_q))
+@pytest.mark.parametrize("use_mask", [True, False])
+def test_forward_rounds_and_tails(B, H, n_q, n_k, d, use_bias, use_mask, device_status):
+    """Query tiles and key blocks that are filled in part, more queries than keys and fewer, batch rows in rounds of one to three,
+    several rounds per CTA: every element, twice the same bits.  What lies behind the last key is NaN.  Bound: P and the output are rounded to
+    bf16 and |v| < 5.5, as above, with logits of order 1."""
+    g = torch.Generator(device=DEV).manual_seed(B + n_k)
+    xq = torch.randn(B, n_q, 3, H, d, device=DEV, generator=g).to(torch.bfloat16)
+    xkv = torch.randn(B, n_k + 3, 3, H, d, device=DEV, generator=g).to(torch.bfloat16)
+    xkv[:, n_k:] = float("nan")
+    bias = torch.randn(H, n_q, n_k, device=DEV, generator=g).to(torch.bfloat16) if use_bias else None
+    mask = None
+    if use_mask:
+        mask = (torch.rand(B, n_k, device=DEV, generator=g) > 0.3).to(torch.bfloat16)
+        mask[:, 0] = 1
+        mask[B // 2:] = 1
+    out = _infer(xq, xkv, bias, mask, n_k)
+    assert torch.equal(out, _infer(xq, xkv, bias, mask, n_k))
     for i in range(0, B, 64):
-        q, k, v = (t.transpose(1, 2) for t in x[i:i + 64].float().unbind(2))
-        ref = attention_core_ref(q[:, :, :n_q], k, v, mask[i:i + 64].float(), None if bias is None else bias.float())
+        q = xq[i:i + 64, :, 0].float().transpose(1, 2)
+        k, v = (xkv[i:i + 64, :n_k, j].float().transpose(1, 2) for j in (1, 2))
+        ref = attention_core_ref(q, k, v, None if mask is None else mask[i:i + 64].float(), None if bias is None else bias.float())
         assert (out[i:i + 64].float() - ref).abs().max().item() < 2.2e-2
 
 
