@@ -285,8 +285,9 @@ __global__ void adam_k(float* w, float* m, float* v, const bf16* grad, bf16* w16
 // the reciprocal, which as tensor operations are six.  Small tiles, since the chain over S is what it takes: 64 x 64 outputs made 36
 // CTAs at 384 residues and 512 sequences.
 // G groups of 256 / G threads take every G-th sequence and F x F outputs a thread, F^2 = 4 G.  G = 4: two 16-byte reads from shared memory
-// for 16 FMAs, where G = 1 has two reads for 4, but the groups' sums are still to be added: 512 x 384 23.9 -> 16.7 us, 200 x 100 8.2 -> 6.7,
-// 128 x 256 5.5 -> 5.0, 64 x 384 the same, 16 x 32 2.6 -> 2.9 (graph replay; up to 64 sequences take G = 1).
+// for 16 FMAs, where G = 1 has two reads for 4, but the groups' sums are still to be added: 512 x 384 25 -> 16.6 us, 200 x 100 8.2 -> 7.2,
+// 128 x 256 5.5 -> 5.1, 65 x 384 6.9 -> 5.3, 64 x 384 the same, 16 x 32 2.6 -> 2.9 (graph replay; up to 64 sequences take G = 1).  The groups
+// add in another order than G = 1: of masks of zeros and ones all sums are exact, of others the last bits differ.
 template <typename T, int G>
 __global__ void __launch_bounds__(256) mask_norm_k(const T* __restrict__ mask, float* __restrict__ out, int S, int N, float eps) {
   pdl_launch_dependents();

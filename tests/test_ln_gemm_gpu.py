@@ -489,8 +489,8 @@ def test_masks_in_host_memory_raise(device_status):
 @pytest.mark.parametrize("S,N", [(64, 40), (65, 40), (128, 33), (129, 64), (515, 70)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_mask_normaliser_of_many_sequences(S, N, dtype, device_status):
-    """One, two and five passes of 128 sequences: fp32 sums of at most 515 products of values in [0, 1], one reciprocal:
-    515 x 2^-24 relative, and 2 ulp.  Of masks of zeros and ones the sums are exact."""
+    """One pass of 64 sequences in one group, and one, two and five passes of 128 in four: fp32 sums of at most 515 products of
+    values in [0, 1], one reciprocal: 515 x 2^-24 relative, and 2 ulp.  Of masks of zeros and ones the sums are exact."""
     torch.manual_seed(N)
     for mask in (torch.rand(1, S, N, device=DEV).to(dtype), (torch.rand(1, S, N, device=DEV) > 0.3).to(dtype)):
         ref = 1.0 / (mask[0].double().t() @ mask[0].double() + 1e-3)
