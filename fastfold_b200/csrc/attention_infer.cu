@@ -96,24 +96,6 @@ struct AttnInferSmem {
   static constexpr int TOTAL = BARS + 576 + 1024;
 };
 
-// two floats in one 64-bit register pair: the FMA pipe does both in one instruction
-__device__ __forceinline__ uint64_t pk2(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ void up2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 // a + the lower / upper bf16 of w
 __device__ __forceinline__ float add_lo(float a, uint32_t w) {
   float d;
@@ -131,29 +113,29 @@ __device__ __forceinline__ float add_hi(float a, uint32_t w) {
 template <bool PLAIN, bool BIAS>
 __device__ __forceinline__ void logits16(uint64_t (&t)[8], const float (&s)[16], const uint8_t* brow, int r, int c0, const float* pen,
                                          float scale_log2e, float add) {
-  const uint64_t sc = pk2(scale_log2e, scale_log2e), ad = pk2(add, add), l2e = pk2(LOG2E, LOG2E);
+  const uint64_t sc = pair2(scale_log2e, scale_log2e), ad = pair2(add, add), l2e = pair2(LOG2E, LOG2E);
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     uint64_t b[4];
     if (BIAS) {
       const uint4 raw = *reinterpret_cast<const uint4*>(brow + ((((c0 >> 3) + u) ^ (r & 7)) << 4));
-      b[0] = fma2(pk2(bf_lo(raw.x), bf_hi(raw.x)), l2e, ad);
-      b[1] = fma2(pk2(bf_lo(raw.y), bf_hi(raw.y)), l2e, ad);
-      b[2] = fma2(pk2(bf_lo(raw.z), bf_hi(raw.z)), l2e, ad);
-      b[3] = fma2(pk2(bf_lo(raw.w), bf_hi(raw.w)), l2e, ad);
+      b[0] = fma2(pair2(bf_lo(raw.x), bf_hi(raw.x)), l2e, ad);
+      b[1] = fma2(pair2(bf_lo(raw.y), bf_hi(raw.y)), l2e, ad);
+      b[2] = fma2(pair2(bf_lo(raw.z), bf_hi(raw.z)), l2e, ad);
+      b[3] = fma2(pair2(bf_lo(raw.w), bf_hi(raw.w)), l2e, ad);
     } else {
 #pragma unroll
       for (int e = 0; e < 4; ++e) b[e] = ad;
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) t[u * 4 + e] = fma2(pk2(s[u * 8 + 2 * e], s[u * 8 + 2 * e + 1]), sc, b[e]);
+    for (int e = 0; e < 4; ++e) t[u * 4 + e] = fma2(pair2(s[u * 8 + 2 * e], s[u * 8 + 2 * e + 1]), sc, b[e]);
     if (!PLAIN) {
       const float4 k0 = *reinterpret_cast<const float4*>(pen + c0 + u * 8);         // same address in every lane: broadcast
       const float4 k1 = *reinterpret_cast<const float4*>(pen + c0 + u * 8 + 4);
-      t[u * 4] = add2(t[u * 4], pk2(k0.x, k0.y));
-      t[u * 4 + 1] = add2(t[u * 4 + 1], pk2(k0.z, k0.w));
-      t[u * 4 + 2] = add2(t[u * 4 + 2], pk2(k1.x, k1.y));
-      t[u * 4 + 3] = add2(t[u * 4 + 3], pk2(k1.z, k1.w));
+      t[u * 4] = add2(t[u * 4], pair2(k0.x, k0.y));
+      t[u * 4 + 1] = add2(t[u * 4 + 1], pair2(k0.z, k0.w));
+      t[u * 4 + 2] = add2(t[u * 4 + 2], pair2(k1.x, k1.y));
+      t[u * 4 + 3] = add2(t[u * 4 + 3], pair2(k1.z, k1.w));
     }
   }
 }
@@ -195,9 +177,8 @@ __device__ __forceinline__ void softmax_block(uint32_t tm_s, const uint8_t* brow
       logits16<PLAIN, BIAS>(t, s[q & 1], brow, r, q * 16, pen, scale_log2e, add);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        float x, y;
-        up2(t[i], x, y);
-        const bf162 h = __floats2bfloat162_rn(ex2f(x), ex2f(y));
+        const float2 f = split2(t[i]);
+        const bf162 h = __floats2bfloat162_rn(ex2f(f.x), ex2f(f.y));
         const uint32_t w = *reinterpret_cast<const uint32_t*>(&h);
         p[q * 8 + i] = w;
         sum.x = add_lo(sum.x, w);
@@ -697,9 +678,8 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_infer_kernel(const __grid_
                 logits16<false, BIAS>(t, s, brow, r, c * 16, pen, a.scale_log2e, 0.f);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                  float x, y;
-                  up2(t[i], x, y);
-                  mx = fmaxf(mx, fmaxf(x, y));
+                  const float2 f = split2(t[i]);
+                  mx = fmaxf(mx, fmaxf(f.x, f.y));
                 }
               }
               const float m2 = (row.l > 0.f && !row.far) ? fmaxf(mx, row.M + log2f(row.l)) : mx;

@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include "gemm_api.h"
+#include "ipa_api.h"
 #include "ln_gemm_api.h"
 
 extern "C" {
@@ -807,7 +808,8 @@ Tensor ipa_layer(const Tensor& q, const Tensor& kv, const Tensor& q_pts, const T
     }
     return t.to(at::kFloat).contiguous();
   };
-  const Tensor w = operand(wb, H * CZ, 1), b = operand(bb, H, 2), g = operand(gamma, H, 4), m = operand(mask, N, 8);
+  const Tensor w = operand(wb, H * CZ, IPA_BF16_WB), b = operand(bb, H, IPA_BF16_BB), g = operand(gamma, H, IPA_BF16_GAMMA),
+               m = operand(mask, N, IPA_BF16_MASK);
   expect(rot.numel() == N * (is_quat ? 4 : 9) && trans.numel() == 3 * N && rot.scalar_type() == at::kFloat && trans.scalar_type() == at::kFloat &&
              rot.device() == z.device() && trans.device() == z.device() && rot.is_contiguous() && trans.is_contiguous(),
          "invariant point attention: frames");

@@ -14,12 +14,12 @@
 // Replaces the PyTorch composite of the reference (fastfold/model/nn/structure_module.py:383-505), which materialises
 // all of the above through cuBLAS and elementwise kernels.
 #include "common.cuh"
+#include "ipa_api.h"
 
 namespace ffb {
 
 constexpr int IPA_THREADS = 384;   // one warp per head
 constexpr int IPA_J = 64;          // keys per chunk
-enum { IPA_BF16_WB = 1, IPA_BF16_BB = 2, IPA_BF16_GAMMA = 4, IPA_BF16_MASK = 8 };
 constexpr int IPA_ZP = 8;          // padding (bf16) of a z row in shared memory: consecutive keys fall into different banks
 
 struct IpaArgs {
@@ -44,28 +44,6 @@ struct IpaArgs {
 
 __device__ __forceinline__ float ipa_load(const void* p, long long i, bool half) {
   return half ? __bfloat162float(reinterpret_cast<const bf16*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
-}
-
-// two floats in one 64-bit register pair: the FMA pipe does both in one instruction
-__device__ __forceinline__ uint64_t ipa_pair(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ float2 ipa_split(uint64_t v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-__device__ __forceinline__ uint64_t ipa_fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t ipa_mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in_range) {
@@ -149,7 +127,7 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
   constexpr int NACC = H > NVA * (R / 2) ? H : NVA * (R / 2);
   uint64_t acc[NACC];
 #pragma unroll
-  for (int i = 0; i < NACC; ++i) acc[i] = ipa_pair(0.f, 0.f);
+  for (int i = 0; i < NACC; ++i) acc[i] = pair2(0.f, 0.f);
   int vhead[NVA], vstep[NVA];
   const float* vbase[NVA];
 #pragma unroll
@@ -176,17 +154,17 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
       const long long jj = on ? j0 + j : 0;
       uint64_t zw[R];                                   // even / odd pair channels
 #pragma unroll
-      for (int r = 0; r < R; ++r) zw[r] = ipa_pair(bb_h, 0.f);
+      for (int r = 0; r < R; ++r) zw[r] = pair2(bb_h, 0.f);
 #pragma unroll 4
       for (int c = 0; c < CZ; c += 8) {
         const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(wbs + warp * CZ + c), w1 = *reinterpret_cast<const ulonglong2*>(wbs + warp * CZ + c + 4);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const uint4 raw = *reinterpret_cast<const uint4*>(zc + (r * IPA_J + j) * ZROW + c);
-          zw[r] = ipa_fma2(ipa_pair(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u)), w0.x, zw[r]);
-          zw[r] = ipa_fma2(ipa_pair(__uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u)), w0.y, zw[r]);
-          zw[r] = ipa_fma2(ipa_pair(__uint_as_float(raw.z << 16), __uint_as_float(raw.z & 0xffff0000u)), w1.x, zw[r]);
-          zw[r] = ipa_fma2(ipa_pair(__uint_as_float(raw.w << 16), __uint_as_float(raw.w & 0xffff0000u)), w1.y, zw[r]);
+          zw[r] = fma2(pair2(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u)), w0.x, zw[r]);
+          zw[r] = fma2(pair2(__uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u)), w0.y, zw[r]);
+          zw[r] = fma2(pair2(__uint_as_float(raw.z << 16), __uint_as_float(raw.z & 0xffff0000u)), w1.x, zw[r]);
+          zw[r] = fma2(pair2(__uint_as_float(raw.w << 16), __uint_as_float(raw.w & 0xffff0000u)), w1.y, zw[r]);
         }
       }
       const float mj = a.mask ? ipa_load(a.mask, jj, a.bf & IPA_BF16_MASK) : 1.f;
@@ -216,7 +194,7 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
       }
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        lg[r][half] = on ? a.w_c * qk[r] + a.w_b * (ipa_split(zw[r]).x + ipa_split(zw[r]).y) - ghalf * d2[r] + a.inf * (mask_i[r] * mj - 1.f) : -INFINITY;
+        lg[r][half] = on ? a.w_c * qk[r] + a.w_b * (split2(zw[r]).x + split2(zw[r]).y) - ghalf * d2[r] + a.inf * (mask_i[r] * mj - 1.f) : -INFINITY;
     }
     float p0[R], p1[R];
 #pragma unroll
@@ -239,8 +217,8 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
 #pragma unroll
       for (int h2 = 0; h2 < H / 2; ++h2) {
         const uint64_t al = *reinterpret_cast<const uint64_t*>(alph + zr * H + 2 * h2);
-        acc[h2] = ipa_mul2(acc[h2], al);
-        acc[H / 2 + h2] = ipa_mul2(acc[H / 2 + h2], al);
+        acc[h2] = mul2(acc[h2], al);
+        acc[H / 2 + h2] = mul2(acc[H / 2 + h2], al);
       }
       const bf16* zp = zc + zr * IPA_J * ZROW + 2 * cp;
       const float* pp = ps + zr * IPA_J * H;
@@ -248,27 +226,27 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
       for (int j = 0; j < IPA_J; ++j) {                 // rows past N: z = 0 and p = 0
         const uint32_t zz = *reinterpret_cast<const uint32_t*>(zp + j * ZROW);
         const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xffff0000u);
-        const uint64_t z00 = ipa_pair(z0, z0), z11 = ipa_pair(z1, z1);
+        const uint64_t z00 = pair2(z0, z0), z11 = pair2(z1, z1);
 #pragma unroll
         for (int h4 = 0; h4 < H / 4; ++h4) {
           const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(pp + j * H + h4 * 4);  // same address in every lane
-          acc[h4 * 2] = ipa_fma2(p.x, z00, acc[h4 * 2]);
-          acc[h4 * 2 + 1] = ipa_fma2(p.y, z00, acc[h4 * 2 + 1]);
-          acc[H / 2 + h4 * 2] = ipa_fma2(p.x, z11, acc[H / 2 + h4 * 2]);
-          acc[H / 2 + h4 * 2 + 1] = ipa_fma2(p.y, z11, acc[H / 2 + h4 * 2 + 1]);
+          acc[h4 * 2] = fma2(p.x, z00, acc[h4 * 2]);
+          acc[h4 * 2 + 1] = fma2(p.y, z00, acc[h4 * 2 + 1]);
+          acc[H / 2 + h4 * 2] = fma2(p.x, z11, acc[H / 2 + h4 * 2]);
+          acc[H / 2 + h4 * 2 + 1] = fma2(p.y, z11, acc[H / 2 + h4 * 2 + 1]);
         }
       }
     } else {
 #pragma unroll
       for (int u = 0; u < NVA; ++u) {
-        acc[u * 2] = ipa_mul2(acc[u * 2], ipa_pair(alph[vhead[u]], alph[H + vhead[u]]));
-        acc[u * 2 + 1] = ipa_mul2(acc[u * 2 + 1], ipa_pair(alph[2 * H + vhead[u]], alph[3 * H + vhead[u]]));
+        acc[u * 2] = mul2(acc[u * 2], pair2(alph[vhead[u]], alph[H + vhead[u]]));
+        acc[u * 2 + 1] = mul2(acc[u * 2 + 1], pair2(alph[2 * H + vhead[u]], alph[3 * H + vhead[u]]));
       }
       auto add = [&](int u, int j, float v) {
         const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(pr + j * PRS + vhead[u] * R);
-        const uint64_t vv = ipa_pair(v, v);
-        acc[u * 2] = ipa_fma2(p.x, vv, acc[u * 2]);
-        acc[u * 2 + 1] = ipa_fma2(p.y, vv, acc[u * 2 + 1]);
+        const uint64_t vv = pair2(v, v);
+        acc[u * 2] = fma2(p.x, vv, acc[u * 2]);
+        acc[u * 2 + 1] = fma2(p.y, vv, acc[u * 2 + 1]);
       };
       // 16 keys on their way at a time: the four warps that do this read from L2 and have nothing else to fill the wait with (the
       // core at 512 residues: 2 keys 180 us, 4 149, 8 135, 16 130).  Keys past the end have probability 0 and get the value 0: with the last
@@ -304,7 +282,7 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
 #pragma unroll
       for (int h = 0; h < H; ++h) {
         const float l = lfin[zr * H + h];
-        const float2 lo = ipa_split(acc[h / 2]), hi = ipa_split(acc[H / 2 + h / 2]);
+        const float2 lo = split2(acc[h / 2]), hi = split2(acc[H / 2 + h / 2]);
         *reinterpret_cast<float2*>(a.o_pair + ((long long)(r0 + zr) * H + h) * CZ + 2 * cp) =
             h & 1 ? make_float2(lo.y / l, hi.y / l) : make_float2(lo.x / l, hi.x / l);
       }
@@ -317,7 +295,7 @@ __global__ void __launch_bounds__(IPA_THREADS, 1) ipa_fwd_kernel(const IpaArgs a
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if (r0 + r >= a.rows) continue;
-        const float2 two = ipa_split(acc[u * 2 + r / 2]);
+        const float2 two = split2(acc[u * 2 + r / 2]);
         const float val = (r & 1 ? two.y : two.x) / lfin[r * H + vhead[u]];
         if (ch < VC) a.o[(long long)(r0 + r) * VC + ch] = val;
         else a.o_pt[(long long)(r0 + r) * VT + ch - VC] = val;
@@ -464,7 +442,7 @@ int ffb_ipa_cat(const float* o, const float* o_pt, const float* o_pair, const fl
 // All pointers are device memory; q / k / v / points / weights / outputs fp32, z bf16 (layouts in IpaArgs).
 // Supported configuration: H = 12 heads, C = 16 channels, 4 query / key points, 8 value points, c_z = 128 (AlphaFold's
 // structure module); anything else returns -2 and the caller uses its PyTorch composite.
-// ..._mixed: wb, bb, gamma and mask in fp32 or, as `bf` says (bits 1, 2, 4, 8), in bf16.
+// ..._mixed: wb, bb, gamma and mask in fp32 or, as `bf` says (IpaBf16), in bf16.
 int ffb_ipa_fwd_mixed(const float* q, const float* k, const float* v, const float* q_pts, const float* k_pts, const float* v_pts, const void* z,
                       const void* wb, const void* bb, const void* gamma, const void* mask, int bf, float* o, float* o_pt, float* o_pair, int N, int H,
                       int C, int Pq, int Pv, int CZ, int row0, int rows, float w_c, float w_b, float inf, void* stream) {

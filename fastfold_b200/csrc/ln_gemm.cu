@@ -114,35 +114,9 @@ __device__ __forceinline__ uint32_t lg_pack2(float a, float b) {
 }
 __device__ __forceinline__ uint4 lg_pack(const float* v) { return make_uint4(lg_pack2(v[0], v[1]), lg_pack2(v[2], v[3]), lg_pack2(v[4], v[5]), lg_pack2(v[6], v[7])); }
 
-// Two floats in one 64-bit register pair: the FMA pipe does both in one instruction.
-__device__ __forceinline__ uint64_t lg_pair(float a, float b) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t lg_bf2(uint32_t w) { return lg_pair(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
-__device__ __forceinline__ float2 lg_split(uint64_t v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-__device__ __forceinline__ uint64_t lg_add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t lg_mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t lg_fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
+__device__ __forceinline__ uint64_t lg_bf2(uint32_t w) { return pair2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 __device__ __forceinline__ uint32_t lg_pack2v(uint64_t v) {
-  const float2 f = lg_split(v);
+  const float2 f = split2(v);
   return lg_pack2(f.x, f.y);
 }
 
@@ -163,9 +137,9 @@ __device__ __forceinline__ void lg_norm_row(uint8_t* tile, int row, const float*
   };
   // the first and the second channel of word w of two pieces
   auto word = [](const uint4& v, int w) { return w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w; };
-  auto even = [&](const uint4& a, const uint4& b, int w) { return lg_pair(__uint_as_float(word(a, w) << 16), __uint_as_float(word(b, w) << 16)); };
+  auto even = [&](const uint4& a, const uint4& b, int w) { return pair2(__uint_as_float(word(a, w) << 16), __uint_as_float(word(b, w) << 16)); };
   auto odd = [&](const uint4& a, const uint4& b, int w) {
-    return lg_pair(__uint_as_float(word(a, w) & 0xffff0000u), __uint_as_float(word(b, w) & 0xffff0000u));
+    return pair2(__uint_as_float(word(a, w) & 0xffff0000u), __uint_as_float(word(b, w) & 0xffff0000u));
   };
   if constexpr (KB == 1) {
     // the row stays unpacked in registers: pieces 2 h and 2 h + 1 side by side, gamma and beta too
@@ -173,39 +147,39 @@ __device__ __forceinline__ void lg_norm_row(uint8_t* tile, int row, const float*
     load(raw, 0);
     uint64_t v[4][8], t[4];
     auto fold = [&]() {
-      const float2 f = lg_split(lg_add2(lg_add2(t[0], t[2]), lg_add2(t[1], t[3])));
+      const float2 f = split2(add2(add2(t[0], t[2]), add2(t[1], t[3])));
       return f.x + f.y;
     };
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
-      t[h] = lg_pair(0.f, 0.f);
+      t[h] = pair2(0.f, 0.f);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         v[h][j] = j & 1 ? odd(raw[2 * h], raw[2 * h + 1], j >> 1) : even(raw[2 * h], raw[2 * h + 1], j >> 1);
-        t[h] = lg_add2(t[h], v[h][j]);
+        t[h] = add2(t[h], v[h][j]);
       }
     }
     const float mean = fold() * (1.f / C);
-    const uint64_t m2 = lg_pair(-mean, -mean);
+    const uint64_t m2 = pair2(-mean, -mean);
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
-      t[h] = lg_pair(0.f, 0.f);
+      t[h] = pair2(0.f, 0.f);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        v[h][j] = lg_add2(v[h][j], m2);
-        t[h] = lg_fma2(v[h][j], v[h][j], t[h]);
+        v[h][j] = add2(v[h][j], m2);
+        t[h] = fma2(v[h][j], v[h][j], t[h]);
       }
     }
     const float rstd = rsqrtf(fold() * (1.f / C) + eps);
-    const uint64_t r2 = lg_pair(rstd, rstd);
+    const uint64_t r2 = pair2(rstd, rstd);
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       uint32_t lo[4], hi[4];
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(gamma + h * 16 + 4 * w), b = *reinterpret_cast<const ulonglong2*>(beta + h * 16 + 4 * w);
-        const float2 e = lg_split(lg_fma2(lg_mul2(v[h][2 * w], r2), g.x, b.x));
-        const float2 o = lg_split(lg_fma2(lg_mul2(v[h][2 * w + 1], r2), g.y, b.y));
+        const float2 e = split2(fma2(mul2(v[h][2 * w], r2), g.x, b.x));
+        const float2 o = split2(fma2(mul2(v[h][2 * w + 1], r2), g.y, b.y));
         lo[w] = lg_pack2(e.x, o.x);
         hi[w] = lg_pack2(e.y, o.y);
       }
@@ -218,13 +192,13 @@ __device__ __forceinline__ void lg_norm_row(uint8_t* tile, int row, const float*
     auto total = [&](auto&& add) {
       uint64_t s[4], half, t;
       auto combine = [&](int n) {
-        const uint64_t u = lg_add2(KB == 4 ? lg_add2(s[0], s[2]) : lg_add2(s[0], s[1]), KB == 4 ? lg_add2(s[1], s[3]) : lg_add2(s[2], s[3]));
+        const uint64_t u = add2(KB == 4 ? add2(s[0], s[2]) : add2(s[0], s[1]), KB == 4 ? add2(s[1], s[3]) : add2(s[2], s[3]));
         if (KB == 4) {
-          const uint64_t w = lg_add2(half, u);
-          if (n & 1) t = n > 1 ? lg_add2(t, w) : w;
+          const uint64_t w = add2(half, u);
+          if (n & 1) t = n > 1 ? add2(t, w) : w;
           half = u;
         } else {
-          t = n ? lg_add2(t, u) : u;
+          t = n ? add2(t, u) : u;
         }
       };
       half = t = 0;
@@ -241,7 +215,7 @@ __device__ __forceinline__ void lg_norm_row(uint8_t* tile, int row, const float*
         }
         if (n) combine(n - 1);          // here, with the loads under way, and not at the end of the pass, where it would wait for the sums
 #pragma unroll
-        for (int c = 0; c < 4; ++c) s[c] = lg_pair(0.f, 0.f);
+        for (int c = 0; c < 4; ++c) s[c] = pair2(0.f, 0.f);
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
 #pragma unroll
@@ -252,17 +226,17 @@ __device__ __forceinline__ void lg_norm_row(uint8_t* tile, int row, const float*
       }
       combine(KB - 1);
       asm volatile("" ::: "memory");
-      const float2 f = lg_split(t);
+      const float2 f = split2(t);
       return f.x + f.y;
     };
-    const float mean = total([](uint64_t s, uint64_t v) { return lg_add2(s, v); }) * (1.f / C);
-    const uint64_t m2 = lg_pair(-mean, -mean);
+    const float mean = total([](uint64_t s, uint64_t v) { return add2(s, v); }) * (1.f / C);
+    const uint64_t m2 = pair2(-mean, -mean);
     const float var = total([&](uint64_t s, uint64_t v) {
-      const uint64_t d = lg_add2(v, m2);
-      return lg_fma2(d, d, s);
+      const uint64_t d = add2(v, m2);
+      return fma2(d, d, s);
     });
     const float rstd = rsqrtf(var * (1.f / C) + eps);
-    const uint64_t r2 = lg_pair(rstd, rstd);
+    const uint64_t r2 = pair2(rstd, rstd);
 #pragma unroll 1
     for (int kb = 0; kb < KB; ++kb) {
       uint4 ra[8];
@@ -273,10 +247,10 @@ __device__ __forceinline__ void lg_norm_row(uint8_t* tile, int row, const float*
         const ulonglong2* b = reinterpret_cast<const ulonglong2*>(beta + kb * 64 + u * 8);
         const ulonglong2 g0 = g[0], g1 = g[1], b0 = b[0], b1 = b[1];
         uint4 o;
-        o.x = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(ra[u].x), m2), r2), g0.x, b0.x));
-        o.y = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(ra[u].y), m2), r2), g0.y, b0.y));
-        o.z = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(ra[u].z), m2), r2), g1.x, b1.x));
-        o.w = lg_pack2v(lg_fma2(lg_mul2(lg_add2(lg_bf2(ra[u].w), m2), r2), g1.y, b1.y));
+        o.x = lg_pack2v(fma2(mul2(add2(lg_bf2(ra[u].x), m2), r2), g0.x, b0.x));
+        o.y = lg_pack2v(fma2(mul2(add2(lg_bf2(ra[u].y), m2), r2), g0.y, b0.y));
+        o.z = lg_pack2v(fma2(mul2(add2(lg_bf2(ra[u].z), m2), r2), g1.x, b1.x));
+        o.w = lg_pack2v(fma2(mul2(add2(lg_bf2(ra[u].w), m2), r2), g1.y, b1.y));
         *reinterpret_cast<uint4*>(p + kb * 16384 + ((u ^ x) << 4)) = o;
       }
     }
@@ -301,13 +275,13 @@ __device__ __forceinline__ void lg_norm_columns(uint8_t* tile, int t, float2* pa
     }
   };
   auto total = [&](float2* at, auto&& quad) {
-    uint64_t first = lg_pair(0.f, 0.f);
+    uint64_t first = pair2(0.f, 0.f);
     sweep([&](int k0, const uint32_t (&raw)[16]) {
-      const uint64_t g = lg_add2(lg_add2(quad(raw), quad(raw + 4)), lg_add2(quad(raw + 8), quad(raw + 12)));
-      if (kb == 0) first = lg_add2(first, g);
-      else at[(1 + (k0 >> 4)) * 64 + pr] = lg_split(g);
+      const uint64_t g = add2(add2(quad(raw), quad(raw + 4)), add2(quad(raw + 8), quad(raw + 12)));
+      if (kb == 0) first = add2(first, g);
+      else at[(1 + (k0 >> 4)) * 64 + pr] = split2(g);
     });
-    if (kb == 0) at[pr] = lg_split(first);
+    if (kb == 0) at[pr] = split2(first);
     asm volatile("bar.sync 2, 128;" ::: "memory");
     float2 sum = at[pr];
 #pragma unroll
@@ -318,18 +292,18 @@ __device__ __forceinline__ void lg_norm_columns(uint8_t* tile, int t, float2* pa
     }
     return sum;
   };
-  const float2 ms = total(part, [&](const uint32_t* r) { return lg_add2(lg_add2(lg_bf2(r[0]), lg_bf2(r[1])), lg_add2(lg_bf2(r[2]), lg_bf2(r[3]))); });
-  const uint64_t m2 = lg_pair(-ms.x * (1.f / 128), -ms.y * (1.f / 128));
+  const float2 ms = total(part, [&](const uint32_t* r) { return add2(add2(lg_bf2(r[0]), lg_bf2(r[1])), add2(lg_bf2(r[2]), lg_bf2(r[3]))); });
+  const uint64_t m2 = pair2(-ms.x * (1.f / 128), -ms.y * (1.f / 128));
   const float2 qs = total(part + 320, [&](const uint32_t* r) {
-    uint64_t q = lg_pair(0.f, 0.f);
+    uint64_t q = pair2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const uint64_t d = lg_add2(lg_bf2(r[k]), m2);
-      q = lg_fma2(d, d, q);
+      const uint64_t d = add2(lg_bf2(r[k]), m2);
+      q = fma2(d, d, q);
     }
     return q;
   });
-  const uint64_t r2 = lg_pair(rsqrtf(qs.x * (1.f / 128) + eps), rsqrtf(qs.y * (1.f / 128) + eps));
+  const uint64_t r2 = pair2(rsqrtf(qs.x * (1.f / 128) + eps), rsqrtf(qs.y * (1.f / 128) + eps));
   sweep([&](int k0, const uint32_t (&raw)[16]) {
 #pragma unroll
     for (int k = 0; k < 16; k += 4) {
@@ -337,7 +311,7 @@ __device__ __forceinline__ void lg_norm_columns(uint8_t* tile, int t, float2* pa
       const float gv[4] = {g.x, g.y, g.z, g.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const uint64_t y = lg_fma2(lg_mul2(lg_add2(lg_bf2(raw[k + i]), m2), r2), lg_pair(gv[i], gv[i]), lg_pair(bv[i], bv[i]));
+        const uint64_t y = fma2(mul2(add2(lg_bf2(raw[k + i]), m2), r2), pair2(gv[i], gv[i]), pair2(bv[i], bv[i]));
         *reinterpret_cast<uint32_t*>(p + (k0 + k + i) * 128 + ((u ^ ((k + i) & 7)) << 4)) = lg_pack2v(y);
       }
     }
