@@ -29,11 +29,11 @@
 // Three groups with two S buffers each (480 of the 512 columns; P takes the place of the S it was made from), not four with one:
 // a group never waits for its S product.  With four of them the products' latency, 1500 - 1900 cycles of 4400 a block, was
 // bare, since all four were in step.
-//   Measured (B200, graph replay, us; four groups with one S buffer -> this): B 384, H 4, n 1536 with bias and mask 1685 -> 1418;
-//   B 64, H 4, n 1024 132 -> 113; B 389, H 4, n 389 192 -> 144; B 256, H 4, n 256 41.6 -> 36.2; B 1024, H 8, D 16, n 256 310 -> 213;
-//   B 300, H 2, n 700 without bias 139 -> 119; B 256, H 8, n 128 without bias 23.2 -> 21.6; B 32, H 8, n 64 5.7 -> 5.0.  Random masks:
-//   1854 -> 1605, 147 -> 136, 205 -> 159, 45.3 -> 41.6, 328 -> 255, 148 -> 131, 24.5 -> 23.9, 6.0 -> 5.1.  Of this 1 - 3 % is the price of
-//   the wait between a P V product and the S product over its P (issue_s).
+//   Measured (B200, graph replay, us; four groups with one S buffer -> this): B 384, H 4, n 1536 with bias and mask 1685 -> 1397;
+//   B 64, H 4, n 1024 132 -> 113; B 389, H 4, n 389 192 -> 142; B 256, H 4, n 256 41.6 -> 36.2; B 1024, H 8, D 16, n 256 310 -> 214;
+//   B 300, H 2, n 700 without bias 139 -> 119; B 256, H 8, n 128 without bias 23.2 -> 21.7; B 32, H 8, n 64 5.7 -> 5.0.  Random masks:
+//   1854 -> 1595, 147 -> 136, 205 -> 157, 45.3 -> 41.6, 328 -> 256, 148 -> 132, 24.5 -> 23.9, 6.0 -> 5.3.  The wait between a P V product
+//   and the S product over its P (issue_s) is in these times; it costs 1 - 2 %.
 // Masked keys get a huge negative logit (replaced, not added; -2^30 here, -1e9 in the reference's
 // softmax kernels, softmax_cuda_kernel.cu:338-423,618-706 - same weights), which is weight 0 next to any ordinary
 // key: there they are left out; keys beyond the sequence end get -inf.
